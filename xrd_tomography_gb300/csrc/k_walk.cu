@@ -19,6 +19,8 @@
 // rays, so that neighbouring lanes mostly share cache lines.  Per voxel each
 // lane sets up its own ray (FP32 with the exact FP64 fallback) and stores its
 // float2; the stores of consecutive voxels of a row merge in L2.
+#include <algorithm>
+
 #include "scatter.cuh"
 
 namespace xrdt {
@@ -28,7 +30,15 @@ namespace {
 constexpr int kWalkThreads = 128;
 constexpr int kWalkWarps = kWalkThreads / 32;
 constexpr int kRays = 32;          // rays per group: neighbouring pixels of one view
-constexpr int kVoxPerStrip = 64;   // voxels per warp item
+// Voxels per warp item (a strip): up to 64, so that the ray's FP64 endpoint is
+// set up seldom, but no more than leaves kItemsPerSM items per SM.  A warp
+// walks its strip's voxels one after the other; with 64 always, a small
+// problem ran as a few warps: 45x33 voxels, 10 views x 75 px (240 warps) took
+// 649 us against 82 now, 12x12, 4 views x 8 px (8 warps) 462 us against 20, and
+// the last wave of 128x128, 32 views x 128 px showed too (7.8 against 6.65 ms).
+// The smallest strips still pay: one voxel's walk outweighs the set-up.
+constexpr int kMaxStrip = 64;
+constexpr int kItemsPerSM = 256;   // 8 times the resident warps
 
 // Ray r of group g.  Linear pairs (pairs == NULL): the tile holds the pixels
 // d0 .. d0+nd-1 of every view, row (det - d0) * SRC + src; group g is view
@@ -59,14 +69,14 @@ __device__ __forceinline__ bool group_ray(const DevProblem &P, const int2 *pairs
 // the 256x256 workload against 1089 ms at 6 blocks and 80 registers.
 __global__ void __launch_bounds__(kWalkThreads, 8)
 k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2 *__restrict__ pairs,
-           long long n_items, int d0, int nd, long long n_groups, const int *__restrict__ vox_xy, int nv,
+           long long n_items, int d0, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,
            const float4 *__restrict__ cells, float2 *__restrict__ tab)
 {
     const int lane = threadIdx.x & 31;
     const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
     const unsigned ncell_m1 = (unsigned)(ncell - 1);
     const float4 *cells_t = cells + 2 * ncell;   // column-major copy
-    const int nstrips = (nv + kVoxPerStrip - 1) / kVoxPerStrip;
+    const int nstrips = (nv + strip_len - 1) / strip_len;
     const long long nwork = n_groups * nstrips;
     const long long wstride = (long long)gridDim.x * kWalkWarps;
     for (long long wk = (long long)blockIdx.x * kWalkWarps + (threadIdx.x >> 5); wk < nwork; wk += wstride) {
@@ -87,8 +97,8 @@ k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2
         // double issue on the FP64 pipe)
         const ff exff = ff_from_double(ex), eyff = ff_from_double(ey);
         float2 *out = tab + (valid ? row : 0) * nv;
-        const int v1 = min(nv, (strip + 1) * kVoxPerStrip);
-        for (int v = strip * kVoxPerStrip; v < v1; v++) {
+        const int v1 = min(nv, (strip + 1) * strip_len);
+        for (int v = strip * strip_len; v < v1; v++) {
             const int xy = vox_xy[v];
             const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
             const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
@@ -133,15 +143,14 @@ cudaError_t launch_det_walk(const DevProblem &P, const SrcGeom *sg, const int2 *
         nd = (int)(n_items / P.n_src);
         n_groups = (long long)P.n_src * ((nd + kRays - 1) / kRays);
     }
-    const long long nwork = n_groups * ((nv + kVoxPerStrip - 1) / kVoxPerStrip);
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
+    const int sms = current_sm_count();
+    const int strip = (int)std::min<long long>(
+        kMaxStrip, std::max<long long>(1, n_groups * nv / ((long long)sms * kItemsPerSM)));
+    const long long nwork = n_groups * ((nv + strip - 1) / strip);
     long long blocks = (nwork + kWalkWarps - 1) / kWalkWarps;
     if (blocks > (long long)sms * 64) blocks = (long long)sms * 64;
     k_det_walk<<<(unsigned)blocks, kWalkThreads, 0, s>>>(P, make_f32_consts(P), sg, pairs, n_items, d0, nd, n_groups,
-                                                          vox_xy, nv, cells, tab);
+                                                          strip, vox_xy, nv, cells, tab);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }
