@@ -52,3 +52,31 @@ def test_forward_over_walk_strips(ctx, oracle_lib, nx, ny, views, px):
     Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
     assert max_rel_err(N[rays], Nr) < FAST_RTOL
     assert max_rel_err(C[rays], Cr) < FAST_RTOL
+
+
+# the forward's splits: tiles of one step, remainders of steps and tiles, two
+# tiles and more; more and fewer energies than runs; source bins wider than
+# detector bins (a range meets many channels) and a detector grid that only
+# part of the source bins reaches; many detector bins per window (fewer warps)
+@pytest.mark.parametrize("nx,ny,es,ed,dnrg,nqf,e_det", [
+    (9, 5, 1, 1, 0, 7, (20.0, 80.0)), (24, 24, 7, 7, 3, 64, (20.0, 80.0)), (44, 40, 12, 12, 2, 96, (20.0, 80.0)),
+    (31, 33, 65, 33, 4, 130, (20.0, 80.0)), (16, 12, 20, 61, 3, 64, (20.0, 80.0)),
+    (20, 16, 16, 300, 4, 64, (20.0, 80.0)), (12, 12, 11, 900, 5, 64, (20.0, 80.0)),
+    (20, 16, 40, 9, 1, 64, (30.0, 70.0)), (18, 18, 128, 128, 5, 64, (20.0, 80.0))])
+def test_forward_over_splits(ctx, oracle_lib, nx, ny, es, ed, dnrg, nqf, e_det):
+    inp = synth.make_inputs(sized_problem(nx, ny, 3, 40, es, ed, dnrg, nqf=nqf, e_det=e_det), 200 + nx + es)
+    p = inp.problem
+    N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    rays = some_rays(p, 300, nx)
+    Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
+    assert max_rel_err(N[rays], Nr) < FAST_RTOL
+    assert max_rel_err(C[rays], Cr) < FAST_RTOL
+    N2, C2, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    assert np.array_equal(N, N2) and np.array_equal(C, C2)
+    S1 = synth.coherent_table(inp)
+    for bilinear in (False, True):
+        Nt, Ct = xt.forward_tables(p, inp.spectrum, inp.seg, inp.a1, inp.a2, S1, inp.S2, *inp.args()[6:],
+                                   bilinear=bilinear, ctx=ctx)
+        Nr, Cr = oracle_lib.forward_tables(inp, S1, rays, bilinear=bilinear)
+        assert max_rel_err(Nt[rays], Nr) < FAST_RTOL
+        assert max_rel_err(Ct[rays], Cr) < FAST_RTOL

@@ -41,7 +41,7 @@ enum Slot {
     S_RAYS, S_PAIRS, S_NC, S_CC, S_AC,
     S_MA, S_MY, S_MC, S_MX, S_MPART, S_MSENS, S_BC, S_BB, S_BI, S_ERR, S_WALK,
     S_SPFINE, S_SPSRC, S_SPDET, S_SPOUT, S_DWALK, S_DNQ,
-    S_S1, S_S1U8, S_VTA,
+    S_S1, S_S1U8, S_VTA, S_FWDEN, S_VORD,
     S_COUNT
 };
 
@@ -307,12 +307,47 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
     t->sl = 1;
     for (int e = 0; e < p->nrg_src; e++)
         if (t->win_n[2 * e + 1] >= t->win_n[2 * e]) t->sl = std::max(t->sl, t->win_n[2 * e + 1] - t->win_n[2 * e] + 1);
-    t->offs_e.assign((size_t)p->nrg_src * t->sl, 0.f);
+    // offsets from each slot's left edge to the source bin's, with a slot below
+    // and one above the window
+    t->offs_e.assign((size_t)p->nrg_src * (t->sl + 2), 0.f);
     for (int e = 0; e < p->nrg_src; e++)
-        for (int s = 0; s < t->sl; s++) {
-            const double Ed1 = P.e_det_min + (double)(t->win_n[2 * e] + s) * P.dEd;
-            t->offs_e[(size_t)e * t->sl + s] = (float)((P.e_src_min + (double)e * P.dEs) - Ed1);
+        for (int s = 0; s < t->sl + 2; s++) {
+            const double Ed1 = P.e_det_min + (double)(t->win_n[2 * e] - 1 + s) * P.dEd;
+            t->offs_e[(size_t)e * (t->sl + 2) + s] = (float)((P.e_src_min + (double)e * P.dEs) - Ed1);
         }
+    t->fwd_energy.resize(p->nrg_src);
+    for (int e = 0; e < p->nrg_src; e++) {
+        const EnergyRow &r = t->energy[e];
+        FwdEnergy &q = t->fwd_energy[e];
+        const double log2e = 1.4426950408889634074;
+        const double f1 = r.ein * r.ein * r.ein, f2 = P.kn0 + P.kn1 * r.ein + P.kn2 * r.ein * r.ein;
+        const double g1 = -log2e / f1, g2 = -log2e / f2, w = 2.0 * r.Esrc / P.hbarc / P.dq_fine;
+        const double h = r.Esrc / P.hbarc / P.dq_fine;
+        q.f1 = (float)g1;
+        q.f1l = (float)(g1 - (double)q.f1);
+        q.f2 = (float)g2;
+        q.f2l = (float)(g2 - (double)q.f2);
+        q.wh = (float)w;
+        q.wl = (float)(w - (double)q.wh);
+        q.c2 = (float)(h * h / 4.0);
+        q.ein = r.einf;
+        const double k1 = P.kn1 * r.ein, k2 = P.kn2 * r.ein * r.ein;
+        q.pe = (float)(k1 + 2.0 * k2);
+        q.qe = (float)(k1 + k2);
+        q.k1 = (float)k1;
+        q.k2 = (float)k2;
+        const int n0 = t->win_n[2 * e];
+        q.ns = t->win_n[2 * e + 1] - n0 + 1;
+        if (q.ns < 1) {   // no window holds the bin: every slot lies above
+            q.ns = 0;
+            q.es = q.edb = 0.f;
+            q.cs = 1e6f;
+        } else {
+            q.es = (float)(r.Esrc1 / P.dEd);
+            q.cs = (float)(-P.e_det_min / P.dEd - 0.5 - (double)(n0 - 1));
+            q.edb = (float)(P.e_det_min + (double)(n0 - 1) * P.dEd);
+        }
+    }
     t->fine_q.resize(p->nqf);
     for (int j = 0; j < p->nqf; j++) {
         const double q = P.q_lo + P.dq_fine * (0.5 + (double)j);
@@ -641,6 +676,9 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
     B.vox_xy = (int *)tmp;
     if ((rc = get_buf(ctx, S_VMAT, sizeof(int) * nvox, &tmp))) return rc;
     B.vox_mat = (int *)tmp;
+    if ((rc = get_buf(ctx, S_VORD, sizeof(int) * 2 * nvox, &tmp))) return rc;
+    B.vox_order = (int *)tmp;
+    B.vox_rank = B.vox_order + nvox;
     if ((rc = get_buf(ctx, S_VNA, sizeof(int) * nvox, &tmp))) return rc;
     B.vox_na = (int *)tmp;
     if ((rc = get_buf(ctx, S_VA2, sizeof(float) * nvox, &tmp))) return rc;
@@ -726,6 +764,10 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         CK(cudaMemcpyAsync(d, offs_e.data(), sizeof(float) * offs_e.size(), cudaMemcpyHostToDevice, st));
         T.offs_e = (const float *)d;
         T.sl = sl;
+        if ((rc = get_buf(ctx, S_FWDEN, sizeof(FwdEnergy) * ht.fwd_energy.size(), &d))) return rc;
+        CK(cudaMemcpyAsync(d, ht.fwd_energy.data(), sizeof(FwdEnergy) * ht.fwd_energy.size(), cudaMemcpyHostToDevice,
+                           st));
+        T.fwd_energy = (const FwdEnergy *)d;
         if ((rc = get_buf(ctx, S_WINLO, sizeof(int) * wlo.size(), &d))) return rc;
         CK(cudaMemcpyAsync(d, wlo.data(), sizeof(int) * wlo.size(), cudaMemcpyHostToDevice, st));
         T.win_lo = (const int *)d;
@@ -766,8 +808,13 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
                                        B.cells, (float2 *)dtab, st, &ctx->launches));
                 }
                 ProfScope ps(ctx, XRDT_KERNEL_FORWARD);
-                CK(launch_fast_forward(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list, n_total,
-                                       p0, (int)n, (const float2 *)dtab, oN, oC, oA, st, &ctx->launches, tab));
+                if (oA)
+                    CK(launch_matrix(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list, n_total, p0,
+                                     (int)n, (const float2 *)dtab, oN, oC, oA, st, &ctx->launches));
+                else
+                    CK(launch_fast_forward(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list,
+                                           n_total, p0, (int)n, (const float2 *)dtab, oN, oC, st, &ctx->launches,
+                                           tab));
             }
             return XRDT_OK;
         };

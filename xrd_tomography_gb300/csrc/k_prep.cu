@@ -72,50 +72,105 @@ __global__ void k_build_cells(int nx, int ny, const float *__restrict__ a1, cons
     }
 }
 
-// One block of 1024 threads: stream compaction in loop order.
+// The position of each of a thread's flags (bit r of `keep`, r < 4, in order)
+// among all flags of the block, after `base`; adds the block's total to base.
+// cnt: [2][32], used in turn, so that one barrier per call is enough.
+__device__ __forceinline__ int block_positions(unsigned keep, int *base, int (*cnt)[32], int turn)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int mine = __popc(keep);
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    if (lane == 31) cnt[turn & 1][wid] = incl;
+    __syncthreads();
+    int w = cnt[turn & 1][lane];   // 32 warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += n;
+    }
+    const int before = wid ? __shfl_sync(0xffffffffu, w, wid ? wid - 1 : 0) : 0;
+    const int pos = *base + before + incl - mine;
+    *base += __shfl_sync(0xffffffffu, w, 31);
+    return pos;
+}
+
+// One block of 1024 threads, four voxels per thread and round: stream
+// compaction in loop order, then (order != NULL) the same voxels once more in
+// tiles of 8 x 4 voxels: order[i] is the loop-order number of the i-th voxel
+// in tile order.  Thirty-two neighbours in tile order lie within 8 x 4 voxels,
+// in loop order within a strip 32 long: the lanes of a warp that takes them see
+// more even scattering angles and distances.  rank: [nx*ny] scratch.
 __global__ void __launch_bounds__(1024)
 k_compact_voxels(int nx, int ny, int n_mat, const int32_t *__restrict__ seg, int *__restrict__ vox_xy,
-                 int *__restrict__ vox_mat, int *__restrict__ counters)
+                 int *__restrict__ vox_mat, int *__restrict__ counters, int *__restrict__ order, int *rank)
 {
-    __shared__ int warp_cnt[32];
-    __shared__ int base_s;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) base_s = 0;
-    __syncthreads();
-    int bad = 0;
+    __shared__ int cnt[2][32];
+    int bad = 0, base = 0, turn = 0;
     const int64_t total = (int64_t)nx * ny;
-    for (int64_t L0 = 0; L0 < total; L0 += blockDim.x) {
-        const int64_t L = L0 + threadIdx.x;
-        int x = 0, y = 0, s = 0;
-        if (L < total) {
-            x = (int)(L / ny);
-            y = (int)(L % ny);
-            s = seg[(int64_t)x + (int64_t)y * nx];
-            bad |= (s > n_mat);
+    for (int64_t L0 = 0; L0 < total; L0 += 4096, turn++) {
+        int s[4], x[4], y[4];
+        unsigned keep = 0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int64_t L = L0 + 4 * (int)threadIdx.x + r;
+            s[r] = 0;
+            x[r] = y[r] = 0;
+            if (L < total) {
+                x[r] = (int)(L / ny);
+                y[r] = (int)(L - (int64_t)x[r] * ny);
+                s[r] = seg[(int64_t)x[r] + (int64_t)y[r] * nx];
+            }
         }
-        const bool keep = (L < total) && (s > 0) && (s <= n_mat);
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) warp_cnt[wid] = __popc(m);
-        __syncthreads();
-        int off = 0, tot = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-            if (w < wid) off += warp_cnt[w];
-            tot += warp_cnt[w];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            bad |= (s[r] > n_mat);
+            if (s[r] > 0 && s[r] <= n_mat) keep |= 1u << r;
         }
-        const int base = base_s;
-        if (keep) {
-            const int pos = base + off + __popc(m & ((1u << lane) - 1u));
-            vox_xy[pos] = x | (y << 16);
-            vox_mat[pos] = s - 1;
+        int pos = block_positions(keep, &base, cnt, turn);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const bool k = keep >> r & 1u;
+            if (k) {
+                vox_xy[pos] = x[r] | (y[r] << 16);
+                vox_mat[pos] = s[r] - 1;
+            }
+            if (order && L0 + 4 * (int)threadIdx.x + r < total) rank[(int64_t)x[r] + (int64_t)y[r] * nx] = k ? pos : -1;
+            pos += k;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) base_s = base + tot;
-        __syncthreads();
     }
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) {
-        counters[0] = base_s;
+        counters[0] = base;
         counters[1] = bad;
+    }
+    if (!order) return;
+    const int nty = (ny + 3) >> 2;
+    const int64_t quads = 8 * (int64_t)((nx + 7) >> 3) * nty;   // columns of four voxels
+    base = 0;
+    for (int64_t Q0 = 0; Q0 < quads; Q0 += 1024, turn++) {
+        const int64_t q = Q0 + threadIdx.x;
+        int v[4] = {-1, -1, -1, -1};
+        unsigned keep = 0;
+        if (q < quads) {
+            const int64_t tile = q >> 3;
+            const int tx = (int)(tile / nty), ty = (int)(tile - (int64_t)tx * nty);
+            const int x = 8 * tx + (int)(q & 7);
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+                if (x < nx && 4 * ty + r < ny) v[r] = rank[(int64_t)x + (int64_t)(4 * ty + r) * nx];
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            if (v[r] >= 0) keep |= 1u << r;
+        int pos = block_positions(keep, &base, cnt, turn);
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            if (v[r] >= 0) order[pos++] = v[r];
     }
 }
 
@@ -179,7 +234,8 @@ cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a
 cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const float *a1,
                                const float *a2, PrepBuffers &B, cudaStream_t s, int64_t *launches)
 {
-    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters);
+    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
+                                        B.vox_rank);
     const int64_t nvox = (int64_t)P.nx * P.ny;
     int blocks = (int)((nvox + 255) / 256);
     if (blocks > 2048) blocks = 2048;
@@ -191,7 +247,8 @@ cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const fl
 cudaError_t launch_compact_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
                                   int64_t *launches)
 {
-    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters);
+    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
+                                        B.vox_rank);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

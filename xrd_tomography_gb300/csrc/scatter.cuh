@@ -163,24 +163,28 @@ __device__ __noinline__ int compton_bin_f64(const DevProblem &P, double ein, flo
     return floor_to_int((l2d - P.q_min) / P.dq_tab);
 }
 
-// Compton table bin nq = floor((log2(w sqrt(eratio + w^2) / eratio) - q_min) / dq)
-// with w = ein sin(theta/2), clamped to [0, NQ) (integrate_diffraction.cu:331-337).
-// Decided in FP32 from the voxel's 1 - cos(theta) (pair (oh, ol)) and
-// sin(theta/2) (hi part sh); within 2e-4 of a bin edge it is decided again in
-// FP64.  eratio = 1 + ein oh and inv_er = 1/eratio as the caller formed them.
-__device__ __forceinline__ int compton_bin(const DevProblem &P, float ein, float eratio, float inv_er, float sh,
-                                           float oh, float ol, double ein_d, float qmin_t, float inv_dqt)
+// log2(w sqrt(eratio + w^2) / eratio), the Compton table's wavevector axis
+// (integrate_diffraction.cu:331-333), with w = ein sin(theta/2).
+__device__ __forceinline__ float compton_log2(float w, float eratio)
 {
-    const float wC = ein * sh;
-    const float arg = eratio + wC * wC;
-    const float l2 = lg2_approx(wC * arg * rsqrt_approx(arg) * inv_er);
-    const float tq = (l2 - qmin_t) * inv_dqt;
-    float ftq;
-    int nq = floor_bounded(tq, &ftq);   // clamped to the table below
-    const float fr = tq - ftq;
-    if (!(fr > 2e-4f && fr < 1.f - 2e-4f))  // near a table edge
-        nq = compton_bin_f64(P, ein_d, oh, ol);
-    return nq < 0 ? 0 : (nq >= P.nq ? P.nq - 1 : nq);
+    const float w2 = w * w;
+    return fmaf(0.5f, lg2_approx(w2 * (eratio + w2)), -lg2_approx(eratio));
+}
+
+// Compton table bin nq = floor((compton_log2 - q_min) / dq), clamped to
+// [0, NQ) (integrate_diffraction.cu:331-337).  Decided in FP32 from the voxel's
+// 1 - cos(theta) (pair (oh, ol)) and sin(theta/2) (hi part sh), by rounding
+// through the float mantissa; within 2e-4 of a bin edge it is decided again
+// in FP64 with the energy row's ein.  eratio = 1 + ein oh without contraction.
+__device__ __forceinline__ int compton_bin(const DevProblem &P, float ein, float eratio, float sh, float oh, float ol,
+                                           const EnergyRow *row, float qmin_t, float inv_dqt)
+{
+    const float h = (compton_log2(ein * sh, eratio) - qmin_t) * inv_dqt - 0.5f;
+    const float t = h + 12582912.f;
+    int nq = __float_as_int(t) - 0x4B400000;            // round(h) = floor(h + 1/2); clamped below
+    if (!(fabsf(h - (t - 12582912.f)) < 0.5f - 2e-4f))   // near a table edge
+        nq = compton_bin_f64(P, row->ein, oh, ol);
+    return max(0, min(nq, P.nq - 1));
 }
 
 // The cross-section table path (code the reference keeps commented out,
@@ -206,19 +210,21 @@ __device__ __forceinline__ int coherent_bin(const DevProblem &P, float ein, floa
     return nq < 0 ? 0 : (nq >= P.nq ? P.nq - 1 : nq);
 }
 
-// Bilinear value of a table [nq, na] (index q + a*nq, values as floats) at
+// Bilinear value of a table [nq, na] (S(q + a*nq) as a float) at
 // grid coordinates (tq, ta): the grid points are the table's entries,
 // q_min + i (q_max - q_min)/(NQ - 1) (XSection_builder.m:121-125); clamped to
 // the table (a NaN coordinate reads the first row or column).
-__device__ __forceinline__ float table_bilinear(const float *S, int nq, int na, float tq, float ta)
+template <class Table>
+__device__ __forceinline__ float table_bilinear(const Table &S, int nq, int na, float tq, float ta)
 {
     tq = fminf(fmaxf(tq, 0.f), (float)(nq - 1));
     ta = fminf(fmaxf(ta, 0.f), (float)(na - 1));
     const int i = min((int)tq, nq - 2), j = min((int)ta, na - 2);
     const float f = tq - (float)i, g = ta - (float)j;
-    const float *r0 = S + i + j * nq, *r1 = r0 + nq;
-    const float lo = fmaf(f, r0[1] - r0[0], r0[0]);
-    const float hi = fmaf(f, r1[1] - r1[0], r1[0]);
+    const int r0 = i + j * nq, r1 = r0 + nq;
+    const float s00 = S(r0), s01 = S(r1);
+    const float lo = fmaf(f, S(r0 + 1) - s00, s00);
+    const float hi = fmaf(f, S(r1 + 1) - s01, s01);
     return fmaf(g, hi - lo, lo);
 }
 

@@ -64,6 +64,21 @@ struct EnergyRow {
     float inv_f1_lo, inv_f2_lo; // low parts of 1/ein^3, 1/KN(ein)
 };
 
+// A source bin's constants as the forward projector reads them (k_fwd.cu),
+// formed in double: exponents in units of log2, wavevectors and sigma in fine
+// q bins, channels as slots of the bin's detector window (slot 0 is the
+// channel below it, ns the last one).
+struct alignas(16) FwdEnergy {
+    float f1, f1l, f2, f2l;     // -log2(e)/ein^3, -log2(e)/KN(ein) as float pairs
+    float wh, wl;               // 2 Esrc/hbarc per fine bin as a float pair
+    float c2;                   // sigma^2 = c1b s^2 + c2 sg/s^2 (bins^2)
+    float ein;
+    float pe, qe, k1, k2;       // k1 = kn1 ein, k2 = kn2 ein^2, pe = k1 + 2 k2, qe = k1 + k2
+    float es, cs;               // slot of an energy E1/eratio: floor(es/eratio + cs + 1/2)
+    float edb;                  // left edge of slot 0
+    int ns;                     // detector bins whose window holds the source bin
+};
+
 std::string fmt(const char *f, ...);
 
 // Per-call tables of the factored kernels, built on the host in double.
@@ -73,7 +88,8 @@ struct HostTables {
     std::vector<int> win_lo;        // [nrg_det]
     std::vector<int> win_n;         // [nrg_src][2]
     int sl = 1;
-    std::vector<float> offs_e;      // [nrg_src][sl]
+    std::vector<float> offs_e;      // [nrg_src][sl + 2]
+    std::vector<FwdEnergy> fwd_energy;   // [nrg_src]
     std::vector<float2> fine_q;     // [nqf]
     std::vector<float4> coarse_q;   // [nwt]
 };
@@ -117,6 +133,8 @@ struct PrepBuffers {
     float4 *cells = nullptr;          // [2][(ny+1)*(nx+1)*2] bilinear cells, row- then column-major
     int *vox_xy = nullptr;            // [nx*ny] packed x | y << 16 of non-empty voxels
     int *vox_mat = nullptr;           // [nx*ny]
+    int *vox_order = nullptr;         // [nx*ny] voxel numbers in tiles of 8 x 4 voxels, or NULL
+    int *vox_rank = nullptr;          // [nx*ny] scratch of vox_order
     int *vox_na = nullptr;            // [nx*ny] Compton table column per voxel
     float *vox_a2 = nullptr;          // [nx*ny] a2 used by the Compton term
     float *vox_ta = nullptr;          // [nx*ny] the same column as a grid coordinate (bilinear lookups), or NULL
@@ -138,7 +156,8 @@ cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, 
 struct FwdTables {
     const EnergyRow *energy;   // [nrg_src]
     const float *rf_win;       // [nrg_det][2*dnrg+1] spectrum window per detector bin
-    const float *offs_e;       // [nrg_src][sl] Esrc1(e) - Edet1(win_n(e) + s)
+    const FwdEnergy *fwd_energy;   // [nrg_src]
+    const float *offs_e;       // [nrg_src][sl + 2] Esrc1(e) - Edet1(win_n(e) - 1 + s)
     int sl;                    // slots per source bin: max over e of the number of
                                // detector bins whose window holds e
     const int *win_lo;         // [nrg_det] first source bin of each window
@@ -147,17 +166,20 @@ struct FwdTables {
     const float4 *coarse_q;    // [nwt] (q_hi, q_lo, dq, 0)
     unsigned long long *work;  // nullable: counts the exp2 evaluations
 };
-size_t fast_forward_smem(const DevProblem &P, int sl, int e_pass, bool with_n, bool with_a, int tab = 0);
 // n_pairs blocks, block b on pair p0 + b: of the list pairs[0 .. n_list)
-// when it is given (outputs then go to the compact layout [nrg_det][n_list],
-// and [nrg_det][n_list][n_mat*nwt] for A), else of the linear index
-// src + det*SRC of the full layout.  walk holds the blocks' detector-side
-// integrals, [n_pairs][nv] (launch_det_walk).
+// when it is given (outputs then go to the compact layout [nrg_det][n_list]),
+// else of the linear index src + det*SRC of the full layout.  walk holds the
+// blocks' detector-side integrals, [n_pairs][nv] (launch_det_walk).
 cudaError_t launch_fast_forward(const DevProblem &P, const SrcGeom *d_src, const FwdTables &T,
                                 const PrepBuffers &B, int nv, const float *Ifine,
                                 const int2 *pairs, long long n_list, long long p0, int n_pairs,
-                                const float2 *walk, float *N, float *C, float *A, cudaStream_t s,
-                                int64_t *launches, int tab = 0);
+                                const float2 *walk, float *N, float *C, cudaStream_t s, int64_t *launches, int tab);
+// k_matrix.cu: the same with the model matrix A (compact layout
+// [nrg_det][n_list][n_mat*nwt] for a list of pairs).
+cudaError_t launch_matrix(const DevProblem &P, const SrcGeom *d_src, const FwdTables &T,
+                          const PrepBuffers &B, int nv, const float *Ifine, const int2 *pairs, long long n_list,
+                          long long p0, int n_pairs, const float2 *walk, float *N, float *C, float *A,
+                          cudaStream_t s, int64_t *launches);
 // k_spectrum.cu: the spectrum-response matrix (spectrum_builder.m:64-95).
 // A fine bin: edges, centre, 1/(2 sigma^2) and n/(sqrt(2 pi) sigma); a coarse
 // bin: edges and the range [h0, h1) of fine bins that overlap it.
