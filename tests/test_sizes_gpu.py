@@ -80,3 +80,34 @@ def test_forward_over_splits(ctx, oracle_lib, nx, ny, es, ed, dnrg, nqf, e_det):
         Nr, Cr = oracle_lib.forward_tables(inp, S1, rays, bilinear=bilinear)
         assert max_rel_err(Nt[rays], Nr) < FAST_RTOL
         assert max_rel_err(Ct[rays], Cr) < FAST_RTOL
+
+
+# line integrals across uniform squares: larger than the largest radius a cell
+# carries (31), cut by the map's edge and by thin borders; with a gradient
+# that leaves no cell uniform; and the empty phantom but for one voxel
+@pytest.mark.parametrize("kind", ["blocks", "gradient", "one voxel"])
+def test_walks_across_uniform_squares(ctx, oracle_lib, kind):
+    p = sized_problem(150, 137, 5, 64, 16, 16, 3)
+    inp = synth.make_inputs(p, 300)
+    seg = np.zeros((150, 137), np.int32)
+    if kind == "one voxel":
+        seg[70, 131] = 2
+    else:
+        seg[8:97, :120:3] = 1
+        seg[20:140, 60] = 2
+        seg[75, 3:130] = 3
+    dens = np.where(seg > 0, 1.0, 0.0)
+    if kind != "one voxel":
+        dens[8:97, :120] = 1.0     # attenuating between the listed voxels, up to the map's edge
+        dens[20:140, 60] = 2.0
+        dens[100:140, 10:100] = 0.5
+    if kind == "gradient":
+        dens = dens + 1e-3 * np.add.outer(np.arange(150) % 7, np.arange(137) % 5)
+    inp.seg = seg.flatten(order="F")
+    inp.a1 = (2e-6 * dens).astype(np.float32).flatten(order="F")
+    inp.a2 = (0.01 * dens).astype(np.float32).flatten(order="F")
+    N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    rays = some_rays(p, 60, 3)
+    Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
+    assert max_rel_err(N[rays], Nr) < FAST_RTOL
+    assert max_rel_err(C[rays], Cr) < FAST_RTOL

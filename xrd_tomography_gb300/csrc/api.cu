@@ -41,7 +41,7 @@ enum Slot {
     S_RAYS, S_PAIRS, S_NC, S_CC, S_AC,
     S_MA, S_MY, S_MC, S_MX, S_MPART, S_MSENS, S_BC, S_BB, S_BI, S_ERR, S_WALK,
     S_SPFINE, S_SPSRC, S_SPDET, S_SPOUT, S_DWALK, S_DNQ,
-    S_S1, S_S1U8, S_VTA, S_FWDEN, S_VORD,
+    S_S1, S_S1U8, S_VTA, S_FWDEN, S_VORD, S_PREC,
     S_COUNT
 };
 
@@ -226,6 +226,7 @@ F32Consts make_f32_consts(const DevProblem &P)
     F32Consts c;
     c.vox = (float)P.vox;
     c.DQ = (float)P.DQ;
+    c.DQ_lo = (float)(P.DQ - (double)c.DQ);
     c.inv_DQ = (float)(1.0 / P.DQ);
     c.nxf = (float)P.nx;
     c.nyf = (float)P.ny;
@@ -800,20 +801,25 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
             void *dtab;
             int r = get_buf(ctx, S_WALK, sizeof(float2) * (size_t)tile * nv, &dtab);
             if (r) return r;
+            void *drec;
+            if ((r = get_buf(ctx, S_PREC, pair_rec_bytes() * (size_t)tile, &drec))) return r;
+            const PairRec *recs = (const PairRec *)drec;
             for (int64_t p0 = 0; p0 < n_total; p0 += tile) {
                 const int64_t n = std::min(tile, n_total - p0);
                 {
                     ProfScope ps(ctx, XRDT_KERNEL_WALK);
-                    CK(launch_det_walk(P, (const SrcGeom *)d_srcg, list ? list + p0 : nullptr, p0, n, B.vox_xy, nv,
-                                       B.cells, (float2 *)dtab, st, &ctx->launches));
+                    CK(launch_pair_table(P, (const SrcGeom *)d_srcg, list ? list + p0 : nullptr, p0, n,
+                                         (PairRec *)drec, st, &ctx->launches));
+                    CK(launch_det_walk(P, recs, list != nullptr, n, B.vox_xy, nv, B.cells, (float2 *)dtab, st,
+                                       &ctx->launches));
                 }
                 ProfScope ps(ctx, XRDT_KERNEL_FORWARD);
                 if (oA)
                     CK(launch_matrix(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list, n_total, p0,
                                      (int)n, (const float2 *)dtab, oN, oC, oA, st, &ctx->launches));
                 else
-                    CK(launch_fast_forward(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list,
-                                           n_total, p0, (int)n, (const float2 *)dtab, oN, oC, st, &ctx->launches,
+                    CK(launch_fast_forward(P, recs, T, B, nv, (const float *)d_ifine, list != nullptr, n_total,
+                                           p0, (int)n, (const float2 *)dtab, oN, oC, st, &ctx->launches,
                                            tab));
             }
             return XRDT_OK;

@@ -7,10 +7,10 @@
 // kernel makes them with the very device functions the production kernels
 // call, on the same inputs:
 //
-//  * the detector-side walk set-up of k_det_walk (k_walk.cu): FP32 with
-//    guard bands, FP64 near a threshold -> ROI edge and sample count
+//  * the detector- and source-side walk set-ups of k_det_walk (k_walk.cu) and
+//    k_src_atten (k_prep.cu): FP32 with guard bands, float pairs near a
+//    threshold, FP64 within 1e-9 of it -> ROI edge and sample count
 //    (GetIntersection.cu:9-57, attenuator.cu:44-52);
-//  * the source-side walk set-up of k_src_atten (k_prep.cu), in FP64;
 //  * the Compton table bin nq of k_fwd (k_fwd.cu) for every source energy of
 //    the ray's window (integrate_diffraction.cu:331-337).
 //
@@ -40,9 +40,6 @@ __global__ void k_decisions(DevProblem P, F32Consts c, const SrcGeom *__restrict
     const int W = 2 * P.dnrg + 1;
     const int lo = win_lo[nrg];
     const SrcGeom gs = sg[src];
-    double ex, ey, ez;
-    det_position(P, gs.sphi, gs.cphi, det, &ex, &ey, &ez);
-    const float exf = (float)ex, eyf = (float)ey;
     PairGeom G;
     double Rdx, Rdy;
     pair_geom(P, gs, det, &G, &Rdx, &Rdy);
@@ -55,12 +52,12 @@ __global__ void k_decisions(DevProblem P, F32Consts c, const SrcGeom *__restrict
         WalkSetup wd;
         wd.n = 0;
         wd.edge = -1;
-        if (!walk_setup_f32(P, c, exf, eyf, vx, vy, &wd)) walk_setup_f64(P, ex, ey, (double)vx, (double)vy, &wd);
+        walk_decide(P, c, G.Rdx, G.Rdy, &Rdx, &Rdy, vx, vy, &wd);
         // source side, as k_src_atten sets it up
-        const double vxd = ((double)(xy & 0xffff) + 0.5) * P.vox;
-        const double vyd = ((double)(xy >> 16) + 0.5) * P.vox;
         WalkSetup wsrc;
-        walk_setup(P, gs.Rsrc_x, gs.Rsrc_y, vxd, vyd, &wsrc);
+        wsrc.n = 0;
+        wsrc.edge = -1;
+        walk_decide(P, c, G.Rsx, G.Rsy, &gs.Rsrc_x, &gs.Rsrc_y, vx, vy, &wsrc);
         walk[(int64_t)blockIdx.x * nv + v] = make_int4(wd.n, wd.edge, wsrc.n, wsrc.edge);
         // Compton bins, as k_fwd forms them
         const VoxGeom vg = vox_geom<false>(G, vx, vy);

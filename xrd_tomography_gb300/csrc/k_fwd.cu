@@ -103,7 +103,7 @@ __host__ __device__ inline Layout fwd_layout(const DevProblem &P, int E, int SL,
 
 struct FwdArgs {
     DevProblem P;
-    const SrcGeom *sg;
+    const PairRec *recs;       // [block] the blocks' pairs
     FwdTables T;
     const int *vox_xy, *vox_mat, *vox_na, *vox_order;
     const float *vox_a2;
@@ -113,8 +113,7 @@ struct FwdArgs {
     const float *vox_ta;         // the table path, bilinear: the Compton column as a grid coordinate
     const float *Ifine;
     float *N, *C;
-    const int2 *pairs;         // a list of pairs, or NULL: the linear pairs src + det*SRC
-    long long p0;              // block b takes pair p0 + b (of the list or of the linear index)
+    long long p0;              // block b writes output column p0 + b
     long long n_cols;          // output columns: the list's length, or SRC*DET
     const float2 *walk;        // [block][nv] detector-side line integrals (k_walk.cu)
     int nv, E, sl;
@@ -188,16 +187,7 @@ k_fwd(const FwdArgs args)
     const float *S1 = (const float *)(sm + L.s1);
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nthr = 32 * nw;
-    int det, src;
     const int64_t colidx = args.p0 + blockIdx.x;   // output column of this block
-    if (args.pairs) {
-        const int2 pr = args.pairs[colidx];
-        src = pr.x;
-        det = pr.y;
-    } else {
-        src = (int)(colidx % P.n_src);
-        det = (int)(colidx / P.n_src);
-    }
     const int64_t ncols = args.n_cols;
     const float2 *walk = args.walk + (int64_t)blockIdx.x * args.nv;
 
@@ -232,8 +222,9 @@ k_fwd(const FwdArgs args)
     auto table2 = [&](int i) { return FAST || args.split.tables ? S2[i] : (float)__ldg(args.s2u8 + i); };
     auto table1 = [&](int i) { return FAST || args.split.tables ? S1[i] : (float)__ldg(args.s1u8 + i); };
 
-    // ---- per-(source, pixel) geometry, integrate_diffraction.cu:81-128 ----
-    if (tid == 0) pair_geom(P, args.sg[src], det, &pair.G, &pair.Rdx, &pair.Rdy);
+    // ---- per-(source, pixel) geometry, integrate_diffraction.cu:81-128 (k_pair_table) ----
+    for (int i = tid; i < (int)(sizeof(PairRec) / 4); i += nthr)
+        reinterpret_cast<int *>(&pair)[i] = reinterpret_cast<const int *>(args.recs + blockIdx.x)[i];
     const float qmin_t = c.qmin_t, inv_dqt = c.inv_dqt;
     const float dEdf = c.dEd, dEsf = c.dEs, kn0 = c.kn0;
     const int jlast = (int)kMagicBits + P.nqf - 1;
@@ -261,7 +252,7 @@ k_fwd(const FwdArgs args)
             // labels as at integrate_diffraction.cu:259-260: the detector-side
             // integral feeds Pin, the source-side one Pout; the coherent term
             // needs their sum only
-            const float2 As = args.atten_src[(int64_t)src * nv + v];
+            const float2 As = args.atten_src[(int64_t)pair.src * nv + v];
             const float2 Ad = walk[v];
             // factors formed once per voxel: the Compton weight gp a2 / 2 over
             // the source bin width (the 1/2 of Cf, :347), the Rayleigh weight
@@ -586,19 +577,18 @@ cudaError_t launch_gather_rays(const int64_t *idx, int64_t n, const float *Nc, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_fast_forward(const DevProblem &P, const SrcGeom *d_src, const FwdTables &T,
-                                const PrepBuffers &B, int nv, const float *Ifine, const int2 *pairs,
+cudaError_t launch_fast_forward(const DevProblem &P, const PairRec *recs, const FwdTables &T,
+                                const PrepBuffers &B, int nv, const float *Ifine, bool list,
                                 long long n_list, long long p0, int n_pairs, const float2 *walk, float *N,
                                 float *C, cudaStream_t s, int64_t *launches, int tab)
 {
     if (!N || !C || !B.vox_order || tab < 0 || tab > 2 || (tab && !B.s1u8) || (tab == 2 && !B.vox_ta)) return cudaErrorInvalidValue;
     FwdArgs a;
-    a.pairs = pairs;
     a.p0 = p0;
-    a.n_cols = pairs ? n_list : (long long)P.n_src * P.n_det;
+    a.n_cols = list ? n_list : (long long)P.n_src * P.n_det;
     a.walk = walk;
     a.P = P;
-    a.sg = d_src;
+    a.recs = recs;
     a.T = T;
     a.vox_xy = B.vox_xy;
     a.vox_mat = B.vox_mat;

@@ -8,7 +8,11 @@
 //    packed FMAs with no border tests.  The map is stored twice: row-major
 //    (ci + cj (NX+1)) and behind it column-major (cj + ci (NY+1)), so that a
 //    warp whose rays lie side by side along y reads neighbouring cells from
-//    one cache line as well as one whose rays lie side by side along x.  Also
+//    one cache line as well as one whose rays lie side by side along x.  A
+//    uniform cell also carries the radius of the uniform square around it
+//    (walk_cells, walk.cuh).  One block per 32 x 32 cells; coefficients from
+//    float pairs (in FP64 the blocks of a small map queued on the FP64 pipes of
+//    a few SMs: 24 us against 14 on 45x33).  Also
 //    quantises the Compton table to u8 (integrate_diffraction.cu:66-74).
 //  * k_compact_voxels: non-empty voxels in the reference's loop order
 //    (nx outer, ny inner; integrate_diffraction.cu:173-178) and the material
@@ -24,36 +28,90 @@ namespace xrdt {
 
 namespace {
 
-__global__ void k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restrict__ a2,
+// (a + b) + (c + d) in float pairs, rounded to float (plain float sums where
+// a pair's low part overflows to NaN).
+__device__ __forceinline__ float sum4(float a, float b, float c, float d)
+{
+    const ff s = ff_add(two_sum(a, b), two_sum(c, d));
+    return isfinite(s.hi) ? s.hi : (a + b) + (c + d);
+}
+
+constexpr int kRows = 32 + 2 * kReach;   // cells of a tile and its surroundings, per side
+
+__global__ void __launch_bounds__(1024)
+k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restrict__ a2,
                               float4 *__restrict__ cells, const float *__restrict__ S2,
                               unsigned char *__restrict__ s2u8, int ns2, const float *__restrict__ S1,
                               unsigned char *__restrict__ s1u8)
 {
+    __shared__ unsigned uneven[kRows][3];
+    __shared__ unsigned char row_dist[kRows][32];
     const int64_t ncell = (int64_t)(nx + 1) * (ny + 1);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncell; c += stride) {
-        const int ci = (int)(c % (nx + 1)), cj = (int)(c / (nx + 1));
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tiles_x = (nx + 1 + 31) >> 5;
+    const int x0 = 32 * (int)(blockIdx.x % tiles_x), y0 = 32 * (int)(blockIdx.x / tiles_x);
+    // texel (i, j) of the map with its zero border
+    auto texel = [&](int i, int j) {
+        const bool in = (i >= 0 && i < nx && j >= 0 && j < ny);
+        const int64_t idx = in ? (int64_t)i + (int64_t)j * nx : 0;
+        return in ? make_float2(a1[idx], a2[idx]) : make_float2(0.f, 0.f);
+    };
+    // ---- which cells of the tile and its surroundings are not uniform ----
+    // row r of `uneven`: cells y0 - kReach + r, bit b: cell x0 - kReach + b;
+    // cells outside the map count as uniform (no sample lies there)
+#pragma unroll 3
+    for (int i = wid; i < kRows * 3; i += 32) {
+        const int r = i / 3, w = i - 3 * r;
+        const int ci = x0 - kReach + 32 * w + lane, cj = y0 - kReach + r;
+        bool odd = false;
+        if (ci >= 0 && ci <= nx && cj >= 0 && cj <= ny && 32 * w + lane < kRows) {
+            const float2 t = texel(ci, cj), l = texel(ci - 1, cj), d = texel(ci, cj - 1), e = texel(ci - 1, cj - 1);
+            odd = !(t.x == l.x && t.x == d.x && t.x == e.x && t.y == l.y && t.y == d.y && t.y == e.y);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, odd);
+        if (lane == 0) uneven[r][w] = m;
+    }
+    __syncthreads();
+    // ---- per row and tile column: distance to the nearest one in the row ----
+    for (int r = wid; r < kRows; r += 32) {
+        const unsigned w0 = uneven[r][0], w1 = uneven[r][1], w2 = uneven[r][2];
+        const int c = lane + kReach;   // this column's bit
+        const unsigned right = c < 32 ? __funnelshift_r(w0, w1, c) : __funnelshift_r(w1, w2, c - 32);   // bits c ..
+        const unsigned left = __funnelshift_r(w0, w1, lane);                                            // bits .. c
+        const int dr = right ? __ffs(right) - 1 : 32, dl = left ? __clz(left) : 32;
+        row_dist[r][lane] = (unsigned char)min(dr, dl);
+    }
+    __syncthreads();
+    const int ci = x0 + lane, cj = y0 + wid;
+    if (ci <= nx && cj <= ny) {
+        int dist = row_dist[kReach + wid][lane];
+        for (int dy = 1; dy < dist; dy++)
+            dist = min(dist, max(dy, min((int)row_dist[kReach + wid - dy][lane], (int)row_dist[kReach + wid + dy][lane])));
+        const int64_t c = (int64_t)ci + (int64_t)cj * (nx + 1);
         float v[2][2][2];
 #pragma unroll
         for (int dj = 0; dj < 2; dj++)
 #pragma unroll
             for (int di = 0; di < 2; di++) {
-                const int i = ci - 1 + di, j = cj - 1 + dj;
-                const bool in = (i >= 0 && i < nx && j >= 0 && j < ny);
-                const int64_t idx = in ? (int64_t)i + (int64_t)j * nx : 0;
-                v[dj][di][0] = in ? a1[idx] : 0.f;
-                v[dj][di][1] = in ? a2[idx] : 0.f;
+                const float2 t = texel(ci - 1 + di, cj - 1 + dj);
+                v[dj][di][0] = t.x;
+                v[dj][di][1] = t.y;
             }
         // bilinear coefficients per component q about the cell centre:
         // f(u,v) = c00 + c10 u + c01 v + c11 u v for u, v in [-1/2, 1/2]
         float c00[2], c10[2], c01[2], c11[2];
         for (int q = 0; q < 2; q++) {
-            const double f00 = v[0][0][q], f10 = v[0][1][q], f01 = v[1][0][q], f11 = v[1][1][q];
-            c00[q] = (float)(0.25 * ((f00 + f10) + (f01 + f11)));
-            c10[q] = (float)(0.5 * ((f10 - f00) + (f11 - f01)));
-            c01[q] = (float)(0.5 * ((f01 - f00) + (f11 - f10)));
-            c11[q] = (float)((f11 - f01) - (f10 - f00));
+            const float f00 = v[0][0][q], f10 = v[0][1][q], f01 = v[1][0][q], f11 = v[1][1][q];
+            c00[q] = 0.25f * sum4(f00, f10, f01, f11);
+            c10[q] = 0.5f * sum4(f10, -f00, f11, -f01);
+            c01[q] = 0.5f * sum4(f01, -f00, f11, -f10);
+            c11[q] = sum4(f11, -f01, f00, -f10);
         }
+        // a uniform cell's c11 is 0: the first one carries twice the radius of
+        // the uniform square around it, scaled below every coefficient that
+        // is kept (walk_cells)
+        if (fabsf(c11[0]) < kReachLimit) c11[0] = dist > 1 ? (float)(2 * (dist - 1)) * kReachUnit : 0.f;
         const float4 lo = make_float4(c00[0], c00[1], c10[0], c10[1]);
         const float4 hi = make_float4(c01[0], c01[1], c11[0], c11[1]);
         const int64_t ct = ncell + (int64_t)cj + (int64_t)ci * (ny + 1);
@@ -198,9 +256,10 @@ __global__ void k_voxel_compton(DevProblem P, const float *__restrict__ a1, cons
 }
 
 // One lane per (source, voxel): attenuator(Rsrc, Rvox) of
-// integrate_diffraction.cu:260, set up in FP64 and walked cell by cell from
-// the voxel (walk_cells).  A warp takes 32 neighbouring voxels of one source.
-__global__ void k_src_atten(DevProblem P, const SrcGeom *__restrict__ sg, const int *__restrict__ vox_xy,
+// integrate_diffraction.cu:260, decided as the detector side's (walk_decide)
+// and walked cell by cell from the voxel (walk_cells).  A warp takes 32
+// neighbouring voxels of one source.
+__global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int *__restrict__ vox_xy,
                             int nv, const float4 *__restrict__ cells, float2 *__restrict__ out)
 {
     const int64_t nwork = (int64_t)P.n_src * nv;
@@ -209,11 +268,12 @@ __global__ void k_src_atten(DevProblem P, const SrcGeom *__restrict__ sg, const 
     for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < nwork; w += stride) {
         const int src = (int)(w / nv), v = (int)(w % nv);
         const int xy = vox_xy[v];
-        const double vx = ((double)(xy & 0xffff) + 0.5) * P.vox;
-        const double vy = ((double)(xy >> 16) + 0.5) * P.vox;
+        const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
+        const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
+        const SrcGeom *g = sg + src;
         WalkSetup ws;
-        walk_setup(P, sg[src].Rsrc_x, sg[src].Rsrc_y, vx, vy, &ws);
-        out[(int64_t)src * nv + v] = walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, (float)vx, (float)vy, (float)P.DQ);
+        walk_decide(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), &g->Rsrc_x, &g->Rsrc_y, vx, vy, &ws);
+        out[(int64_t)src * nv + v] = walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ);
     }
 }
 
@@ -222,10 +282,9 @@ __global__ void k_src_atten(DevProblem P, const SrcGeom *__restrict__ sg, const 
 cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a2, const float *S2,
                             PrepBuffers &B, cudaStream_t s, int64_t *launches, const float *S1)
 {
-    const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
-    int blocks = (int)((ncell + 255) / 256);
-    if (blocks > 4096) blocks = 4096;
-    k_build_cells<<<blocks, 256, 0, s>>>(P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8, S2 ? P.nq * P.na : 0,
+    // one block of 1024 threads per tile of 32 x 32 cells
+    const int64_t blocks = (int64_t)((P.nx + 1 + 31) / 32) * ((P.ny + 1 + 31) / 32);
+    k_build_cells<<<(unsigned)blocks, 1024, 0, s>>>(P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8, S2 ? P.nq * P.na : 0,
                                          B.s1u8 ? S1 : nullptr, B.s1u8);
     if (launches) (*launches)++;
     return cudaGetLastError();
@@ -282,7 +341,7 @@ cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, 
     const int64_t items = (int64_t)P.n_src * nv;
     int64_t blocks = (items + 127) / 128;
     if (blocks > (int64_t)sms * 16) blocks = (int64_t)sms * 16;
-    k_src_atten<<<(int)blocks, 128, 0, s>>>(P, d_src, B.vox_xy, nv, B.cells, B.atten_src);
+    k_src_atten<<<(int)blocks, 128, 0, s>>>(P, make_f32_consts(P), d_src, B.vox_xy, nv, B.cells, B.atten_src);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

@@ -640,16 +640,19 @@ __global__ void k_vox_scatter(const VoxBatch B)
     }
 }
 
-// Pair table: the (source, pixel) constants of every pair, once per operator.
-__global__ void k_pair_table(DevProblem P, const SrcGeom *__restrict__ sg, PairRec *__restrict__ out)
+// Pair table: the (source, pixel) constants of a list of pairs or of the
+// linear pairs from p0 on.
+__global__ void k_pair_table(DevProblem P, const SrcGeom *__restrict__ sg, const int2 *__restrict__ list, int64_t p0,
+                             int64_t n, PairRec *__restrict__ out)
 {
-    const int64_t npairs = (int64_t)P.n_src * P.n_det;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npairs;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int src = (int)(p % P.n_src), det = (int)(p / P.n_src);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = p0 + i;
+        const int2 pr = list ? list[i] : make_int2((int)(p % P.n_src), (int)(p / P.n_src));
         PairRec r;
-        pair_geom(P, sg[src], det, &r.G, &r.Rdx, &r.Rdy);
-        out[p] = r;
+        pair_geom(P, sg[pr.x], pr.y, &r.G, &r.Rdx, &r.Rdy);
+        r.src = pr.x;
+        r.pad = 0;
+        out[i] = r;
     }
 }
 
@@ -687,11 +690,11 @@ size_t static_smem(F *kernel)
 
 size_t pair_rec_bytes() { return sizeof(PairRec); }
 
-cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, PairRec *out, cudaStream_t s,
-                              int64_t *launches)
+cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, const int2 *list, long long p0, long long n,
+                              PairRec *out, cudaStream_t s, int64_t *launches)
 {
-    const int64_t n = (int64_t)P.n_src * P.n_det;
-    k_pair_table<<<grid_for(n, 128), 128, 0, s>>>(P, sg, out);
+    // small blocks: the records are FP64 work, spread over the SMs
+    k_pair_table<<<grid_for(n, 32), 32, 0, s>>>(P, sg, list, p0, n, out);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

@@ -40,36 +40,28 @@ constexpr int kRays = 32;          // rays per group: neighbouring pixels of one
 constexpr int kMaxStrip = 64;
 constexpr int kItemsPerSM = 256;   // 8 times the resident warps
 
-// Ray r of group g.  Linear pairs (pairs == NULL): the tile holds the pixels
-// d0 .. d0+nd-1 of every view, row (det - d0) * SRC + src; group g is view
-// g % SRC and pixels d0 + 32 (g / SRC) + r.  A list: entries 32g + r.
-__device__ __forceinline__ bool group_ray(const DevProblem &P, const int2 *pairs, long long n_items, int nd,
-                                          long long g, int r, int *src, int *det, long long *row)
+// Row of ray r of group g.  Linear pairs: the tile holds whole pixels (nd of
+// them) of every view, row pixel * SRC + view; group g is view g % SRC and
+// pixels 32 (g / SRC) + r.  A list: entries 32g + r.
+__device__ __forceinline__ bool group_row(const DevProblem &P, int list, long long n_items, int nd, long long g, int r,
+                                          long long *row)
 {
-    if (pairs) {
-        const long long e = g * kRays + r;
-        if (e >= n_items) return false;
-        const int2 pr = pairs[e];
-        *src = pr.x;
-        *det = pr.y;
-        *row = e;
-        return true;
+    if (list) {
+        *row = g * kRays + r;
+        return *row < n_items;
     }
     const int s = (int)(g % P.n_src);
     const int dl = (int)(g / P.n_src) * kRays + r;
-    if (dl >= nd) return false;
-    *src = s;
-    *det = dl;   // relative to d0
     *row = (long long)dl * P.n_src + s;
-    return true;
+    return dl < nd;
 }
 
 // 8 blocks (32 warps) per SM: the walk waits on L1 latency, and at 64
 // registers (8 bytes spilled around the FP64 fallback call) it ran 1016 ms on
 // the 256x256 workload against 1089 ms at 6 blocks and 80 registers.
 __global__ void __launch_bounds__(kWalkThreads, 8)
-k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2 *__restrict__ pairs,
-           long long n_items, int d0, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,
+k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list,
+           long long n_items, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,
            const float4 *__restrict__ cells, float2 *__restrict__ tab)
 {
     const int lane = threadIdx.x & 31;
@@ -82,20 +74,12 @@ k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2
     for (long long wk = (long long)blockIdx.x * kWalkWarps + (threadIdx.x >> 5); wk < nwork; wk += wstride) {
         const long long g = wk / nstrips;
         const int strip = (int)(wk - g * nstrips);
-        int src = 0, det = 0;
         long long row = -1;
-        const bool valid = group_ray(P, pairs, n_items, nd, g, lane, &src, &det, &row);
-        double ex = 0.0, ey = 0.0;
-        if (valid) {
-            if (!pairs) det += d0;
-            const SrcGeom gs = sg[src];
-            double ez;
-            det_position(P, gs.sphi, gs.cphi, det, &ex, &ey, &ez);
-        }
-        const float exf = (float)ex, eyf = (float)ey;
-        // the endpoint as float pairs, once per ray group (conversions from
-        // double issue on the FP64 pipe)
-        const ff exff = ff_from_double(ex), eyff = ff_from_double(ey);
+        const bool valid = group_row(P, list, n_items, nd, g, lane, &row);
+        // the pixel's position, tabulated per pair, as float pairs (and as
+        // double for the rare FP64 set-up)
+        const PairRec *rec = recs + (valid ? row : 0);
+        const ff exff = rec->G.Rdx, eyff = rec->G.Rdy;
         float2 *out = tab + (valid ? row : 0) * nv;
         const int v1 = min(nv, (strip + 1) * strip_len);
         for (int v = strip * strip_len; v < v1; v++) {
@@ -106,14 +90,7 @@ k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2
             ws.Lx = ws.Ly = 0.f;
             ws.n = 0;
             ws.dlt = ws.ux = ws.uy = ff{0.f, 0.f};
-            if (valid) {
-                // decided in FP32 (guard bands) or FP64; the anchor of an FP32
-                // decision comes from the endpoint as a float pair
-                if (walk_setup_f32(P, c, exf, eyf, vx, vy, &ws))
-                    walk_anchor_ff(c, exff, eyff, vx, vy, &ws);
-                else
-                    walk_setup_f64(P, ex, ey, (double)vx, (double)vy, &ws);
-            }
+            if (valid) walk_decide(P, c, exff, eyff, &rec->Rdx, &rec->Rdy, vx, vy, &ws);
             // rays mostly along x lie side by side along y: column-major copy
             const unsigned along_x = __ballot_sync(0xffffffffu, valid && fabsf(ws.Lx) > fabsf(ws.Ly));
             const unsigned any = __ballot_sync(0xffffffffu, valid);
@@ -127,19 +104,17 @@ k_det_walk(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int2
 
 } // namespace
 
-cudaError_t launch_det_walk(const DevProblem &P, const SrcGeom *sg, const int2 *pairs, long long p0,
-                            long long n_items, const int *vox_xy, int nv, const float4 *cells, float2 *tab,
-                            cudaStream_t s, int64_t *launches)
+cudaError_t launch_det_walk(const DevProblem &P, const PairRec *recs, bool list, long long n_items, const int *vox_xy,
+                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches)
 {
     if (n_items <= 0 || nv <= 0) return cudaSuccess;
-    int d0 = 0, nd = 0;
+    int nd = 0;
     long long n_groups;
-    if (pairs) {
+    if (list) {
         n_groups = (n_items + kRays - 1) / kRays;
     } else {
         // whole pixels of every view
-        if (p0 % P.n_src != 0 || n_items % P.n_src != 0) return cudaErrorInvalidValue;
-        d0 = (int)(p0 / P.n_src);
+        if (n_items % P.n_src != 0) return cudaErrorInvalidValue;
         nd = (int)(n_items / P.n_src);
         n_groups = (long long)P.n_src * ((nd + kRays - 1) / kRays);
     }
@@ -149,7 +124,7 @@ cudaError_t launch_det_walk(const DevProblem &P, const SrcGeom *sg, const int2 *
     const long long nwork = n_groups * ((nv + strip - 1) / strip);
     long long blocks = (nwork + kWalkWarps - 1) / kWalkWarps;
     if (blocks > (long long)sms * 64) blocks = (long long)sms * 64;
-    k_det_walk<<<(unsigned)blocks, kWalkThreads, 0, s>>>(P, make_f32_consts(P), sg, pairs, n_items, d0, nd, n_groups,
+    k_det_walk<<<(unsigned)blocks, kWalkThreads, 0, s>>>(P, make_f32_consts(P), recs, list ? 1 : 0, n_items, nd, n_groups,
                                                           strip, vox_xy, nv, cells, tab);
     if (launches) (*launches)++;
     return cudaGetLastError();

@@ -314,7 +314,8 @@ cudaError_t tile_walks(const Plan *pl, const Plan::Tile &t, cudaStream_t st, int
     for (const Plan::Seg &sg : t.segs) {
         if (sg.woff < 0) continue;
         const xrdt_op *op = pl->ops[sg.op];
-        cudaError_t e = launch_det_walk(op->v.P, op->src, nullptr, sg.p0, sg.p1 - sg.p0, op->v.vox_xy, op->v.nv,
+        const char *recs = (const char *)op->v.pairs + pair_rec_bytes() * sg.p0;
+        cudaError_t e = launch_det_walk(op->v.P, (const PairRec *)recs, false, sg.p1 - sg.p0, op->v.vox_xy, op->v.nv,
                                         op->v.cells, pl->walkbuf + sg.woff, st, launches);
         if (e != cudaSuccess) return e;
     }
@@ -932,7 +933,7 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     e = cudaMemcpyAsync(d_src, hsg.data(), sizeof(SrcGeom) * p->n_src, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = launch_compact_voxels(P, op->seg, B, st, &ctx->launches);
     if (e == cudaSuccess) e = launch_prep_map(P, op->a1, op->a2, nullptr, B, st, &ctx->launches);
-    if (e == cudaSuccess) e = launch_pair_table(P, d_src, d_pairs, st, &ctx->launches);
+    if (e == cudaSuccess) e = launch_pair_table(P, d_src, nullptr, 0, npairs, d_pairs, st, &ctx->launches);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_counters, B.counters, sizeof(int) * 2, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
@@ -967,7 +968,7 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
             void *w;
             if ((rc = op_alloc(op, bytes, &w))) return bail(rc);
             d_walk = (float2 *)w;
-            if ((e = launch_det_walk(P, d_src, nullptr, 0, npairs, B.vox_xy, nv, B.cells, d_walk, st,
+            if ((e = launch_det_walk(P, d_pairs, false, npairs, B.vox_xy, nv, B.cells, d_walk, st,
                                      &ctx->launches)) != cudaSuccess) {
                 cudaGetLastError();
                 fail(ctx, XRDT_ERR_CUDA, fmt("detector-side integrals: %s", cudaGetErrorString(e)));

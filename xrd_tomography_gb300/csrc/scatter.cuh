@@ -36,11 +36,12 @@ struct VoxGeom {
     float cos2;  // cos^2(theta)
 };
 
-// A pair's constants with its detector position in double, tabulated once
-// per operator (k_vox.cu).
+// A pair's constants with its detector position in double and its source,
+// tabulated once per operator or forward call (k_pair_table, k_vox.cu).
 struct PairRec {
     PairGeom G;
     double Rdx, Rdy;
+    int src, pad;
 };
 
 namespace {
@@ -226,14 +227,6 @@ __device__ __forceinline__ float table_bilinear(const Table &S, int nq, int na, 
     const float lo = fmaf(f, S(r0 + 1) - s00, s00);
     const float hi = fmaf(f, S(r1 + 1) - s01, s01);
     return fmaf(g, hi - lo, lo);
-}
-
-// FP64 walk set-up out of line: the rare fallback of walk_setup_f32 stays a
-// real branch instead of being predicated into the caller's loop.
-__device__ __noinline__ void walk_setup_f64(const DevProblem &P, double ex, double ey, double vx, double vy,
-                                            WalkSetup *w)
-{
-    walk_setup(P, ex, ey, vx, vy, w);
 }
 
 // integrate_diffraction.cu:93-128 for source g and pixel det: the pair's

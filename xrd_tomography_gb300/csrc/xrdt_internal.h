@@ -38,7 +38,7 @@ struct DevProblem {
 // holding it in a register) runs on the FP64 pipe, which on this GPU issues
 // at 1/64 of the FP32 rate.
 struct F32Consts {
-    float vox, DQ, inv_DQ, nxf, nyf, rsqrt2pi;
+    float vox, DQ, DQ_lo, inv_DQ, nxf, nyf, rsqrt2pi;
     float dqf_hi, dqf_lo, inv_dqf, q_lo, q_hi;
     float kn0, kn1, kn2;
     float edmin, inv_dEd, dEd, dEs, inv_dEs;
@@ -152,6 +152,8 @@ cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const fl
 cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, PrepBuffers &B,
                              cudaStream_t s, int64_t *launches);
 
+// The constants of one (source, pixel) pair (scatter.cuh).
+struct PairRec;
 // k_fwd.cu: factored FP32 forward over (src, det) pairs.
 struct FwdTables {
     const EnergyRow *energy;   // [nrg_src]
@@ -168,11 +170,12 @@ struct FwdTables {
 };
 // n_pairs blocks, block b on pair p0 + b: of the list pairs[0 .. n_list)
 // when it is given (outputs then go to the compact layout [nrg_det][n_list]),
-// else of the linear index src + det*SRC of the full layout.  walk holds the
-// blocks' detector-side integrals, [n_pairs][nv] (launch_det_walk).
-cudaError_t launch_fast_forward(const DevProblem &P, const SrcGeom *d_src, const FwdTables &T,
+// else of the linear index src + det*SRC of the full layout.  recs and walk
+// hold the blocks' pair records and detector-side integrals, [n_pairs] and
+// [n_pairs][nv] (launch_pair_table, launch_det_walk).
+cudaError_t launch_fast_forward(const DevProblem &P, const PairRec *recs, const FwdTables &T,
                                 const PrepBuffers &B, int nv, const float *Ifine,
-                                const int2 *pairs, long long n_list, long long p0, int n_pairs,
+                                bool list, long long n_list, long long p0, int n_pairs,
                                 const float2 *walk, float *N, float *C, cudaStream_t s, int64_t *launches, int tab);
 // k_matrix.cu: the same with the model matrix A (compact layout
 // [nrg_det][n_list][n_mat*nwt] for a list of pairs).
@@ -194,12 +197,15 @@ struct SpecCoarseBin {
 cudaError_t launch_spectrum(const SpecFineBin *fb, const SpecCoarseBin *sb, int ns, const SpecCoarseBin *db, int nd,
                             float *out, cudaStream_t s, int64_t *launches);
 
+size_t pair_rec_bytes();
+// out[i] = the record of pair list[i], or of the linear pair p0 + i, i < n.
+cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, const int2 *list, long long p0, long long n,
+                              PairRec *out, cudaStream_t s, int64_t *launches);
 // k_walk.cu: tab[item][v] = detector-side line integral of voxel v for the
-// pair pairs[item] (or the linear pair p0 + item), item < n_items.  Linear
-// pairs come in whole pixels: p0 and n_items multiples of SRC.
-cudaError_t launch_det_walk(const DevProblem &P, const SrcGeom *sg, const int2 *pairs, long long p0,
-                            long long n_items, const int *vox_xy, int nv, const float4 *cells, float2 *tab,
-                            cudaStream_t s, int64_t *launches);
+// pair of recs[item], item < n_items.  Pairs that are not a list come in
+// whole pixels of every view, from a multiple of SRC on.
+cudaError_t launch_det_walk(const DevProblem &P, const PairRec *recs, bool list, long long n_items, const int *vox_xy,
+                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches);
 // k_bop.cu: rows of R values per non-empty voxel between the full grid
 // [NX*NY][R] and the compact voxel order [nv][R]; the coefficient-space MLEM
 // update c <- c g / (s + 1e-7) with the fix-ups of main.m:163,176.
@@ -236,8 +242,6 @@ cudaError_t launch_mlem_iteration(const float *A, long long rays, int K, const f
                                   int64_t *launches);
 
 // k_vox.cu: the per-voxel-coefficient model (forward, adjoint, MLEM update).
-struct PairRec;
-size_t pair_rec_bytes();
 struct VoxOp {
     DevProblem P;
     int nv;                    // non-empty voxels
@@ -253,8 +257,6 @@ struct VoxOp {
 };
 cudaError_t launch_compact_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
                                   int64_t *launches);
-cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, PairRec *out, cudaStream_t s,
-                              int64_t *launches);
 
 // One problem of an operator batch as the kernels read it (device memory):
 // its tables, its adjoint split and its buffers.
