@@ -111,3 +111,25 @@ def test_walks_across_uniform_squares(ctx, oracle_lib, kind):
     Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
     assert max_rel_err(N[rays], Nr) < FAST_RTOL
     assert max_rel_err(C[rays], Cr) < FAST_RTOL
+
+
+# the model matrix over groups of 32 coarse bins: part of one, one and a part,
+# exact ones, a second block of eight groups; several passes over the energies
+# (large rows); voxels at the materials' borders; tiles and remainders of steps
+@pytest.mark.parametrize("nx,ny,es,ed,nwt,mats", [(9, 5, 5, 5, 8, 2), (23, 30, 12, 12, 40, 3), (40, 44, 17, 13, 64, 4),
+                                                  (16, 12, 9, 9, 130, 5), (12, 12, 64, 64, 256, 9),
+                                                  (12, 14, 12, 12, 300, 2)])
+def test_model_matrix_over_bin_groups(ctx, oracle_lib, nx, ny, es, ed, nwt, mats):
+    inp = synth.make_inputs(sized_problem(nx, ny, 3, 34, es, ed, 2, nwt=nwt, mats=mats), 400 + nwt)
+    p = inp.problem
+    if nwt > 100:
+        p.dq0 = 0.005
+    rays = some_rays(p, 60, nwt)
+    Nr, Cr, Ar = oracle_lib.forward_rays(inp, rays, want_a=True)[:3]
+    N, C, A = xt.forward_rays(p, rays, *inp.args(), want_amatrix=True, ctx=ctx)
+    assert max_rel_err(N, Nr) < FAST_RTOL
+    assert max_rel_err(C, Cr) < FAST_RTOL
+    assert max_rel_err(A, np.asarray(Ar).reshape(A.shape)) < FAST_RTOL
+    N, C, A = xt.forward(p, *inp.args(), ctx=ctx)
+    assert max_rel_err(A.reshape(p.rays, p.n_mat, p.nwt)[rays], np.asarray(Ar).reshape(len(rays), p.n_mat, p.nwt)) < FAST_RTOL
+    assert np.array_equal(A, xt.forward(p, *inp.args(), ctx=ctx)[2])

@@ -814,13 +814,11 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
                                        &ctx->launches));
                 }
                 ProfScope ps(ctx, XRDT_KERNEL_FORWARD);
+                CK(launch_fast_forward(P, recs, T, B, nv, (const float *)d_ifine, list != nullptr, n_total, p0, (int)n,
+                                       (const float2 *)dtab, oN, oC, st, &ctx->launches, tab));
                 if (oA)
-                    CK(launch_matrix(P, (const SrcGeom *)d_srcg, T, B, nv, (const float *)d_ifine, list, n_total, p0,
-                                     (int)n, (const float2 *)dtab, oN, oC, oA, st, &ctx->launches));
-                else
-                    CK(launch_fast_forward(P, recs, T, B, nv, (const float *)d_ifine, list != nullptr, n_total,
-                                           p0, (int)n, (const float2 *)dtab, oN, oC, st, &ctx->launches,
-                                           tab));
+                    CK(launch_matrix(P, recs, T, B, nv, list != nullptr, n_total, p0, (int)n, (const float2 *)dtab, oA,
+                                     st, &ctx->launches));
             }
             return XRDT_OK;
         };

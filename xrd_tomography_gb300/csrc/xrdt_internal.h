@@ -177,11 +177,10 @@ cudaError_t launch_fast_forward(const DevProblem &P, const PairRec *recs, const 
                                 const PrepBuffers &B, int nv, const float *Ifine,
                                 bool list, long long n_list, long long p0, int n_pairs,
                                 const float2 *walk, float *N, float *C, cudaStream_t s, int64_t *launches, int tab);
-// k_matrix.cu: the same with the model matrix A (compact layout
-// [nrg_det][n_list][n_mat*nwt] for a list of pairs).
-cudaError_t launch_matrix(const DevProblem &P, const SrcGeom *d_src, const FwdTables &T,
-                          const PrepBuffers &B, int nv, const float *Ifine, const int2 *pairs, long long n_list,
-                          long long p0, int n_pairs, const float2 *walk, float *N, float *C, float *A,
+// k_matrix.cu: the model matrix of the same pairs (rows of n_mat*nwt; the
+// compact layout [nrg_det][n_list][n_mat*nwt] for a list).
+cudaError_t launch_matrix(const DevProblem &P, const PairRec *recs, const FwdTables &T, const PrepBuffers &B, int nv,
+                          bool list, long long n_list, long long p0, int n_pairs, const float2 *walk, float *A,
                           cudaStream_t s, int64_t *launches);
 // k_spectrum.cu: the spectrum-response matrix (spectrum_builder.m:64-95).
 // A fine bin: edges, centre, 1/(2 sigma^2) and n/(sqrt(2 pi) sigma); a coarse
