@@ -133,3 +133,49 @@ def test_model_matrix_over_bin_groups(ctx, oracle_lib, nx, ny, es, ed, nwt, mats
     N, C, A = xt.forward(p, *inp.args(), ctx=ctx)
     assert max_rel_err(A.reshape(p.rays, p.n_mat, p.nwt)[rays], np.asarray(Ar).reshape(len(rays), p.n_mat, p.nwt)) < FAST_RTOL
     assert np.array_equal(A, xt.forward(p, *inp.args(), ctx=ctx)[2])
+
+
+def vox_case(nx, ny, views, px, es, ed, dnrg, nwt, seed):
+    p = sized_problem(nx, ny, views, px, es, ed, dnrg, nwt=nwt)
+    if nwt > 100:
+        p.dq0 = 0.004
+    inp = synth.make_inputs(p, seed)
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0.0, 1.0, (nx * ny, nwt)).astype(np.float32)
+    x[inp.seg == 0] = 0.0
+    return inp, x.reshape(-1), rng.uniform(0.0, 2.0, p.rays).astype(np.float32)
+
+
+# the per-voxel operator: one chunk of voxels, remainders of chunks and tiles;
+# an odd number of energies and of coarse bins (both come in twos); one bin;
+# more bins than a tile has room for twice
+@pytest.mark.parametrize("nx,ny,es,ed,dnrg,nwt", [(5, 4, 1, 1, 0, 1), (24, 20, 7, 5, 2, 33), (30, 34, 12, 12, 2, 32),
+                                                  (44, 48, 17, 13, 3, 41), (20, 18, 12, 12, 2, 257),
+                                                  (12, 12, 65, 64, 5, 24)])
+def test_operator_over_splits(ctx, oracle_lib, nx, ny, es, ed, dnrg, nwt):
+    inp, x, w = vox_case(nx, ny, 3, 33, es, ed, dnrg, nwt, 500 + nwt)
+    p = inp.problem
+    op = xt.Operator(p, inp.spectrum, inp.seg, inp.a1, inp.a2, ctx=ctx)
+    rays = some_rays(p, 150, nwt)
+    ws = np.zeros_like(w)
+    ws[rays] = w[rays]
+    y_ref, g_ref = oracle_lib.vox_rays(inp, rays, x=x, w=w[rays])
+    y = op.forward(x)
+    assert max_rel_err(y[rays], y_ref) < FAST_RTOL
+    assert max_rel_err(op.adjoint(ws), g_ref.reshape(-1)) < FAST_RTOL
+    assert np.array_equal(y, op.forward(x))
+    op.close()
+
+
+def test_window_table_takes_any_order_of_bins(ctx, oracle_lib):
+    """Coarse bins whose edges turn back (dq0 NWT far beyond the range): their
+    centres are not in order, and the window table must still hold them all."""
+    inp, x, w = vox_case(20, 16, 3, 33, 12, 12, 2, 32, 77)
+    inp.problem.dq0 = 0.3
+    p = inp.problem
+    op = xt.Operator(p, inp.spectrum, inp.seg, inp.a1, inp.a2, ctx=ctx)
+    rays = np.arange(p.rays)
+    y_ref, g_ref = oracle_lib.vox_rays(inp, rays, x=x, w=w)
+    assert max_rel_err(op.forward(x), y_ref) < FAST_RTOL
+    assert max_rel_err(op.adjoint(w), g_ref.reshape(-1)) < FAST_RTOL
+    op.close()

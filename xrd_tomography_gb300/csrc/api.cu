@@ -349,6 +349,12 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
             q.edb = (float)(P.e_det_min + (double)(n0 - 1) * P.dEd);
         }
     }
+    t->vox_energy.resize(p->nrg_src);
+    for (int e = 0; e < p->nrg_src; e++) {
+        const EnergyRow &r = t->energy[e];
+        const FwdEnergy &q = t->fwd_energy[e];
+        t->vox_energy[e] = VoxEnergy{q.f1, q.f1l, q.f2, q.f2l, r.wfac_hi, r.wfac_lo, r.sig_c2, r.sig_c2_lo};
+    }
     t->fine_q.resize(p->nqf);
     for (int j = 0; j < p->nqf; j++) {
         const double q = P.q_lo + P.dq_fine * (0.5 + (double)j);
@@ -369,6 +375,24 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         t->coarse_q[k].z = (float)(e2 - e1);
         t->coarse_q[k].w = 0.f;
     }
+    // window table: the bins whose centres may lie beyond a wavevector's cell,
+    // each cell a little wider against the rounding of the index; any order of
+    // the centres gives a range that holds them all
+    t->qlut.assign(kLutCells + 2, 0u);
+    const double cell = (p->q_hi - p->q_lo) / kLutCells;
+    const double margin = std::max(1e-3, 1e-6 * std::max(std::fabs(p->q_lo), std::fabs(p->q_hi)) / cell) * cell;
+    for (int i = 0; i < kLutCells + 2; i++) {
+        const double a = i == 0 ? -HUGE_VAL : p->q_lo + (i - 1) * cell - margin;
+        const double b = i == kLutCells + 1 ? HUGE_VAL : p->q_lo + i * cell + margin;
+        int lo = p->nwt, hi = -1;
+        for (int k = 0; k < p->nwt; k++) {
+            const double q = (double)t->coarse_q[k].x;
+            if (q >= a && k < lo) lo = k;
+            if (q <= b) hi = k;
+        }
+        t->qlut[i] = (unsigned)lo | (unsigned)hi << 16;
+    }
+    t->lut_scale = (float)(1.0 / cell);
 }
 
 } // namespace xrdt

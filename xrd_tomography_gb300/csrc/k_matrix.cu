@@ -122,11 +122,12 @@ k_matrix(const MatrixArgs args)
                 const int xy = args.vox_xy[v];
                 const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
                 const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
-                const VoxGeom vg = vox_geom<false>(pair.G, vx, vy);
+                // sigma through pairs: a row's small entries are Gaussian tails
+                const VoxGeom vg = vox_geom<true>(pair.G, vx, vy);
                 const float2 As = args.atten_src[(int64_t)pair.src * nv + v];
                 const float2 Ad = walk[v];
                 const float wr = t0 + i < nv ? vg.Wg * c.rsqrt2pi : 0.f;
-                rec[i] = make_float4(Ad.x + As.x, Ad.y + As.y, __fdividef(vg.sg.hi, vg.s.hi * vg.s.hi), wr);
+                rec[i] = make_float4(Ad.x + As.x, Ad.y + As.y, ff_mul(vg.sg, ffl_rcp(vg.s2)).hi, wr);
                 rec[32 * nst + i] = make_float4(vg.s.hi, vg.s.lo, __int_as_float(args.vox_mat[v]), 0.f);
             }
             __syncthreads();

@@ -158,14 +158,15 @@ __device__ __forceinline__ int block_positions(unsigned keep, int *base, int (*c
 }
 
 // One block of 1024 threads, four voxels per thread and round: stream
-// compaction in loop order, then (order != NULL) the same voxels once more in
-// tiles of 8 x 4 voxels: order[i] is the loop-order number of the i-th voxel
-// in tile order.  Thirty-two neighbours in tile order lie within 8 x 4 voxels,
+// compaction in loop order, then (order or tile_xy != NULL) the same voxels
+// once more in tiles of 8 x 4 voxels: order[i] is the loop-order number of the
+// i-th voxel in tile order, tile_xy[i] its packed coordinates.  Thirty-two neighbours in tile order lie within 8 x 4 voxels,
 // in loop order within a strip 32 long: the lanes of a warp that takes them see
 // more even scattering angles and distances.  rank: [nx*ny] scratch.
 __global__ void __launch_bounds__(1024)
 k_compact_voxels(int nx, int ny, int n_mat, const int32_t *__restrict__ seg, int *__restrict__ vox_xy,
-                 int *__restrict__ vox_mat, int *__restrict__ counters, int *__restrict__ order, int *rank)
+                 int *__restrict__ vox_mat, int *__restrict__ counters, int *__restrict__ order, int *rank,
+                 int *__restrict__ tile_xy)
 {
     __shared__ int cnt[2][32];
     int bad = 0, base = 0, turn = 0;
@@ -197,7 +198,7 @@ k_compact_voxels(int nx, int ny, int n_mat, const int32_t *__restrict__ seg, int
                 vox_xy[pos] = x[r] | (y[r] << 16);
                 vox_mat[pos] = s[r] - 1;
             }
-            if (order && L0 + 4 * (int)threadIdx.x + r < total) rank[(int64_t)x[r] + (int64_t)y[r] * nx] = k ? pos : -1;
+            if (rank && L0 + 4 * (int)threadIdx.x + r < total) rank[(int64_t)x[r] + (int64_t)y[r] * nx] = k ? pos : -1;
             pos += k;
         }
     }
@@ -206,7 +207,7 @@ k_compact_voxels(int nx, int ny, int n_mat, const int32_t *__restrict__ seg, int
         counters[0] = base;
         counters[1] = bad;
     }
-    if (!order) return;
+    if (!rank) return;
     const int nty = (ny + 3) >> 2;
     const int64_t quads = 8 * (int64_t)((nx + 7) >> 3) * nty;   // columns of four voxels
     base = 0;
@@ -228,7 +229,11 @@ k_compact_voxels(int nx, int ny, int n_mat, const int32_t *__restrict__ seg, int
         int pos = block_positions(keep, &base, cnt, turn);
 #pragma unroll
         for (int r = 0; r < 4; r++)
-            if (v[r] >= 0) order[pos++] = v[r];
+            if (v[r] >= 0) {
+                if (order) order[pos] = v[r];
+                if (tile_xy) tile_xy[pos] = vox_xy[v[r]];
+                pos++;
+            }
     }
 }
 
@@ -294,7 +299,7 @@ cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const fl
                                const float *a2, PrepBuffers &B, cudaStream_t s, int64_t *launches)
 {
     k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
-                                        B.vox_rank);
+                                        B.vox_rank, nullptr);
     const int64_t nvox = (int64_t)P.nx * P.ny;
     int blocks = (int)((nvox + 255) / 256);
     if (blocks > 2048) blocks = 2048;
@@ -306,8 +311,8 @@ cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const fl
 cudaError_t launch_compact_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
                                   int64_t *launches)
 {
-    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
-                                        B.vox_rank);
+    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_order, B.vox_mat, B.counters, nullptr,
+                                        B.vox_rank, B.vox_xy);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

@@ -24,107 +24,149 @@
 // created) or the current tile of a walk streamed inside the call.
 //
 //  * forward (k_vox_fwd): one item = one (source, pixel) pair, as in
-//    k_fwd.cu; lane = source energy (or, for windows that are not a multiple
-//    of 32 energies, the chunk's (voxel, energy) items 32 at a time) sums the
-//    coarse bins within 7.5 sigma of the wavevector transfer, weighted by
-//    x[v, k] dq_k, into compensated per-energy sums; the banded spectrum
-//    weights give the detector bins.  In
-//    MLEM mode the block goes on to form the ratios y / (Av x + c + 1e-20) of
-//    main.m:162 for its detector bins and folds them back through the same
-//    spectrum band into per-energy weights what[pair, e] = sum_nrg RF[e,nrg]
-//    ratio[nrg].
+//    k_fwd.cu: tiles of voxels with their scattering geometry and their
+//    coefficients x[v, k] dq_k in shared memory, runs of 32-voxel steps of one
+//    energy off a counter, lane = voxel; a lane sums the coarse bins within
+//    7.5 sigma of its wavevector transfer, two per instruction.  The banded
+//    spectrum weights give the detector bins.  In MLEM mode the block goes on
+//    to form the ratios y / (Av x + c + 1e-20) of main.m:162 for its detector
+//    bins and folds them back through the same weights, what[pair, e].
 //  * adjoint (k_vox_adj): voxel-major, so that g stays on chip.  A warp owns
-//    32 voxels and loops over a group of pairs; per (pair, voxel) lane =
-//    energy forms what[pair,e] * (the energy's prefactor) and its coarse-bin
-//    window (13.25 sigma), then lane = coarse bin k adds the terms of the
-//    energies whose windows can hold k to the voxel's compensated sum.  The
-//    groups' partial sums (float pairs) are added in FP64 by k_vox_reduce,
-//    which also applies the MLEM update (main.m:163-176).
+//    32 voxels, one per lane, and loops over a group of pairs: geometry once
+//    per pair, then per two energies the lane adds what[pair,e] times their
+//    terms to its own column of sums over the bins within 13.25 sigma, two
+//    bins per instruction; at a pair's end the column goes into the partial
+//    row with a two-sum.  The groups' partial sums
+//    (float pairs) are added in FP64 by k_vox_reduce, which also applies the
+//    MLEM update (main.m:163-176).
+//
+// Both are bound by instruction issue.  The bins of a window come from a table
+// over the wavevector axis (VoxOp::qlut) instead of two square roots and
+// quotients.  Measured on 128x128 voxels, 32 views x 128 px, 40 energies, 32 bins:
+// forward 5.5 ms, 10.1 with lane = energy; 7.9 before the scattering geometry lost
+// its component-wise form (vox_geom) and the coefficients' transposition moved
+// out of the tiles.  Adjoint of 96x78 voxels, 27 views x 110 px, 40 energies, 40
+// bins: 2.2 ms, 8.7 with lane = energy for the terms, scans over the energies for
+// each bin's range and lane = bin for the sums; 3.8 with compensated sums in
+// shared memory, one energy per visit to a bin.
 #include "scatter.cuh"
 
 namespace xrdt {
 
 namespace {
 
-constexpr int kFwdThreads = 256;
-constexpr int kFwdWarps = kFwdThreads / 32;
+constexpr int kFwdWarps = 8;
+constexpr int kFwdThreads = 32 * kFwdWarps;
+constexpr int kMaxSteps = 24;   // 32-voxel steps of a tile
+
+// A voxel's constants against one (source, pixel) pair.
+struct VoxTerm {
+    ff ax, ay;        // sums of both line integrals, unrounded: the rounding would be
+                      // one error in every energy's and bin's term of the pair
+    ff t1, b;         // sigma^2 = t1 + c2(e) b: c1 s^2 and sg / s^2 as pairs
+    float sh, sl;     // sin(theta/2)
+    float wr;         // geom Rayleigh / sqrt(2 pi)
+};
 
 // Per-(voxel, energy) factors shared by the forward and the adjoint: the
 // prefactor pref = Pin Pout geom Rayleigh / (sigma sqrt(2 pi)) without RF,
 // the wavevector transfer as a pair, the Gaussian exponent scale (log2
-// units, as a pair) and the window half-width.
+// units, as a pair) and sigma.
 struct EnergyTerm {
-    float pref, w_hi, w_lo, c_hi, c_lo, half;
+    float pref, w_hi, w_lo, c_hi, c_lo, sigma;
 };
 
-// Per-(pair, voxel) parts of sigma^2 = c1 s^2 + c2(e) sg / s^2 as pairs:
-// c1 s^2 (c1, the energy-bin width term, is the same for every source bin)
-// and sg / s^2.
-struct SigmaGeom {
-    ff t1, sg_s2;
-};
-
-__device__ __forceinline__ SigmaGeom sigma_geom(float sh, float sl, ff sg, ff c1)
+__device__ __forceinline__ EnergyTerm energy_term(const VoxEnergy &q, const VoxTerm &v)
 {
-    SigmaGeom g;
-    const ff s2 = ff_sqr(ff{sh, sl});
-    g.t1 = ff_mul(c1, s2);
-    g.sg_s2 = ff_div(sg, s2);
-    return g;
-}
-
-__device__ __forceinline__ EnergyTerm energy_term(const float *en, int E, int el, float Adx, float Ady, float Asx,
-                                                  float Asy, float sh, float sl, const SigmaGeom &sgm, float Wg,
-                                                  float rsqrt2pi)
-{
-    const float if1 = en[el], if2 = en[E + el];
-    const float Xin = fmaf(Adx, if1, Ady * if2);
-    const float Xout = fmaf(Asx, if1, Asy * if2);
-    const float wh0 = en[2 * E + el], wl0 = en[3 * E + el];
     EnergyTerm t;
-    float w_hi = wh0 * sh;
-    float w_lo = fmaf(wh0, sh, -w_hi) + fmaf(wh0, sl, wl0 * sh);
-    {
-        const float s = w_hi + w_lo;
-        w_lo = w_lo - (s - w_hi);
-        w_hi = s;
-    }
+    // exp(-X) with 1/f1 and 1/f2 as pairs in units of log2
+    const float low = fmaf(v.ax.hi, q.f1l, fmaf(v.ay.hi, q.f2l, fmaf(v.ax.lo, q.f1, v.ay.lo * q.f2)));
+    const float PP = ex2_approx(fmaf(v.ax.hi, q.f1, fmaf(v.ay.hi, q.f2, low)));
+    const float w = __fmul_rn(q.wh, v.sh);
+    const float wr = fmaf(q.wh, v.sh, -w) + fmaf(q.wh, v.sl, q.wl * v.sh);
+    t.w_hi = w + wr;
+    t.w_lo = wr - (t.w_hi - w);
     // sigma^2 as a pair: deep in the Gaussian's tail the exponent amplifies
     // its relative error by (q distance / sigma)^2 / 2
-    const ff sig2 = ff_add(sgm.t1, ff_mul(ff{en[5 * E + el], en[7 * E + el]}, sgm.sg_s2));
+    const float p = __fmul_rn(q.c2, v.b.hi);
+    const float e = fmaf(q.c2, v.b.lo, fmaf(q.c2l, v.b.hi, fmaf(q.c2, v.b.hi, -p)));
+    ff s2 = two_sum(v.t1.hi, p);
+    s2.lo += e + v.t1.lo;
+    s2 = fast_two_sum(s2.hi, s2.lo);
     // 1/sigma to within an ulp: one Newton step on rsqrt, with the low part
-    const float r0 = rsqrtf(sig2.hi);
-    const float h = fmaf(-0.5f * sig2.hi * r0, r0, 0.5f) - 0.5f * sig2.lo * r0 * r0;
+    const float r0 = rsqrt_approx(s2.hi);
+    const float h = fmaf(-0.5f * s2.hi * r0, r0, 0.5f) - 0.5f * s2.lo * r0 * r0;
     const float rs = fmaf(r0, h, r0);
-    const ff c = gauss_scale(sig2);
+    const ff c = gauss_scale(s2, rs * rs);
     t.c_hi = c.hi;
     t.c_lo = c.lo;
-    // exp(-X) as 2^(-X log2 e) with log2 e as a pair
-    const float X = Xin + Xout;
-    const float PP = ex2_approx(-fmaf(X, kLog2e, X * kLog2e_lo));
-    t.pref = PP * Wg * rsqrt2pi * rs;
-    t.half = kSig * sig2.hi * rs;
-    t.w_hi = w_hi;
-    t.w_lo = w_lo;
+    t.pref = PP * v.wr * rs;
+    t.sigma = s2.hi * rs;
     return t;
 }
 
-// Energy rows in shared memory: 1/f1, 1/f2, wfac_hi, wfac_lo, sig_c1,
-// sig_c2, and the low parts of sig_c1, sig_c2.
-constexpr int kEnRows = 8;
-__device__ __forceinline__ void stage_energy_rows(const VoxJob &J, float *en, int tid, int nthreads)
+// The scattering geometry and line integrals of a voxel against a pair.
+__device__ __forceinline__ VoxTerm vox_term(const PairGeom &G, const F32Consts &c, ff c1, int xy, float2 As, float2 Ad)
 {
-    for (int i = tid; i < J.E; i += nthreads) {
-        const EnergyRow r = J.op.energy[J.op.P.e_lo + i];
-        en[i] = r.inv_f1;
-        en[J.E + i] = r.inv_f2;
-        en[2 * J.E + i] = r.wfac_hi;
-        en[3 * J.E + i] = r.wfac_lo;
-        en[4 * J.E + i] = r.sig_c1;
-        en[5 * J.E + i] = r.sig_c2;
-        en[6 * J.E + i] = r.sig_c1_lo;
-        en[7 * J.E + i] = r.sig_c2_lo;
+    const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
+    const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
+    const VoxGeom g = vox_geom<true>(G, vx, vy);
+    VoxTerm v;
+    v.ax = two_sum(Ad.x, As.x);
+    v.ay = two_sum(Ad.y, As.y);
+    v.t1 = ff_mul(c1, g.s2);
+    v.b = ff_mul(g.sg, ffl_rcp(g.s2));
+    v.sh = g.s.hi;
+    v.sl = g.s.lo;
+    v.wr = g.Wg * c.rsqrt2pi;
+    return v;
+}
+
+// The first and last coarse bin that may lie within `half` of w: the table's
+// cells of both ends, entry 0 below the grid and kLutCells + 1 above it.
+__device__ __forceinline__ void bin_window(const unsigned *lut, float scale, float q_lo, float w, float half, int *k0,
+                                           int *k1)
+{
+    // round(x + 1/2) through the float mantissa
+    const float x0 = fmaf((w - half) - q_lo, scale, 0.5f), x1 = fmaf((w + half) - q_lo, scale, 0.5f);
+    const int i0 = __float_as_int(x0 + 12582912.f) - 0x4B400000, i1 = __float_as_int(x1 + 12582912.f) - 0x4B400000;
+    *k0 = (int)(lut[max(0, min(i0, kLutCells + 1))] & 0xffffu);
+    *k1 = (int)lut[max(0, min(i1, kLutCells + 1))] >> 16;
+}
+
+// 2^(c (w - q)^2) at two neighbouring bins, q = (hi, hi, lo, lo): the
+// argument in FP32 but c as a pair -- the scale carries the systematic part of
+// the error (sigma), the difference and its square round independently per
+// term.
+__device__ __forceinline__ float2 gauss2(const EnergyTerm &t, float4 q)
+{
+    const float2 d = __fadd2_rn(__fadd2_rn(make_float2(t.w_hi, t.w_hi), make_float2(-q.x, -q.y)),
+                                __fadd2_rn(make_float2(t.w_lo, t.w_lo), make_float2(-q.z, -q.w)));
+    const float2 d2 = __fmul2_rn(d, d);
+    const float2 x = __ffma2_rn(make_float2(t.c_hi, t.c_hi), d2, __fmul2_rn(make_float2(t.c_lo, t.c_lo), d2));
+    return make_float2(ex2_approx(x.x), ex2_approx(x.y));
+}
+
+__device__ __forceinline__ VoxEnergy load_energy(const VoxEnergy *en, int el)
+{
+    const float4 a = ((const float4 *)en)[2 * el], b = ((const float4 *)en)[2 * el + 1];
+    return VoxEnergy{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+}
+
+// Stages the tables of a job with every thread of the block: energy rows, bin
+// pairs (negative would be the pad of an odd count: far off the grid) and the
+// window table.
+__device__ __forceinline__ void stage_tables(const VoxJob &J, VoxEnergy *en, float4 *cq, unsigned *lut)
+{
+    const int K = J.op.P.nwt;
+    const float4 *src = (const float4 *)(J.op.vox_energy + J.op.P.e_lo);
+    for (int i = threadIdx.x; i < 2 * J.E; i += blockDim.x) ((float4 *)en)[i] = __ldg(src + i);
+    for (int i = threadIdx.x; 2 * i < K; i += blockDim.x) {
+        const float4 a = J.op.coarse_q[2 * i];
+        const float4 b = 2 * i + 1 < K ? J.op.coarse_q[2 * i + 1] : make_float4(1e15f, 0.f, 0.f, 0.f);
+        cq[i] = make_float4(a.x, b.x, a.y, b.y);
     }
+    for (int i = threadIdx.x; i < kLutCells + 2; i += blockDim.x) lut[i] = __ldg(J.op.qlut + i);
 }
 
 // The problem that work item t belongs to: the last p with off[p] <= t.
@@ -149,147 +191,131 @@ __device__ __forceinline__ void load_job(const VoxJob *__restrict__ jobs, int p,
 }
 
 struct FwdLayout {
-    size_t tn, tns, en, rf, winlo, wn, cq, ratio, total;
+    size_t rec, xs, en, cq, lut, tns, tn, ratio, total;
+    int xstride;   // floats of a row of two bins
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-__host__ __device__ inline FwdLayout vox_fwd_layout(const DevProblem &P, int E)
+__host__ __device__ inline FwdLayout vox_fwd_layout(const DevProblem &P, int E, int steps, int runs)
 {
-    const int W = 2 * P.dnrg + 1;
     FwdLayout L;
+    L.xstride = 64 * steps;   // two bins of every voxel of the tile side by side
     size_t o = 0;
+    L.rec = o; o = al16(o + sizeof(float4) * 3 * 32 * (size_t)steps);
+    L.xs = o; o = al16(o + sizeof(float) * (size_t)((P.nwt + 1) / 2) * L.xstride);
+    L.en = o; o = al16(o + sizeof(VoxEnergy) * E);
+    L.cq = o; o = al16(o + sizeof(float4) * ((P.nwt + 1) / 2));
+    L.lut = o; o = al16(o + sizeof(unsigned) * (kLutCells + 2));
+    L.tns = o; o = al16(o + sizeof(float2) * (size_t)E * runs);
     L.tn = o; o = al16(o + sizeof(double) * E);
-    L.tns = o; o = al16(o + sizeof(float2) * kFwdWarps * E);
-    L.en = o; o = al16(o + sizeof(float) * kEnRows * E);
-    L.rf = o; o = al16(o + sizeof(float) * P.nrg_det * W);
-    L.winlo = o; o = al16(o + sizeof(int) * P.nrg_det);
-    L.wn = o; o = al16(o + sizeof(int) * 2 * E);
-    L.cq = o; o = al16(o + sizeof(float4) * P.nwt);
     L.ratio = o; o = al16(o + sizeof(double) * P.nrg_det);
     L.total = o;
     return L;
 }
 
-// One (source, pixel) pair of job J, by the whole block.
+// One (source, pixel) pair of job J, by the whole block; the job's tables are
+// staged.
 template <bool MLEM>
-__device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsigned char *sm, PairRec &pair)
+__device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsigned char *sm, PairRec &pair,
+                                             int &next_run)
 {
     const DevProblem &P = J.op.P;
     const F32Consts &c = J.c;
-    const int E = J.E, K = P.nwt, W = 2 * P.dnrg + 1;
-    const FwdLayout L = vox_fwd_layout(P, E);
+    const int E = J.E, K = P.nwt, W = 2 * P.dnrg + 1, nv = J.op.nv;
+    const int nst = J.steps, H = J.runs, run_len = (nst + H - 1) / H;
+    const FwdLayout L = vox_fwd_layout(P, E, nst, H);
+    float4 *rec = (float4 *)(sm + L.rec);          // [3][32 nst]
+    float *xs = (float *)(sm + L.xs);              // [(K + 1)/2][32 nst] x dq of bins 2i, 2i + 1
+    const VoxEnergy *en = (const VoxEnergy *)(sm + L.en);
+    const float4 *cq = (const float4 *)(sm + L.cq);
+    const unsigned *lut = (const unsigned *)(sm + L.lut);
+    float2 *TNs = (float2 *)(sm + L.tns);          // [E][runs] compensated sums
     double *TN = (double *)(sm + L.tn);
-    float2 *TNs = (float2 *)(sm + L.tns);
-    float *en = (float *)(sm + L.en);
-    float *rf = (float *)(sm + L.rf);
-    int *winlo = (int *)(sm + L.winlo);
-    int *wn = (int *)(sm + L.wn);
-    float4 *cq = (float4 *)(sm + L.cq);
-    double *ratio = (double *)(sm + L.ratio);   // kept in FP64: see the weights below
-
+    double *ratio = (double *)(sm + L.ratio);      // kept in FP64: see the weights below
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
-    const int src = (int)(pidx % P.n_src);
 
-    stage_energy_rows(J, en, tid, kFwdThreads);
-    for (int i = tid; i < kFwdWarps * E; i += kFwdThreads) TNs[i] = make_float2(0.f, 0.f);
-    for (int i = tid; i < 2 * E; i += kFwdThreads) wn[i] = J.op.win_n[2 * P.e_lo + i];
-    for (int i = tid; i < P.nrg_det * W; i += kFwdThreads) rf[i] = J.op.rf_win[i];
-    for (int i = tid; i < P.nrg_det; i += kFwdThreads) winlo[i] = J.op.win_lo[i];
-    for (int i = tid; i < K; i += kFwdThreads) cq[i] = J.op.coarse_q[i];
-    static_assert(sizeof(PairRec) / 4 <= kFwdThreads, "one word per thread");
-    if (tid < (int)(sizeof(PairRec) / 4))
-        reinterpret_cast<int *>(&pair)[tid] = reinterpret_cast<const int *>(J.op.pairs + pidx)[tid];
-    const float rsqrt2pi = c.rsqrt2pi;
-    const float qlo_f = c.q_lo;
-    const float *__restrict__ xd = J.xd;
-    __syncthreads();
+    for (int i = tid; i < (int)(sizeof(PairRec) / 4); i += kFwdThreads)
+        reinterpret_cast<int *>(&pair)[i] = reinterpret_cast<const int *>(J.op.pairs + pidx)[i];
+    for (int i = tid; i < E * H; i += kFwdThreads) TNs[i] = make_float2(0.f, 0.f);
+    const ff c1 = {J.op.c1, J.op.c1l};
+    const float scale = J.op.lut_scale, q_lo = J.c.q_lo;
+    const int x_row = L.xstride;
 
-    float2 *TNw = TNs + wid * E;
-    const int nv = J.op.nv;
-    const int nchunks = (nv + 31) >> 5;
-    for (int chunk = wid; chunk < nchunks; chunk += kFwdWarps) {
-        const int v = min(chunk * 32 + lane, nv - 1);
-        const int xy = J.op.vox_xy[v];
-        const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
-        const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
-        const VoxGeom vg = vox_geom<true>(pair.G, vx, vy);
-        const float2 Asv = J.op.atten_src[(int64_t)src * nv + v];
-        // the detector-side integral feeds Pin (integrate_diffraction.cu:259-260),
-        // read from the table of this job's pairs (kept, or walked for the tile)
-        const float2 Adv = J.op.walk[(pidx - J.pair0) * nv + v];
-
-        const int nin = min(32, nv - chunk * 32);
-        // the (voxel, energy) term: lane's energy el for voxel i of the chunk
-        auto term = [&](int i, int el, float2 Ad, float sh, float sl, float Wg, float Asx, float Asy,
-                        const SigmaGeom &sgm) {
-            const float *xrow = xd + (int64_t)(chunk * 32 + i) * K;
-            const EnergyTerm t = energy_term(en, E, el, Ad.x, Ad.y, Asx, Asy, sh, sl, sgm, Wg, rsqrt2pi);
-            if (t.pref == 0.f) return;   // attenuation underflow: no contribution
-            int klo, khi;
-            coarse_window(t.w_hi, t.half, qlo_f, c.qpar_a, c.qpar_b, K, &klo, &khi);
-            float acc = 0.f;
-            for (int k = klo; k <= khi; k++) {
-                const float4 q = cq[k];
-                acc = fmaf(gauss_f32(t.w_hi, t.w_lo, q.x, q.y, t.c_hi, t.c_lo), __ldg(xrow + k), acc);
-            }
-            float2 s = TNw[el];
-            kahan_add(s.x, s.y, t.pref * acc);
-            TNw[el] = s;
-        };
-        if (E > 32 && (E & 31)) {
-            // E not a multiple of 32 (40 on the 128x128 workload): the chunk's
-            // (voxel, energy) items nin*E, 32 consecutive ones per step, so
-            // that no step runs with a few lanes.  Consecutive items of a step
-            // have distinct energies (32 < E), hence distinct sums TNw[el].
-            // Each lane's voxel constants come from the lane that holds them.
-            const SigmaGeom sgv = sigma_geom(vg.s.hi, vg.s.lo, vg.sg, ff{en[4 * E], en[6 * E]});
-            int i = 0, el = lane;
-            for (int t0 = 0; t0 < nin * E; t0 += 32) {
-                const bool act = i < nin;
-                const float2 Ad = make_float2(__shfl_sync(0xffffffffu, Adv.x, i), __shfl_sync(0xffffffffu, Adv.y, i));
-                const float sh = __shfl_sync(0xffffffffu, vg.s.hi, i);
-                const float sl = __shfl_sync(0xffffffffu, vg.s.lo, i);
-                const float Wg = __shfl_sync(0xffffffffu, vg.Wg, i);
-                const float Asx = __shfl_sync(0xffffffffu, Asv.x, i);
-                const float Asy = __shfl_sync(0xffffffffu, Asv.y, i);
-                SigmaGeom sgm;
-                sgm.t1 = ff{__shfl_sync(0xffffffffu, sgv.t1.hi, i), __shfl_sync(0xffffffffu, sgv.t1.lo, i)};
-                sgm.sg_s2 = ff{__shfl_sync(0xffffffffu, sgv.sg_s2.hi, i), __shfl_sync(0xffffffffu, sgv.sg_s2.lo, i)};
-                if (act) term(i, el, Ad, sh, sl, Wg, Asx, Asy, sgm);
-                el += 32;
-                if (el >= E) {
-                    el -= E;
-                    i++;
+    for (int tile = 0; tile < J.tiles; tile++) {
+        const int t0 = 32 * nst * tile;
+        __syncthreads();   // the tables and the pair are staged; the last tile is no longer read
+        if (tid == 0) next_run = 0;
+        // the tile's coefficients (rows of two bins of the tile's voxels),
+        // copied while the geometry is formed
+        const int steps = min(nst, (nv - t0 + 31) >> 5);
+        for (int k = wid; k < (K + 1) >> 1; k += kFwdWarps) {
+            const float *src = J.xd + 2 * ((int64_t)k * J.xd_stride + t0) + 4 * lane;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs + k * x_row + 4 * lane);
+            for (int i = 0; i < 16 * steps; i += 32)
+                if (i + lane < 16 * steps)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(src + 4 * i)
+                                 : "memory");
+        }
+        for (int i = tid; i < 32 * nst && t0 + (i & ~31) < nv; i += kFwdThreads) {
+            const int v = min(t0 + i, nv - 1);
+            const VoxTerm t = vox_term(pair.G, c, c1, J.op.vox_xy[v], J.op.atten_src[(int64_t)pair.src * nv + v],
+                                       J.op.walk[(pidx - J.pair0) * nv + v]);
+            rec[i] = make_float4(t.ax.hi, t.ay.hi, t.t1.hi, t.t1.lo);
+            rec[32 * nst + i] = make_float4(t.sh, t.sl, t.b.hi, t.b.lo);
+            // a lane past the last voxel repeats it with a weight of zero
+            rec[64 * nst + i] = make_float4(t0 + i < nv ? t.wr : 0.f, t.ax.lo, t.ay.lo, 0.f);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        // ---- lane = voxel: runs of 32-voxel steps of one energy, the widest windows first ----
+        for (;;) {
+            int item = 0;
+            if (lane == 0) item = atomicAdd(&next_run, 1);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            if (item >= E * H) break;
+            const int el = E - 1 - item / H, row = el * H + item % H;
+            const int s0 = item % H * run_len, s1 = min(s0 + run_len, steps);
+            const VoxEnergy q = load_energy(en, el);
+            float sum = 0.f;
+            for (int st = s0; st < s1; st++) {
+                const int i = 32 * st + lane;
+                const float4 r0 = rec[i], r1 = rec[32 * nst + i], r2 = rec[64 * nst + i];
+                const VoxTerm v = {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
+                const EnergyTerm t = energy_term(q, v);
+                int k0, k1;
+                bin_window(lut, scale, q_lo, t.w_hi, kSig * t.sigma, &k0, &k1);
+                if (k0 <= k1 && t.pref != 0.f) {   // pref 0: attenuation underflow, no contribution
+                    float2 acc = make_float2(0.f, 0.f);
+                    const float2 *x2 = (const float2 *)xs + i;
+                    for (int k = k0 >> 1; k <= k1 >> 1; k++)
+                        acc = __ffma2_rn(gauss2(t, cq[k]), x2[k * (x_row >> 1)], acc);
+                    sum = fmaf(t.pref, acc.x + acc.y, sum);
                 }
             }
-        } else {
-            for (int i = 0; i < nin; i++) {
-                const float2 Ad = make_float2(__shfl_sync(0xffffffffu, Adv.x, i), __shfl_sync(0xffffffffu, Adv.y, i));
-                const float sh = __shfl_sync(0xffffffffu, vg.s.hi, i);
-                const float sl = __shfl_sync(0xffffffffu, vg.s.lo, i);
-                const ff sg = {__shfl_sync(0xffffffffu, vg.sg.hi, i), __shfl_sync(0xffffffffu, vg.sg.lo, i)};
-                const float Wg = __shfl_sync(0xffffffffu, vg.Wg, i);
-                const float Asx = __shfl_sync(0xffffffffu, Asv.x, i);
-                const float Asy = __shfl_sync(0xffffffffu, Asv.y, i);
-                const SigmaGeom sgm = sigma_geom(sh, sl, sg, ff{en[4 * E], en[6 * E]});
-#pragma unroll 1
-                for (int el = lane; el < E; el += 32) term(i, el, Ad, sh, sl, Wg, Asx, Asy, sgm);
+            sum = warp_sum(sum);
+            if (lane == 0) {
+                float2 k = TNs[row];
+                kahan_add(k.x, k.y, sum);
+                TNs[row] = k;
             }
         }
     }
     __syncthreads();
     for (int el = tid; el < E; el += kFwdThreads) {
         double s = 0.0;
-        for (int w = 0; w < kFwdWarps; w++) s += (double)TNs[w * E + el].x - (double)TNs[w * E + el].y;
+        for (int h = 0; h < H; h++) s += (double)TNs[el * H + h].x - (double)TNs[el * H + h].y;
         TN[el] = s;
     }
     __syncthreads();
     const int lo_e = P.e_lo;
+    const float *rf = J.op.rf_win;
+    const int *winlo = J.op.win_lo, *wn = J.op.win_n;
     for (int n = tid; n < P.nrg_det; n += kFwdThreads) {
         double acc = 0.0;
-        for (int j = 0; j < W; j++) acc += (double)rf[n * W + j] * TN[winlo[n] + j - lo_e];
+        const int w0 = __ldg(winlo + n) - lo_e;
+        for (int j = 0; j < W; j++) acc += (double)__ldg(rf + n * W + j) * TN[w0 + j];
         const int64_t ray = pidx + (int64_t)n * npairs;
         if (MLEM) ratio[n] = (double)J.ymeas[ray] / (acc + (double)J.cbg[ray] + 1e-20);   // main.m:162
         else J.y[ray] = (float)acc;
@@ -300,9 +326,10 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
         for (int el = tid; el < E; el += kFwdThreads) {
             const int e = lo_e + el;
             double s = 0.0;
-            for (int n = wn[2 * el]; n <= wn[2 * el + 1]; n++) {
-                const int j = e - winlo[n];
-                if (j >= 0 && j < W) s += (double)rf[n * W + j] * ratio[n];
+            const int n1 = __ldg(wn + 2 * e + 1);
+            for (int n = __ldg(wn + 2 * e); n <= n1; n++) {
+                const int j = e - __ldg(winlo + n);
+                if (j >= 0 && j < W) s += (double)__ldg(rf + n * W + j) * ratio[n];
             }
             J.what[pidx * E + el] = (float)s;
         }
@@ -318,6 +345,7 @@ k_vox_fwd(const VoxBatch B)
     __shared__ PairRec pair;
     __shared__ VoxJob job;
     __shared__ long long item_s;
+    __shared__ int next_run;
     const int64_t *off = B.off + 0 * (B.n + 1);
     const int64_t total = off[B.n];
     int cur = -1;
@@ -332,16 +360,46 @@ k_vox_fwd(const VoxBatch B)
             load_job(B.jobs, p, &job);
             cur = p;
             __syncthreads();
+            const FwdLayout L = vox_fwd_layout(job.op.P, job.E, job.steps, job.runs);
+            stage_tables(job, (VoxEnergy *)(sm + L.en), (float4 *)(sm + L.cq), (unsigned *)(sm + L.lut));
         }
-        vox_fwd_pair<MLEM>(job, job.pair0 + (item - off[p]), sm, pair);
+        vox_fwd_pair<MLEM>(job, job.pair0 + (item - off[p]), sm, pair, next_run);
     }
 }
 
-// Adjoint tile (voxel-chunk block bx, pair group by) of job J.  Shared
-// memory: energy rows and coarse bins, then per warp E rows of (coefficient,
-// wvt pair, exponent scale), 32 x K compensated sums and the current pair's
-// record.
-__global__ void __launch_bounds__(128)
+// Shared memory of the adjoint: the job's tables, then per warp the current
+// pair's record and weights and its sums, [(K + 1)/2][32] of two bins side by
+// side.
+struct AdjLayout {
+    size_t en, cq, lut, warp0, per_warp, sums, weights, total;
+};
+
+__host__ __device__ inline AdjLayout vox_adj_layout(const DevProblem &P, int E, int warps)
+{
+    AdjLayout L;
+    size_t o = 0;
+    L.en = o; o = al16(o + sizeof(VoxEnergy) * E);
+    L.cq = o; o = al16(o + sizeof(float4) * ((P.nwt + 1) / 2));
+    L.lut = o; o = al16(o + sizeof(unsigned) * (kLutCells + 2));
+    L.warp0 = o;
+    size_t w = al16(sizeof(PairRec));
+    L.weights = w; w = al16(w + sizeof(float) * E);
+    L.sums = w; w = al16(w + sizeof(float2) * 32 * (size_t)((P.nwt + 1) / 2));
+    L.per_warp = w;
+    L.total = L.warp0 + w * warps;
+    return L;
+}
+
+// Adjoint tile (voxel-chunk block bx, pair group by) of job J.  A pair's sums
+// over the energies are plain FP32 sums in shared memory, two energies per
+// visit to a bin (the visits' loads and stores would bind before the FMA
+// pipe); at the pair's end they go into the tile's partial rows in global
+// memory with a two-sum, whose low parts are kept: rounded to one float, each
+// row would carry the same relative error into every MLEM iteration, where
+// the update multiplies it in again and again.  The rows of the tiles in
+// flight stay in L2, and shared memory holds twice the warps that it would
+// with compensated sums beside the plain ones.
+__global__ void __launch_bounds__(128, 6)
 k_vox_adj(const VoxBatch B)
 {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -363,168 +421,82 @@ k_vox_adj(const VoxBatch B)
             load_job(B.jobs, p, &J);
             cur = p;
             __syncthreads();
+            const AdjLayout L = vox_adj_layout(J.op.P, J.E, nwarps);
+            stage_tables(J, (VoxEnergy *)(sm + L.en), (float4 *)(sm + L.cq), (unsigned *)(sm + L.lut));
+            __syncthreads();
         }
         const DevProblem &P = J.op.P;
-        const F32Consts &c = J.c;
-        const int E = J.E, K = P.nwt;
-        float *en = (float *)sm;                                            // [6][E]
-        float4 *cq = (float4 *)(sm + al16(sizeof(float) * kEnRows * E));    // [K]
-        float4 *rows = cq + K;                                              // [warps][E]
-        float2 *gacc = (float2 *)(rows + (size_t)nwarps * E);               // [warps][32][K]
-        PairRec *prs = (PairRec *)(gacc + (size_t)nwarps * 32 * K);         // [warps]
-        float *rows_lo = (float *)(prs + nwarps);                           // [warps][E]
-        int2 *wins = (int2 *)(sm + al16((size_t)((unsigned char *)(rows_lo + (size_t)nwarps * E) - sm)));
-                                                                            // [warps][E]
-        unsigned char *eranges = (unsigned char *)(wins + (size_t)nwarps * E);   // [warps][2][K]
-        float4 *rw = rows + (size_t)wid * E;
-        float *rwl = rows_lo + (size_t)wid * E;
-        int2 *ww = wins + (size_t)wid * E;
-        unsigned char *e_first = eranges + (size_t)wid * 2 * K, *e_end = e_first + K;
-        float2 *gw = gacc + (size_t)wid * 32 * K;
-        PairRec &pr = prs[wid];
-        stage_energy_rows(J, en, tid, blockDim.x);
-        for (int i = tid; i < K; i += blockDim.x) cq[i] = J.op.coarse_q[i];
-        for (int i = lane; i < 32 * K; i += 32) gw[i] = make_float2(0.f, 0.f);
-        __syncthreads();
+        const int E = J.E, K2 = (P.nwt + 1) >> 1;
+        const AdjLayout L = vox_adj_layout(P, E, nwarps);
+        const VoxEnergy *en = (const VoxEnergy *)(sm + L.en);
+        const float4 *cq = (const float4 *)(sm + L.cq);
+        const unsigned *lut = (const unsigned *)(sm + L.lut);
+        unsigned char *mine = sm + L.warp0 + L.per_warp * wid;
+        PairRec &pr = *(PairRec *)mine;
+        float *ws = (float *)(mine + L.weights);
+        float2 *sums = (float2 *)(mine + L.sums) + lane;   // this lane's column
 
         const int64_t r = item - off[p];
         const int bx = (int)(r % J.chunk_blocks), by = (int)(r / J.chunk_blocks);
-        const int nv = J.op.nv;
+        const int nv = J.op.nv, chunks = (nv + 31) >> 5;
         const int chunk = bx * nwarps + wid;
-        if (chunk * 32 >= nv) continue;   // an idle warp; the next item starts with a barrier
+        if (chunk >= chunks) continue;   // an idle warp; the next item starts with a barrier
         const int64_t p0 = J.pair0 + (int64_t)by * J.ppg;
         const int64_t p1 = min(J.pair1, p0 + J.ppg);
-        const float rsqrt2pi = c.rsqrt2pi;
-        const float q_lo = c.q_lo, q_hi = c.q_hi;
-        const int nin = min(32, nv - chunk * 32);
-        const int v = chunk * 32 + min(lane, nin - 1);
+        const int v = min(chunk * 32 + lane, nv - 1);   // a lane past the last voxel repeats it
         const int xy = J.op.vox_xy[v];
-        const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
-        const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
+        const ff c1 = {J.op.c1, J.op.c1l};
+        const float scale = J.op.lut_scale, q_lo = J.c.q_lo;
+        // this lane's column of the partial row: sums of two bins and their low parts
+        float4 *row = J.part + ((int64_t)by * chunks + chunk) * K2 * 32 + lane;
+        for (int k = 0; k < K2; k++) sums[32 * k] = make_float2(0.f, 0.f);
+        // a job that is one tile of a problem adds to what the earlier tiles left
+        // (tiles run in a fixed order on one stream)
+        if (!J.accumulate)
+            for (int k = 0; k < K2; k++) row[32 * k] = make_float4(0.f, 0.f, 0.f, 0.f);
 
         for (int64_t pp = p0; pp < p1; pp++) {
             __syncwarp();   // the previous pair's constants are no longer read
             for (int i = lane; i < (int)(sizeof(PairRec) / 4); i += 32)
                 reinterpret_cast<int *>(&pr)[i] = reinterpret_cast<const int *>(J.op.pairs + pp)[i];
+            for (int i = lane; i < E; i += 32) ws[i] = __ldg(J.what + pp * E + i);
             __syncwarp();
-            const int src = (int)(pp % P.n_src);
-            const VoxGeom vg = vox_geom<true>(pr.G, vx, vy);
-            const float2 Asv = J.op.atten_src[(int64_t)src * nv + v];
-            const float2 Adv = J.op.walk[(pp - J.pair0) * nv + v];
-            const float *wp = J.what + pp * E;
-            for (int i = 0; i < nin; i++) {
-                const float2 Ad = make_float2(__shfl_sync(0xffffffffu, Adv.x, i), __shfl_sync(0xffffffffu, Adv.y, i));
-                const float sh = __shfl_sync(0xffffffffu, vg.s.hi, i);
-                const float sl = __shfl_sync(0xffffffffu, vg.s.lo, i);
-                const ff sg = {__shfl_sync(0xffffffffu, vg.sg.hi, i), __shfl_sync(0xffffffffu, vg.sg.lo, i)};
-                const float Wg = __shfl_sync(0xffffffffu, vg.Wg, i);
-                const float Asx = __shfl_sync(0xffffffffu, Asv.x, i);
-                const float Asy = __shfl_sync(0xffffffffu, Asv.y, i);
-                const SigmaGeom sgm = sigma_geom(sh, sl, sg, ff{en[4 * E], en[6 * E]});
-                // lane = energy: the energy's factors and its coarse-bin
-                // window (the bins within 13.25 sigma: every term FP32 can
-                // represent), with the running maximum of the windows' upper
-                // ends in ww[e].x
-                int run_max = -1;
-                for (int eb = 0; eb < E; eb += 32) {
-                    const int el = eb + lane;
-                    int klo = K, khi = -1;
-                    if (el < E) {
-                        const EnergyTerm t =
-                            energy_term(en, E, el, Ad.x, Ad.y, Asx, Asy, sh, sl, sgm, Wg, rsqrt2pi);
-                        const float cf = __ldg(wp + el) * t.pref;
-                        const float half = t.half * (kSigAdj / kSig);
-                        // a window entirely outside the coarse grid contributes nothing
-                        if (cf != 0.f && !(t.w_hi + half < q_lo || t.w_hi - half > q_hi))
-                            coarse_window(t.w_hi, half, q_lo, c.qpar_a, c.qpar_b, K, &klo, &khi);
-                        rw[el] = make_float4(cf, t.w_hi, t.w_lo, t.c_hi);
-                        rwl[el] = t.c_lo;
-                        ww[el].y = klo;
-                    }
-                    int m = khi;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int n = __shfl_up_sync(0xffffffffu, m, o);
-                        if (lane >= o) m = max(m, n);
-                    }
-                    m = max(m, run_max);
-                    if (el < E) ww[el].x = m;
-                    run_max = __shfl_sync(0xffffffffu, m, 31);
-                }
-                __syncwarp();
-                // running minimum of the windows' lower ends from the top
-                // energy down, in ww[e].y
-                int run_min = K;
-                for (int eb = ((E - 1) >> 5) << 5; eb >= 0; eb -= 32) {
-                    const int el = eb + lane;
-                    int m = el < E ? ww[el].y : K;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int n = __shfl_down_sync(0xffffffffu, m, o);
-                        if (lane + o < 32) m = min(m, n);
-                    }
-                    m = min(m, run_min);
-                    if (el < E) ww[el].y = m;
-                    run_min = __shfl_sync(0xffffffffu, m, 0);
-                }
-                __syncwarp();
-                // The energies whose window holds bin k lie in [e0(k), e1(k)):
-                // below e0 every window ends before k (the running maximum of
-                // the upper ends is below k), from e1 on every window starts
-                // after it (the running minimum of the lower ends is above
-                // k).  Both bounds are monotone in k, so energy e is e0 for the
-                // bins (M[e-1], M[e]] and e1 for [m[e-1], m[e]); lane = energy
-                // writes those entries for the bins in [kmin, kmax].
-                const int kmin = run_min, kmax = run_max;
-                for (int eb = 0; eb < E && kmin <= kmax; eb += 32) {
-                    const int el = eb + lane;
-                    if (el < E) {
-                        const int2 cur = ww[el];
-                        const int2 prv = el > 0 ? ww[el - 1] : make_int2(-1, kmin);
-                        for (int k = max(prv.x + 1, kmin); k <= min(cur.x, kmax); k++) e_first[k] = (unsigned char)el;
-                        if (el > 0)
-                            for (int k = max(prv.y, kmin); k <= min(cur.y - 1, kmax); k++) e_end[k] = (unsigned char)el;
-                        if (el == E - 1)
-                            for (int k = max(cur.y, kmin); k <= kmax; k++) e_end[k] = (unsigned char)E;
-                    }
-                }
-                __syncwarp();
-                // lane = coarse bin k over the bins some window reaches
-                float2 *gi = gw + i * K;
-                for (int kb = kmin; kb <= kmax; kb += 32) {
-                    const int k = kb + lane;
-                    if (k > kmax) break;
-                    const int e0 = e_first[k], e1 = e_end[k];
+            const VoxTerm vt = vox_term(pr.G, J.c, c1, xy, J.op.atten_src[(int64_t)pr.src * nv + v],
+                                        J.op.walk[(pp - J.pair0) * nv + v]);
+            int kmin = K2, kmax = -1;   // the pairs of bins this lane adds to
+            for (int el = 0; el < E; el += 2) {
+                const EnergyTerm t = energy_term(load_energy(en, el), vt);
+                const int e1 = min(el + 1, E - 1);
+                const EnergyTerm u = energy_term(load_energy(en, e1), vt);
+                const float ct = ws[el] * t.pref, cu = el + 1 < E ? ws[e1] * u.pref : 0.f;
+                // the bins within 13.25 sigma: every term FP32 can represent
+                int k0, k1, l0, l1;
+                bin_window(lut, scale, q_lo, t.w_hi, kSigAdj * t.sigma, &k0, &k1);
+                bin_window(lut, scale, q_lo, u.w_hi, kSigAdj * u.sigma, &l0, &l1);
+                if (ct == 0.f || k0 > k1) k0 = 0xffff, k1 = -1;
+                if (cu == 0.f || l0 > l1) l0 = 0xffff, l1 = -1;
+                k0 = min(k0, l0) >> 1;
+                k1 = max(k1, l1) >> 1;
+                if (k0 > k1) continue;
+                kmin = min(kmin, k0);
+                kmax = max(kmax, k1);
+                for (int k = k0; k <= k1; k++) {
                     const float4 q = cq[k];
-                    float acc = 0.f;
-                    for (int e = e0; e < e1; e++) {
-                        const float4 rr = rw[e];
-                        acc = fmaf(rr.x, gauss_f32(rr.y, rr.z, q.x, q.y, rr.w, rwl[e]), acc);
-                    }
-                    float2 sacc = gi[k];
-                    kahan_add(sacc.x, sacc.y, acc * q.z);
-                    gi[k] = sacc;
+                    const float2 g = gauss2(t, q), h = gauss2(u, q);
+                    sums[32 * k] = __ffma2_rn(make_float2(cu, cu), h, __ffma2_rn(make_float2(ct, ct), g, sums[32 * k]));
                 }
-                __syncwarp();
+            }
+            kmin = __reduce_min_sync(0xffffffffu, kmin);
+            kmax = __reduce_max_sync(0xffffffffu, kmax);
+            for (int k = kmin; k <= kmax; k++) {
+                const float4 o = row[32 * k];
+                const float2 b = sums[32 * k];
+                sums[32 * k] = make_float2(0.f, 0.f);
+                const ff x = two_sum(o.x, b.x), y = two_sum(o.y, b.y);
+                row[32 * k] = make_float4(x.hi, y.hi, o.z + x.lo, o.w + y.lo);
             }
         }
-        // The partial rows keep the compensated sums as pairs (sum, minus
-        // the compensation): rounded to one float, each row would carry the
-        // same relative error into every MLEM iteration, where the update
-        // multiplies it in again and again.  A job that is one tile of a
-        // problem adds to the rows the earlier tiles left (tiles run in a
-        // fixed order on one stream), with a two-sum.
-        float2 *out = J.part + ((int64_t)by * nv + (int64_t)chunk * 32) * K;
-        if (J.accumulate)
-            for (int i = lane; i < nin * K; i += 32) {
-                const float2 o = out[i];
-                const float s = o.x + gw[i].x;
-                const float bb = s - o.x;
-                const float err = (o.x - (s - bb)) + (gw[i].x - bb);
-                out[i] = make_float2(s, o.y + (err - gw[i].y));
-            }
-        else
-            for (int i = lane; i < nin * K; i += 32) out[i] = make_float2(gw[i].x, -gw[i].y);
+        __syncwarp();
     }
 }
 
@@ -560,46 +532,81 @@ __global__ void k_vox_wtab(const VoxBatch B, int mode)
     }
 }
 
-// Sum of the adjoint's partial rows in FP64 and what follows from it:
+// Where x dq of (voxel, bin) lies: rows of two bins, [(K + 1)/2][xd_stride][2],
+// as the forward's tiles copy them.
+__device__ __forceinline__ int64_t xd_index(const VoxJob &J, int64_t v, int k)
+{
+    return 2 * ((int64_t)(k >> 1) * J.xd_stride + v) + (k & 1);
+}
+
+// Sum of the adjoint's partial rows in FP64, times the bins' widths, and what
+// follows from it:
 //   mode 0: sens = sum (the sensitivity, Av^T 1)
 //   mode 4: sens += sum (its second part, k_vox_wtab)
 //   mode 1: the MLEM update x <- x * sum / (sens + 1e-7), non-finite -> 0,
 //           negative -> 0 (main.m:162-176), and xd = x dq
 //   mode 2: g[voxel] = sum in the full-grid layout (nx + ny*NX)*nwt + k
 //   mode 3: g = sum in the compact voxel order [nv][nwt]
-__global__ void k_vox_reduce(const VoxBatch B, int mode)
+// A block takes 32 voxels and two bins, 512 bytes of every partial row.  Its
+// warps split the rows and add theirs with two-sums (whose low parts FP32
+// holds as well as it held the rows'), then the warps' sums are added in FP64:
+// in FP64 throughout and by one thread per entry, 200 rows of 2224 voxels x 40
+// bins took 250 us against 65, on a pipe of 1/64 of the FP32 rate.
+constexpr int kReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kReduceWarps)
+k_vox_reduce(const VoxBatch B, int mode)
 {
-    const int64_t *off = B.off + 2 * (B.n + 1);
-    const int64_t total = off[B.n];
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int pj = find_job(off, B.n, t);
+    __shared__ double part_s[kReduceWarps][2][32];
+    const int64_t *off = B.off + 5 * (B.n + 1);
+    const int64_t total = off[B.n] >> 5;   // (chunk, pair of bins) of every job
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+        const int pj = find_job(off, B.n, 32 * t);
         const VoxJob &J = B.jobs[pj];
-        const int K = J.op.P.nwt;
-        const int64_t loc = t - off[pj];
-        const int64_t n = (int64_t)J.op.nv * K;
-        double s = 0.0;
-        for (int gi = 0; gi < J.groups; gi++) {
-            const float2 pv = J.part[(int64_t)gi * n + loc];
-            s += (double)pv.x + (double)pv.y;
+        const int K = J.op.P.nwt, K2 = (K + 1) >> 1, nv = J.op.nv;
+        const int64_t loc = t - (off[pj] >> 5);
+        const int64_t chunk = loc / K2;
+        const int k2 = (int)(loc - chunk * K2);
+        const int64_t n = off[pj + 1] - off[pj];
+        const float4 *part = J.part + 32 * loc + lane;
+        ff a = {0.f, 0.f}, b = {0.f, 0.f};
+#pragma unroll 4
+        for (int gi = wid; gi < J.groups; gi += kReduceWarps) {
+            const float4 pv = part[(int64_t)gi * n];
+            const ff x = two_sum(a.hi, pv.x), y = two_sum(b.hi, pv.y);
+            a = ff{x.hi, a.lo + (x.lo + pv.z)};
+            b = ff{y.hi, b.lo + (y.lo + pv.w)};
         }
-        if (mode == 0) {
-            J.sens[loc] = s;
-        } else if (mode == 4) {
-            J.sens[loc] += s;
-        } else if (mode == 1) {
-            float v = (float)((double)J.xc[loc] * s / (J.sens[loc] + 1e-7));
-            if (!isfinite(v)) v = 0.f;
-            if (v < 0.f) v = 0.f;
-            J.xc[loc] = v;
-            J.xd[loc] = v * J.op.coarse_q[loc % K].z;
-        } else if (mode == 2) {
-            const int64_t vi = loc / K;
-            const int xy = J.op.vox_xy[vi];
-            J.g[((int64_t)(xy & 0xffff) + (int64_t)(xy >> 16) * J.op.P.nx) * K + (loc - vi * K)] = (float)s;
-        } else {
-            J.g[loc] = (float)s;   // compact voxel order [nv][NWT]
+        part_s[wid][0][lane] = (double)a.hi + (double)a.lo;
+        part_s[wid][1][lane] = (double)b.hi + (double)b.lo;
+        __syncthreads();
+        const int64_t vi = 32 * chunk + lane;
+        const int k = 2 * k2 + wid;
+        if (wid < 2 && vi < nv && k < K) {
+            double sum = 0.0;
+#pragma unroll
+            for (int w = 0; w < kReduceWarps; w++) sum += part_s[w][wid][lane];
+            const float dq = J.op.coarse_q[k].z;
+            const double s = sum * (double)dq;
+            const int64_t i = vi * K + k;
+            if (mode == 0) {
+                J.sens[i] = s;
+            } else if (mode == 4) {
+                J.sens[i] += s;
+            } else if (mode == 1) {
+                float v = (float)((double)J.xc[i] * s / (J.sens[i] + 1e-7));
+                if (!isfinite(v)) v = 0.f;
+                if (v < 0.f) v = 0.f;
+                J.xc[i] = v;
+                J.xd[xd_index(J, vi, k)] = v * dq;
+            } else if (mode == 2) {
+                const int xy = J.op.vox_xy[vi];
+                J.g[((int64_t)(xy & 0xffff) + (int64_t)(xy >> 16) * J.op.P.nx) * K + k] = (float)s;
+            } else {
+                J.g[i] = (float)s;
+            }
         }
+        __syncthreads();
     }
 }
 
@@ -619,7 +626,17 @@ __global__ void k_vox_gather(const VoxBatch B, int with_xc)
         const int xy = J.op.vox_xy[vi];
         const float v = J.xfull[((int64_t)(xy & 0xffff) + (int64_t)(xy >> 16) * J.op.P.nx) * K + k];
         if (with_xc) J.xc[loc] = v;
-        J.xd[loc] = v * J.op.coarse_q[k].z;
+        J.xd[xd_index(J, vi, k)] = v * J.op.coarse_q[k].z;
+    }
+}
+
+// Rows [nv][K] of x dq into the forward's layout.
+__global__ void k_vox_pack(const float *__restrict__ rows, int64_t nv, int K, int64_t stride, float *__restrict__ xd)
+{
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nv * K; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = t / K;
+        const int k = (int)(t - v * K);
+        xd[2 * ((int64_t)(k >> 1) * stride + v) + (k & 1)] = rows[t];
     }
 }
 
@@ -711,15 +728,39 @@ cudaError_t vox_set_attributes(int max_smem)
 size_t vox_fwd_static_smem() { return static_smem(k_vox_fwd<true>); }
 size_t vox_adj_static_smem() { return static_smem(k_vox_adj); }
 
-size_t vox_fwd_smem(const DevProblem &P) { return vox_fwd_layout(P, P.e_hi - P.e_lo + 1).total; }
-
-size_t vox_adj_smem(const DevProblem &P, int warps)
+// Bytes of one block with the sums of 32 voxels, as the operator's limit on
+// the coarse bins is stated: 256 bytes per bin and the tables.
+size_t vox_limit_smem(const DevProblem &P)
 {
     const int E = P.e_hi - P.e_lo + 1, K = P.nwt;
-    return al16(sizeof(float) * kEnRows * E) + sizeof(float4) * K + sizeof(float4) * (size_t)warps * E +
-           sizeof(float2) * (size_t)warps * 32 * K + sizeof(PairRec) * warps + sizeof(float) * (size_t)warps * E +
-           16 + sizeof(int2) * (size_t)warps * E + (size_t)warps * 2 * K;
+    return al16(sizeof(float) * 8 * E) + sizeof(float4) * K + sizeof(float4) * E + sizeof(float2) * 32 * (size_t)K +
+           sizeof(PairRec) + sizeof(float) * E + 16 + sizeof(int2) * E + 2 * K;
 }
+
+// The forward's tiles and runs: as many voxels per tile as three blocks per SM
+// leave room for (up to 768; a voxel takes 48 bytes and 4 per coarse bin), fewer
+// blocks only where not even one step of 32 voxels would fit; four runs or
+// more per warp.  They depend on the problem alone, so that a batch gives
+// the same bits as the operators by themselves.
+size_t vox_fwd_split(const DevProblem &P, int nv, int *steps, int *tiles, int *runs)
+{
+    const int E = P.e_hi - P.e_lo + 1;
+    const int chunks = nv > 0 ? (nv + 31) / 32 : 1;
+    const size_t stat = vox_fwd_static_smem() + 1024;
+    auto runs_of = [&](int st) {
+        const int r = (4 * kFwdWarps + E - 1) / E;
+        return r < 1 ? 1 : (r > st ? st : r);
+    };
+    int cap = 1;
+    for (int st = 2; st <= kMaxSteps; st++)
+        if (vox_fwd_layout(P, E, st, runs_of(st)).total + stat <= 76 * 1024) cap = st;
+    *tiles = (chunks + cap - 1) / cap;
+    *steps = (chunks + *tiles - 1) / *tiles;
+    *runs = runs_of(*steps);
+    return vox_fwd_layout(P, E, *steps, *runs).total;
+}
+
+size_t vox_adj_smem(const DevProblem &P, int warps) { return vox_adj_layout(P, P.e_hi - P.e_lo + 1, warps).total; }
 
 int vox_fwd_blocks_per_sm(size_t smem)
 {
@@ -770,7 +811,7 @@ cudaError_t launch_vox_wtab(const VoxBatch &B, int64_t total, int mode, cudaStre
 
 cudaError_t launch_vox_reduce(const VoxBatch &B, int64_t total, int mode, cudaStream_t s, int64_t *launches)
 {
-    k_vox_reduce<<<grid_for(total, 256), 256, 0, s>>>(B, mode);
+    k_vox_reduce<<<grid_for(total, 32), 32 * kReduceWarps, 0, s>>>(B, mode);   // a block per 32 entries
     if (launches) (*launches)++;
     return cudaGetLastError();
 }
@@ -778,6 +819,14 @@ cudaError_t launch_vox_reduce(const VoxBatch &B, int64_t total, int mode, cudaSt
 cudaError_t launch_vox_gather(const VoxBatch &B, int64_t total, bool with_xc, cudaStream_t s, int64_t *launches)
 {
     k_vox_gather<<<grid_for(total, 256), 256, 0, s>>>(B, with_xc ? 1 : 0);
+    if (launches) (*launches)++;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_vox_pack(const float *rows, int64_t nv, int K, int64_t stride, float *xd, cudaStream_t s,
+                            int64_t *launches)
+{
+    k_vox_pack<<<grid_for(nv * K, 256), 256, 0, s>>>(rows, nv, K, stride, xd);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

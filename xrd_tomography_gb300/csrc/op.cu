@@ -41,9 +41,10 @@ struct xrdt_op {
     // device buffers
     int32_t *seg = nullptr;
     float *a1 = nullptr, *a2 = nullptr;
-    float *xc = nullptr, *xd = nullptr;   // unknowns, compact; xd = x * dq
+    float *xc = nullptr, *xd = nullptr;   // unknowns, compact; xd = x * dq in the forward's layout
+    int64_t xd_stride = 0;
     float *what = nullptr;                // [pairs][E]
-    float2 *part = nullptr;               // [groups][nv][NWT] as float pairs
+    float4 *part = nullptr;               // [groups][row_len] (VoxJob::part)
     double *sens = nullptr;               // [nv][NWT]
     float *xfull = nullptr;               // staging of the full-grid layout
     float *ray_a = nullptr, *ray_b = nullptr;   // staging of ray vectors
@@ -67,7 +68,7 @@ struct Plan {
     VoxJob *jobs_d = nullptr;
     int64_t *off_d = nullptr;
     unsigned long long *counters_d = nullptr;
-    std::vector<int64_t> off;          // 5 x (n + 1)
+    std::vector<int64_t> off;          // 6 x (n + 1)
     int sms = 0;
     int adj_warps = 1;
     int64_t adj_tiles = 0;             // target number of adjoint tiles
@@ -200,6 +201,8 @@ int begin(xrdt_op *op)
 
 int64_t pairs_of(const xrdt_op *op) { return (int64_t)op->p.n_src * op->v.P.n_det; }
 int chunks_of(const xrdt_op *op) { return (op->v.nv + 31) / 32; }
+// float4 entries of one partial row of the adjoint
+int64_t row_len(const xrdt_op *op) { return (int64_t)chunks_of(op) * 32 * ((op->p.nwt + 1) / 2); }
 
 // Adjoint split for a warps-per-block count and a target tile count: one
 // pairs-per-group for the whole batch, so that tiles carry similar work.
@@ -213,7 +216,7 @@ void plan_split(Plan *pl, int warps, int64_t tiles)
     }
     int64_t ppg = (int64_t)std::ceil(work / (double)std::max<int64_t>(tiles, 1));
     if (ppg < 1) ppg = 1;
-    pl->off.assign(5 * (size_t)(n + 1), 0);
+    pl->off.assign(6 * (size_t)(n + 1), 0);
     size_t smem = 0;
     for (int i = 0; i < n; i++) {
         const xrdt_op *op = pl->ops[i];
@@ -232,6 +235,7 @@ void plan_split(Plan *pl, int warps, int64_t tiles)
         o[2 * N1 + i + 1] = o[2 * N1 + i] + (int64_t)op->v.nv * op->p.nwt;
         o[3 * N1 + i + 1] = o[3 * N1 + i] + (int64_t)op->p.nx * op->p.ny * op->p.nwt;
         o[4 * N1 + i + 1] = o[4 * N1 + i] + np * J.E;
+        o[5 * N1 + i + 1] = o[5 * N1 + i] + row_len(op);
         smem = std::max(smem, vox_adj_smem(op->v.P, warps));
     }
     pl->adj_warps = warps;
@@ -328,7 +332,7 @@ cudaError_t zero_rows(const Plan *pl, cudaStream_t st)
     for (size_t i = 0; i < pl->ops.size(); i++) {
         const xrdt_op *op = pl->ops[i];
         if (op->v.nv == 0) continue;
-        cudaError_t e = cudaMemsetAsync(op->part, 0, sizeof(float2) * (size_t)pl->rows[i] * op->v.nv * op->p.nwt, st);
+        cudaError_t e = cudaMemsetAsync(op->part, 0, sizeof(float4) * (size_t)pl->rows[i] * row_len(op), st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -454,7 +458,7 @@ int plan_create(xrdt_ctx *ctx, xrdt_op *const *ops, int n, Plan **out)
     cudaError_t e = test_alloc_fails() ? cudaErrorMemoryAllocation
                                        : cudaMallocHost((void **)&pl->jobs_h, sizeof(VoxJob) * n);
     if (e == cudaSuccess) e = cudaMalloc((void **)&pl->jobs_d, sizeof(VoxJob) * n);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&pl->off_d, sizeof(int64_t) * 5 * (n + 1));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&pl->off_d, sizeof(int64_t) * 6 * (n + 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&pl->counters_d, sizeof(unsigned long long) * 2);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&pl->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e != cudaSuccess) {
@@ -471,6 +475,7 @@ int plan_create(xrdt_ctx *ctx, xrdt_op *const *ops, int n, Plan **out)
         J.c = make_f32_consts(op->v.P);
         J.E = op->v.P.e_hi - op->v.P.e_lo + 1;
         J.xd = op->xd;
+        J.xd_stride = op->xd_stride;
         J.xc = op->xc;
         J.what = op->what;
         J.part = op->part;
@@ -478,7 +483,7 @@ int plan_create(xrdt_ctx *ctx, xrdt_op *const *ops, int n, Plan **out)
         J.pair0 = 0;
         J.pair1 = pairs_of(op);
         J.accumulate = 0;
-        fsmem = std::max(fsmem, vox_fwd_smem(op->v.P));
+        fsmem = std::max(fsmem, vox_fwd_split(op->v.P, op->v.nv, &J.steps, &J.tiles, &J.runs));
         if (op->v.nv > 0 && !op->v.walk) pl->streamed = true;
     }
     pl->fwd_smem = fsmem;
@@ -489,16 +494,26 @@ int plan_create(xrdt_ctx *ctx, xrdt_op *const *ops, int n, Plan **out)
             return rc;
         }
     }
-    // the widest adjoint block the shared memory allows
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    int warps = 4;
-    for (; warps > 1; warps /= 2) {
+    // the adjoint's block that keeps the most warps on an SM (the narrowest of
+    // them: a block's warps wait for one another between tiles), and four
+    // tiles for every block that is resident at once (96x78 voxels: 2.23 ms; two
+    // 2.49, one 2.79: the tiles' lengths differ)
+    int warps = 1, most = 0;
+    int64_t tiles = 1;
+    for (int w = 1; w <= 4; w *= 2) {
         size_t sm = 0;
-        for (int i = 0; i < n; i++) sm = std::max(sm, vox_adj_smem(ops[i]->v.P, warps));
-        if ((int64_t)(sm + vox_adj_static_smem()) <= optin) break;
+        for (int i = 0; i < n; i++) sm = std::max(sm, vox_adj_smem(ops[i]->v.P, w));
+        if ((int64_t)(sm + vox_adj_static_smem()) > optin) break;
+        const int bps = vox_adj_blocks_per_sm(w, sm);
+        if (bps * w > most) {
+            most = bps * w;
+            warps = w;
+            tiles = (int64_t)pl->sms * bps * 4;
+        }
     }
-    plan_split(pl, warps, (int64_t)pl->sms * 4 * vox_adj_blocks_per_sm(warps, 0));
+    plan_split(pl, warps, tiles);
     const int64_t items = plan_total(pl, 0);
     pl->fwd_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)pl->sms * vox_fwd_blocks_per_sm(fsmem), items));
     *out = pl;
@@ -532,7 +547,7 @@ int plan_sens(Plan *pl)
         }
         {
             ProfScope ps(ctx, XRDT_KERNEL_VOX_UPDATE);
-            CK(launch_vox_reduce(B, plan_total(pl, 2), part ? 4 : 0, st, &ctx->launches));
+            CK(launch_vox_reduce(B, plan_total(pl, 5), part ? 4 : 0, st, &ctx->launches));
         }
     }
     for (xrdt_op *op : pl->ops) op->sens_ready = true;
@@ -566,7 +581,8 @@ std::string tune_key(const Plan *pl)
     std::string key;
     if (cudaGetDeviceProperties(&prop, pl->ctx->device) == cudaSuccess) {
         for (const char *c = prop.name; *c; c++) key += (*c == ' ') ? '_' : *c;
-        key += fmt("-sm%d", prop.multiProcessorCount);
+        // (the suffix names the adjoint's layout: a split tuned for another one says nothing)
+        key += fmt("-sm%d-lane_voxel", prop.multiProcessorCount);
     } else {
         cudaGetLastError();
         key = "gpu";
@@ -761,7 +777,7 @@ int plan_adjoint(Plan *pl, const float *const *w, float *const *g, bool compact 
         else CK(launch_vox_adjoint(B, pl->adj_grid, pl->adj_smem, st, &ctx->launches));
     }
     ProfScope ps(ctx, XRDT_KERNEL_VOX_UPDATE);
-    CK(launch_vox_reduce(B, plan_total(pl, 2), compact ? 3 : 2, st, &ctx->launches));
+    CK(launch_vox_reduce(B, plan_total(pl, 5), compact ? 3 : 2, st, &ctx->launches));
     return XRDT_OK;
 }
 
@@ -785,7 +801,7 @@ int plan_ratio_backprojection(Plan *pl)
         CK(launch_vox_adjoint(B, pl->adj_grid, pl->adj_smem, st, &ctx->launches));
     }
     ProfScope ps(ctx, XRDT_KERNEL_VOX_UPDATE);
-    CK(launch_vox_reduce(B, plan_total(pl, 2), 3, st, &ctx->launches));
+    CK(launch_vox_reduce(B, plan_total(pl, 5), 3, st, &ctx->launches));
     return XRDT_OK;
 }
 
@@ -830,7 +846,7 @@ int plan_mlem(Plan *pl, const float *const *y, const float *const *c, float *con
                 le = launch_vox_forward(B, true, pl->fwd_grid, pl->fwd_smem, st, &dummy);
                 if (le == cudaSuccess) le = launch_vox_adjoint(B, pl->adj_grid, pl->adj_smem, st, &dummy);
             }
-            if (le == cudaSuccess) le = launch_vox_reduce(B, plan_total(pl, 2), 1, st, &dummy);
+            if (le == cudaSuccess) le = launch_vox_reduce(B, plan_total(pl, 5), 1, st, &dummy);
             pl->mlem_launches = dummy;
             cudaError_t ce = cudaStreamEndCapture(st, &graph);
             if (le != cudaSuccess) {
@@ -923,6 +939,7 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     PairRec *d_pairs;
     if ((rc = op_alloc_t(op, 4 * (size_t)(p->nx + 1) * (p->ny + 1), &B.cells)) ||
         (rc = op_alloc_t(op, nvox, &B.vox_xy)) || (rc = op_alloc_t(op, nvox, &B.vox_mat)) ||
+        (rc = op_alloc_t(op, nvox, &B.vox_order)) || (rc = op_alloc_t(op, nvox, &B.vox_rank)) ||
         (rc = op_alloc_t(op, 4, &B.counters)) || (rc = op_alloc_t(op, p->n_src, &d_src)))
         return bail(rc);
     void *pp;
@@ -985,14 +1002,19 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     float *d_rf;
     int *d_wlo, *d_wn;
     float4 *d_cq;
+    VoxEnergy *d_ven;
+    unsigned *d_lut;
     if ((rc = op_alloc_t(op, ht.energy.size(), &d_energy)) || (rc = op_alloc_t(op, ht.rf_win.size(), &d_rf)) ||
         (rc = op_alloc_t(op, ht.win_lo.size(), &d_wlo)) || (rc = op_alloc_t(op, ht.win_n.size(), &d_wn)) ||
-        (rc = op_alloc_t(op, ht.coarse_q.size(), &d_cq)))
+        (rc = op_alloc_t(op, ht.coarse_q.size(), &d_cq)) || (rc = op_alloc_t(op, ht.vox_energy.size(), &d_ven)) ||
+        (rc = op_alloc_t(op, ht.qlut.size(), &d_lut)))
         return bail(rc);
     e = cudaMemcpyAsync(d_energy, ht.energy.data(), sizeof(EnergyRow) * ht.energy.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_rf, ht.rf_win.data(), sizeof(float) * ht.rf_win.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_wlo, ht.win_lo.data(), sizeof(int) * ht.win_lo.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_wn, ht.win_n.data(), sizeof(int) * ht.win_n.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_ven, ht.vox_energy.data(), sizeof(VoxEnergy) * ht.vox_energy.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_lut, ht.qlut.data(), sizeof(unsigned) * ht.qlut.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_cq, ht.coarse_q.data(), sizeof(float4) * ht.coarse_q.size(), cudaMemcpyHostToDevice, st);
 
     op->src = d_src;
@@ -1027,6 +1049,11 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     op->v.cells = B.cells;
     op->v.atten_src = B.atten_src;
     op->v.walk = d_walk;
+    op->v.vox_energy = d_ven;
+    op->v.qlut = d_lut;
+    op->v.lut_scale = ht.lut_scale;
+    op->v.c1 = ht.energy[P.e_lo].sig_c1;   // the same for every source bin
+    op->v.c1l = ht.energy[P.e_lo].sig_c1_lo;
 
     // work buffers
     int sms = 0;
@@ -1043,19 +1070,25 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
         op->groups_cap = (int)std::max<int64_t>(1, std::min<int64_t>(npairs, ((int64_t)sms * 64 + cb - 1) / cb));
     }
     const size_t nx_k = (size_t)std::max(nv, 1) * K;
-    if ((rc = op_alloc_t(op, nx_k, &op->xc)) || (rc = op_alloc_t(op, nx_k, &op->xd)) ||
+    op->xd_stride = ((int64_t)std::max(nv, 1) + 31) / 32 * 32;
+    const size_t n_xd = 2 * (size_t)op->xd_stride * ((K + 1) / 2);
+    if ((rc = op_alloc_t(op, nx_k, &op->xc)) || (rc = op_alloc_t(op, n_xd, &op->xd)) ||
         (rc = op_alloc_t(op, (size_t)npairs * E, &op->what)) ||
-        (rc = op_alloc_t(op, (size_t)op->groups_cap * nx_k, &op->part)) || (rc = op_alloc_t(op, nx_k, &op->sens)) ||
+        (rc = op_alloc_t(op, (size_t)op->groups_cap * std::max<int64_t>(row_len(op), 1), &op->part)) || (rc = op_alloc_t(op, nx_k, &op->sens)) ||
         (rc = op_alloc_t(op, (size_t)nvox * K, &op->xfull)) || (rc = op_alloc_t(op, (size_t)op->rays, &op->ray_a)) ||
         (rc = op_alloc_t(op, (size_t)op->rays, &op->ray_b)))
         return bail(rc);
     int optin = 0;
     e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-    if (e == cudaSuccess && ((int64_t)(vox_fwd_smem(P) + vox_fwd_static_smem()) > optin ||
+    int st_, ti_, ru_;
+    if (e == cudaSuccess && ((int64_t)(vox_fwd_split(P, nv, &st_, &ti_, &ru_) + vox_fwd_static_smem()) > optin ||
+                           (int64_t)(vox_limit_smem(P) + vox_adj_static_smem()) > optin ||
                            (int64_t)(vox_adj_smem(P, 1) + vox_adj_static_smem()) > optin)) {
         fail(ctx, XRDT_ERR_UNSUPPORTED, "the problem's tables exceed the shared memory of one block");
         return bail(XRDT_ERR_UNSUPPORTED);
     }
+    // the pads of xd are read (and multiplied by 0): never leave them unset
+    if (e == cudaSuccess) e = cudaMemsetAsync(op->xd, 0, sizeof(float) * n_xd, st);
     if (e == cudaSuccess) e = vox_set_attributes(optin);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
@@ -1428,7 +1461,8 @@ int bop_expand(xrdt_bop *b)
     xrdt_ctx *ctx = op->ctx;
     if (op->v.nv == 0) return XRDT_OK;
     ProfScope ps(ctx, XRDT_KERNEL_BASIS);
-    CK(launch_basis_expand(b->coef, op->v.nv, b->J, b->Bdq, op->p.nwt, op->xd, b->err, ctx->stream, &ctx->launches));
+    CK(launch_basis_expand(b->coef, op->v.nv, b->J, b->Bdq, op->p.nwt, b->gx, b->err, ctx->stream, &ctx->launches));
+    CK(launch_vox_pack(b->gx, op->v.nv, op->p.nwt, op->xd_stride, op->xd, ctx->stream, &ctx->launches));
     return XRDT_OK;
 }
 

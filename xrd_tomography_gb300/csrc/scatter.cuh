@@ -17,18 +17,20 @@ namespace xrdt {
 
 // Per-(source, pixel) constants of the scattering geometry.
 struct PairGeom {
-    ff Rsx, Rsy, Rdx, Rdy, Rdz;   // source and detector positions
-    ff k1;                        // tan(geomphi/2) / |nsrc_xy|
-    ff nsx2, nsy2;                // in-plane source orientation as pairs
+    ff Rsx, Rsy, Rdx, Rdy;        // source and detector positions (in plane)
+    ff Dx, Dy, Dz, DD;            // source -> detector vector and its square
+    ff mx, my;                    // the voxel's height over the source: az = ax mx + ay my
+    ff Dn;                        // D . n_det
+    ff hz;                        // Hvox = az hz
     float nsx, nsy, nsz, ndx, ndy, sphi, cphi;
-    float k2;                     // tan(geomphi) / |nsrc_xy|
-    ff k2f;                       // the same as a pair
-    float tan_full, adet12, vox2, focal2_12;
+    float tan_full, adet12, focal2_12;
+    ff vox2_12;                   // vox^2 / 12
 };
 
 // Per-voxel results of the scattering geometry.
 struct VoxGeom {
     ff s;        // sin(theta/2)
+    ff s2;       // sin^2(theta/2)
     ff omc;      // 1 - cos(theta)
     ff sg;       // (sS2 + vV2 + dD2) / (|a|^2 |b|^2)
     float gp;    // geom_src2vox * geom_vox2det
@@ -106,48 +108,15 @@ constexpr double kHalfLog2e = 0.72134752044448170368;
 constexpr float kHalfLog2e_hi = (float)kHalfLog2e;
 constexpr float kHalfLog2e_lo = (float)(kHalfLog2e - (double)kHalfLog2e_hi);
 
-// c = -0.5 log2(e) / sigma^2 as a float pair, from sigma^2 as a pair.  The
-// residual of the correctly rounded quotient is exact through the FMA.
-__device__ __forceinline__ ff gauss_scale(ff sig2)
+// c = -0.5 log2(e) / sigma^2 as a float pair, from sigma^2 as a pair and its
+// reciprocal to FP32.  The residual of the quotient is exact through the FMA
+// to a bit or two.
+__device__ __forceinline__ ff gauss_scale(ff sig2, float rcp)
 {
-    const float rcp = rcp_approx(sig2.hi);
     const float ch = -kHalfLog2e_hi * rcp;
-    // the quotient's residual, exact through the FMA to a bit or two
     float r = fmaf(-ch, sig2.hi, -kHalfLog2e_hi);
     r = fmaf(-ch, sig2.lo, r) - kHalfLog2e_lo;
     return {ch, r * rcp};
-}
-
-// 2^(c (w - q)^2) with the argument in FP32 but c as a pair: the scale c
-// carries the systematic part of the error (sigma), the difference and its
-// square round independently per term.
-__device__ __forceinline__ float gauss_f32(float wh, float wl, float qh, float ql, float ch, float cl)
-{
-    const float d = (wh - qh) + (wl - ql);
-    const float d2 = d * d;
-    return ex2_approx(fmaf(ch, d2, cl * d2));
-}
-
-// 2^(c (w - q)^2) with w, q and c as float pairs.  The argument is formed
-// as a pair (exact difference, exact square through the FMA), so its error
-// is a few units of 2^-44 relative instead of a few FP32 ulps: deep in the
-// Gaussian's tail, where the argument is tens, an FP32 argument would move
-// the term by about 1e-6 relative.  The low part enters as 2^lo = 1 + lo ln2.
-__device__ __forceinline__ float gauss_ff(float wh, float wl, float qh, float ql, float ch, float cl)
-{
-    const float t = wh - qh;   // exact while w and q are within a factor of two
-    const float u = wl - ql;
-    const float dh = t + u;
-    const float dl = u - (dh - t);
-    const float d2h = dh * dh;
-    float d2l = fmaf(dh, dh, -d2h);
-    d2l = fmaf(dh + dh, dl, d2l);
-    const float ah = ch * d2h;
-    float al = fmaf(ch, d2h, -ah);
-    al = fmaf(ch, d2l, al);
-    al = fmaf(cl, d2h, al);
-    const float e = ex2_approx(ah);
-    return fmaf(e, al * kLn2, e);
 }
 
 // Compton table bin of integrate_diffraction.cu:331-337 decided in FP64, as
@@ -240,112 +209,113 @@ __device__ __forceinline__ void pair_geom(const DevProblem &P, const SrcGeom &g,
     G->Rsy = ff_from_double(g.Rsrc_y);
     G->Rdx = ff_from_double(*Rdet_x);
     G->Rdy = ff_from_double(*Rdet_y);
-    G->Rdz = ff_from_double(Rdz);
+    const double Dx = *Rdet_x - g.Rsrc_x, Dy = *Rdet_y - g.Rsrc_y;   // Rsrc_z = 0
+    G->Dx = ff_from_double(Dx);
+    G->Dy = ff_from_double(Dy);
+    G->Dz = ff_from_double(Rdz);
+    G->DD = ff_from_double(Dx * Dx + Dy * Dy + Rdz * Rdz);
     const double nsx = -g.sphi * P.sta, nsy = g.cphi * P.sta, nsz = -P.cta;
     const double nsxy = sqrt(nsx * nsx + nsy * nsy);
     G->nsx = (float)nsx;
     G->nsy = (float)nsy;
-    G->nsx2 = ff_from_double(nsx);
-    G->nsy2 = ff_from_double(nsy);
     G->nsz = (float)nsz;
-    G->k1 = ff_from_double(P.tan_half / nsxy);
-    G->k2 = (float)(P.tan_full / nsxy);
-    G->k2f = ff_from_double(P.tan_full / nsxy);
+    // Rvox_z = -(a . nsrc_xy) tan(geomphi/2) / |nsrc_xy|, Hvox with tan(geomphi)
+    G->mx = ff_from_double(-nsx * P.tan_half / nsxy);
+    G->my = ff_from_double(-nsy * P.tan_half / nsxy);
+    G->hz = ff_from_double(-P.tan_full / P.tan_half);
     G->ndx = (float)g.sphi;
     G->ndy = (float)(-g.cphi);
+    G->Dn = ff_from_double(Dx * (double)G->ndx + Dy * (double)G->ndy);
     G->sphi = (float)g.sphi;
     G->cphi = (float)g.cphi;
     G->tan_full = (float)P.tan_full;
     G->adet12 = (float)(P.geomAdet / 12.0);
-    G->vox2 = (float)(P.vox * P.vox);
+    G->vox2_12 = ff_from_double(P.vox * P.vox / 12.0);
     G->focal2_12 = (float)(P.focal * P.focal / 12.0);
 }
 
-// integrate_diffraction.cu:196-255 for one voxel.  a = voxel - source and
-// b = detector - voxel as float pairs; 1 - cos(theta) from the cross product
-// |a x b|^2 / (|a||b| (|a||b| + a.b)), which has no cancellation at small
-// angles; the blur vectors S = ((a x b) x a)/|a|^2 = b - (a.b/|a|^2) a and
-// D = ((a x b) x b)/|b|^2 = -a + (a.b/|b|^2) b in FP32.
-// SIGMA_PAIR: sigma's blur terms as float pairs (the per-voxel operator,
-// whose adjoint sums deep Gaussian tails); otherwise in FP32 (the material
-// forward projector, whose counts are dominated by the Gaussians' cores).
+// integrate_diffraction.cu:196-255 for one voxel.  a = voxel - source as
+// float pairs, b = detector - voxel = D - a; 1 - cos(theta) from the cross
+// product a x b = a x D, |a x b|^2 / (|a||b| (|a||b| + a.b)), which has no
+// cancellation at small angles.  The blur vectors S = ((a x b) x a)/|a|^2,
+// D' = ((a x b) x b)/|b|^2 and V = -(S + D') = u x (a x b), u = a/|a|^2 +
+// b/|b|^2, are perpendicular to a, b and a x b in turn, so with c = a x b
+//   |S|^2 = |c|^2/|a|^2,  |D'|^2 = |c|^2/|b|^2,  |V|^2 = |D|^2 |c|^2/(|a|^2 |b|^2)
+// and only their components along the source's, the detector's and the z axis
+// are left to find.  (The z component is no small one where the detector sits
+// high over the fan plane.)
+// SIGMA_PAIR: the terms that make up most of sigma^2 as pairs (the per-voxel
+// operator, whose adjoint sums deep Gaussian tails: a tail amplifies sigma^2's
+// relative error by (q distance / sigma)^2 / 2, and FP32 leaves it about two
+// ulps off); otherwise in FP32 (the material forward projector, whose counts
+// are dominated by the Gaussians' cores).  About 500 and 300 instructions per
+// voxel; component by component with correctly rounded quotients and roots
+// they were 2700 and 700, a third of the operator's forward and a tenth of
+// the projector.
 template <bool SIGMA_PAIR>
 __device__ __forceinline__ VoxGeom vox_geom(const PairGeom &G, float vx, float vy)
 {
     const ff ax = ff_fsub(vx, G.Rsx), ay = ff_fsub(vy, G.Rsy);
-    const ff proj = ff_add(ff_mul(ax, G.nsx2), ff_mul(ay, G.nsy2));
-    const ff az = ff_neg(ff_mul(proj, G.k1));          // Rvox_z; Rsrc_z = 0
-    const float Hvox = proj.hi * G.k2;
-    const ff bx = ff_add(G.Rdx, ff{-vx, 0.f}), by = ff_add(G.Rdy, ff{-vy, 0.f});
-    const ff bz = ff_sub(G.Rdz, az);
-    const ff ab = ff_add(ff_add(ff_mul(ax, bx), ff_mul(ay, by)), ff_mul(az, bz));
-    const ff an = ff_add(ff_add(ff_sqr(ax), ff_sqr(ay)), ff_sqr(az));
-    const ff bn = ff_add(ff_add(ff_sqr(bx), ff_sqr(by)), ff_sqr(bz));
-    const ff cx = ff_sub(ff_mul(ay, bz), ff_mul(az, by));
-    const ff cy = ff_sub(ff_mul(az, bx), ff_mul(ax, bz));
-    const ff cz = ff_sub(ff_mul(ax, by), ff_mul(ay, bx));
-    const ff cn = ff_add(ff_add(ff_sqr(cx), ff_sqr(cy)), ff_sqr(cz));
-    const ff nab = ff_sqrt(ff_mul(an, bn));
+    const ff az = ffl_dot2(ax, G.mx, ay, G.my);
+    const ff aD = ffl_dot3(ax, G.Dx, ay, G.Dy, az, G.Dz);
+    const ff an = ffl_dot3(ax, ax, ay, ay, az, az);
+    const ff ab = ffl_sub(aD, an), bD = ffl_sub(G.DD, aD);
+    // (tight where terms cancel: these high parts are used as floats, too)
+    const ff bn = ff_sub(bD, ab);
+    const ff cx = ff_dot2(ay, G.Dz, ff_neg(az), G.Dy);
+    const ff cy = ff_dot2(az, G.Dx, ff_neg(ax), G.Dz);
+    const ff cz = ff_dot2(ax, G.Dy, ff_neg(ay), G.Dx);
+    const ff cn = ffl_dot3(cx, cx, cy, cy, cz, cz);
+    const ff nab = ffl_sqrt(ffl_mul(an, bn));
     VoxGeom r;
-    if (ab.hi > 0.f) r.omc = ff_div(cn, ff_mul(nab, ff_add(nab, ab)));
-    else r.omc = ff_fsub(1.f, ff_div(ab, nab));
-    r.s = ff_sqrt(ff_mulf(r.omc, 0.5f));
+    if (ab.hi > 0.f) r.omc = ff_tight(ffl_mul(cn, ffl_rcp(ffl_mul(nab, ffl_add(nab, ab)))));
+    else r.omc = ff_fsub(1.f, ffl_mul(ab, ffl_rcp(nab)));
+    r.s2 = ff{0.5f * r.omc.hi, 0.5f * r.omc.lo};
+    r.s = ff_sqrt(r.s2);
     const float costh = 1.f - r.omc.hi;
     r.cos2 = costh * costh;
     // FP32 remainder of the geometry
-    const float Ax = ax.hi, Ay = ay.hi, Az = az.hi, Bx = bx.hi, By = by.hi, Bz = bz.hi;
-    const float Cx = cx.hi, Cy = cy.hi, Cz = cz.hi, An = an.hi, Bn = bn.hi;
-    const float ia = __fdividef(1.f, An);
-    const float Sx = (Cy * Az - Cz * Ay) * ia, Sy = (Cz * Ax - Cx * Az) * ia, Sz = (Cx * Ay - Cy * Ax) * ia;
-    const float Snsrc = Sx * G.nsx + Sy * G.nsy + Sz * G.nsz;
-    const float sS2 = (Sx * Sx + Sy * Sy + Sz * Sz - Snsrc * Snsrc) * G.focal2_12;
+    const float Ax = ax.hi, Ay = ay.hi, Az = az.hi, Cx = cx.hi, Cy = cy.hi, Cz = cz.hi;
+    // (from the pixel: D - a would round at the size of D)
+    const float Bx = (G.Rdx.hi - vx) + G.Rdx.lo, By = (G.Rdy.hi - vy) + G.Rdy.lo;
+    const ff ian = ff_rcp(an), ibn = ff_rcp(bn);
+    const float ia = ian.hi, ib = ibn.hi;
+    const float Sn = ((Cy * Az - Cz * Ay) * G.nsx + (Cz * Ax - Cx * Az) * G.nsy + (Cx * Ay - Cy * Ax) * G.nsz) * ia;
+    const float sS2 = (cn.hi * ia - Sn * Sn) * G.focal2_12;
     if (!SIGMA_PAIR) {
-        const float ib = __fdividef(1.f, Bn);
-        const float Dx = (Cy * Bz - Cz * By) * ib, Dy = (Cz * Bx - Cx * Bz) * ib, Dz = (Cx * By - Cy * Bx) * ib;
-        const float Vx = -(Sx + Dx), Vy = -(Sy + Dy), Vz = -(Sz + Dz);
-        const float Dndet = Dx * G.ndx + Dy * G.ndy;
-        const float dD2 = (Dx * Dx + Dy * Dy + Dz * Dz - Dndet * Dndet) * G.adet12;
-        const float vV2 = (G.vox2 * (Vx * Vx + Vy * Vy) + Hvox * Hvox * Vz * Vz) * (1.f / 12.f);
-        r.sg = ff{(sS2 + vV2 + dD2) * ia * ib, 0.f};
+        const float ux = fmaf(Ax, ia, Bx * ib), uy = fmaf(Ay, ia, By * ib);
+        const float Vz = ux * Cy - uy * Cx, Bz = G.Dz.hi - Az;
+        const float Dn = ((Cy * Bz - Cz * By) * G.ndx + (Cz * Bx - Cx * Bz) * G.ndy) * ib;
+        const float cb = cn.hi * ib;
+        const float H = Az * G.hz.hi;
+        const float rest = fmaf(Vz * Vz, fmaf(H * H, 1.f / 12.f, -G.vox2_12.hi), sS2);
+        r.sg = ff{fmaf(G.DD.hi * (cb * ia), G.vox2_12.hi, fmaf(cb - Dn * Dn, G.adet12, rest)) * ia * ib, 0.f};
     } else {
-        // The blur terms that make up most of sigma^2 as pairs: the Gaussian's
-        // tail amplifies their relative error by (q distance / sigma)^2 / 2, and
-        // FP32 leaves them about two ulps off.  V = -(S + D) = u x C with
-        // u = a/|a|^2 + b/|b|^2 (S = C x a/|a|^2, D = C x b/|b|^2, C = a x b), and
-        // |D|^2 - (D.n_det)^2 = Dz^2 + (Dx n_y - Dy n_x)^2 for the in-plane unit
-        // normal n_det.
-        const ff iaf = ff_div(ff{1.f, 0.f}, an), ibf = ff_div(ff{1.f, 0.f}, bn);
-        const ff ux = ff_add(ff_mul(ax, iaf), ff_mul(bx, ibf));
-        const ff uy = ff_add(ff_mul(ay, iaf), ff_mul(by, ibf));
-        const ff uz = ff_add(ff_mul(az, iaf), ff_mul(bz, ibf));
-        const ff Vx = ff_sub(ff_mul(uy, cz), ff_mul(uz, cy));
-        const ff Vy = ff_sub(ff_mul(uz, cx), ff_mul(ux, cz));
-        const ff Vz = ff_sub(ff_mul(ux, cy), ff_mul(uy, cx));
-        const ff Hv = ff_mul(proj, G.k2f);
-        const ff vV = ff_add(ff_mulf(ff_add(ff_sqr(Vx), ff_sqr(Vy)), G.vox2), ff_mul(ff_sqr(Hv), ff_sqr(Vz)));
-        const ff Dx = ff_mul(ff_sub(ff_mul(cy, bz), ff_mul(cz, by)), ibf);
-        const ff Dy = ff_mul(ff_sub(ff_mul(cz, bx), ff_mul(cx, bz)), ibf);
-        const ff Dz = ff_mul(ff_sub(ff_mul(cx, by), ff_mul(cy, bx)), ibf);
-        const ff Dt = ff_sub(ff_mulf(Dx, G.ndy), ff_mulf(Dy, G.ndx));
-        const ff dD = ff_mulf(ff_add(ff_sqr(Dz), ff_sqr(Dt)), G.adet12);
-        const ff blur = ff_add(ff_add(ff_mul(vV, ff{kTwelfth_hi, kTwelfth_lo}), dD), ff{sS2, 0.f});
-        r.sg = ff_mul(ff_mul(blur, iaf), ibf);
+        const ff cb = ffl_mul(cn, ibn);
+        const ff VV = ffl_mul(G.DD, ffl_mul(cb, ian));
+        // Vz of V = a (u.D) - D (u.a)
+        const ff ua = ffl_add(ff{1.f, 0.f}, ffl_mul(ab, ibn));
+        const ff Vz = ffl_dot2(az, ffl_dot2(aD, ian, bD, ibn), ff_neg(G.Dz), ua);
+        const ff Vz2 = ffl_mul(Vz, Vz);
+        // D'.n_det = c.(b x n)/|b|^2 = ((a.b)(D.n) - (a.n)(D.b))/|b|^2
+        const ff adn = ffl_dot2(ax, ff{G.ndx, 0.f}, ay, ff{G.ndy, 0.f});
+        const ff Dn = ffl_mul(ffl_dot2(ab, G.Dn, ff_neg(adn), bD), ibn);
+        const ff dD = ffl_sub(cb, ffl_mul(Dn, Dn));
+        const ff H = ffl_mul(az, G.hz);
+        const ff blur = ffl_add(ffl_dot3(ffl_sub(VV, Vz2), G.vox2_12, ffl_mul(Vz2, ffl_mul(H, H)),
+                                         ff{kTwelfth_hi, kTwelfth_lo}, dD, ff{G.adet12, 0.f}),
+                                ff{sS2, 0.f});
+        r.sg = ffl_mul(ffl_mul(blur, ian), ibn);
     }
+    // geom_src2vox geom_vox2det = (a.n_src,xy / |a_xy|) (b.n_det) tan / (|a| |b|^3);
+    // the roots and quotients with a correction step: the adjoint's column
+    // sums inherit any bias of these factors, and MLEM amplifies it tenfold
     const float Rdotn = -G.sphi * Ax + G.cphi * Ay;
-    if (!SIGMA_PAIR) {
-        const float cospsi = Rdotn * rsqrtf(Ax * Ax + Ay * Ay);
-        const float gsv = cospsi * rsqrtf(An) * G.tan_full;
-        const float gvd = -(G.ndx * Bx + G.ndy * By) * rsqrtf(Bn * Bn * Bn);
-        r.gp = gsv * gvd;
-    } else {
-        // correctly rounded roots and quotients: the adjoint's column sums
-        // inherit any bias of these factors, and MLEM amplifies it tenfold
-        const float axy = __fsqrt_rn(fmaf(Ax, Ax, Ay * Ay));
-        const float gsv = __fdiv_rn(__fdiv_rn(Rdotn, axy), __fsqrt_rn(An)) * G.tan_full;
-        const float nb = __fsqrt_rn(Bn);
-        const float gvd = __fdiv_rn(-(G.ndx * Bx + G.ndy * By), Bn * nb);
-        r.gp = gsv * gvd;
-    }
+    const float axy2 = fmaf(Ax, Ax, Ay * Ay);
+    float rxy = rsqrt_approx(axy2);
+    rxy = fmaf(0.5f * rxy, fmaf(-axy2 * rxy, rxy, 1.f), rxy);
+    const float inab = ff_rcp(nab).hi;   // (tight: rounded once)
+    r.gp = (Rdotn * rxy) * (-(G.ndx * Bx + G.ndy * By) * ib) * inab * G.tan_full;
     r.Wg = r.gp * ((1.f + r.cos2) * 0.5f);
     return r;
 }

@@ -77,18 +77,14 @@ __device__ __forceinline__ void walk_anchor_ff(const F32Consts &C, ff ex, ff ey,
         return;
     }
     const ff Dx = ff_fsub(vx, ex), Dy = ff_fsub(vy, ey);
-    const ff D = ff_sqrt(ff_add(ff_sqr(Dx), ff_sqr(Dy)));
-    ff ratio;
-    switch (w->edge) {
-    case 0: ratio = ff_div(ff{vy, 0.f}, Dy); break;              // y = 0
-    case 1: ratio = ff_div(ff{vx - C.nxf, 0.f}, Dx); break;      // x = NX
-    case 2: ratio = ff_div(ff{vy - C.nyf, 0.f}, Dy); break;      // y = NY
-    default: ratio = ff_div(ff{vx, 0.f}, Dx); break;             // x = 0
-    }
-    const ff Lr = ff_mul(D, ratio);
+    const ff D = ff_sqrt(ff_dot2(Dx, Dx, Dy, Dy));
+    const bool horizontal = w->edge == 0 || w->edge == 2;        // y = 0 or NY, else x = NX or 0
+    const float far_edge = w->edge == 1 ? C.nxf : (w->edge == 2 ? C.nyf : 0.f);
+    const ff ratio = ff_mulf(ff_rcp(horizontal ? Dy : Dx), (horizontal ? vy : vx) - far_edge);
+    const ff Lr = ff_mul(D, ratio), iD = ff_rcp(D);
     w->dlt = ff_sub(Lr, ff_mulf(ff{(float)(w->n - 1), 0.f}, C.DQ));
-    w->ux = ff_neg(ff_div(Dx, D));
-    w->uy = ff_neg(ff_div(Dy, D));
+    w->ux = ff_neg(ff_mul(Dx, iD));
+    w->uy = ff_neg(ff_mul(Dy, iD));
 }
 
 // FP32 version of walk_setup for the endpoint (ex, ey) rounded to float.
@@ -198,7 +194,7 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
         }
     }
     if (edge < 0) return false;
-    const ff D = ff_sqrt(ff_add(ff_sqr(dx), ff_sqr(dy)));
+    const ff D = ff_sqrt(ff_dot2(dx, dx, dy, dy));
     const ff Lr = ff_mul(D, ff_fsub(1.f, ua));
     const ff t = ff_div(Lr, ff{C.DQ, C.DQ_lo});
     if (!(t.hi > 0.f && t.hi < 4194304.f)) return false;

@@ -79,6 +79,18 @@ struct alignas(16) FwdEnergy {
     int ns;                     // detector bins whose window holds the source bin
 };
 
+// A source bin's constants as the per-voxel operator reads them (k_vox.cu):
+// -log2(e)/ein^3, -log2(e)/KN(ein), 2 Esrc/hbarc and c2 of sigma^2 = c1 s^2 +
+// c2 sg/s^2, each as a float pair.
+struct alignas(16) VoxEnergy {
+    float f1, f1l, f2, f2l;
+    float wh, wl, c2, c2l;
+};
+// Cells of the operator's window table over the q grid, besides one below and
+// one above it: per cell the first coarse bin whose centre lies above the
+// cell's left end and (<< 16) the last one below its right end.
+constexpr int kLutCells = 512;
+
 std::string fmt(const char *f, ...);
 
 // Per-call tables of the factored kernels, built on the host in double.
@@ -90,6 +102,9 @@ struct HostTables {
     int sl = 1;
     std::vector<float> offs_e;      // [nrg_src][sl + 2]
     std::vector<FwdEnergy> fwd_energy;   // [nrg_src]
+    std::vector<VoxEnergy> vox_energy;   // [nrg_src]
+    std::vector<unsigned> qlut;          // [kLutCells + 2]
+    float lut_scale = 0.f;          // cells per wavevector unit
     std::vector<float2> fine_q;     // [nqf]
     std::vector<float4> coarse_q;   // [nwt]
 };
@@ -253,7 +268,13 @@ struct VoxOp {
     const float4 *cells;
     const float2 *atten_src;
     const float2 *walk;        // [n_src * n_det][nv] detector-side integrals, or NULL
+    const VoxEnergy *vox_energy;   // [nrg_src]
+    const unsigned *qlut;      // [kLutCells + 2] window table
+    float lut_scale;
+    float c1, c1l;             // sigma^2 of the source bin width over s^2, as a pair
 };
+// The voxel list in tiles of 8 x 4 voxels, B.vox_xy; B.vox_mat, B.vox_order
+// and B.vox_rank are scratch.
 cudaError_t launch_compact_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
                                   int64_t *launches);
 
@@ -266,11 +287,14 @@ struct VoxJob {
     int groups;                // adjoint pair groups (rows of part)
     int ppg;                   // pairs per group
     int chunk_blocks;          // adjoint blocks along the voxel chunks
-    float *xd, *xc;            // [nv][nwt] unknowns times dq, unknowns
+    float *xd;                 // unknowns times dq, [(nwt + 1)/2][xd_stride][2], 0 past the last voxel and bin
+    float *xc;                 // [nv][nwt] unknowns
+    int64_t xd_stride;         // nv rounded up to whole steps of 32 voxels
     float *y;                  // [rays] forward output
     const float *ymeas, *cbg;  // [rays] MLEM counts and background
     float *what;               // [pairs][E] per-energy weights
-    float2 *part;              // [groups][nv][nwt] adjoint partial sums, each as a float pair
+    float4 *part;              // [groups][chunks of 32 voxels][(nwt + 1)/2][32] adjoint partial sums of two
+                               // bins, each as a float pair (both high parts first), without dq
     double *sens;              // [nv][nwt] sensitivity
     float *g;                  // [nx*ny*nwt] adjoint output
     const float *w;            // [rays] adjoint weights
@@ -280,12 +304,13 @@ struct VoxJob {
     // or one tile); op.walk holds their detector-side integrals from row 0
     int64_t pair0, pair1;
     int accumulate;            // adjoint: add to the partial rows instead of writing them
-    int pad;
+    int steps, tiles, runs;    // the forward's tiles and runs (vox_fwd_split)
 };
-// Kernel argument of the batched operator kernels.  off holds five prefix
+// Kernel argument of the batched operator kernels.  off holds six prefix
 // sums over the n jobs, each of n + 1 entries: 0 forward items (pairs),
 // 1 adjoint items (chunk blocks x groups), 2 unknowns (nv*nwt), 3 full-grid
-// entries (nx*ny*nwt), 4 per-energy weights (pairs*E).
+// entries (nx*ny*nwt), 4 per-energy weights (pairs*E), 5 entries of a partial row.
+// (A tile's hold rows 0 and 1.)
 struct VoxBatch {
     const VoxJob *jobs;
     const int64_t *off;
@@ -297,7 +322,9 @@ struct VoxBatch {
 cudaError_t vox_set_attributes(int max_smem);
 size_t vox_fwd_static_smem();
 size_t vox_adj_static_smem();
-size_t vox_fwd_smem(const DevProblem &P);
+size_t vox_limit_smem(const DevProblem &P);
+// The forward's tiles for a problem; returns its shared memory.
+size_t vox_fwd_split(const DevProblem &P, int nv, int *steps, int *tiles, int *runs);
 size_t vox_adj_smem(const DevProblem &P, int warps);
 int vox_fwd_blocks_per_sm(size_t smem);
 int vox_adj_blocks_per_sm(int warps, size_t smem);
@@ -309,6 +336,9 @@ cudaError_t launch_vox_adjoint(const VoxBatch &B, int grid, size_t smem, cudaStr
 cudaError_t launch_vox_wtab(const VoxBatch &B, int64_t total, int mode, cudaStream_t s, int64_t *launches);
 cudaError_t launch_vox_reduce(const VoxBatch &B, int64_t total, int mode, cudaStream_t s, int64_t *launches);
 cudaError_t launch_vox_gather(const VoxBatch &B, int64_t total, bool with_xc, cudaStream_t s, int64_t *launches);
+// rows [nv][K] of x dq into the layout of VoxJob::xd
+cudaError_t launch_vox_pack(const float *rows, int64_t nv, int K, int64_t stride, float *xd, cudaStream_t s,
+                            int64_t *launches);
 cudaError_t launch_vox_scatter(const VoxBatch &B, int64_t total, cudaStream_t s, int64_t *launches);
 
 } // namespace xrdt
