@@ -179,3 +179,20 @@ def test_window_table_takes_any_order_of_bins(ctx, oracle_lib):
     assert max_rel_err(op.forward(x), y_ref) < FAST_RTOL
     assert max_rel_err(op.adjoint(w), g_ref.reshape(-1)) < FAST_RTOL
     op.close()
+
+
+# CT chords: fewer than a warp, remainders, chords along the grid (views at
+# multiples of 90 degrees), chords that miss the phantom, source bins in one
+# pass, in several, and windows wider than a pass holds
+@pytest.mark.parametrize("nx,ny,views,px,es,ed,dnrg", [(5, 4, 1, 3, 1, 1, 0), (33, 20, 4, 41, 12, 12, 2),
+                                                       (70, 64, 9, 150, 64, 48, 5), (20, 24, 5, 33, 300, 290, 4),
+                                                       (12, 12, 3, 7, 3401, 3, 1700)])
+def test_ct_over_passes(ctx, oracle_lib, nx, ny, views, px, es, ed, dnrg):
+    p = sized_problem(nx, ny, views, px, es, ed, dnrg)
+    p.col_pitch *= 1.6
+    inp = synth.make_inputs(p, 600 + nx)
+    T, G = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=ctx)
+    rays = some_rays(p, 500, nx)
+    Tr, Gr = oracle_lib.ct_rays(inp, rays)
+    assert max_rel_err(T[rays], Tr) < FAST_RTOL
+    assert max_rel_err(G[rays], Gr) < 1e-5

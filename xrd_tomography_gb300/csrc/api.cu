@@ -1177,11 +1177,12 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
     for (int s = 0; s < p->n_src; s++) src_geom(p, s, &hsg[s]);
     void *d_srcg, *d_energy, *d_rf, *d_wlo;
     if ((rc = get_buf(ctx, S_SRCG, sizeof(SrcGeom) * p->n_src, &d_srcg))) return rc;
-    if ((rc = get_buf(ctx, S_ENERGY, sizeof(EnergyRow) * ht.energy.size(), &d_energy))) return rc;
+    if ((rc = get_buf(ctx, S_FWDEN, sizeof(FwdEnergy) * ht.fwd_energy.size(), &d_energy))) return rc;
     if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * ht.rf_win.size(), &d_rf))) return rc;
     if ((rc = get_buf(ctx, S_WINLO, sizeof(int) * ht.win_lo.size(), &d_wlo))) return rc;
     CK(cudaMemcpyAsync(d_srcg, hsg.data(), sizeof(SrcGeom) * p->n_src, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_energy, ht.energy.data(), sizeof(EnergyRow) * ht.energy.size(), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_energy, ht.fwd_energy.data(), sizeof(FwdEnergy) * ht.fwd_energy.size(), cudaMemcpyHostToDevice,
+                       st));
     CK(cudaMemcpyAsync(d_rf, ht.rf_win.data(), sizeof(float) * ht.rf_win.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_wlo, ht.win_lo.data(), sizeof(int) * ht.win_lo.size(), cudaMemcpyHostToDevice, st));
     PrepBuffers B;
@@ -1194,7 +1195,7 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
     }
     {
         ProfScope ps(ctx, XRDT_KERNEL_CT);
-        CK(launch_ct_sinogram(P, (const SrcGeom *)d_srcg, B.cells, (const EnergyRow *)d_energy, (const float *)d_rf,
+        CK(launch_ct_sinogram(P, (const SrcGeom *)d_srcg, B.cells, (const FwdEnergy *)d_energy, (const float *)d_rf,
                               (const int *)d_wlo, dT, dG, st, &ctx->launches));
     }
     if (hostT) CK(cudaMemcpyAsync(Tphotons, dT, sizeof(float) * rays, cudaMemcpyDeviceToHost, st));

@@ -18,18 +18,32 @@
 //
 // with the energy window and spectrum weights of find_src_nrg_range.cu and
 // the attenuation model of integrate_diffraction.cu:291-296.  Outputs use the
-// Nphotons layout, index src + det*SRC + nrg*SRC*DET.  One warp per
-// (source, pixel): the chord is walked cooperatively, then lane = energy
-// channel forms the two sums.
+// Nphotons layout, index src + det*SRC + nrg*SRC*DET.
+//
+// Lane = chord, 32 consecutive output columns per warp: the stores of every
+// detector bin are whole rows, at the cost of chords of different views side by
+// side in the walk.  The chord's entry point and sample count are decided in
+// float pairs, near a threshold in FP64 (which issues at 1/64 of the FP32 rate:
+// all chords in FP64 took 16 us more), the chord is walked cell by cell
+// (walk_cells), then the transmission of every source bin is formed once per
+// chord -- each detector bin's window holds 2 DNRG + 1 of them -- and the windows
+// are summed out of shared memory.  256x256 voxels, 180 views x
+// 512 px, 64 energies: 82 us; with a warp per chord, one sample per lane, the set-up
+// in FP64 by all 32 lanes alike and every window's exponentials on their own
+// 660 us, and its line integrals were off by 1e-6 (positions in FP32).
+#include <algorithm>
+
 #include "scatter.cuh"
 
 namespace xrdt {
 
 namespace {
 
-// Slab clipping of (sx,sy) -> (dx,dy) against [0,NX] x [0,NY].  Returns the
-// walk of the clipped chord (n = 0 when the segment misses the region).
-__device__ void chord_setup(const DevProblem &P, double sx, double sy, double dx, double dy, WalkSetup *w)
+// Slab clipping of (sx,sy) -> (dx,dy) against [0,NX] x [0,NY]: the walk of the
+// clipped chord, anchored at its entry point r (n = 0 when the segment misses
+// the region).
+__device__ void chord_setup(const DevProblem &P, double sx, double sy, double dx, double dy, WalkSetup *w, double *rx,
+                            double *ry)
 {
     const double ex = dsub(dx, sx), ey = dsub(dy, sy);
     double t0 = 0.0, t1 = 1.0;
@@ -50,66 +64,210 @@ __device__ void chord_setup(const DevProblem &P, double sx, double sy, double dx
         if (tb < t1) t1 = tb;
     }
     w->n = 0;
-    w->rx = w->ry = w->Lx = w->Ly = 0.f;
+    w->dlt = w->ux = w->uy = ff{0.f, 0.f};
+    *rx = *ry = 0.0;
     if (!(t1 > t0)) return;
     const double len = sqrt(dadd(dmul(ex, ex), dmul(ey, ey)));
-    const double rx = dadd(sx, dmul(t0, ex)), ry = dadd(sy, dmul(t0, ey));
+    *rx = dadd(sx, dmul(t0, ex));
+    *ry = dadd(sy, dmul(t0, ey));
     const double L = dmul(dsub(t1, t0), len);
     long long k = (long long)floor(L / P.DQ);
     while (dmul(P.DQ, (double)(k + 1)) <= L) k++;
     while (k >= 0 && !(dmul(P.DQ, (double)k) <= L)) k--;
     long long n = k + 1;
     if (n > P.kmax) n = P.kmax;
-    w->rx = (float)(rx - 1.0);
-    w->ry = (float)(ry - 1.0);
-    w->Lx = (float)(ex / len * P.DQ);
-    w->Ly = (float)(ey / len * P.DQ);
+    const double inv = 1.0 / len;
     w->n = (int)n;
+    w->ux = ff_from_double(ex * inv);
+    w->uy = ff_from_double(ey * inv);
 }
 
-__global__ void __launch_bounds__(256)
-k_ct_sinogram(DevProblem P, const SrcGeom *__restrict__ sg, const float4 *__restrict__ cells,
-              const EnergyRow *__restrict__ energy, const float *__restrict__ rf_win, const int *__restrict__ win_lo,
-              float *__restrict__ T, float *__restrict__ G0)
+// The same in float pairs (about 2^-44 of the lengths): false within 1e-9 of
+// a threshold, 1e-8 of a step for the sample count, and for rays along an axis.
+__device__ __forceinline__ bool chord_setup_pairs(const DevProblem &P, const F32Consts &C, ff sx, ff sy, ff dx, ff dy,
+                                                  WalkSetup *w, ff *rx, ff *ry)
 {
-    const int lane = threadIdx.x & 31;
+    const ff ex = ff_sub(dx, sx), ey = ff_sub(dy, sy);
+    if (!(fabsf(ex.hi) > 1e-3f && fabsf(ey.hi) > 1e-3f)) return false;
+    const ff ix = ff_rcp(ex), iy = ff_rcp(ey);
+    // entry and exit of both slabs
+    const ff x0 = ff_neg(ff_mul(sx, ix)), x1 = ff_mul(ff_fsub(C.nxf, sx), ix);
+    const ff y0 = ff_neg(ff_mul(sy, iy)), y1 = ff_mul(ff_fsub(C.nyf, sy), iy);
+    const ff tx0 = ex.hi > 0.f ? x0 : x1, tx1 = ex.hi > 0.f ? x1 : x0;
+    const ff ty0 = ey.hi > 0.f ? y0 : y1, ty1 = ey.hi > 0.f ? y1 : y0;
+    auto less = [](ff a, ff b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); };
+    ff t0 = {0.f, 0.f}, t1 = {1.f, 0.f};
+    if (less(t0, tx0)) t0 = tx0;
+    if (less(t0, ty0)) t0 = ty0;
+    if (less(tx1, t1)) t1 = tx1;
+    if (less(ty1, t1)) t1 = ty1;
+    const ff dt = ff_sub(t1, t0);
+    if (!(fabsf(dt.hi) > 1e-9f)) return false;
+    w->n = 0;
+    w->dlt = w->ux = w->uy = ff{0.f, 0.f};
+    *rx = *ry = ff{0.f, 0.f};
+    if (dt.hi < 0.f) return true;
+    const ff len = ff_sqrt(ff_dot2(ex, ex, ey, ey));
+    const ff t = ff_div(ff_mul(dt, len), ff{C.DQ, C.DQ_lo});
+    if (!(t.hi < 4194304.f)) return false;
+    float ft = floorf(t.hi);
+    float fr = (t.hi - ft) + t.lo;
+    if (fr < 0.f) {
+        ft -= 1.f;
+        fr = (t.hi - ft) + t.lo;
+    }
+    const float gt = fmaf(1e-12f, len.hi * C.inv_DQ, 1e-8f);
+    if (!(fr > gt && fr < 1.f - fmaxf(gt, 1e-7f))) return false;
+    long long n = (long long)ft + 1;
+    if (n > P.kmax) n = P.kmax;
+    const ff il = ff_rcp(len);
+    w->n = (int)n;
+    w->ux = ff_mul(ex, il);
+    w->uy = ff_mul(ey, il);
+    *rx = ff_add(sx, ff_mul(t0, ex));
+    *ry = ff_add(sy, ff_mul(t0, ey));
+    return true;
+}
+
+// FP64 out of line, for the chords that the pairs leave open.
+__device__ __noinline__ void chord_setup_f64(const DevProblem &P, const SrcGeom *g, int det, WalkSetup *w, ff *rx,
+                                             ff *ry)
+{
+    double Rdx, Rdy, Rdz, x, y;
+    det_position(P, g->sphi, g->cphi, det, &Rdx, &Rdy, &Rdz);
+    chord_setup(P, g->Rsrc_x, g->Rsrc_y, Rdx, Rdy, w, &x, &y);
+    *rx = ff_from_double(x);
+    *ry = ff_from_double(y);
+}
+
+constexpr int kCtWarps = 4;
+
+// A detector's position per column pitch and a source's trigonometry as pairs.
+struct CtConsts {
+    ff cx, cy, r_det, pitch;
+    int n_col;
+};
+
+// Shared memory: per warp the transmission of a pass's source bins
+// [e_pass][32], then (STAGED) the spectrum windows [nrg_det][W] and their sums.
+// Windows too wide for that (!STAGED) are read through L1, and every bin forms
+// its own transmissions.
+template <bool STAGED>
+__global__ void __launch_bounds__(32 * kCtWarps)
+k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__ sg, const float4 *__restrict__ cells,
+              const FwdEnergy *__restrict__ energy, const float *__restrict__ rf_win, const int *__restrict__ win_lo,
+              float *__restrict__ T, float *__restrict__ G0, int e_pass)
+{
+    extern __shared__ float att_s[];
+    const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    float *att = att_s + (size_t)(threadIdx.x >> 5) * 32 * e_pass + lane;   // [e_pass][32], this lane's column
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
     const int W = 2 * P.dnrg + 1;
-    const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t p = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); p < npairs; p += wstride) {
+    const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
+    const int64_t wstride = 32 * (int64_t)gridDim.x * nwarps;
+    float *rf_s = att_s + (size_t)nwarps * 32 * e_pass, *g0_s = rf_s + P.nrg_det * W;
+    if (STAGED) {
+        for (int i = threadIdx.x; i < P.nrg_det * W; i += blockDim.x) rf_s[i] = rf_win[i];
+        for (int n = threadIdx.x; n < P.nrg_det; n += blockDim.x) {
+            float g0 = 0.f;
+            for (int j = 0; j < W; j++) g0 += rf_win[n * W + j];
+            g0_s[n] = g0;
+        }
+        __syncthreads();
+    }
+    for (int64_t p0 = 32 * (blockIdx.x * (int64_t)nwarps + (threadIdx.x >> 5)); p0 < npairs; p0 += wstride) {
+        const int64_t p = min(p0 + lane, npairs - 1);   // a lane past the last chord repeats it
+        const bool mine = p0 + lane < npairs;
         const int src = (int)(p % P.n_src), det = (int)(p / P.n_src);
-        const SrcGeom g = sg[src];
-        double Rdx, Rdy, Rdz;
-        det_position(P, g.sphi, g.cphi, det, &Rdx, &Rdy, &Rdz);
+        const SrcGeom *g = sg + src;
+        // det_position in pairs: the column's offset is a multiple of 1/2
+        const ff sphi = ff_from_double(g->sphi), cphi = ff_from_double(g->cphi);
+        const ff rdet = ff_mulf(q.pitch, (float)(det % q.n_col) - 0.5f * (float)q.n_col + 0.5f);
+        const ff dx = ff_add(ff_sub(q.cx, ff_mul(q.r_det, sphi)), ff_mul(rdet, cphi));
+        const ff dy = ff_add(ff_add(q.cy, ff_mul(q.r_det, cphi)), ff_mul(rdet, sphi));
         WalkSetup ws;
-        chord_setup(P, g.Rsrc_x, g.Rsrc_y, Rdx, Rdy, &ws);
-        const float2 A = walk_coop(cells, P.nx, P.ny, ws, (float)P.DQ, lane);
-        for (int n = lane; n < P.nrg_det; n += 32) {
-            const int lo = win_lo[n];
-            float t = 0.f, g0 = 0.f;
-            for (int j = 0; j < W; j++) {
-                const EnergyRow r = energy[lo + j];
-                const float rf = rf_win[n * W + j];
-                t = fmaf(rf, expf(-fmaf(A.x, r.inv_f1, A.y * r.inv_f2)), t);
-                g0 += rf;
+        ff ax, ay;
+        if (!chord_setup_pairs(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), dx, dy, &ws, &ax, &ay))
+            chord_setup_f64(P, g, det, &ws, &ax, &ay);
+        const float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
+                                          make_float2(ax.lo, ay.lo));
+        auto transmission = [&](int e) {   // -log2(e)/f1, -log2(e)/f2 as pairs
+            const float4 f = __ldg(reinterpret_cast<const float4 *>(energy + e));
+            return ex2_approx(fmaf(A.x, f.x, fmaf(A.y, f.z, fmaf(A.x, f.y, A.y * f.w))));
+        };
+        auto store = [&](int n, float t, float g0) {
+            if (mine) {
+                const int64_t ray = p + (int64_t)n * npairs;
+                T[ray] = t;
+                G0[ray] = g0;
             }
-            const int64_t ray = p + (int64_t)n * npairs;
-            T[ray] = t;
-            G0[ray] = g0;
+        };
+        if (STAGED) {
+            // per pass the bins whose windows lie in its source bins (win_lo rises with n)
+            for (int n = 0; n < P.nrg_det;) {
+                const int e0 = __ldg(win_lo + n);
+                const int ne = min(e_pass, P.nrg_src - e0);
+#pragma unroll 4
+                for (int e = 0; e < ne; e++) att[32 * e] = transmission(e0 + e);
+                for (; n < P.nrg_det; n++) {
+                    const int lo = __ldg(win_lo + n) - e0;
+                    if (lo + W > ne) break;
+                    const float *a = att + 32 * lo, *rf = rf_s + n * W;
+                    float t = 0.f;
+#pragma unroll 4
+                    for (int j = 0; j < W; j++) t = fmaf(rf[j], a[32 * j], t);
+                    store(n, t, g0_s[n]);
+                }
+            }
+        } else {
+            for (int n = 0; n < P.nrg_det; n++) {
+                float t = 0.f, g0 = 0.f;
+                for (int j = 0; j < W; j++) {
+                    const float rf = __ldg(rf_win + n * W + j);
+                    t = fmaf(rf, transmission(__ldg(win_lo + n) + j), t);
+                    g0 += rf;
+                }
+                store(n, t, g0);
+            }
         }
     }
 }
 
 } // namespace
 
-cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const float4 *cells, const EnergyRow *energy,
+cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const float4 *cells, const FwdEnergy *energy,
                                const float *rf_win, const int *win_lo, float *T, float *G0, cudaStream_t s,
                                int64_t *launches)
 {
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
-    int64_t blocks = (npairs + 7) / 8;
+    const int W = 2 * P.dnrg + 1;
+    // the source bins of a pass: all that the windows reach, or as many as one
+    // warp's columns have room for beside the windows, one window at least
+    const int E = P.e_hi - P.e_lo + 1;
+    const size_t tables = sizeof(float) * ((size_t)P.nrg_det * W + P.nrg_det);
+    int warps = kCtWarps;
+    int64_t e_pass = E;
+    size_t smem = 128 * (size_t)warps * E + tables;
+    if (smem > 56 * 1024) {   // four blocks per SM
+        warps = 1;
+        e_pass = tables < 200 * 1024 ? std::min<int64_t>(E, (int64_t)(200 * 1024 - tables) / 128) : 0;
+        smem = 128 * (size_t)e_pass + tables;
+    }
+    const bool staged = e_pass >= W;
+    if (!staged) {
+        warps = kCtWarps;
+        e_pass = 0;
+        smem = 0;
+    }
+    auto *kernel = staged ? k_ct_sinogram<true> : k_ct_sinogram<false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int64_t blocks = (npairs + 32 * warps - 1) / (32 * warps);
     if (blocks > 64LL * current_sm_count()) blocks = 64LL * current_sm_count();
-    k_ct_sinogram<<<(int)blocks, 256, 0, s>>>(P, sg, cells, energy, rf_win, win_lo, T, G0);
+    const CtConsts q = {ff_from_double(P.cx), ff_from_double(P.cy), ff_from_double(P.r_det), ff_from_double(P.col_pitch),
+                        P.n_col};
+    kernel<<<(int)blocks, 32 * warps, smem, s>>>(P, make_f32_consts(P), q, sg, cells, energy, rf_win, win_lo, T, G0,
+                                                 (int)e_pass);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

@@ -2,12 +2,11 @@
 // bilinear cell map.
 //
 // The integer decisions (which ROI edge is entered, how many samples the ray
-// takes) are those of the reference, made in FP32 with guard bands
-// (walk_setup_f32) or in FP64 (walk_setup).  Two ways to sum the samples:
-// walk_cells, one lane per ray, cell by cell with closed-form sums over the
-// samples inside each cell, anchored at the voxel with float-pair offsets
-// (the projector's and the operators' walks); and walk_coop, the 32 lanes of
-// a warp on one ray, lane l taking samples l, l+32, ... (the CT sinogram).
+// takes) are those of the reference, made in FP32 with guard bands, then in
+// float pairs, then in FP64 (walk_decide).  walk_cells sums the samples, one
+// lane per ray, cell by cell with closed-form sums over the samples inside
+// each cell, with float-pair offsets from an anchor: the voxel for the
+// projector's and the operators' walks, the entry point for the CT chords.
 #pragma once
 
 #include "xrdt_device.cuh"
@@ -233,63 +232,19 @@ __device__ __forceinline__ void walk_decide(const DevProblem &P, const F32Consts
     else walk_setup_f64(P, *exd, *eyd, (double)vx, (double)vy, w);
 }
 
-// One bilinear sample of the cell map at texture coordinates (X+1, Y+1),
-// P = (X, Y).  Cell (ci, cj) holds the coefficients of the texels
-// (ci-1..ci, cj-1..cj) of the zero-bordered map in the frame of the cell
-// centre: f = d00 + d10 u + d01 v + d11 u v with u = X - round(X) and
-// v = Y - round(Y) in [-0.5, 0.5] (k_prep.cu).  The interpolant is
-// continuous, so any base cell whose square holds the point gives the same
-// value, and rounding through the float mantissa (adding 1.5 * 2^23) needs
-// no conversion instruction.  Valid for |X| < 2^22; the cell index is
-// clamped for memory safety.  Both components are evaluated with packed
-// FP32 instructions (two lanes of one register pair: a1 and a2).
-__device__ __forceinline__ float2 cell_sample(const float4 *__restrict__ cells, int nx, unsigned ncell_m1, float2 P)
-{
-    const float2 t = __fadd2_rn(P, make_float2(12582912.f, 12582912.f));
-    const int ix = __float_as_int(t.x) - 0x4B400000, iy = __float_as_int(t.y) - 0x4B400000;
-    const float2 r = __fadd2_rn(t, make_float2(-12582912.f, -12582912.f));   // round(P), exact
-    const float2 d = __ffma2_rn(r, make_float2(-1.f, -1.f), P);               // P - round(P), exact
-    const unsigned c = min((unsigned)(ix + 1 + (iy + 1) * (nx + 1)), ncell_m1);
-    const float4 c0 = __ldg(cells + 2 * c), c1 = __ldg(cells + 2 * c + 1);
-    const float2 lo = __ffma2_rn(make_float2(d.y, d.y), make_float2(c1.x, c1.y), make_float2(c0.x, c0.y));
-    const float2 hi = __ffma2_rn(make_float2(d.y, d.y), make_float2(c1.z, c1.w), make_float2(c0.z, c0.w));
-    return __ffma2_rn(make_float2(d.x, d.x), hi, lo);
-}
-
-// Sum of the n samples times DQ; every lane returns the total.  Lane l takes
-// samples l, l+32, l+64, ... two per iteration; the sample index is carried
-// as a float (no int-to-float conversion per sample) and the sample point
-// r + k L is formed for x and y in one packed FMA.
-__device__ __forceinline__ float2 walk_coop(const float4 *__restrict__ cells, int nx, int ny,
-                                            const WalkSetup &w, float DQ, int lane)
-{
-    const unsigned ncell_m1 = (unsigned)((nx + 1) * (ny + 1) - 1);
-    const float2 L2 = make_float2(w.Lx, w.Ly), R2 = make_float2(w.rx, w.ry);
-    float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
-    float kf = __int_as_float(0x4B000000 | lane) - 8388608.f;   // (float)lane
-    int k = lane;
-    for (; k + 32 < w.n; k += 64, kf += 64.f) {
-        const float2 a = cell_sample(cells, nx, ncell_m1, __ffma2_rn(L2, make_float2(kf, kf), R2));
-        const float kg = kf + 32.f;
-        const float2 b = cell_sample(cells, nx, ncell_m1, __ffma2_rn(L2, make_float2(kg, kg), R2));
-        sa = __fadd2_rn(sa, a);
-        sb = __fadd2_rn(sb, b);
-    }
-    if (k < w.n) sa = __fadd2_rn(sa, cell_sample(cells, nx, ncell_m1, __ffma2_rn(L2, make_float2(kf, kf), R2)));
-    const float s1 = warp_sum(sa.x + sb.x);
-    const float s2 = warp_sum(sa.y + sb.y);
-    return make_float2(s1 * DQ, s2 * DQ);
-}
-
-// The same sum walked cell by cell by one lane.  The bilinear patch of a
-// cell is a polynomial in the sample index, so the samples j = 0 .. m-1 of
+// Sum of the n samples times DQ, walked cell by cell by one lane.  Cell (ci,
+// cj) holds the coefficients of the texels (ci-1..ci, cj-1..cj) of the
+// zero-bordered map in the frame of the cell centre: f = c00 + c10 u + c01 v +
+// c11 u v with u = x - ci and v = y - cj in [-0.5, 0.5] (k_prep.cu).  The
+// bilinear patch of a cell is a polynomial in the sample index, so the samples j = 0 .. m-1 of
 // a run inside one cell add up in closed form: with (u0, v0) the first
 // sample's offset from the cell centre, S1 = m(m-1)/2 and
 // S2 = (m-1)m(2m-1)/6,
 //     sum u = m u0 + Lx S1,   sum v = m v0 + Ly S1,
 //     sum uv = m u0 v0 + (u0 Ly + v0 Lx) S1 + Lx Ly S2,
 //     sum f = m c00 + c10 sum u + c01 sum v + c11 sum uv.
-// Each step takes the cell of its first sample (as cell_sample does) and
+// Each step takes the cell of its first sample (the nearest centre: rounding
+// through the float mantissa, valid for |x| < 2^22) and
 // the run up to the first sample beyond the cell's exit edge, at least one
 // sample.  A sample within rounding of an edge may fall on either side; the
 // interpolant is continuous there, so the sum changes only by rounding.  The
@@ -325,8 +280,11 @@ __device__ __forceinline__ void ld_cell256(const float4 *p, float4 &c0, float4 &
 constexpr int kReach = 31;
 constexpr float kReachUnit = 0x1p-125f, kReachScale = 0x1p125f, kReachLimit = 0x1p-115f;
 
+// LOW: the anchor is the pair (v, vlow), not an exact float.
+template <bool LOW = false>
 __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, int sx, int sy, unsigned ncell_m1,
-                                             const WalkSetup &w, float vx, float vy, float DQ)
+                                             const WalkSetup &w, float vx, float vy, float DQ,
+                                             float2 vlow = make_float2(0.f, 0.f))
 {
     const float magic = 12582912.f;
     const float nf = (float)w.n;
@@ -365,8 +323,9 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
         }
         const float2 s2 = make_float2(sh, sh);
         const float2 p = __fmul2_rn(s2, uhi);
-        const float2 e = __fadd2_rn(__ffma2_rn(s2, uhi, make_float2(-p.x, -p.y)),
-                                    __ffma2_rn(s2, ulo, __fmul2_rn(make_float2(sl, sl), uhi)));
+        float2 e = __fadd2_rn(__ffma2_rn(s2, uhi, make_float2(-p.x, -p.y)),
+                              __ffma2_rn(s2, ulo, __fmul2_rn(make_float2(sl, sl), uhi)));
+        if (LOW) e = __fadd2_rn(e, vlow);
         // the cell whose centre is nearest (any cell holding the point gives
         // the same value: the interpolant is continuous), then the offset
         const float2 t = __fadd2_rn(__fadd2_rn(v2, p), make_float2(magic, magic));
