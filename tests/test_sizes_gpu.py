@@ -196,3 +196,23 @@ def test_ct_over_passes(ctx, oracle_lib, nx, ny, views, px, es, ed, dnrg):
     Tr, Gr = oracle_lib.ct_rays(inp, rays)
     assert max_rel_err(T[rays], Tr) < FAST_RTOL
     assert max_rel_err(G[rays], Gr) < 1e-5
+
+
+@pytest.mark.parametrize("N", [16, 48, 64, 80, 192, 256])
+@pytest.mark.parametrize("M,K,off", [(1, 8, 0), (127, 24, 0), (145, 64, 1), (152 * 128 + 17, 40, 0), (40000, 64, 1),
+                                     (60000, 16, 0)])
+def test_basis_read_back(ctx, M, K, N, off):
+    """Column blocks of 64 and 16 of the accumulator's read-back, ragged last
+    tiles, several tiles per block, C and I off a 16-byte boundary.  The bound
+    is that of the basis tests: each product to about 2^-21, the sum in FP32."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    C = torch.randn(M * K + off, device="cuda", generator=g)[off:].view(M, K)
+    B = torch.randn(K, N, device="cuda", generator=g)
+    I = torch.full((M * N + off + 8,), -7.0, device="cuda")
+    torch.cuda.synchronize()
+    xt.basis_expand(C, B, I[off:off + M * N].view(M, N), ctx=ctx)
+    got = I[off:off + M * N].view(M, N).double()
+    bound = C.double().abs() @ B.double().abs()
+    assert bool(((got - C.double() @ B.double()).abs() <= 4e-6 * bound + 1e-30).all())
+    assert bool((I[:off] == -7.0).all()) and bool((I[off + M * N:] == -7.0).all())

@@ -9,15 +9,15 @@
 // bytes per row for 6KN flops, so it is bound by HBM, not by the tensor
 // rate; the kernel is built to keep HBM busy:
 //
-//  * persistent CTAs (4 warps) loop over 128-row tiles of C; the basis is
+//  * persistent CTAs (8 warps) loop over 128-row tiles of C; the basis is
 //    split and staged in shared memory once per CTA, in the canonical
 //    K-major layout without swizzle (core matrices of 8 rows x 16 bytes);
 //  * FP32 accuracy from TF32 inputs: x = hi + lo with hi, lo rounded to TF32,
 //    and D = A_hi B_hi + A_hi B_lo + A_lo B_hi accumulated in FP32 in tensor
 //    memory (the dropped A_lo B_lo term is below 2^-22 of the product);
 //  * two accumulators in tensor memory: while the MMAs of tile g run, the
-//    four warps read tile g-1's accumulator back (tcgen05.ld) and store its
-//    rows;
+//    warps read tile g-1's accumulator back (tcgen05.ld, 16 rows x 64 columns
+//    at a time, in the shape that lets a store write whole sectors);
 //  * the tiles of C arrive ahead of use: through the bulk-copy engine into a
 //    ring of shared-memory stages (one cp.async.bulk per tile, completing on
 //    the stage's mbarrier) when C is 16-byte aligned and two stages fit,
@@ -26,6 +26,14 @@
 //    stores of the split free of bank conflicts;
 //  * one thread issues the MMAs (K = 8 each) and commits each tile's to the
 //    mbarrier of its accumulator.
+//
+// What is left between this and HBM is the sequence of a tile (its rows land,
+// are split, the MMAs run, the accumulator is read back) with one CTA on an SM
+// where the basis fills shared memory.  147456 x 64 x 256: 54 us (3.5 TB/s)
+// where four warps with a row per lane -- 32 lines per store -- took 105;
+// 400000 x 64 x 64: 83 against 123; 1245184 x 32 x 32: 104 against 125.  Rows
+// through shared memory and whole-line stores: 67, 109 and 135; 16 warps: 53,
+// 94 and 125 (fewer CTAs per SM where K and N are small).
 //
 // Every mbarrier wait is bounded: on time-out the kernel raises an error
 // flag, stops taking tiles, waits (again bounded) for the MMAs it committed
@@ -38,7 +46,8 @@ namespace xrdt {
 namespace {
 
 constexpr int kTileM = 128;
-constexpr int kBasisThreads = 128;
+constexpr int kBasisThreads = 256;
+constexpr int kBasisWarps = kBasisThreads / 32;
 constexpr int kMaxK = 64;
 constexpr unsigned kSpinLimit = 1u << 26;
 
@@ -96,22 +105,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 }
 
 // The row chunks of one tile that a thread loads: warp instruction j of warp
-// w covers rows 8 rg .. 8 rg + 7 (lane % 8) and the 16-byte columns
-// 4 cg .. 4 cg + 3 (lane / 8), with (rg, cg) = item j*4 + w of
-// 16 row groups x ceil(K/16) column groups.
+// w covers rows 8 rg .. 8 rg + 7 (lane % 8) of the row group rg = 8 (j / 4) + w
+// and the 16-byte columns 4 cg .. 4 cg + 3 (lane / 8), cg = j % 4.
+constexpr int kChunks = (16 / kBasisWarps) * 4;   // of a thread, at K = 64
 struct ChunkPos {
     int r, c4;
     bool ok;
 };
 __device__ __forceinline__ ChunkPos chunk_pos(int j, int wid, int lane, int K)
 {
-    const int ncg = (K + 15) >> 4;
-    const int item = j * 4 + wid;
-    const int rg = item / ncg, cg = item - rg * ncg;
     ChunkPos p;
-    p.r = rg * 8 + (lane & 7);
-    p.c4 = cg * 4 + (lane >> 3);
-    p.ok = rg < 16 && p.c4 < (K >> 2);
+    p.r = ((j >> 2) * kBasisWarps + wid) * 8 + (lane & 7);
+    p.c4 = (j & 3) * 4 + (lane >> 3);
+    p.ok = p.c4 < (K >> 2);
     return p;
 }
 
@@ -124,7 +130,7 @@ __device__ __forceinline__ ChunkPos chunk_pos(int j, int wid, int lane, int K)
 template <bool BULK>
 __global__ void __launch_bounds__(kBasisThreads)
 k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__restrict__ B, int N,
-               float *__restrict__ I, unsigned *__restrict__ err, int aligned, int aligned_b, int test_timeout,
+               float *__restrict__ I, unsigned *__restrict__ err, int aligned, int test_timeout,
                int stages)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -140,8 +146,6 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(full + nst);
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const long long tiles = (M + kTileM - 1) / kTileM;
-    const int nitems = 16 * ((K + 15) >> 4);   // warp instructions per tile, all warps
-    const int per_warp = (nitems + 3) >> 2;
 
     uint32_t ncols = 32;   // accumulator columns: a power of two >= N, two accumulators
     while (ncols < (uint32_t)N) ncols <<= 1;
@@ -157,29 +161,23 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
         for (int st = 0; st < nst; st++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(full + st)));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
-    // the basis, split into TF32 pairs, once: B[k][n .. n+3] per load (N is
-    // a multiple of 16), four loads in flight per thread
-    {
-        const int n4 = N >> 2;
+    // the basis, split into TF32 pairs, once: four rows' elements of one column
+    // per thread, neighbouring threads on neighbouring columns, so that a warp
+    // stores whole core-matrix rows (with lanes along the row the 4-byte stores
+    // of a 64 x 256 basis conflicted 16 ways, 8 us before the first tile)
 #pragma unroll 4
-        for (int i = tid; i < n4 * K; i += kBasisThreads) {
-            const int k = i / n4, n = 4 * (i - k * n4);
-            const float *src = B + (size_t)k * N + n;
-            float x[4];
-            if (aligned_b) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(src));
-                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-            } else {
-                x[0] = __ldg(src); x[1] = __ldg(src + 1); x[2] = __ldg(src + 2); x[3] = __ldg(src + 3);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float hi = tf32_rna(x[q]), lo = tf32_rna(x[q] - hi);
-                const int o = kmajor_offset(n + q, k, K);
-                *reinterpret_cast<float *>(b_hi + o) = hi;
-                *reinterpret_cast<float *>(b_lo + o) = lo;
-            }
-        }
+    for (int i = tid; i < N * (K >> 2); i += kBasisThreads) {
+        const int k = 4 * (i / N), n = i - (k >> 2) * N;
+        const float *src = B + (size_t)k * N + n;
+        const float4 x = make_float4(__ldg(src), __ldg(src + N), __ldg(src + 2 * N), __ldg(src + 3 * N));
+        float4 h, l;
+        h.x = tf32_rna(x.x); l.x = tf32_rna(x.x - h.x);
+        h.y = tf32_rna(x.y); l.y = tf32_rna(x.y - h.y);
+        h.z = tf32_rna(x.z); l.z = tf32_rna(x.z - h.z);
+        h.w = tf32_rna(x.w); l.w = tf32_rna(x.w - h.w);
+        const int o = kmajor_offset(n, k, K);
+        *reinterpret_cast<float4 *>(b_hi + o) = h;
+        *reinterpret_cast<float4 *>(b_lo + o) = l;
     }
 
     // BULK: one thread copies tile t's rows (contiguous in C, 16-byte
@@ -203,8 +201,8 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
     auto split_stage = [&](int st) {
         const unsigned char *src = raw + (size_t)st * kTileM * rs;
 #pragma unroll
-        for (int j = 0; j < kMaxK / 4; j++) {
-            if (j < per_warp) {
+        for (int j = 0; j < kChunks; j++) {
+            {
                 const ChunkPos p = chunk_pos(j, wid, lane, K);
                 if (p.ok) {
                     const float4 x = *reinterpret_cast<const float4 *>(src + p.r * rs + 16 * p.c4);
@@ -222,13 +220,13 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
     };
 
     // this thread's chunks of a tile of C, loaded into registers ahead of use
-    float4 ra[BULK ? 1 : kMaxK / 4];
+    float4 ra[BULK ? 1 : kChunks];
     auto load_tile = [&](long long tile) {
         const long long m0 = tile * kTileM;
 #pragma unroll
-        for (int j = 0; j < (BULK ? 0 : kMaxK / 4); j++) {
+        for (int j = 0; j < (BULK ? 0 : kChunks); j++) {
             ra[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j < per_warp) {
+            {
                 const ChunkPos p = chunk_pos(j, wid, lane, K);
                 const long long row = m0 + p.r;
                 if (p.ok && row < M) {
@@ -245,8 +243,8 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
     // the registers, split, into the K-major A buffers
     auto store_tile = [&]() {
 #pragma unroll
-        for (int j = 0; j < (BULK ? 0 : kMaxK / 4); j++) {
-            if (j < per_warp) {
+        for (int j = 0; j < (BULK ? 0 : kChunks); j++) {
+            {
                 const ChunkPos p = chunk_pos(j, wid, lane, K);
                 if (p.ok) {
                     const float4 x = ra[j];
@@ -306,46 +304,51 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
     uint32_t full_phase = 0u;   // bit st: the next phase of stage st's barrier
     long long consumed = -1;    // the last tile index g whose stage has landed
 
-    // accumulator acc_i (tile ptile) back to HBM: warp w holds lanes
-    // 32w .. 32w+31 = rows of the tile; 32 columns per wait
+    // accumulator acc_i (tile ptile) back to HBM: warps w and w + 4 read lanes
+    // 32 (w % 4) .. + 31 = rows of the tile, 16 each.  In the 16x256b shape a
+    // lane holds two neighbouring columns of rows lane / 4 and lane / 4 + 8, so
+    // a store instruction writes whole 32-byte sectors of 8 rows.
     auto read_back = [&](int acc_i, long long ptile) {
-        const long long row = ptile * kTileM + wid * 32 + lane;
-        const uint32_t tbase = tmem + ((uint32_t)(wid * 32) << 16) + (uint32_t)acc_i * ncols;
-        for (int c = 0; c < N; c += 32) {
+        const int sub = (wid & 3) * 32 + (wid >> 2) * 16;   // the warp's first row of the tile
+        const uint32_t tbase = tmem + ((uint32_t)sub << 16) + (uint32_t)acc_i * ncols;
+        const long long row = ptile * kTileM + sub + (lane >> 2);
+        const bool in0 = row < M, in1 = row + 8 < M;
+        float *o0 = I + row * N + 2 * (lane & 3), *o1 = o0 + 8 * (long long)N;
+        auto put = [&](const uint32_t *v, int c) {   // 8 columns: two rows' pairs
+            if (aligned) {
+                if (in0) *reinterpret_cast<uint2 *>(o0 + c) = make_uint2(v[0], v[1]);
+                if (in1) *reinterpret_cast<uint2 *>(o1 + c) = make_uint2(v[2], v[3]);
+            } else {
+                if (in0) o0[c] = __uint_as_float(v[0]), o0[c + 1] = __uint_as_float(v[1]);
+                if (in1) o1[c] = __uint_as_float(v[2]), o1[c + 1] = __uint_as_float(v[3]);
+            }
+        };
+        int c = 0;
+        for (; c + 64 <= N; c += 64) {
             uint32_t v[32];
             asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                "%12, %13, %14, %15}, [%16];"
+                "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, "
+                "%31}, [%32];"
                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15])
+                  "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+                  "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+                  "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                 : "r"(tbase + (uint32_t)c));
-            const bool two = c + 16 < N;
-            if (two)
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                    "%12, %13, %14, %15}, [%16];"
-                    : "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-                      "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-                      "=r"(v[30]), "=r"(v[31])
-                    : "r"(tbase + (uint32_t)(c + 16)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-            if (row < M) {
-                float *o = I + row * N + c;
-                const int nq = two ? 8 : 4;
-                if (aligned) {
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        if (q < nq)
-                            reinterpret_cast<float4 *>(o)[q] =
-                                make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
-                                            __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 32; q++)
-                        if (q < 4 * nq) o[q] = __uint_as_float(v[q]);
-                }
-            }
+            for (int j = 0; j < 8; j++) put(v + 4 * j, c + 8 * j);
+        }
+        for (; c < N; c += 16) {
+            uint32_t v[8];
+            asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                           "=r"(v[7])
+                         : "r"(tbase + (uint32_t)c));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            put(v, c);
+            put(v + 4, c + 8);
         }
     };
 
@@ -439,7 +442,10 @@ k_basis_expand(const float *__restrict__ C, long long M, int K, const float *__r
 
 // Shared memory of the register path (the bound xrdt_basis_expand checks);
 // the bulk path adds its stages of padded rows and their barriers.
-size_t basis_smem(int K, int N) { return 2 * (size_t)kTileM * K * 4 + 2 * (size_t)N * K * 4 + 32; }
+size_t basis_smem(int K, int N)
+{
+    return 2 * (size_t)kTileM * K * 4 + 2 * (size_t)N * K * 4 + 32;
+}
 
 namespace {
 
@@ -450,7 +456,7 @@ size_t basis_smem_bulk(int K, int N, int stages)
 
 template <bool BULK>
 cudaError_t launch_basis_variant(const float *C, long long M, int K, const float *B, int N, float *I, unsigned *err,
-                                 cudaStream_t s, size_t smem, int stages, int aligned, int aligned_b, int sms,
+                                 cudaStream_t s, size_t smem, int stages, int aligned, int sms,
                                  int smem_sm, int optin)
 {
     cudaError_t e = cudaFuncSetAttribute(k_basis_expand<BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -468,13 +474,13 @@ cudaError_t launch_basis_variant(const float *C, long long M, int K, const float
     if (e != cudaSuccess) return e;
     // registers are allocated per warp in units of 256
     const int regs_warp = ((fa.numRegs * 32 + 255) / 256) * 256;
-    const int reg_ctas = regs_warp > 0 ? 65536 / (regs_warp * (kBasisThreads / 32)) : 16;
+    const int reg_ctas = regs_warp > 0 ? 65536 / (regs_warp * kBasisWarps) : 16;
     const size_t per_cta = smem + fa.sharedSizeBytes + 1024;   // 1 KB reserved per block
     const int smem_ctas = (int)((size_t)smem_sm / per_cta);
     int ctas = tmem_ctas;
     if (reg_ctas < ctas) ctas = reg_ctas;
     if (smem_ctas < ctas) ctas = smem_ctas;
-    if (ctas > 16) ctas = 16;
+    if (ctas > 2048 / kBasisThreads) ctas = 2048 / kBasisThreads;
     if (ctas < 1) return cudaErrorInvalidConfiguration;
     if (smem_ctas > tmem_ctas && reg_ctas > tmem_ctas) {
         const size_t padded = (size_t)smem_sm / (tmem_ctas + 1) + 1 - fa.sharedSizeBytes - 1024;
@@ -488,8 +494,8 @@ cudaError_t launch_basis_variant(const float *C, long long M, int K, const float
     // freed)
     const char *tt = getenv("XRDT_TEST_BASIS_TIMEOUT");
     const int test_timeout = (tt && tt[0] == '1') ? 1 : 0;
-    k_basis_expand<BULK><<<(unsigned)grid, kBasisThreads, smem, s>>>(C, M, K, B, N, I, err, aligned, aligned_b,
-                                                                       test_timeout, stages);
+    k_basis_expand<BULK><<<(unsigned)grid, kBasisThreads, smem, s>>>(C, M, K, B, N, I, err, aligned, test_timeout,
+                                                                       stages);
     return cudaGetLastError();
 }
 
@@ -507,7 +513,6 @@ cudaError_t launch_basis_expand(const float *C, long long M, int K, const float 
     if (e != cudaSuccess) return e;
     if (basis_smem(K, N) > (size_t)optin) return cudaErrorInvalidConfiguration;
     const int aligned = (((uintptr_t)C | (uintptr_t)I) & 15) == 0 ? 1 : 0;
-    const int aligned_b = ((uintptr_t)B & 15) == 0 ? 1 : 0;
     if (launches) (*launches)++;
     // the bulk-copy ring when C allows it: two or three stages, whichever
     // leaves more CTAs on an SM (the per-tile work is latency-bound, so CTAs
@@ -525,9 +530,9 @@ cudaError_t launch_basis_expand(const float *C, long long M, int K, const float 
         }
         if (best)
             return launch_basis_variant<true>(C, M, K, B, N, I, err, s, basis_smem_bulk(K, N, best), best, aligned,
-                                              aligned_b, sms, smem_sm, optin);
+                                              sms, smem_sm, optin);
     }
-    return launch_basis_variant<false>(C, M, K, B, N, I, err, s, basis_smem(K, N), 0, aligned, aligned_b, sms,
+    return launch_basis_variant<false>(C, M, K, B, N, I, err, s, basis_smem(K, N), 0, aligned, sms,
                                        smem_sm, optin);
 }
 
