@@ -216,3 +216,21 @@ def test_basis_read_back(ctx, M, K, N, off):
     bound = C.double().abs() @ B.double().abs()
     assert bool(((got - C.double() @ B.double()).abs() <= 4e-6 * bound + 1e-30).all())
     assert bool((I[:off] == -7.0).all()) and bool((I[off + M * N:] == -7.0).all())
+
+
+# chords shared by 32, 16, 8, 4, 2 lanes and by one, counts that leave ragged
+# warps; one lane with several passes of source bins, and with windows wider
+# than a pass
+@pytest.mark.parametrize("nx,ny,views,px,es,ed,dnrg", [(60, 50, 37, 43, 16, 12, 2), (60, 50, 37, 143, 16, 12, 2),
+                                                       (60, 50, 61, 211, 16, 12, 2), (30, 34, 121, 211, 16, 12, 2),
+                                                       (30, 34, 241, 211, 16, 12, 2), (30, 34, 401, 211, 16, 12, 2),
+                                                       (12, 12, 401, 211, 2400, 8, 100), (12, 12, 401, 211, 2400, 8, 1000)])
+def test_ct_lanes_per_chord(ctx, oracle_lib, nx, ny, views, px, es, ed, dnrg):
+    p = sized_problem(nx, ny, views, px, es, ed, dnrg)
+    p.col_pitch *= 1.6
+    inp = synth.make_inputs(p, 700 + nx)
+    T, G = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=ctx)
+    rays = some_rays(p, 400, nx + px)
+    Tr, Gr = oracle_lib.ct_rays(inp, rays)
+    assert max_rel_err(T[rays], Tr) < FAST_RTOL
+    assert max_rel_err(G[rays], Gr) < 1e-5

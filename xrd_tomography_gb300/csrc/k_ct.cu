@@ -22,7 +22,8 @@
 //
 // Lane = chord, 32 consecutive output columns per warp: the stores of every
 // detector bin are whole rows, at the cost of chords of different views side by
-// side in the walk.  The chord's entry point and sample count are decided in
+// side in the walk.  Few chords are split among 2 to 32 lanes each (see the
+// launch).  The chord's entry point and sample count are decided in
 // float pairs, near a threshold in FP64 (which issues at 1/64 of the FP32 rate:
 // all chords in FP64 took 16 us more), the chord is walked cell by cell
 // (walk_cells), then the transmission of every source bin is formed once per
@@ -156,16 +157,18 @@ template <bool STAGED>
 __global__ void __launch_bounds__(32 * kCtWarps)
 k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__ sg, const float4 *__restrict__ cells,
               const FwdEnergy *__restrict__ energy, const float *__restrict__ rf_win, const int *__restrict__ win_lo,
-              float *__restrict__ T, float *__restrict__ G0, int e_pass)
+              float *__restrict__ T, float *__restrict__ G0, int e_pass, int lg_split)
 {
     extern __shared__ float att_s[];
     const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    float *att = att_s + (size_t)(threadIdx.x >> 5) * 32 * e_pass + lane;   // [e_pass][32], this lane's column
+    // 2^lg_split neighbouring lanes share a chord: its samples, source bins and detector bins
+    const int split = 1 << lg_split, sub = lane & (split - 1), col = lane >> lg_split, cols = 32 >> lg_split;
+    float *att = att_s + (size_t)(threadIdx.x >> 5) * cols * e_pass + col;   // [e_pass][cols], this chord's column
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
     const int W = 2 * P.dnrg + 1;
     const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
-    const int64_t wstride = 32 * (int64_t)gridDim.x * nwarps;
-    float *rf_s = att_s + (size_t)nwarps * 32 * e_pass, *g0_s = rf_s + P.nrg_det * W;
+    const int64_t wstride = cols * (int64_t)gridDim.x * nwarps;
+    float *rf_s = att_s + (size_t)nwarps * cols * e_pass, *g0_s = rf_s + P.nrg_det * W;
     if (STAGED) {
         for (int i = threadIdx.x; i < P.nrg_det * W; i += blockDim.x) rf_s[i] = rf_win[i];
         for (int n = threadIdx.x; n < P.nrg_det; n += blockDim.x) {
@@ -175,9 +178,9 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
         }
         __syncthreads();
     }
-    for (int64_t p0 = 32 * (blockIdx.x * (int64_t)nwarps + (threadIdx.x >> 5)); p0 < npairs; p0 += wstride) {
-        const int64_t p = min(p0 + lane, npairs - 1);   // a lane past the last chord repeats it
-        const bool mine = p0 + lane < npairs;
+    for (int64_t p0 = cols * (blockIdx.x * (int64_t)nwarps + (threadIdx.x >> 5)); p0 < npairs; p0 += wstride) {
+        const int64_t p = min(p0 + col, npairs - 1);   // lanes past the last chord repeat it
+        const bool mine = p0 + col < npairs;
         const int src = (int)(p % P.n_src), det = (int)(p / P.n_src);
         const SrcGeom *g = sg + src;
         // det_position in pairs: the column's offset is a multiple of 1/2
@@ -189,8 +192,14 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
         ff ax, ay;
         if (!chord_setup_pairs(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), dx, dy, &ws, &ax, &ay))
             chord_setup_f64(P, g, det, &ws, &ax, &ay);
-        const float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
-                                          make_float2(ax.lo, ay.lo));
+        const int per = (ws.n + split - 1) >> lg_split;
+        ws.n = min(ws.n, (sub + 1) * per);
+        float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
+                                    make_float2(ax.lo, ay.lo), (float)(sub * per));
+        for (int o = split >> 1; o > 0; o >>= 1) {
+            A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
+            A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
+        }
         auto transmission = [&](int e) {   // -log2(e)/f1, -log2(e)/f2 as pairs
             const float4 f = __ldg(reinterpret_cast<const float4 *>(energy + e));
             return ex2_approx(fmaf(A.x, f.x, fmaf(A.y, f.z, fmaf(A.x, f.y, A.y * f.w))));
@@ -207,20 +216,23 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
             for (int n = 0; n < P.nrg_det;) {
                 const int e0 = __ldg(win_lo + n);
                 const int ne = min(e_pass, P.nrg_src - e0);
+                __syncwarp();   // the windows of the pass before are done with their bins
 #pragma unroll 4
-                for (int e = 0; e < ne; e++) att[32 * e] = transmission(e0 + e);
-                for (; n < P.nrg_det; n++) {
+                for (int e = sub; e < ne; e += split) att[cols * e] = transmission(e0 + e);
+                __syncwarp();
+                for (n += sub; n < P.nrg_det; n += split) {
                     const int lo = __ldg(win_lo + n) - e0;
                     if (lo + W > ne) break;
-                    const float *a = att + 32 * lo, *rf = rf_s + n * W;
+                    const float *a = att + cols * lo, *rf = rf_s + n * W;
                     float t = 0.f;
 #pragma unroll 4
-                    for (int j = 0; j < W; j++) t = fmaf(rf[j], a[32 * j], t);
+                    for (int j = 0; j < W; j++) t = fmaf(rf[j], a[cols * j], t);
                     store(n, t, g0_s[n]);
                 }
+                n = __reduce_min_sync(0xffffffffu, n);   // the first bin of the next pass
             }
         } else {
-            for (int n = 0; n < P.nrg_det; n++) {
+            for (int n = sub; n < P.nrg_det; n += split) {
                 float t = 0.f, g0 = 0.f;
                 for (int j = 0; j < W; j++) {
                     const float rf = __ldg(rf_win + n * W + j);
@@ -241,17 +253,25 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
 {
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
     const int W = 2 * P.dnrg + 1;
+    // lanes per chord: as many as 32 warps per SM have.  Kernel time at 1, 2, 4,
+    // 8, 16, 32 lanes: 38400 chords (200x180 voxels, 64 bins) 62.4, 46.6, 38.4,
+    // 40.5, 52.7, 75.3 us; 9600 (110x100, 32 bins) 42.1, 27.2, 22.0, 18.0, 17.2,
+    // 21.9; 1000 (72x56, 48 bins) 44.6, 28.2, 20.0, 14.9, 11.8, 11.8; a warp's
+    // serial walk and its serial bins are what the small ones wait for.
+    int lg_split = 0;
+    while (lg_split < 5 && (npairs << (lg_split + 1)) <= 1024LL * current_sm_count()) lg_split++;
+    const size_t bin_bytes = sizeof(float) * (32 >> lg_split);
     // the source bins of a pass: all that the windows reach, or as many as one
     // warp's columns have room for beside the windows, one window at least
     const int E = P.e_hi - P.e_lo + 1;
     const size_t tables = sizeof(float) * ((size_t)P.nrg_det * W + P.nrg_det);
     int warps = kCtWarps;
     int64_t e_pass = E;
-    size_t smem = 128 * (size_t)warps * E + tables;
+    size_t smem = bin_bytes * warps * E + tables;
     if (smem > 56 * 1024) {   // four blocks per SM
         warps = 1;
-        e_pass = tables < 200 * 1024 ? std::min<int64_t>(E, (int64_t)(200 * 1024 - tables) / 128) : 0;
-        smem = 128 * (size_t)e_pass + tables;
+        e_pass = tables < 200 * 1024 ? std::min<int64_t>(E, (int64_t)((200 * 1024 - tables) / bin_bytes)) : 0;
+        smem = bin_bytes * (size_t)e_pass + tables;
     }
     const bool staged = e_pass >= W;
     if (!staged) {
@@ -262,12 +282,13 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
     auto *kernel = staged ? k_ct_sinogram<true> : k_ct_sinogram<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int64_t blocks = (npairs + 32 * warps - 1) / (32 * warps);
+    const int64_t per_block = (int64_t)(32 >> lg_split) * warps;
+    int64_t blocks = (npairs + per_block - 1) / per_block;
     if (blocks > 64LL * current_sm_count()) blocks = 64LL * current_sm_count();
     const CtConsts q = {ff_from_double(P.cx), ff_from_double(P.cy), ff_from_double(P.r_det), ff_from_double(P.col_pitch),
                         P.n_col};
     kernel<<<(int)blocks, 32 * warps, smem, s>>>(P, make_f32_consts(P), q, sg, cells, energy, rf_win, win_lo, T, G0,
-                                                 (int)e_pass);
+                                                 (int)e_pass, lg_split);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

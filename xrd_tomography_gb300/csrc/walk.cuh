@@ -280,11 +280,11 @@ __device__ __forceinline__ void ld_cell256(const float4 *p, float4 &c0, float4 &
 constexpr int kReach = 31;
 constexpr float kReachUnit = 0x1p-125f, kReachScale = 0x1p125f, kReachLimit = 0x1p-115f;
 
-// LOW: the anchor is the pair (v, vlow), not an exact float.
+// LOW: the anchor is the pair (v, vlow), not an exact float.  k0: the first sample to take.
 template <bool LOW = false>
 __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, int sx, int sy, unsigned ncell_m1,
                                              const WalkSetup &w, float vx, float vy, float DQ,
-                                             float2 vlow = make_float2(0.f, 0.f))
+                                             float2 vlow = make_float2(0.f, 0.f), float k0 = 0.f)
 {
     const float magic = 12582912.f;
     const float nf = (float)w.n;
@@ -302,7 +302,7 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
     // sample count was capped: then a two-sum that needs no ordering
     const bool small_dlt = w.dlt.hi <= DQ;
     float2 acc = make_float2(0.f, 0.f), comp = make_float2(0.f, 0.f);
-    for (float k0 = 0.f; k0 < nf;) {
+    while (k0 < nf) {
         // distance s = dlt + k0 DQ and displacement t = s u as float pairs
         // (exact products through the FMA): the sample's offset from its cell
         // centre is then good to about 1e-7 voxel, where a position formed
