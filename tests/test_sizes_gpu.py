@@ -234,3 +234,33 @@ def test_ct_lanes_per_chord(ctx, oracle_lib, nx, ny, views, px, es, ed, dnrg):
     Tr, Gr = oracle_lib.ct_rays(inp, rays)
     assert max_rel_err(T[rays], Tr) < FAST_RTOL
     assert max_rel_err(G[rays], Gr) < 1e-5
+
+
+@pytest.mark.parametrize("K", [4, 8, 12, 16, 20, 32, 36, 64, 68, 128, 132, 256, 260, 384, 388, 512, 516, 640, 644, 768,
+                               772, 896, 900, 1024])
+@pytest.mark.parametrize("rays", [1, 37, 2433, 20011])
+def test_matrix_mlem_row_shapes(ctx, K, rays):
+    """Every lanes-per-row and chunk count of the pass, at both ends of its
+    range of K, with fewer rows than warps, ragged visits and several steps of
+    the ring, both directions.  A, x, y and c are positive, so errors are
+    relative: a chain of 4 products per chunk and 5 partner sums, the ratio, a
+    chain of the warp's rows, its row groups, 16 warps and the update round
+    e = (4 * 8 + 5 + 4 + rows + 5 + 16 + 4) 2^-24 at most, and an error of x
+    comes back as twice that after an iteration: 7 e after three."""
+    torch = pytest.importorskip("torch")
+    it = 3
+    g = torch.Generator(device="cuda").manual_seed(K + rays)
+    A = torch.rand(rays, K, device="cuda", generator=g) + 0.1
+    x0 = torch.rand(K, device="cuda", generator=g) + 0.1
+    c = torch.rand(rays, device="cuda", generator=g) + 0.1
+    y = (torch.rand(rays, device="cuda", generator=g) + 0.1) * K
+    want, a = x0.double(), A.double()
+    for _ in range(it):
+        want = want * (a.T @ (y.double() / (a @ want + c.double() + 1e-20))) / (a.sum(0) + 1e-7)
+    got = x0.clone()
+    torch.cuda.synchronize()
+    xt.mlem_matrix(A, y, c, got, it, ctx=ctx)
+    per_warp = -(-rays // (152 * 8))
+    tol = 7 * (66 + per_warp) * 2.0 ** -24
+    rel = float(((got.double() - want).abs() / want).max())
+    assert rel <= tol, (rel, tol)

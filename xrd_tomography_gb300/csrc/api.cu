@@ -590,7 +590,6 @@ int32_t xrdt_ctx_destroy(xrdt_ctx *ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     fold_pending(ctx);
-    if (ctx->mlem_exec) cudaGraphExecDestroy(ctx->mlem_exec);
     if (ctx->d_work) cudaFree(ctx->d_work);
     for (void *p : ctx->buf)
         if (p) cudaFree(p);
@@ -1232,43 +1231,14 @@ int32_t xrdt_mlem_matrix(xrdt_ctx *ctx, const float *A, int64_t rays, int32_t K,
         return fail(ctx, XRDT_ERR_UNSUPPORTED, "device arrays A and x must be 16-byte aligned");
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    const int nparts = mlem_pass_blocks(sms, K);
+    const int nparts = mlem_pass_blocks(sms, rays, K);
     void *dpart, *dsens;
-    if ((rc = get_buf(ctx, S_MPART, sizeof(float) * (size_t)nparts * K, &dpart))) return rc;
+    if ((rc = get_buf(ctx, S_MPART, sizeof(float) * 2 * (size_t)nparts * K, &dpart))) return rc;
     if ((rc = get_buf(ctx, S_MSENS, sizeof(double) * K, &dsens))) return rc;
     {
         ProfScope ps(ctx, XRDT_KERNEL_MLEM);
-        CK(launch_mlem_sensitivity((const float *)dA, rays, K, (float *)dpart, nparts, (double *)dsens, st,
-                                   &ctx->launches));
-    }
-    if (iters > 0) {
-        const void *key[6] = {dA, dy, dc, dx, dpart, dsens};
-        bool same = ctx->mlem_exec && ctx->mlem_rays == rays && ctx->mlem_K == K;
-        for (int i = 0; i < 6 && same; i++) same = ctx->mlem_key[i] == key[i];
-        if (!same) {
-            if (ctx->mlem_exec) {
-                cudaGraphExecDestroy(ctx->mlem_exec);
-                ctx->mlem_exec = nullptr;
-            }
-            cudaGraph_t graph;
-            CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            int64_t dummy = 0;
-            cudaError_t le = launch_mlem_iteration((const float *)dA, rays, K, (const float *)dy,
-                                                   (const float *)dc, dx, (float *)dpart, nparts,
-                                                   (const double *)dsens, st, &dummy);
-            cudaError_t ce = cudaStreamEndCapture(st, &graph);
-            if (le != cudaSuccess) return fail(ctx, XRDT_ERR_CUDA, fmt("MLEM capture: %s", cudaGetErrorString(le)));
-            CK(ce);
-            cudaError_t ie = cudaGraphInstantiate(&ctx->mlem_exec, graph, 0);
-            cudaGraphDestroy(graph);
-            CK(ie);
-            for (int i = 0; i < 6; i++) ctx->mlem_key[i] = key[i];
-            ctx->mlem_rays = rays;
-            ctx->mlem_K = K;
-        }
-        ProfScope ps(ctx, XRDT_KERNEL_MLEM);
-        for (int it = 0; it < iters; it++) CK(cudaGraphLaunch(ctx->mlem_exec, st));
-        ctx->launches += 2 * (int64_t)iters;
+        CK(launch_mlem_matrix((const float *)dA, rays, K, (const float *)dy, (const float *)dc, dx, iters,
+                              (float *)dpart, nparts, (double *)dsens, st, &ctx->launches));
     }
     if (hostX) CK(cudaMemcpyAsync(x, dx, sizeof(float) * K, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -27,11 +27,6 @@ struct xrdt_ctx {
     int64_t prof_launches[XRDT_KERNEL_COUNT] = {};
     double prof_ms[XRDT_KERNEL_COUNT] = {};
     unsigned long long *d_work = nullptr;  // exp2 evaluations of the forward kernel
-    // MLEM iteration captured as a graph, keyed by its arguments
-    cudaGraphExec_t mlem_exec = nullptr;
-    const void *mlem_key[6] = {};
-    long long mlem_rays = 0;
-    int mlem_K = 0;
 };
 
 namespace xrdt {

@@ -97,13 +97,11 @@ extern "C" int32_t xrdt_mlem_matrix_noalloc(const float *A, int64_t rays, int32_
     int rc = scratch_addresses(device, &partial, &sens);
     if (rc) return rc;
     // as many partial rows as the pass wants, up to what the scratch holds
-    int nparts = xrdt::mlem_pass_blocks(sms, K);
-    const int cap = (int)(kScratchFloats / (size_t)K);
+    int nparts = xrdt::mlem_pass_blocks(sms, rays, K);
+    const int cap = (int)(kScratchFloats / (2 * (size_t)K));
     if (nparts > cap) nparts = cap;
     cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = xrdt::launch_mlem_sensitivity(A, rays, K, partial, nparts, sens, st, nullptr);
-    for (int it = 0; it < iters && e == cudaSuccess; it++)
-        e = xrdt::launch_mlem_iteration(A, rays, K, y, c, x, partial, nparts, sens, st, nullptr);
+    cudaError_t e = xrdt::launch_mlem_matrix(A, rays, K, y, c, x, iters, partial, nparts, sens, st, nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         cudaGetLastError();

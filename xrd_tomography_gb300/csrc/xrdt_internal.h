@@ -247,13 +247,12 @@ cudaError_t launch_gather_rays(const int64_t *idx, int64_t n, const float *Nc, c
 int current_sm_count();
 
 // k_mlem.cu: MLEM with an explicit model matrix (rows of K floats, K % 4 == 0,
-// K <= 1024); partial holds nparts rows of K floats.
-int mlem_pass_blocks(int sm_count, int K);
-cudaError_t launch_mlem_sensitivity(const float *A, long long rays, int K, float *partial, int nparts,
-                                    double *sens, cudaStream_t s, int64_t *launches);
-cudaError_t launch_mlem_iteration(const float *A, long long rays, int K, const float *y, const float *c,
-                                  float *x, float *partial, int nparts, const double *sens, cudaStream_t s,
-                                  int64_t *launches);
+// K <= 1024); partial holds 2 nparts rows of K floats, sens K doubles.
+// Blocks of a pass: at most one per SM.
+int mlem_pass_blocks(int sm_count, long long rays, int K);
+// `iters` iterations on x, with nparts <= mlem_pass_blocks() blocks.
+cudaError_t launch_mlem_matrix(const float *A, long long rays, int K, const float *y, const float *c, float *x,
+                               int iters, float *partial, int nparts, double *sens, cudaStream_t s, int64_t *launches);
 
 // k_vox.cu: the per-voxel-coefficient model (forward, adjoint, MLEM update).
 struct VoxOp {
