@@ -37,11 +37,11 @@ namespace {
 enum Slot {
     S_SPEC, S_IFINE, S_SEG, S_A1, S_A2, S_S2, S_N, S_C, S_A,
     S_CELLS, S_VXY, S_VMAT, S_VNA, S_VA2, S_CNT, S_ASRC, S_S2U8,
-    S_SRCG, S_ENERGY, S_RFWIN, S_OFFS, S_WINLO, S_WINN, S_FINEQ, S_COARSEQ, S_COARSEQD,
+    S_SRCG, S_ENERGY, S_RFWIN, S_WINLO, S_COARSEQD,
     S_RAYS, S_PAIRS, S_NC, S_CC, S_AC,
-    S_MA, S_MY, S_MC, S_MX, S_MPART, S_MSENS, S_BC, S_BB, S_BI, S_ERR, S_WALK,
+    S_MA, S_MY, S_MC, S_MX, S_MPART, S_MSENS, S_BC, S_BB, S_BI, S_WALK,
     S_SPFINE, S_SPSRC, S_SPDET, S_SPOUT, S_DWALK, S_DNQ,
-    S_S1, S_S1U8, S_VTA, S_FWDEN, S_VORD, S_PREC,
+    S_S1, S_S1U8, S_VTA, S_TABLES, S_VORD, S_PREC,
     S_COUNT
 };
 
@@ -116,6 +116,50 @@ int stage_in(xrdt_ctx *ctx, int slot, const void *p, size_t bytes, const void **
     *dev = d;
     return XRDT_OK;
 }
+
+// The per-call tables of the forward and the CT sinogram: put together in a
+// pinned buffer and copied to the device in one go.  (As ten copies from
+// pageable memory they took 27 us of a call and as many gaps between its
+// kernels.)  The buffer belongs to the context.  Each call that fills it
+// synchronises its stream after the copy, so the next call may overwrite it.
+struct TablePack {
+    xrdt_ctx *ctx;
+    size_t used = 0;
+    std::vector<std::pair<const void **, size_t>> views;   // where each table's address goes, and its offset
+    std::vector<std::pair<const void *, size_t>> sources;  // what is copied, and its size
+
+    template <class T, class U>
+    void add(const std::vector<T> &v, const U **out)
+    {
+        views.push_back({(const void **)out, used});
+        sources.push_back({v.data(), sizeof(T) * v.size()});
+        used = (used + sizeof(T) * v.size() + 255) & ~(size_t)255;
+    }
+    int upload(int slot)
+    {
+        void *d;
+        int rc = get_buf(ctx, slot, used, &d);
+        if (rc) return rc;
+        if (ctx->stage_cap < used) {
+            if (ctx->h_stage) {
+                CK(cudaFreeHost(ctx->h_stage));
+                ctx->h_stage = nullptr;
+                ctx->stage_cap = 0;
+            }
+            if (cudaMallocHost((void **)&ctx->h_stage, used) != cudaSuccess) {
+                cudaGetLastError();
+                return fail(ctx, XRDT_ERR_ALLOC, fmt("cudaMallocHost(%zu bytes) failed", used));
+            }
+            ctx->stage_cap = used;
+        }
+        for (size_t i = 0; i < views.size(); i++) {
+            memcpy(ctx->h_stage + views[i].second, sources[i].first, sources[i].second);
+            *views[i].first = (const char *)d + views[i].second;
+        }
+        CK(cudaMemcpyAsync(d, ctx->h_stage, used, cudaMemcpyHostToDevice, ctx->stream));
+        return XRDT_OK;
+    }
+};
 
 bool finite_all(const xrdt_problem *p)
 {
@@ -286,7 +330,7 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
     // with weights RF = spectrum[e + n*nrg_src]; win_n[e] = the detector bins
     // whose window holds e
     const int same = (p->nrg_src == p->nrg_det && p->e_src_min == p->e_det_min && p->e_src_max == p->e_det_max);
-    t->rf_win.assign((size_t)p->nrg_det * W, 0.f);
+    if (spec_h) t->rf_win.assign((size_t)p->nrg_det * W, 0.f);
     t->win_lo.assign(p->nrg_det, 0);
     t->win_n.assign(2 * (size_t)p->nrg_src, 0);
     for (int e = 0; e < p->nrg_src; e++) {
@@ -298,7 +342,7 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         src_nrg_range(P, same, n, &lo, &hi);
         t->win_lo[n] = lo;
         for (int j = 0; j < W; j++) {
-            t->rf_win[(size_t)n * W + j] = spec_h[(lo + j) + (size_t)n * p->nrg_src];
+            if (spec_h) t->rf_win[(size_t)n * W + j] = spec_h[(lo + j) + (size_t)n * p->nrg_src];
             const int e = lo + j;
             if (n < t->win_n[2 * e]) t->win_n[2 * e] = n;
             if (n > t->win_n[2 * e + 1]) t->win_n[2 * e + 1] = n;
@@ -375,6 +419,10 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         t->coarse_q[k].z = (float)(e2 - e1);
         t->coarse_q[k].w = 0.f;
     }
+}
+
+void build_window_table(const xrdt_problem *p, HostTables *t)
+{
     // window table: the bins whose centres may lie beyond a wavevector's cell,
     // each cell a little wider against the rounding of the index; any order of
     // the centres gives a range that holds them all
@@ -481,22 +529,29 @@ int32_t xrdt_problem_validate(const xrdt_problem *p)
         return XRDT_ERR_DIMS;
     if (!(p->dq0 > 0) || !(p->dq_step > 0) || !(p->hbarc > 0) || !(p->mec2 > 0) || !(p->vox_side > 0))
         return XRDT_ERR_DIMS;
+    // the detector panel of a view is a segment; its end pixels and 63 points
+    // between them must lie outside the region of interest
+    const double r0 = (0.0 - (double)p->n_col / 2.0 + 0.5) * p->col_pitch;
+    const double r1 = ((double)(p->n_col - 1) - (double)p->n_col / 2.0 + 0.5) * p->col_pitch;
+    const double wx = p->nx * p->vox_side, wy = p->ny * p->vox_side;
     for (int s = 0; s < p->n_src; s++) {
         SrcGeom g;
         src_geom(p, s, &g);
         if (inside_roi(p, g.Rsrc_x, g.Rsrc_y)) return XRDT_ERR_GEOMETRY;
-        // the detector panel is a segment; its end pixels bound it
-        for (int c = 0; c < p->n_col; c += (p->n_col > 1 ? p->n_col - 1 : 1)) {
-            const double rdet = ((double)c - (double)p->n_col / 2.0 + 0.5) * p->col_pitch;
-            const double x = p->cx - p->r_det * g.sphi + rdet * g.cphi;
-            const double y = p->cy + p->r_det * g.cphi + rdet * g.sphi;
-            if (inside_roi(p, x, y)) return XRDT_ERR_GEOMETRY;
+        // The panel lies on the line (x - cx) (-sphi) + (y - cy) cphi = r_det.  Where
+        // that line passes the region's corners by more than the rounding of
+        // all this, no point of it lies inside, and the points need no look.
+        double far_corner = -HUGE_VAL, near_corner = HUGE_VAL;
+        for (int k = 0; k < 4; k++) {
+            const double h = ((k & 1 ? wx : 0.0) - p->cx) * -g.sphi + ((k & 2 ? wy : 0.0) - p->cy) * g.cphi;
+            far_corner = std::max(far_corner, h);
+            near_corner = std::min(near_corner, h);
         }
-        // the segment between the end pixels must not cross the ROI either
-        const double r0 = (0.0 - (double)p->n_col / 2.0 + 0.5) * p->col_pitch;
-        const double r1 = ((double)(p->n_col - 1) - (double)p->n_col / 2.0 + 0.5) * p->col_pitch;
-        for (int k = 1; k < 64; k++) {
-            const double r = r0 + (r1 - r0) * k / 64.0;
+        const double slack = 0.01 + 1e-9 * (std::fabs(p->r_det) + std::fabs(r0) + std::fabs(r1) + std::fabs(p->cx) +
+                                            std::fabs(p->cy) + wx + wy);
+        if (p->r_det > far_corner + slack || p->r_det < near_corner - slack) continue;
+        for (int k = 0; k < 65; k++) {
+            const double r = k == 64 ? r1 : r0 + (r1 - r0) * k / 64.0;
             if (inside_roi(p, p->cx - p->r_det * g.sphi + r * g.cphi, p->cy + p->r_det * g.cphi + r * g.sphi))
                 return XRDT_ERR_GEOMETRY;
         }
@@ -594,6 +649,7 @@ int32_t xrdt_ctx_destroy(xrdt_ctx *ctx)
     for (void *p : ctx->buf)
         if (p) cudaFree(p);
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return XRDT_OK;
@@ -688,12 +744,7 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
     if (hostA) { if ((rc = get_buf(ctx, S_A, sizeof(float) * aelems, &tmp))) return rc; dA = (float *)tmp; }
 
     // ---- per-call tables (host, double) ----
-    std::vector<SrcGeom> hsg(p->n_src);
-    for (int s = 0; s < p->n_src; s++) src_geom(p, s, &hsg[s]);
     PrepBuffers B;
-    void *d_srcg;
-    if ((rc = get_buf(ctx, S_SRCG, sizeof(SrcGeom) * p->n_src, &d_srcg))) return rc;
-    CK(cudaMemcpyAsync(d_srcg, hsg.data(), sizeof(SrcGeom) * p->n_src, cudaMemcpyHostToDevice, st));
     if ((rc = get_buf(ctx, S_CELLS, sizeof(float4) * 4 * (size_t)(p->nx + 1) * (p->ny + 1), &tmp))) return rc;
     B.cells = (float4 *)tmp;
     if ((rc = get_buf(ctx, S_VXY, sizeof(int) * nvox, &tmp))) return rc;
@@ -725,6 +776,33 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
     CK(launch_prep_voxels(P, (const int32_t *)d_seg, (const float *)d_a1, (const float *)d_a2, B, st,
                           &ctx->launches)); }
     CK(cudaMemcpyAsync(ctx->h_counters, B.counters, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
+    // the tables and what needs no voxel count go out while the voxels are counted
+    std::vector<SrcGeom> hsg(p->n_src);
+    for (int s = 0; s < p->n_src; s++) src_geom(p, s, &hsg[s]);
+    const SrcGeom *d_srcg;
+    FwdTables T;
+    TablePack pack{ctx};
+    pack.add(hsg, &d_srcg);
+    HostTables ht;
+    if (!plain) {
+        build_host_tables(p, P, nullptr, &ht);
+        pack.add(ht.energy, &T.energy);
+        pack.add(ht.fwd_energy, &T.fwd_energy);
+        pack.add(ht.offs_e, &T.offs_e);
+        pack.add(ht.win_lo, &T.win_lo);
+        pack.add(ht.win_n, &T.win_n);
+        pack.add(ht.fine_q, &T.fine_q);
+        pack.add(ht.coarse_q, &T.coarse_q);
+        T.sl = ht.sl;
+    }
+    if ((rc = pack.upload(S_TABLES))) return rc;
+    if (!plain) {
+        if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * (size_t)p->nrg_det * (2 * p->dnrg + 1), &tmp))) return rc;
+        T.rf_win = (const float *)tmp;
+        ProfScope ps(ctx, XRDT_KERNEL_PREP_MAP);
+        CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, (const float *)d_S2, B, st, &ctx->launches,
+                           (const float *)d_S1, (const float *)d_spec, T.win_lo, (float *)tmp));
+    }
     CK(cudaStreamSynchronize(st));
     const int nv = ctx->h_counters[0];
     if (ctx->h_counters[1])
@@ -751,7 +829,7 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
             d_rays = (const int64_t *)dr;
         }
         ProfScope ps(ctx, XRDT_KERNEL_PLAIN);
-        CK(launch_plain_forward(P, (const SrcGeom *)d_srcg, (const float *)d_spec, (const float *)d_ifine,
+        CK(launch_plain_forward(P, d_srcg, (const float *)d_spec, (const float *)d_ifine,
                                 (const int32_t *)d_seg, (const float *)d_a1, (const float *)d_a2,
                                 (const float *)d_S2, (const double *)tmp, d_rays, n_list, dN, dC, dA, st,
                                 &ctx->launches));
@@ -761,57 +839,10 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         CK(cudaMemsetAsync(dC, 0, sizeof(float) * rays, st));
         if (dA) CK(cudaMemsetAsync(dA, 0, sizeof(float) * aelems, st));
     } else {
-        std::vector<float> hspec;
-        const float *spec_h = spectrum;
-        if (is_device_ptr(spectrum)) {
-            hspec.resize((size_t)p->nrg_src * p->nrg_det);
-            CK(cudaMemcpy(hspec.data(), spectrum, sizeof(float) * hspec.size(), cudaMemcpyDeviceToHost));
-            spec_h = hspec.data();
-        }
-        HostTables ht;
-        build_host_tables(p, P, spec_h, &ht);
-        const std::vector<EnergyRow> &er = ht.energy;
-        const std::vector<float> &rfw = ht.rf_win, &offs_e = ht.offs_e;
-        const std::vector<int> &wlo = ht.win_lo, &wn = ht.win_n;
-        const std::vector<float2> &fq = ht.fine_q;
-        const std::vector<float4> &cqf = ht.coarse_q;
-        const int sl = ht.sl;
-        FwdTables T;
-        void *d;
-        if ((rc = get_buf(ctx, S_ENERGY, sizeof(EnergyRow) * er.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, er.data(), sizeof(EnergyRow) * er.size(), cudaMemcpyHostToDevice, st));
-        T.energy = (const EnergyRow *)d;
-        if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * rfw.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, rfw.data(), sizeof(float) * rfw.size(), cudaMemcpyHostToDevice, st));
-        T.rf_win = (const float *)d;
-        if ((rc = get_buf(ctx, S_OFFS, sizeof(float) * offs_e.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, offs_e.data(), sizeof(float) * offs_e.size(), cudaMemcpyHostToDevice, st));
-        T.offs_e = (const float *)d;
-        T.sl = sl;
-        if ((rc = get_buf(ctx, S_FWDEN, sizeof(FwdEnergy) * ht.fwd_energy.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, ht.fwd_energy.data(), sizeof(FwdEnergy) * ht.fwd_energy.size(), cudaMemcpyHostToDevice,
-                           st));
-        T.fwd_energy = (const FwdEnergy *)d;
-        if ((rc = get_buf(ctx, S_WINLO, sizeof(int) * wlo.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, wlo.data(), sizeof(int) * wlo.size(), cudaMemcpyHostToDevice, st));
-        T.win_lo = (const int *)d;
-        if ((rc = get_buf(ctx, S_WINN, sizeof(int) * wn.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, wn.data(), sizeof(int) * wn.size(), cudaMemcpyHostToDevice, st));
-        T.win_n = (const int *)d;
-        if ((rc = get_buf(ctx, S_FINEQ, sizeof(float2) * fq.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, fq.data(), sizeof(float2) * fq.size(), cudaMemcpyHostToDevice, st));
-        T.fine_q = (const float2 *)d;
-        if ((rc = get_buf(ctx, S_COARSEQ, sizeof(float4) * cqf.size(), &d))) return rc;
-        CK(cudaMemcpyAsync(d, cqf.data(), sizeof(float4) * cqf.size(), cudaMemcpyHostToDevice, st));
-        T.coarse_q = (const float4 *)d;
-
         if ((rc = get_buf(ctx, S_ASRC, sizeof(float2) * (size_t)p->n_src * nv, &tmp))) return rc;
         B.atten_src = (float2 *)tmp;
-        { ProfScope ps(ctx, XRDT_KERNEL_PREP_MAP);
-          CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, (const float *)d_S2, B, st, &ctx->launches,
-                             (const float *)d_S1)); }
         { ProfScope ps(ctx, XRDT_KERNEL_SRC_ATTEN);
-          CK(launch_src_atten(P, (const SrcGeom *)d_srcg, nv, B, st, &ctx->launches)); }
+          CK(launch_src_atten(P, d_srcg, nv, B, st, &ctx->launches)); }
         T.work = ctx->profiling ? ctx->d_work : nullptr;
         // pairs go through in tiles: the detector-side integrals of a tile
         // (k_walk.cu), then the projector over the same pairs
@@ -831,7 +862,7 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
                 const int64_t n = std::min(tile, n_total - p0);
                 {
                     ProfScope ps(ctx, XRDT_KERNEL_WALK);
-                    CK(launch_pair_table(P, (const SrcGeom *)d_srcg, list ? list + p0 : nullptr, p0, n,
+                    CK(launch_pair_table(P, d_srcg, list ? list + p0 : nullptr, p0, n,
                                          (PairRec *)drec, st, &ctx->launches));
                     CK(launch_det_walk(P, recs, list != nullptr, n, B.vox_xy, nv, B.cells, (float2 *)dtab, st,
                                        &ctx->launches));
@@ -1046,14 +1077,14 @@ int32_t xrdt_basis_expand(xrdt_ctx *ctx, const float *C, int64_t M, int32_t K, c
         if ((rc = get_buf(ctx, S_BI, sizeof(float) * (size_t)M * N, &tmp))) return rc;
         dI = (float *)tmp;
     }
-    if ((rc = get_buf(ctx, S_ERR, sizeof(unsigned), &tmp))) return rc;
-    unsigned *derr = (unsigned *)tmp;
-    CK(cudaMemsetAsync(derr, 0, sizeof(unsigned), st));
+    // the error flag is a word of pinned host memory that the kernel only
+    // touches when a wait runs out
+    unsigned *derr = (unsigned *)(ctx->h_counters + 2);
+    *derr = 0;
     {
         ProfScope ps(ctx, XRDT_KERNEL_BASIS);
         CK(launch_basis_expand((const float *)dC, M, K, (const float *)dB, N, dI, derr, st, &ctx->launches));
     }
-    CK(cudaMemcpyAsync(ctx->h_counters + 2, derr, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     if (hostI) CK(cudaMemcpyAsync(I, dI, sizeof(float) * (size_t)M * N, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (ctx->h_counters[2]) return fail(ctx, XRDT_ERR_TIMEOUT, "the tensor-core accumulator never completed");
@@ -1168,34 +1199,32 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
     void *tmp;
     if (hostT) { if ((rc = get_buf(ctx, S_N, sizeof(float) * rays, &tmp))) return rc; dT = (float *)tmp; }
     if (hostG) { if ((rc = get_buf(ctx, S_C, sizeof(float) * rays, &tmp))) return rc; dG = (float *)tmp; }
-    std::vector<float> hspec((size_t)p->nrg_src * p->nrg_det);
-    CK(cudaMemcpy(hspec.data(), spectrum, sizeof(float) * hspec.size(), cudaMemcpyDefault));
-    HostTables ht;
-    build_host_tables(p, P, hspec.data(), &ht);
     std::vector<SrcGeom> hsg(p->n_src);
     for (int s = 0; s < p->n_src; s++) src_geom(p, s, &hsg[s]);
-    void *d_srcg, *d_energy, *d_rf, *d_wlo;
-    if ((rc = get_buf(ctx, S_SRCG, sizeof(SrcGeom) * p->n_src, &d_srcg))) return rc;
-    if ((rc = get_buf(ctx, S_FWDEN, sizeof(FwdEnergy) * ht.fwd_energy.size(), &d_energy))) return rc;
-    if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * ht.rf_win.size(), &d_rf))) return rc;
-    if ((rc = get_buf(ctx, S_WINLO, sizeof(int) * ht.win_lo.size(), &d_wlo))) return rc;
-    CK(cudaMemcpyAsync(d_srcg, hsg.data(), sizeof(SrcGeom) * p->n_src, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_energy, ht.fwd_energy.data(), sizeof(FwdEnergy) * ht.fwd_energy.size(), cudaMemcpyHostToDevice,
-                       st));
-    CK(cudaMemcpyAsync(d_rf, ht.rf_win.data(), sizeof(float) * ht.rf_win.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_wlo, ht.win_lo.data(), sizeof(int) * ht.win_lo.size(), cudaMemcpyHostToDevice, st));
+    HostTables ht;
+    build_host_tables(p, P, nullptr, &ht);
+    const SrcGeom *d_srcg;
+    const FwdEnergy *d_energy;
+    const int *d_wlo;
+    void *d_rf;
+    TablePack pack{ctx};
+    pack.add(hsg, &d_srcg);
+    pack.add(ht.fwd_energy, &d_energy);
+    pack.add(ht.win_lo, &d_wlo);
+    if ((rc = pack.upload(S_TABLES))) return rc;
+    if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * (size_t)p->nrg_det * (2 * p->dnrg + 1), &d_rf))) return rc;
     PrepBuffers B;
     memset(&B, 0, sizeof B);
     if ((rc = get_buf(ctx, S_CELLS, sizeof(float4) * 4 * (size_t)(p->nx + 1) * (p->ny + 1), &tmp))) return rc;
     B.cells = (float4 *)tmp;
     {
         ProfScope ps(ctx, XRDT_KERNEL_PREP_MAP);
-        CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, nullptr, B, st, &ctx->launches));
+        CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, nullptr, B, st, &ctx->launches, nullptr,
+                           (const float *)d_spec, d_wlo, (float *)d_rf));
     }
     {
         ProfScope ps(ctx, XRDT_KERNEL_CT);
-        CK(launch_ct_sinogram(P, (const SrcGeom *)d_srcg, B.cells, (const FwdEnergy *)d_energy, (const float *)d_rf,
-                              (const int *)d_wlo, dT, dG, st, &ctx->launches));
+        CK(launch_ct_sinogram(P, d_srcg, B.cells, d_energy, (const float *)d_rf, d_wlo, dT, dG, st, &ctx->launches));
     }
     if (hostT) CK(cudaMemcpyAsync(Tphotons, dT, sizeof(float) * rays, cudaMemcpyDeviceToHost, st));
     if (hostG) CK(cudaMemcpyAsync(gain0, dG, sizeof(float) * rays, cudaMemcpyDeviceToHost, st));

@@ -17,6 +17,8 @@ struct xrdt_ctx {
     std::vector<void *> buf;
     std::vector<size_t> cap;
     int *h_counters = nullptr;  // pinned
+    char *h_stage = nullptr;    // pinned: the per-call tables on their way to the device
+    size_t stage_cap = 0;
     // profiling: events bracketing launches, folded into totals on query
     bool profiling = false;
     struct Pending {

@@ -13,7 +13,8 @@
 //    (walk_cells, walk.cuh).  One block per 32 x 32 cells; coefficients from
 //    float pairs (in FP64 the blocks of a small map queued on the FP64 pipes of
 //    a few SMs: 24 us against 14 on 45x33).  Also
-//    quantises the Compton table to u8 (integrate_diffraction.cu:66-74).
+//    quantises the Compton table to u8 (integrate_diffraction.cu:66-74) and
+//    gathers the spectrum windows.
 //  * k_compact_voxels: non-empty voxels in the reference's loop order
 //    (nx outer, ny inner; integrate_diffraction.cu:173-178) and the material
 //    id check (ids above n_mat would index past Ifine in the reference).
@@ -42,7 +43,8 @@ __global__ void __launch_bounds__(1024)
 k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restrict__ a2,
                               float4 *__restrict__ cells, const float *__restrict__ S2,
                               unsigned char *__restrict__ s2u8, int ns2, const float *__restrict__ S1,
-                              unsigned char *__restrict__ s1u8)
+                              unsigned char *__restrict__ s1u8, const float *__restrict__ spec,
+                              const int *__restrict__ win_lo, float *__restrict__ rf_win, int nrg_src, int nrf, int W)
 {
     __shared__ unsigned uneven[kRows][3];
     __shared__ unsigned char row_dist[kRows][32];
@@ -127,6 +129,11 @@ k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restr
             const int q1 = floor_to_int((double)S1[i]);
             s1u8[i] = (unsigned char)(q1 < 0 ? 0 : (q1 > 255 ? 255 : q1));
         }
+    }
+    // the spectrum windows: rf_win[n][j] = spectrum[win_lo[n] + j, n]
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nrf; i += stride) {
+        const int n = (int)(i / W), j = (int)(i - (int64_t)n * W);
+        rf_win[i] = spec[win_lo[n] + j + (int64_t)n * nrg_src];
     }
 }
 
@@ -285,12 +292,14 @@ __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict
 } // namespace
 
 cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a2, const float *S2,
-                            PrepBuffers &B, cudaStream_t s, int64_t *launches, const float *S1)
+                            PrepBuffers &B, cudaStream_t s, int64_t *launches, const float *S1, const float *spec,
+                            const int *win_lo, float *rf_win)
 {
     // one block of 1024 threads per tile of 32 x 32 cells
     const int64_t blocks = (int64_t)((P.nx + 1 + 31) / 32) * ((P.ny + 1 + 31) / 32);
     k_build_cells<<<(unsigned)blocks, 1024, 0, s>>>(P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8, S2 ? P.nq * P.na : 0,
-                                         B.s1u8 ? S1 : nullptr, B.s1u8);
+                                         B.s1u8 ? S1 : nullptr, B.s1u8, spec, win_lo, rf_win, P.nrg_src,
+                                         rf_win ? P.nrg_det * (2 * P.dnrg + 1) : 0, 2 * P.dnrg + 1);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

@@ -998,6 +998,7 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     // per-energy tables
     HostTables ht;
     build_host_tables(p, P, hspec.data(), &ht);
+    build_window_table(p, &ht);
     EnergyRow *d_energy;
     float *d_rf;
     int *d_wlo, *d_wn;

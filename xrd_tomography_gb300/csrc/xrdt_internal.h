@@ -109,7 +109,10 @@ struct HostTables {
     std::vector<float4> coarse_q;   // [nwt]
 };
 // spectrum: host copy [nrg_src][nrg_det] column-major as passed to Forward_XRD.
+// (NULL: rf_win is left empty, for launch_prep_map to fill on the device.)
 void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *spectrum, HostTables *t);
+// qlut and lut_scale, from coarse_q.
+void build_window_table(const xrdt_problem *p, HostTables *t);
 
 // ---- host-side builders (api.cu) ----
 int build_dev_problem(const xrdt_problem *p, float q_min, float q_max, float a_min,
@@ -158,10 +161,13 @@ struct PrepBuffers {
     unsigned char *s2u8 = nullptr;    // [nq*na]
     unsigned char *s1u8 = nullptr;    // [nq*na] the coherent table of the table path, or NULL
 };
-// S1 (with B.s1u8): the coherent table, quantised like S2.
+// S1 (with B.s1u8): the coherent table, quantised like S2.  rf_win (or NULL):
+// [nrg_det][2*dnrg+1], filled from the spectrum spec [nrg_src, nrg_det] and the
+// windows win_lo.
 cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a2,
                             const float *S2, PrepBuffers &B, cudaStream_t s, int64_t *launches,
-                            const float *S1 = nullptr);
+                            const float *S1 = nullptr, const float *spec = nullptr,
+                            const int *win_lo = nullptr, float *rf_win = nullptr);
 cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const float *a1,
                                const float *a2, PrepBuffers &B, cudaStream_t s, int64_t *launches);
 cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, PrepBuffers &B,
