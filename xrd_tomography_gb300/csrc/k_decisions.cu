@@ -66,7 +66,8 @@ __global__ void k_decisions(DevProblem P, F32Consts c, const SrcGeom *__restrict
             const EnergyRow r = energy[lo + j];
             const float ein = r.einf;
             const float eratio = __fadd_rn(1.f, __fmul_rn(ein, vg.omc.hi));   // as k_fwd forms it
-            out[j] = compton_bin(P, ein, eratio, vg.s.hi, vg.omc.hi, vg.omc.lo, energy + lo + j, qmin_t, inv_dqt);
+            out[j] = compton_bin(P, ein, eratio, vg.s.hi, vg.omc.hi, vg.omc.lo, energy + lo + j, qmin_t, inv_dqt,
+                                 c.bin_guard);
         }
     }
 }

@@ -35,12 +35,15 @@
 // The kernel is bound by instruction issue.  With lane = energy (an energy's
 // constants loaded for every voxel, a voxel's constants shuffled, a window loop
 // as long as the warp's longest window) 32 terms took about 390 instructions;
-// here they take about 250, and k_fwd went from 12.5 to 7.8 ms on 128x128 voxels,
-// 32 views x 128 px, 40 energies, from 314 to 145 ms on the reference's own sizes
-// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 355 ms
-// on 256x256 voxels, 45 views x 512 px, 64 energies.  Measured on the way, 128x128:
-// equal contiguous shares instead of the counter 9.3 (reference sizes 227) ms,
-// the counter 9.6 (192) ms, and voxels in tiles instead of strips 8.2 (149) ms.
+// here they take about 240, and k_fwd went from 12.5 to 7.1 ms on 128x128 voxels,
+// 32 views x 128 px, 40 energies, from 314 to 139 ms on the reference's own sizes
+// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 327 ms
+// on 256x256 voxels, 45 views x 512 px, 64 energies.  Two neighbouring energies per
+// step, packed two to an instruction, took 18 % fewer instructions but no less
+// time (7.0, 147 and 314 ms at best): a packed FMA holds its pipe for two cycles.
+// Measured on the way, 128x128: equal contiguous shares instead of the counter 9.3
+// (reference sizes 227) ms, the counter 9.6 (192) ms, and voxels in tiles instead
+// of strips 8.2 (149) ms.
 //
 // Compton counts: per step each lane adds its two channel overlaps to its own
 // column of the warp's cells [channel][32] (no conflicts, no atomics); at the
@@ -327,7 +330,7 @@ k_fwd(const FwdArgs args)
                     // extra bins are exact terms of the full sum or zero pads);
                     // bin numbers stay in the magic number's mantissa, where
                     // they are integers and floats at once
-                    int jb = max(__float_as_int((y - half) + kMagic) & ~3, (int)kMagicBits);
+                    const int jb = max(__float_as_int((y - half) + kMagic) & ~3, (int)kMagicBits);
                     const int je = min(__float_as_int((y + half) + kMagic), jlast);
                     if (jb <= je && pref != 0.f) {
                         // c (u - frac)^2 as a quadratic in u = j - j0: near the
@@ -342,8 +345,9 @@ k_fwd(const FwdArgs args)
                         float2 U = make_float2(u, u + 1.f);
                         float2 acc = make_float2(0.f, 0.f);
                         uint32_t a = ifine_a + 4u * (uint32_t)((__float_as_int(r2.w) & 0xffff) + jb);
+                        const uint32_t end = a + 4u * (uint32_t)(je - jb);
                         if (COUNT) nexp += (unsigned)((je - jb + 4) & ~3);
-                        for (; jb <= je; jb += 4, a += 16) {
+                        for (; a <= end; a += 16) {
                             const float4 I = lds128(a);
                             const float2 g0 = __ffma2_rn(__ffma2_rn(C2, U, B2), U, A2);
                             U = __fadd2_rn(U, make_float2(2.f, 2.f));
@@ -394,7 +398,7 @@ k_fwd(const FwdArgs args)
                                              (compton_log2(q.ein * sh, er) - qmin_t) * c.inv_dqg, r2.w);
                     else
                         s2v = table2(compton_bin(P, q.ein, er, sh, oh, r1.w, args.T.energy + P.e_lo + el, qmin_t,
-                                                 inv_dqt) +
+                                                 inv_dqt, c.bin_guard) +
                                      (TAB ? __float_as_int(r2.w) : (int)((unsigned)__float_as_int(r2.w) >> 16)));
                     // twice Cf of :347 (gpa holds the 1/2): eratio^2 (eratio + 1/eratio - 1 + cos^2)
                     const float ct = 1.f - oh;

@@ -120,8 +120,8 @@ __device__ __forceinline__ ff gauss_scale(ff sig2, float rcp)
 }
 
 // Compton table bin of integrate_diffraction.cu:331-337 decided in FP64, as
-// the oracle decides it; used only when the FP32 value lies within 2e-4 of a
-// bin edge.  Kept out of line so that the rare FP64 path is a real branch
+// the oracle decides it; used only when the FP32 value lies within its error of
+// a bin edge.  Kept out of line so that the rare FP64 path is a real branch
 // and not predicated into every iteration of the energy loop.
 __device__ __noinline__ int compton_bin_f64(const DevProblem &P, double ein, float omc_hi, float omc_lo)
 {
@@ -138,21 +138,22 @@ __device__ __noinline__ int compton_bin_f64(const DevProblem &P, double ein, flo
 __device__ __forceinline__ float compton_log2(float w, float eratio)
 {
     const float w2 = w * w;
-    return fmaf(0.5f, lg2_approx(w2 * (eratio + w2)), -lg2_approx(eratio));
+    return fmaf(0.5f, lg2_approx(w2 * (eratio + w2)), lg2_approx(rcp_approx(eratio)));
 }
 
 // Compton table bin nq = floor((compton_log2 - q_min) / dq), clamped to
 // [0, NQ) (integrate_diffraction.cu:331-337).  Decided in FP32 from the voxel's
 // 1 - cos(theta) (pair (oh, ol)) and sin(theta/2) (hi part sh), by rounding
-// through the float mantissa; within 2e-4 of a bin edge it is decided again
+// through the float mantissa; near a bin edge, where the value lies bin_guard
+// or more from the middle of its bin (make_f32_consts), it is decided again
 // in FP64 with the energy row's ein.  eratio = 1 + ein oh without contraction.
 __device__ __forceinline__ int compton_bin(const DevProblem &P, float ein, float eratio, float sh, float oh, float ol,
-                                           const EnergyRow *row, float qmin_t, float inv_dqt)
+                                           const EnergyRow *row, float qmin_t, float inv_dqt, float bin_guard)
 {
     const float h = (compton_log2(ein * sh, eratio) - qmin_t) * inv_dqt - 0.5f;
     const float t = h + 12582912.f;
     int nq = __float_as_int(t) - 0x4B400000;            // round(h) = floor(h + 1/2); clamped below
-    if (!(fabsf(h - (t - 12582912.f)) < 0.5f - 2e-4f))   // near a table edge
+    if (!(fabsf(h - (t - 12582912.f)) < bin_guard))   // near a table edge
         nq = compton_bin_f64(P, row->ein, oh, ol);
     return max(0, min(nq, P.nq - 1));
 }
