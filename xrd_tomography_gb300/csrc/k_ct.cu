@@ -20,16 +20,19 @@
 // the attenuation model of integrate_diffraction.cu:291-296.  Outputs use the
 // Nphotons layout, index src + det*SRC + nrg*SRC*DET.
 //
-// Lane = chord, 32 consecutive output columns per warp: the stores of every
-// detector bin are whole rows, at the cost of chords of different views side by
-// side in the walk.  Few chords are split among 2 to 32 lanes each (see the
-// launch).  The chord's entry point and sample count are decided in
+// Lane = chord.  A block walks 8 views x 16 pixels with neighbouring pixels side
+// by side -- their rays cross the same cells -- and then turns the line integrals
+// round in shared memory, so that the stores of every detector bin, views fastest,
+// are whole sectors: 71 us at the size below against 89 with 32 views side by side
+// in both (12 of them in the walk, the rest from two bins' sums at a time and
+// tables staged without a chain of loads).  Few chords are split among 2 to 32 lanes
+// each (see the launch).  The chord's entry point and sample count are decided in
 // float pairs, near a threshold in FP64 (which issues at 1/64 of the FP32 rate:
 // all chords in FP64 took 16 us more), the chord is walked cell by cell
 // (walk_cells), then the transmission of every source bin is formed once per
 // chord -- each detector bin's window holds 2 DNRG + 1 of them -- and the windows
 // are summed out of shared memory.  256x256 voxels, 180 views x
-// 512 px, 64 energies: 82 us; with a warp per chord, one sample per lane, the set-up
+// 512 px, 64 energies: 71 us; with a warp per chord, one sample per lane, the set-up
 // in FP64 by all 32 lanes alike and every window's exponentials on their own
 // 660 us, and its line integrals were off by 1e-6 (positions in FP32).
 #include <algorithm>
@@ -149,57 +152,85 @@ struct CtConsts {
     int n_col;
 };
 
+// Views of a strip of chords: 8 floats of an output row are a 32-byte sector.
+constexpr int kStrip = 8;
+
 // Shared memory: per warp the transmission of a pass's source bins
-// [e_pass][32], then (STAGED) the spectrum windows [nrg_det][W] and their sums.
-// Windows too wide for that (!STAGED) are read through L1, and every bin forms
-// its own transmissions.
+// [e_pass][chords of the warp], then (STAGED) the spectrum windows [nrg_det][W],
+// their sums and their first bins.  Windows too wide for that (!STAGED) are read
+// through L1, and every bin forms its own transmissions.
 template <bool STAGED>
 __global__ void __launch_bounds__(32 * kCtWarps)
 k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__ sg, const float4 *__restrict__ cells,
               const FwdEnergy *__restrict__ energy, const float *__restrict__ rf_win, const int *__restrict__ win_lo,
-              float *__restrict__ T, float *__restrict__ G0, int e_pass, int lg_split)
+              float *__restrict__ T, float *__restrict__ G0, int e_pass, int lg_split, int strip_w)
 {
     extern __shared__ float att_s[];
+    __shared__ float2 A_s[32 * kCtWarps];   // the block's line integrals
     const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     // 2^lg_split neighbouring lanes share a chord: its samples, source bins and detector bins
-    const int split = 1 << lg_split, sub = lane & (split - 1), col = lane >> lg_split, cols = 32 >> lg_split;
-    float *att = att_s + (size_t)(threadIdx.x >> 5) * cols * e_pass + col;   // [e_pass][cols], this chord's column
+    const int split = 1 << lg_split, sub = lane & (split - 1), cols = 32 >> lg_split;
+    const int nch = blockDim.x >> lg_split, ch = threadIdx.x >> lg_split;   // chords of the block, this thread's
+    float *att = att_s + (size_t)(threadIdx.x >> 5) * cols * e_pass + (lane >> lg_split);   // this chord's column
     const int64_t npairs = (int64_t)P.n_src * P.n_det;
     const int W = 2 * P.dnrg + 1;
     const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
-    const int64_t wstride = cols * (int64_t)gridDim.x * nwarps;
     float *rf_s = att_s + (size_t)nwarps * cols * e_pass, *g0_s = rf_s + P.nrg_det * W;
+    int *lo_s = (int *)(g0_s + P.nrg_det);
     if (STAGED) {
         for (int i = threadIdx.x; i < P.nrg_det * W; i += blockDim.x) rf_s[i] = rf_win[i];
+        for (int i = threadIdx.x; i < P.nrg_det; i += blockDim.x) lo_s[i] = win_lo[i];
+        __syncthreads();
         for (int n = threadIdx.x; n < P.nrg_det; n += blockDim.x) {
             float g0 = 0.f;
-            for (int j = 0; j < W; j++) g0 += rf_win[n * W + j];
+            for (int j = 0; j < W; j++) g0 += rf_s[n * W + j];
             g0_s[n] = g0;
         }
-        __syncthreads();
     }
-    for (int64_t p0 = cols * (blockIdx.x * (int64_t)nwarps + (threadIdx.x >> 5)); p0 < npairs; p0 += wstride) {
-        const int64_t p = min(p0 + col, npairs - 1);   // lanes past the last chord repeat it
-        const bool mine = p0 + col < npairs;
-        const int src = (int)(p % P.n_src), det = (int)(p / P.n_src);
-        const SrcGeom *g = sg + src;
-        // det_position in pairs: the column's offset is a multiple of 1/2
-        const ff sphi = ff_from_double(g->sphi), cphi = ff_from_double(g->cphi);
-        const ff rdet = ff_mulf(q.pitch, (float)(det % q.n_col) - 0.5f * (float)q.n_col + 0.5f);
-        const ff dx = ff_add(ff_sub(q.cx, ff_mul(q.r_det, sphi)), ff_mul(rdet, cphi));
-        const ff dy = ff_add(ff_add(q.cy, ff_mul(q.r_det, cphi)), ff_mul(rdet, sphi));
-        WalkSetup ws;
-        ff ax, ay;
-        if (!chord_setup_pairs(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), dx, dy, &ws, &ax, &ay))
-            chord_setup_f64(P, g, det, &ws, &ax, &ay);
-        const int per = (ws.n + split - 1) >> lg_split;
-        ws.n = min(ws.n, (sub + 1) * per);
-        float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
-                                    make_float2(ax.lo, ay.lo), (float)(sub * per));
-        for (int o = split >> 1; o > 0; o >>= 1) {
-            A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
-            A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
+    // Blocks take the chords of a strip of strip_w views (the last may be
+    // narrower) in the order of the outputs, views fastest, nch at a time.
+    const int64_t full = ((int64_t)strip_w * P.n_det + nch - 1) / nch;   // blocks of a full strip
+    const int strips = P.n_src / strip_w, rest = P.n_src - strips * strip_w;
+    const int64_t nblocks = strips * full + ((int64_t)rest * P.n_det + nch - 1) / nch;
+    for (int64_t blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
+        const int strip = (int)min(blk / full, (int64_t)strips);
+        const int width = strip < strips ? strip_w : rest;
+        const int64_t first = (blk - strip * full) * nch;     // of the strip's chords
+        const int count = (int)min((int64_t)nch, (int64_t)width * P.n_det - first);
+        // ---- line integrals, in a strip of kStrip with neighbouring lanes on
+        // neighbouring pixels of one view, whose rays cross the same cells (a
+        // chord past the end repeats the last) ----
+        {
+            int k = ch;
+            if (width == kStrip && nch >= 2 * kStrip) k = (ch % (nch / kStrip)) * kStrip + ch / (nch / kStrip);
+            const int64_t s = first + min(k, count - 1);
+            const int src = strip * strip_w + (int)(s % width), det = (int)(s / width);
+            const SrcGeom *g = sg + src;
+            // det_position in pairs: the column's offset is a multiple of 1/2
+            const ff sphi = ff_from_double(g->sphi), cphi = ff_from_double(g->cphi);
+            const ff rdet = ff_mulf(q.pitch, (float)(det % q.n_col) - 0.5f * (float)q.n_col + 0.5f);
+            const ff dx = ff_add(ff_sub(q.cx, ff_mul(q.r_det, sphi)), ff_mul(rdet, cphi));
+            const ff dy = ff_add(ff_add(q.cy, ff_mul(q.r_det, cphi)), ff_mul(rdet, sphi));
+            WalkSetup ws;
+            ff ax, ay;
+            if (!chord_setup_pairs(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), dx, dy, &ws, &ax, &ay))
+                chord_setup_f64(P, g, det, &ws, &ax, &ay);
+            const int per = (ws.n + split - 1) >> lg_split;
+            ws.n = min(ws.n, (sub + 1) * per);
+            float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
+                                        make_float2(ax.lo, ay.lo), (float)(sub * per));
+            for (int o = split >> 1; o > 0; o >>= 1) {
+                A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
+                A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
+            }
+            if (sub == 0) A_s[k] = A;
         }
+        __syncthreads();
+        // ---- energies: neighbouring lanes on neighbouring outputs ----
+        const float2 A = A_s[ch];
+        const bool mine = ch < count;
+        const int64_t s = first + min(ch, count - 1);
+        const int64_t p = strip * strip_w + s % width + s / width * P.n_src;
         auto transmission = [&](int e) {   // -log2(e)/f1, -log2(e)/f2 as pairs
             const float4 f = __ldg(reinterpret_cast<const float4 *>(energy + e));
             return ex2_approx(fmaf(A.x, f.x, fmaf(A.y, f.z, fmaf(A.x, f.y, A.y * f.w))));
@@ -214,20 +245,36 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
         if (STAGED) {
             // per pass the bins whose windows lie in its source bins (win_lo rises with n)
             for (int n = 0; n < P.nrg_det;) {
-                const int e0 = __ldg(win_lo + n);
+                const int e0 = lo_s[n];
                 const int ne = min(e_pass, P.nrg_src - e0);
                 __syncwarp();   // the windows of the pass before are done with their bins
 #pragma unroll 4
                 for (int e = sub; e < ne; e += split) att[cols * e] = transmission(e0 + e);
                 __syncwarp();
                 for (n += sub; n < P.nrg_det; n += split) {
-                    const int lo = __ldg(win_lo + n) - e0;
+                    const int lo = lo_s[n] - e0;
                     if (lo + W > ne) break;
                     const float *a = att + cols * lo, *rf = rf_s + n * W;
-                    float t = 0.f;
+                    // two bins at a time, for their loads to overlap
+                    const int m = n + split;
+                    const int lo1 = m < P.nrg_det ? lo_s[m] - e0 : ne;
+                    if (lo1 + W <= ne) {
+                        const float *a1 = att + cols * lo1, *rf1 = rf_s + m * W;
+                        float t = 0.f, t1 = 0.f;
 #pragma unroll 4
-                    for (int j = 0; j < W; j++) t = fmaf(rf[j], a[cols * j], t);
-                    store(n, t, g0_s[n]);
+                        for (int j = 0; j < W; j++) {
+                            t = fmaf(rf[j], a[cols * j], t);
+                            t1 = fmaf(rf1[j], a1[cols * j], t1);
+                        }
+                        store(n, t, g0_s[n]);
+                        store(m, t1, g0_s[m]);
+                        n = m;
+                    } else {
+                        float t = 0.f;
+#pragma unroll 4
+                        for (int j = 0; j < W; j++) t = fmaf(rf[j], a[cols * j], t);
+                        store(n, t, g0_s[n]);
+                    }
                 }
                 n = __reduce_min_sync(0xffffffffu, n);   // the first bin of the next pass
             }
@@ -242,6 +289,7 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
                 store(n, t, g0);
             }
         }
+        __syncthreads();   // before the next chords' line integrals
     }
 }
 
@@ -264,7 +312,7 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
     // the source bins of a pass: all that the windows reach, or as many as one
     // warp's columns have room for beside the windows, one window at least
     const int E = P.e_hi - P.e_lo + 1;
-    const size_t tables = sizeof(float) * ((size_t)P.nrg_det * W + P.nrg_det);
+    const size_t tables = sizeof(float) * ((size_t)P.nrg_det * W + 2 * P.nrg_det);
     int warps = kCtWarps;
     int64_t e_pass = E;
     size_t smem = bin_bytes * warps * E + tables;
@@ -282,13 +330,17 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
     auto *kernel = staged ? k_ct_sinogram<true> : k_ct_sinogram<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int64_t per_block = (int64_t)(32 >> lg_split) * warps;
-    int64_t blocks = (npairs + per_block - 1) / per_block;
+    const int64_t nch = (int64_t)(32 >> lg_split) * warps;
+    // strips of kStrip views where a lane has a chord to itself (38400 chords,
+    // four lanes each: 39 us either way; 9600, sixteen: 20 us in strips, 17 in rows)
+    const int strip_w = lg_split == 0 && P.n_src >= kStrip ? kStrip : P.n_src;
+    const int strips = P.n_src / strip_w, rest = P.n_src - strips * strip_w;
+    int64_t blocks = strips * (((int64_t)strip_w * P.n_det + nch - 1) / nch) + ((int64_t)rest * P.n_det + nch - 1) / nch;
     if (blocks > 64LL * current_sm_count()) blocks = 64LL * current_sm_count();
     const CtConsts q = {ff_from_double(P.cx), ff_from_double(P.cy), ff_from_double(P.r_det), ff_from_double(P.col_pitch),
                         P.n_col};
     kernel<<<(int)blocks, 32 * warps, smem, s>>>(P, make_f32_consts(P), q, sg, cells, energy, rf_win, win_lo, T, G0,
-                                                 (int)e_pass, lg_split);
+                                                 (int)e_pass, lg_split, strip_w);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }
