@@ -54,6 +54,21 @@ def test_forward_over_walk_strips(ctx, oracle_lib, nx, ny, views, px):
     assert max_rel_err(C[rays], Cr) < FAST_RTOL
 
 
+# line integrals shared by 8, 4, 2 lanes and by one, on both sides of a voxel
+@pytest.mark.parametrize("nx,ny,views,px", [(9, 7, 3, 11), (16, 14, 5, 29), (16, 15, 6, 45), (31, 29, 7, 61)])
+def test_walk_lanes_per_ray(ctx, oracle_lib, nx, ny, views, px):
+    inp = synth.make_inputs(sized_problem(nx, ny, views, px, 12, 12, 2), 900 + nx + px)
+    p = inp.problem
+    N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    rays = some_rays(p, 300, px)
+    Nr, Cr, _, _ = oracle_lib.forward_rays(inp, rays)
+    assert max_rel_err(N[rays], Nr) < FAST_RTOL
+    assert max_rel_err(C[rays], Cr) < FAST_RTOL
+    # a few rays by themselves: the same bits
+    Ns, Cs, _ = xt.forward_rays(p, rays[:5], *inp.args(), ctx=ctx)
+    assert np.array_equal(Ns, N[rays[:5]]) and np.array_equal(Cs, C[rays[:5]])
+
+
 # the forward's splits: tiles of one step, remainders of steps and tiles, two
 # tiles and more; more and fewer energies than runs; source bins wider than
 # detector bins (a range meets many channels) and a detector grid that only

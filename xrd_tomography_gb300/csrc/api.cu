@@ -121,7 +121,7 @@ int stage_in(xrdt_ctx *ctx, int slot, const void *p, size_t bytes, const void **
 // pinned buffer and copied to the device in one go.  (As ten copies from
 // pageable memory they took 27 us of a call and as many gaps between its
 // kernels.)  The buffer belongs to the context.  Each call that fills it
-// synchronises its stream after the copy, so the next call may overwrite it.
+// waits until the copy is through before it returns, so the next may overwrite it.
 struct TablePack {
     xrdt_ctx *ctx;
     size_t used = 0;
@@ -657,6 +657,7 @@ int32_t xrdt_ctx_destroy(xrdt_ctx *ctx)
         if (p) cudaFree(p);
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    if (ctx->counted) cudaEventDestroy(ctx->counted);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return XRDT_OK;
@@ -780,8 +781,7 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
     }
 
     { ProfScope ps(ctx, XRDT_KERNEL_PREP_VOXELS);
-    CK(launch_prep_voxels(P, (const int32_t *)d_seg, (const float *)d_a1, (const float *)d_a2, B, st,
-                          &ctx->launches)); }
+      CK(launch_list_voxels(P, (const int32_t *)d_seg, B, st, &ctx->launches)); }
     CK(cudaMemcpyAsync(ctx->h_counters, B.counters, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
     // the tables and what needs no voxel count go out while the voxels are counted
     std::vector<SrcGeom> hsg(p->n_src);
@@ -803,17 +803,27 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         T.sl = ht.sl;
     }
     if ((rc = pack.upload(S_TABLES))) return rc;
+    if (!ctx->counted) CK(cudaEventCreateWithFlags(&ctx->counted, cudaEventDisableTiming));
+    CK(cudaEventRecord(ctx->counted, st));
+    { ProfScope ps(ctx, XRDT_KERNEL_PREP_VOXELS);
+      CK(launch_voxel_compton(P, (const float *)d_a1, (const float *)d_a2, B, st, &ctx->launches)); }
     if (!plain) {
         if ((rc = get_buf(ctx, S_RFWIN, sizeof(float) * (size_t)p->nrg_det * (2 * p->dnrg + 1), &tmp))) return rc;
         T.rf_win = (const float *)tmp;
         ProfScope ps(ctx, XRDT_KERNEL_PREP_MAP);
         CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, (const float *)d_S2, B, st, &ctx->launches,
-                           (const float *)d_S1, (const float *)d_spec, T.win_lo, (float *)tmp));
+                           (const float *)d_S1, (const float *)d_spec, T.win_lo, (float *)tmp, true));
     }
-    CK(cudaStreamSynchronize(st));
+    // (a stream in capture refuses the wait, and the call ends as a refused capture)
+    if (cudaEventSynchronize(ctx->counted) != cudaSuccess) {
+        cudaGetLastError();
+        CK(cudaStreamSynchronize(st));
+    }
     const int nv = ctx->h_counters[0];
-    if (ctx->h_counters[1])
+    if (ctx->h_counters[1]) {
+        cudaStreamSynchronize(st);   // nothing reads the caller's arrays after a refusal
         return fail(ctx, XRDT_ERR_INPUT, fmt("segmentation holds a material id above n_mat = %d", p->n_mat));
+    }
 
     if (plain) {
         std::vector<double> cq(2 * (size_t)p->nwt);
@@ -870,9 +880,9 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
                 {
                     ProfScope ps(ctx, XRDT_KERNEL_WALK);
                     CK(launch_pair_table(P, d_srcg, list ? list + p0 : nullptr, p0, n,
-                                         (PairRec *)drec, st, &ctx->launches));
+                                         (PairRec *)drec, st, &ctx->launches, !list && p0 == 0));
                     CK(launch_det_walk(P, recs, list != nullptr, n, B.vox_xy, nv, B.cells, (float2 *)dtab, st,
-                                       &ctx->launches));
+                                       &ctx->launches, true));
                 }
                 ProfScope ps(ctx, XRDT_KERNEL_FORWARD);
                 CK(launch_fast_forward(P, recs, T, B, nv, (const float *)d_ifine, list != nullptr, n_total, p0, (int)n,

@@ -19,6 +19,7 @@ struct xrdt_ctx {
     int *h_counters = nullptr;  // pinned
     char *h_stage = nullptr;    // pinned: the per-call tables on their way to the device
     size_t stage_cap = 0;
+    cudaEvent_t counted = nullptr;   // forward: the voxel counters are back, h_stage is free
     // profiling: events bracketing launches, folded into totals on query
     bool profiling = false;
     struct Pending {

@@ -108,7 +108,7 @@ k_mlem_pass(const float *__restrict__ A, long long rays, int K, const float *__r
     const long long visits = (rays + G - 1) / G;
     const int mine = gw < visits ? (int)((visits - 1 - gw) / nw + 1) : 0;   // visits of this warp
     const int steps = (mine + P - 1) / P;
-    asm volatile("griddepcontrol.launch_dependents;");
+    allow_dependents();
 
     float4 *const slot0 = ring + wid * P * KC * 32 + lane;
     constexpr int kStride = S::kWarps * P * KC * 32;
@@ -158,7 +158,7 @@ k_mlem_pass(const float *__restrict__ A, long long rays, int K, const float *__r
     for (int s = 0; s < S::kSteps - 1; s++) issue(s);
     load_yc();
     // x and the partial rows belong to the update before until here
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    await_predecessor();
     float4 xv[KC], g[KC], h[FIRST ? KC : 1];
 #pragma unroll
     for (int i = 0; i < KC; i++) {
@@ -260,8 +260,8 @@ k_mlem_update(const float *partial, int nparts, int K, double *sens, float *x, i
 {
     __shared__ double part[2][kUpdateThreads / 32][4];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    asm volatile("griddepcontrol.launch_dependents;");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    allow_dependents();
+    await_predecessor();
     for (int at = 0; at <= first; at++) {
         double v[4] = {0.0, 0.0, 0.0, 0.0};
         for (int p = threadIdx.x; p < nparts; p += kUpdateThreads) {
@@ -289,24 +289,6 @@ k_mlem_update(const float *partial, int nparts, int K, double *sens, float *x, i
     if (!isfinite(v)) v = 0.f;   // main.m:163
     if (v < 0.f) v = 0.f;        // main.m:176
     x[k] = v;
-}
-
-// Launch `f` behind the kernel before it in the stream; `early` lets it start
-// before that one is through (its own griddepcontrol.wait then waits).
-template <class F, class... Args>
-cudaError_t launch_after(F *f, int blocks, int threads, int smem, cudaStream_t s, bool early, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, f, args...);
 }
 
 template <int L, int KC>

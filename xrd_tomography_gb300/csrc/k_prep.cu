@@ -22,6 +22,8 @@
 //    (integrate_diffraction.cu:181-189), honouring the stale-coordinate quirk.
 //  * k_src_atten: the source-side line integral per (source, voxel), which
 //    the reference recomputes in every block (integrate_diffraction.cu:260).
+#include <algorithm>
+
 #include "xrdt_device.cuh"
 #include "walk.cuh"
 
@@ -135,6 +137,7 @@ k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restr
         const int n = (int)(i / W), j = (int)(i - (int64_t)n * W);
         rf_win[i] = spec[win_lo[n] + j + (int64_t)n * nrg_src];
     }
+    await_predecessor();   // launched early it must not end before what came before
 }
 
 // The position of each of a thread's flags (bit r of `keep`, r < 4, in order)
@@ -248,6 +251,7 @@ __global__ void k_voxel_compton(DevProblem P, const float *__restrict__ a1, cons
                                 const int *__restrict__ vox_xy, const int *__restrict__ counters,
                                 int *__restrict__ vox_na, float *__restrict__ vox_a2, float *__restrict__ vox_ta)
 {
+    allow_dependents();
     const int nv = counters[0];
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         double sx = 0.0, sy = 0.0;  // stale coordinates start at (0,0)
@@ -267,17 +271,21 @@ __global__ void k_voxel_compton(DevProblem P, const float *__restrict__ a1, cons
     }
 }
 
-// One lane per (source, voxel): attenuator(Rsrc, Rvox) of
+// 2^lg_split lanes per (source, voxel): attenuator(Rsrc, Rvox) of
 // integrate_diffraction.cu:260, decided as the detector side's (walk_decide)
-// and walked cell by cell from the voxel (walk_cells).  A warp takes 32
-// neighbouring voxels of one source.
+// and walked cell by cell from the voxel (walk_cells), each lane its share of the
+// samples.  A warp takes neighbouring voxels of one source.
 __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int *__restrict__ vox_xy,
-                            int nv, const float4 *__restrict__ cells, float2 *__restrict__ out)
+                            int nv, const float4 *__restrict__ cells, float2 *__restrict__ out, int lg_split)
 {
+    allow_dependents();
     const int64_t nwork = (int64_t)P.n_src * nv;
     const unsigned ncell_m1 = (unsigned)((P.nx + 1) * (P.ny + 1) - 1);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < nwork; w += stride) {
+    const int split = 1 << lg_split, sub = threadIdx.x & (split - 1);
+    // (the loop runs by whole warps: lanes past the end repeat the last walk)
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; (t & ~31) < nwork << lg_split; t += stride) {
+        const int64_t w = min(t >> lg_split, nwork - 1);
         const int src = (int)(w / nv), v = (int)(w % nv);
         const int xy = vox_xy[v];
         const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
@@ -285,7 +293,14 @@ __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict
         const SrcGeom *g = sg + src;
         WalkSetup ws;
         walk_decide(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), &g->Rsrc_x, &g->Rsrc_y, vx, vy, &ws);
-        out[(int64_t)src * nv + v] = walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ);
+        const int per = (ws.n + split - 1) >> lg_split;
+        ws.n = min(ws.n, (sub + 1) * per);
+        float2 A = walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ, make_float2(0.f, 0.f), (float)(sub * per));
+        for (int o = split >> 1; o > 0; o >>= 1) {
+            A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
+            A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
+        }
+        if (sub == 0 && t >> lg_split < nwork) out[(int64_t)src * nv + v] = A;
     }
 }
 
@@ -293,13 +308,33 @@ __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict
 
 cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a2, const float *S2,
                             PrepBuffers &B, cudaStream_t s, int64_t *launches, const float *S1, const float *spec,
-                            const int *win_lo, float *rf_win)
+                            const int *win_lo, float *rf_win, bool early)
 {
     // one block of 1024 threads per tile of 32 x 32 cells
     const int64_t blocks = (int64_t)((P.nx + 1 + 31) / 32) * ((P.ny + 1 + 31) / 32);
-    k_build_cells<<<(unsigned)blocks, 1024, 0, s>>>(P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8, S2 ? P.nq * P.na : 0,
-                                         B.s1u8 ? S1 : nullptr, B.s1u8, spec, win_lo, rf_win, P.nrg_src,
-                                         rf_win ? P.nrg_det * (2 * P.dnrg + 1) : 0, 2 * P.dnrg + 1);
+    if (launches) (*launches)++;
+    return launch_after(k_build_cells, (int)blocks, 1024, 0, s, early, P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8,
+                        S2 ? P.nq * P.na : 0, B.s1u8 ? S1 : nullptr, B.s1u8, spec, win_lo, rf_win, P.nrg_src,
+                        rf_win ? P.nrg_det * (2 * P.dnrg + 1) : 0, 2 * P.dnrg + 1);
+}
+
+cudaError_t launch_list_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
+                               int64_t *launches)
+{
+    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
+                                        B.vox_rank, nullptr);
+    if (launches) (*launches)++;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_voxel_compton(const DevProblem &P, const float *a1, const float *a2, PrepBuffers &B, cudaStream_t s,
+                                 int64_t *launches)
+{
+    // blocks of a warp: an FP64 logarithm per voxel, spread over the SMs (in
+    // blocks of 256 a 45x33 map took 10.9 us on six of them, now 7)
+    const int64_t nvox = (int64_t)P.nx * P.ny;
+    int blocks = (int)std::min<int64_t>((nvox + 31) / 32, 16384);
+    k_voxel_compton<<<blocks, 32, 0, s>>>(P, a1, a2, B.vox_xy, B.counters, B.vox_na, B.vox_a2, B.vox_ta);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }
@@ -307,14 +342,8 @@ cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a
 cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const float *a1,
                                const float *a2, PrepBuffers &B, cudaStream_t s, int64_t *launches)
 {
-    k_compact_voxels<<<1, 1024, 0, s>>>(P.nx, P.ny, P.n_mat, seg, B.vox_xy, B.vox_mat, B.counters, B.vox_order,
-                                        B.vox_rank, nullptr);
-    const int64_t nvox = (int64_t)P.nx * P.ny;
-    int blocks = (int)((nvox + 255) / 256);
-    if (blocks > 2048) blocks = 2048;
-    k_voxel_compton<<<blocks, 256, 0, s>>>(P, a1, a2, B.vox_xy, B.counters, B.vox_na, B.vox_a2, B.vox_ta);
-    if (launches) (*launches) += 2;
-    return cudaGetLastError();
+    cudaError_t e = launch_list_voxels(P, seg, B, s, launches);
+    return e == cudaSuccess ? launch_voxel_compton(P, a1, a2, B, s, launches) : e;
 }
 
 cudaError_t launch_compact_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
@@ -352,10 +381,13 @@ cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, 
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
+    // lanes per walk: up to 8, as far as 32 warps per SM have them
     const int64_t items = (int64_t)P.n_src * nv;
-    int64_t blocks = (items + 127) / 128;
+    int lg_split = 0;
+    while (lg_split < 3 && items << (lg_split + 1) <= 1024LL * sms) lg_split++;
+    int64_t blocks = ((items << lg_split) + 127) / 128;
     if (blocks > (int64_t)sms * 16) blocks = (int64_t)sms * 16;
-    k_src_atten<<<(int)blocks, 128, 0, s>>>(P, make_f32_consts(P), d_src, B.vox_xy, nv, B.cells, B.atten_src);
+    k_src_atten<<<(int)blocks, 128, 0, s>>>(P, make_f32_consts(P), d_src, B.vox_xy, nv, B.cells, B.atten_src, lg_split);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

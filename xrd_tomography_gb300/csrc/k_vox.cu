@@ -662,6 +662,7 @@ __global__ void k_vox_scatter(const VoxBatch B)
 __global__ void k_pair_table(DevProblem P, const SrcGeom *__restrict__ sg, const int2 *__restrict__ list, int64_t p0,
                              int64_t n, PairRec *__restrict__ out)
 {
+    allow_dependents();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = p0 + i;
         const int2 pr = list ? list[i] : make_int2((int)(p % P.n_src), (int)(p / P.n_src));
@@ -671,6 +672,7 @@ __global__ void k_pair_table(DevProblem P, const SrcGeom *__restrict__ sg, const
         r.pad = 0;
         out[i] = r;
     }
+    await_predecessor();   // launched early it must not end before what came before
 }
 
 // a grid-stride loop over n items: at most 32 blocks per SM
@@ -708,12 +710,11 @@ size_t static_smem(F *kernel)
 size_t pair_rec_bytes() { return sizeof(PairRec); }
 
 cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, const int2 *list, long long p0, long long n,
-                              PairRec *out, cudaStream_t s, int64_t *launches)
+                              PairRec *out, cudaStream_t s, int64_t *launches, bool early)
 {
     // small blocks: the records are FP64 work, spread over the SMs
-    k_pair_table<<<grid_for(n, 32), 32, 0, s>>>(P, sg, list, p0, n, out);
     if (launches) (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_pair_table, grid_for(n, 32), 32, 0, s, early, P, sg, list, (int64_t)p0, (int64_t)n, out);
 }
 
 cudaError_t vox_set_attributes(int max_smem)

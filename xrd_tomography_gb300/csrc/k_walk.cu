@@ -29,7 +29,6 @@ namespace {
 
 constexpr int kWalkThreads = 128;
 constexpr int kWalkWarps = kWalkThreads / 32;
-constexpr int kRays = 32;          // rays per group: neighbouring pixels of one view
 // Voxels per warp item (a strip): up to 64, so that the ray's FP64 endpoint is
 // set up seldom, but no more than leaves kItemsPerSM items per SM.  A warp
 // walks its strip's voxels one after the other; with 64 always, a small
@@ -40,18 +39,18 @@ constexpr int kRays = 32;          // rays per group: neighbouring pixels of one
 constexpr int kMaxStrip = 64;
 constexpr int kItemsPerSM = 256;   // 8 times the resident warps
 
-// Row of ray r of group g.  Linear pairs: the tile holds whole pixels (nd of
-// them) of every view, row pixel * SRC + view; group g is view g % SRC and
-// pixels 32 (g / SRC) + r.  A list: entries 32g + r.
-__device__ __forceinline__ bool group_row(const DevProblem &P, int list, long long n_items, int nd, long long g, int r,
-                                          long long *row)
+// Row of ray r of group g of `rays` rays.  Linear pairs: the tile holds whole
+// pixels (nd of them) of every view, row pixel * SRC + view; group g is view
+// g % SRC and pixels rays (g / SRC) + r.  A list: entries rays g + r.
+__device__ __forceinline__ bool group_row(const DevProblem &P, int list, long long n_items, int nd, int rays,
+                                          long long g, int r, long long *row)
 {
     if (list) {
-        *row = g * kRays + r;
+        *row = g * rays + r;
         return *row < n_items;
     }
     const int s = (int)(g % P.n_src);
-    const int dl = (int)(g / P.n_src) * kRays + r;
+    const int dl = (int)(g / P.n_src) * rays + r;
     *row = (long long)dl * P.n_src + s;
     return dl < nd;
 }
@@ -62,9 +61,12 @@ __device__ __forceinline__ bool group_row(const DevProblem &P, int list, long lo
 __global__ void __launch_bounds__(kWalkThreads, 8)
 k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list,
            long long n_items, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,
-           const float4 *__restrict__ cells, float2 *__restrict__ tab)
+           const float4 *__restrict__ cells, float2 *__restrict__ tab, int lg_split)
 {
     const int lane = threadIdx.x & 31;
+    // 2^lg_split neighbouring lanes share a ray's samples
+    const int split = 1 << lg_split, sub = lane & (split - 1);
+    await_predecessor();
     const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
     const unsigned ncell_m1 = (unsigned)(ncell - 1);
     const float4 *cells_t = cells + 2 * ncell;   // column-major copy
@@ -75,7 +77,7 @@ k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list
         const long long g = wk / nstrips;
         const int strip = (int)(wk - g * nstrips);
         long long row = -1;
-        const bool valid = group_row(P, list, n_items, nd, g, lane, &row);
+        const bool valid = group_row(P, list, n_items, nd, 32 >> lg_split, g, lane >> lg_split, &row);
         // the pixel's position, tabulated per pair, as float pairs (and as
         // double for the rare FP64 set-up)
         const PairRec *rec = recs + (valid ? row : 0);
@@ -95,9 +97,17 @@ k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list
             const unsigned along_x = __ballot_sync(0xffffffffu, valid && fabsf(ws.Lx) > fabsf(ws.Ly));
             const unsigned any = __ballot_sync(0xffffffffu, valid);
             const bool colmajor = 2 * __popc(along_x) > __popc(any);
-            const float2 A = colmajor ? walk_cells(cells_t, P.ny + 1, 1, ncell_m1, ws, vx, vy, c.DQ)
-                                      : walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ);
-            if (valid) out[v] = A;
+            const int per = (ws.n + split - 1) >> lg_split;
+            ws.n = min(ws.n, (sub + 1) * per);
+            const float2 none = make_float2(0.f, 0.f);
+            const float k0 = (float)(sub * per);
+            float2 A = colmajor ? walk_cells(cells_t, P.ny + 1, 1, ncell_m1, ws, vx, vy, c.DQ, none, k0)
+                                : walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ, none, k0);
+            for (int o = split >> 1; o > 0; o >>= 1) {
+                A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
+                A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
+            }
+            if (valid && sub == 0) out[v] = A;
         }
     }
 }
@@ -105,29 +115,35 @@ k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list
 } // namespace
 
 cudaError_t launch_det_walk(const DevProblem &P, const PairRec *recs, bool list, long long n_items, const int *vox_xy,
-                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches)
+                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches, bool early)
 {
     if (n_items <= 0 || nv <= 0) return cudaSuccess;
+    // Lanes per ray: up to 8, as far as 32 warps per SM have them with every
+    // pair of the problem -- not of this launch, so that a pair's integrals do
+    // not depend on the others that are asked for.
+    const int sms = current_sm_count();
+    const long long walks = (long long)P.n_src * P.n_det * nv;
+    int lg_split = 0;
+    while (lg_split < 3 && walks << (lg_split + 1) <= 1024LL * sms) lg_split++;
+    const int rays = 32 >> lg_split;
     int nd = 0;
     long long n_groups;
     if (list) {
-        n_groups = (n_items + kRays - 1) / kRays;
+        n_groups = (n_items + rays - 1) / rays;
     } else {
         // whole pixels of every view
         if (n_items % P.n_src != 0) return cudaErrorInvalidValue;
         nd = (int)(n_items / P.n_src);
-        n_groups = (long long)P.n_src * ((nd + kRays - 1) / kRays);
+        n_groups = (long long)P.n_src * ((nd + rays - 1) / rays);
     }
-    const int sms = current_sm_count();
     const int strip = (int)std::min<long long>(
         kMaxStrip, std::max<long long>(1, n_groups * nv / ((long long)sms * kItemsPerSM)));
     const long long nwork = n_groups * ((nv + strip - 1) / strip);
     long long blocks = (nwork + kWalkWarps - 1) / kWalkWarps;
     if (blocks > (long long)sms * 64) blocks = (long long)sms * 64;
-    k_det_walk<<<(unsigned)blocks, kWalkThreads, 0, s>>>(P, make_f32_consts(P), recs, list ? 1 : 0, n_items, nd, n_groups,
-                                                          strip, vox_xy, nv, cells, tab);
     if (launches) (*launches)++;
-    return cudaGetLastError();
+    return launch_after(k_det_walk, (int)blocks, kWalkThreads, 0, s, early, P, make_f32_consts(P), recs, list ? 1 : 0,
+                        n_items, nd, n_groups, strip, vox_xy, nv, cells, tab, lg_split);
 }
 
 } // namespace xrdt

@@ -118,6 +118,31 @@ __host__ __device__ inline bool get_intersection(double x1, double y1, double x2
     return false;
 }
 
+// Kernels of one stream that overlap (programmatic dependent launch): after
+// allow_dependents() in every block the next kernel may start if it was launched
+// `early` (launch_after); await_predecessor() there waits until this one, and
+// all before it, are through and their writes visible.
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void await_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_after(void (*kernel)(Params...), int blocks, int threads, size_t smem, cudaStream_t s, bool early,
+                         Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+
 // tex2D of Forward_XRD.cu:229-233 evaluated exactly in double from the
 // float maps: texel (i,j) centred at (i+0.5, j+0.5), zero outside.
 __device__ inline void bilinear_f64(const float *__restrict__ a1, const float *__restrict__ a2,

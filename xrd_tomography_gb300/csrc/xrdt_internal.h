@@ -164,11 +164,18 @@ struct PrepBuffers {
 };
 // S1 (with B.s1u8): the coherent table, quantised like S2.  rf_win (or NULL):
 // [nrg_det][2*dnrg+1], filled from the spectrum spec [nrg_src, nrg_det] and the
-// windows win_lo.
+// windows win_lo.  early: it may overlap the kernel launched before it, which
+// must not touch its buffers.
 cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a2,
                             const float *S2, PrepBuffers &B, cudaStream_t s, int64_t *launches,
                             const float *S1 = nullptr, const float *spec = nullptr,
-                            const int *win_lo = nullptr, float *rf_win = nullptr);
+                            const int *win_lo = nullptr, float *rf_win = nullptr, bool early = false);
+// launch_prep_voxels in two: the list of voxels with its counters, then their
+// Compton columns.
+cudaError_t launch_list_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,
+                               int64_t *launches);
+cudaError_t launch_voxel_compton(const DevProblem &P, const float *a1, const float *a2, PrepBuffers &B, cudaStream_t s,
+                                 int64_t *launches);
 cudaError_t launch_prep_voxels(const DevProblem &P, const int32_t *seg, const float *a1,
                                const float *a2, PrepBuffers &B, cudaStream_t s, int64_t *launches);
 cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, PrepBuffers &B,
@@ -221,12 +228,14 @@ cudaError_t launch_spectrum(const SpecFineBin *fb, const SpecCoarseBin *sb, int 
 size_t pair_rec_bytes();
 // out[i] = the record of pair list[i], or of the linear pair p0 + i, i < n.
 cudaError_t launch_pair_table(const DevProblem &P, const SrcGeom *sg, const int2 *list, long long p0, long long n,
-                              PairRec *out, cudaStream_t s, int64_t *launches);
+                              PairRec *out, cudaStream_t s, int64_t *launches,
+                              bool early = false);
 // k_walk.cu: tab[item][v] = detector-side line integral of voxel v for the
 // pair of recs[item], item < n_items.  Pairs that are not a list come in
 // whole pixels of every view, from a multiple of SRC on.
 cudaError_t launch_det_walk(const DevProblem &P, const PairRec *recs, bool list, long long n_items, const int *vox_xy,
-                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches);
+                            int nv, const float4 *cells, float2 *tab, cudaStream_t s, int64_t *launches,
+                              bool early = false);
 // k_bop.cu: rows of R values per non-empty voxel between the full grid
 // [NX*NY][R] and the compact voxel order [nv][R]; the coefficient-space MLEM
 // update c <- c g / (s + 1e-7) with the fix-ups of main.m:163,176.
