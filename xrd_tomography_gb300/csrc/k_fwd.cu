@@ -225,6 +225,9 @@ k_fwd(const FwdArgs args)
     auto table2 = [&](int i) { return FAST || args.split.tables ? S2[i] : (float)__ldg(args.s2u8 + i); };
     auto table1 = [&](int i) { return FAST || args.split.tables ? S1[i] : (float)__ldg(args.s1u8 + i); };
 
+    // the tables were written long before; the pair's record and walk are from here
+    await_predecessor();
+    allow_dependents();
     // ---- per-(source, pixel) geometry, integrate_diffraction.cu:81-128 (k_pair_table) ----
     for (int i = tid; i < (int)(sizeof(PairRec) / 4); i += nthr)
         reinterpret_cast<int *>(&pair)[i] = reinterpret_cast<const int *>(args.recs + blockIdx.x)[i];
@@ -511,8 +514,8 @@ cudaError_t launch_variant(const FwdArgs &a, int n_pairs, size_t smem, cudaStrea
     auto *kernel = k_fwd<TAB, FAST, COUNT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kernel<<<(unsigned)n_pairs, 32 * a.split.warps, smem, s>>>(a);
-    return cudaGetLastError();
+    // early: the tables are staged while the walk ends
+    return launch_after(kernel, n_pairs, 32 * a.split.warps, smem, s, true, a);
 }
 
 template <int TAB>

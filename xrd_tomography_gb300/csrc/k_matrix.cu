@@ -281,6 +281,7 @@ k_matrix(const MatrixArgs args)
             }
         }
     }
+    await_predecessor();   // launched early it must not end before what came before
     if (COUNT) {
         unsigned long long w = nexp;
 #pragma unroll
@@ -295,8 +296,8 @@ cudaError_t launch_groups(const MatrixArgs &a, int n_pairs, size_t smem, cudaStr
     auto *kernel = a.T.work ? k_matrix<NG, true> : k_matrix<NG, false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kernel<<<(unsigned)n_pairs, 32 * a.split.warps, smem, s>>>(a);
-    return cudaGetLastError();
+    // early: it reads nothing of the projection's, so the two overlap
+    return launch_after(kernel, n_pairs, 32 * a.split.warps, smem, s, true, a);
 }
 
 // Two blocks of 12 warps per SM, or three of 8 -- whichever leaves fewer warps

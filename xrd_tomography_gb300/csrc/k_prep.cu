@@ -39,6 +39,15 @@ __device__ __forceinline__ float sum4(float a, float b, float c, float d)
     return isfinite(s.hi) ? s.hi : (a + b) + (c + d);
 }
 
+// floor(x) clamped to 0 .. 255 (NaN: 0, as floor_to_int's lowest int), without
+// a conversion: those share the FP64 pipe.
+__device__ __forceinline__ unsigned char floor_u8(float x)
+{
+    if (!(x > 0.f)) return 0;
+    if (x >= 255.f) return 255;
+    return (unsigned char)(__float_as_uint(__fadd_rd(x, 8388608.f)) & 255u);   // 2^23
+}
+
 constexpr int kRows = 32 + 2 * kReach;   // cells of a tile and its surroundings, per side
 
 __global__ void __launch_bounds__(1024)
@@ -46,12 +55,28 @@ k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restr
                               float4 *__restrict__ cells, const float *__restrict__ S2,
                               unsigned char *__restrict__ s2u8, int ns2, const float *__restrict__ S1,
                               unsigned char *__restrict__ s1u8, const float *__restrict__ spec,
-                              const int *__restrict__ win_lo, float *__restrict__ rf_win, int nrg_src, int nrf, int W)
+                              const int *__restrict__ win_lo, float *__restrict__ rf_win, int nrg_src, int nrf, int W,
+                              int tiles)
 {
+    if ((int)blockIdx.x >= tiles) {
+        // ---- the blocks behind the cells: the tables ----
+        const int i0 = ((int)blockIdx.x - tiles) * blockDim.x + threadIdx.x;
+        const int step = ((int)gridDim.x - tiles) * blockDim.x;
+        for (int i = i0; i < ns2; i += step) {
+            s2u8[i] = floor_u8(S2[i]);
+            if (S1) s1u8[i] = floor_u8(S1[i]);
+        }
+        // the spectrum windows: rf_win[n][j] = spectrum[win_lo[n] + j, n]
+        for (int i = i0; i < nrf; i += step) {
+            const int n = i / W, j = i - n * W;
+            rf_win[i] = spec[win_lo[n] + j + (int64_t)n * nrg_src];
+        }
+        await_predecessor();
+        return;
+    }
     __shared__ unsigned uneven[kRows][3];
     __shared__ unsigned char row_dist[kRows][32];
     const int64_t ncell = (int64_t)(nx + 1) * (ny + 1);
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int tiles_x = (nx + 1 + 31) >> 5;
     const int x0 = 32 * (int)(blockIdx.x % tiles_x), y0 = 32 * (int)(blockIdx.x / tiles_x);
@@ -123,19 +148,6 @@ k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restr
         cells[2 * c + 1] = hi;
         cells[2 * ct] = lo;
         cells[2 * ct + 1] = hi;
-    }
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ns2; i += stride) {
-        const int q = floor_to_int((double)S2[i]);
-        s2u8[i] = (unsigned char)(q < 0 ? 0 : (q > 255 ? 255 : q));
-        if (S1) {
-            const int q1 = floor_to_int((double)S1[i]);
-            s1u8[i] = (unsigned char)(q1 < 0 ? 0 : (q1 > 255 ? 255 : q1));
-        }
-    }
-    // the spectrum windows: rf_win[n][j] = spectrum[win_lo[n] + j, n]
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nrf; i += stride) {
-        const int n = (int)(i / W), j = (int)(i - (int64_t)n * W);
-        rf_win[i] = spec[win_lo[n] + j + (int64_t)n * nrg_src];
     }
     await_predecessor();   // launched early it must not end before what came before
 }
@@ -310,12 +322,14 @@ cudaError_t launch_prep_map(const DevProblem &P, const float *a1, const float *a
                             PrepBuffers &B, cudaStream_t s, int64_t *launches, const float *S1, const float *spec,
                             const int *win_lo, float *rf_win, bool early)
 {
-    // one block of 1024 threads per tile of 32 x 32 cells
-    const int64_t blocks = (int64_t)((P.nx + 1 + 31) / 32) * ((P.ny + 1 + 31) / 32);
+    // one block of 1024 threads per tile of 32 x 32 cells, and up to eight for
+    // the tables
+    const int tiles = ((P.nx + 1 + 31) / 32) * ((P.ny + 1 + 31) / 32);
+    const int ns2 = S2 ? P.nq * P.na : 0, W = 2 * P.dnrg + 1, nrf = rf_win ? P.nrg_det * W : 0;
+    const int more = std::min(8, (std::max(ns2, nrf) + 1023) / 1024);
     if (launches) (*launches)++;
-    return launch_after(k_build_cells, (int)blocks, 1024, 0, s, early, P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8,
-                        S2 ? P.nq * P.na : 0, B.s1u8 ? S1 : nullptr, B.s1u8, spec, win_lo, rf_win, P.nrg_src,
-                        rf_win ? P.nrg_det * (2 * P.dnrg + 1) : 0, 2 * P.dnrg + 1);
+    return launch_after(k_build_cells, tiles + more, 1024, 0, s, early, P.nx, P.ny, a1, a2, B.cells, S2, B.s2u8, ns2,
+                        B.s1u8 ? S1 : nullptr, B.s1u8, spec, win_lo, rf_win, P.nrg_src, nrf, W, tiles);
 }
 
 cudaError_t launch_list_voxels(const DevProblem &P, const int32_t *seg, PrepBuffers &B, cudaStream_t s,

@@ -67,6 +67,7 @@ k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list
     // 2^lg_split neighbouring lanes share a ray's samples
     const int split = 1 << lg_split, sub = lane & (split - 1);
     await_predecessor();
+    allow_dependents();   // (not before: the next kernel may then take every earlier result as written)
     const int64_t ncell = (int64_t)(P.nx + 1) * (P.ny + 1);
     const unsigned ncell_m1 = (unsigned)(ncell - 1);
     const float4 *cells_t = cells + 2 * ncell;   // column-major copy
