@@ -42,11 +42,12 @@
 //
 // Both are bound by instruction issue.  The bins of a window come from a table
 // over the wavevector axis (VoxOp::qlut) instead of two square roots and
-// quotients.  Measured on 128x128 voxels, 32 views x 128 px, 40 energies, 32 bins:
-// forward 5.5 ms, 10.1 with lane = energy; 7.9 before the scattering geometry lost
+// quotients, whose index is clamped by the addition that forms it.  Measured on
+// 128x128 voxels, 32 views x 128 px, 40 energies, 32 bins: forward 5.3 ms (5.5 with
+// integer clamps and renormalised pairs), 10.1 with lane = energy; 7.9 before the scattering geometry lost
 // its component-wise form (vox_geom) and the coefficients' transposition moved
 // out of the tiles.  Adjoint of 96x78 voxels, 27 views x 110 px, 40 energies, 40
-// bins: 2.2 ms, 8.7 with lane = energy for the terms, scans over the energies for
+// bins: 2.1 ms (2.2), 8.7 with lane = energy for the terms, scans over the energies for
 // each bin's range and lane = bin for the sums; 3.8 with compensated sums in
 // shared memory, one energy per visit to a bin.
 #include "scatter.cuh"
@@ -82,17 +83,16 @@ __device__ __forceinline__ EnergyTerm energy_term(const VoxEnergy &q, const VoxT
     // exp(-X) with 1/f1 and 1/f2 as pairs in units of log2
     const float low = fmaf(v.ax.hi, q.f1l, fmaf(v.ay.hi, q.f2l, fmaf(v.ax.lo, q.f1, v.ay.lo * q.f2)));
     const float PP = ex2_approx(fmaf(v.ax.hi, q.f1, fmaf(v.ay.hi, q.f2, low)));
-    const float w = __fmul_rn(q.wh, v.sh);
-    const float wr = fmaf(q.wh, v.sh, -w) + fmaf(q.wh, v.sl, q.wl * v.sh);
-    t.w_hi = w + wr;
-    t.w_lo = wr - (t.w_hi - w);
+    // (the pairs here stay as they come out: their low parts are an ulp or two
+    // of the high ones, and every use takes both)
+    t.w_hi = __fmul_rn(q.wh, v.sh);
+    t.w_lo = fmaf(q.wh, v.sh, -t.w_hi) + fmaf(q.wh, v.sl, q.wl * v.sh);
     // sigma^2 as a pair: deep in the Gaussian's tail the exponent amplifies
     // its relative error by (q distance / sigma)^2 / 2
     const float p = __fmul_rn(q.c2, v.b.hi);
     const float e = fmaf(q.c2, v.b.lo, fmaf(q.c2l, v.b.hi, fmaf(q.c2, v.b.hi, -p)));
     ff s2 = two_sum(v.t1.hi, p);
     s2.lo += e + v.t1.lo;
-    s2 = fast_two_sum(s2.hi, s2.lo);
     // 1/sigma to within an ulp: one Newton step on rsqrt, with the low part
     const float r0 = rsqrt_approx(s2.hi);
     const float h = fmaf(-0.5f * s2.hi * r0, r0, 0.5f) - 0.5f * s2.lo * r0 * r0;
@@ -122,16 +122,37 @@ __device__ __forceinline__ VoxTerm vox_term(const PairGeom &G, const F32Consts &
     return v;
 }
 
-// The first and last coarse bin that may lie within `half` of w: the table's
-// cells of both ends, entry 0 below the grid and kLutCells + 1 above it.
-__device__ __forceinline__ void bin_window(const unsigned *lut, float scale, float q_lo, float w, float half, int *k0,
-                                           int *k1)
+// The window table as the kernels index it: entry round(M u) of shared memory,
+// u = w scale + offset clamped to [0, 1] by the addition that forms it.
+struct WindowTable {
+    float scale, offset;   // ((w - q_lo) cells + 1/2) / M
+    uint32_t base;         // address of entry 0, less the magic number's bits
+};
+constexpr float kLutM = (float)(kLutCells + 1);
+
+__device__ __forceinline__ WindowTable window_table(const unsigned *lut, float scale, float q_lo)
 {
-    // round(x + 1/2) through the float mantissa
-    const float x0 = fmaf((w - half) - q_lo, scale, 0.5f), x1 = fmaf((w + half) - q_lo, scale, 0.5f);
-    const int i0 = __float_as_int(x0 + 12582912.f) - 0x4B400000, i1 = __float_as_int(x1 + 12582912.f) - 0x4B400000;
-    *k0 = (int)(lut[max(0, min(i0, kLutCells + 1))] & 0xffffu);
-    *k1 = (int)lut[max(0, min(i1, kLutCells + 1))] >> 16;
+    WindowTable t;
+    t.scale = scale * (1.f / kLutM);
+    t.offset = fmaf(-q_lo, t.scale, 0.5f / kLutM);
+    t.base = (uint32_t)__cvta_generic_to_shared(lut) - (0x4B400000u << 2);
+    return t;
+}
+
+// The first and last coarse bin that may lie within `half` (times the table's
+// scale) of w: the table's cells of both ends, entry 0 below the grid and
+// kLutCells + 1 above it.
+__device__ __forceinline__ void bin_window(const WindowTable &L, float w, float half, int *k0, int *k1)
+{
+    const float x = fmaf(w, L.scale, L.offset);
+    // to the nearest entry through the float mantissa
+    const uint32_t i0 = __float_as_uint(fmaf(__saturatef(x - half), kLutM, 12582912.f));
+    const uint32_t i1 = __float_as_uint(fmaf(__saturatef(x + half), kLutM, 12582912.f));
+    unsigned short lo, hi;   // the entry's halves: first bin, last bin
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(lo) : "r"(L.base + (i0 << 2)));
+    asm volatile("ld.shared.s16 %0, [%1+2];" : "=h"(hi) : "r"(L.base + (i1 << 2)));
+    *k0 = lo;
+    *k1 = (short)hi;
 }
 
 // 2^(c (w - q)^2) at two neighbouring bins, q = (hi, hi, lo, lo): the
@@ -240,7 +261,8 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
         reinterpret_cast<int *>(&pair)[i] = reinterpret_cast<const int *>(J.op.pairs + pidx)[i];
     for (int i = tid; i < E * H; i += kFwdThreads) TNs[i] = make_float2(0.f, 0.f);
     const ff c1 = {J.op.c1, J.op.c1l};
-    const float scale = J.op.lut_scale, q_lo = J.c.q_lo;
+    const WindowTable window = window_table(lut, J.op.lut_scale, J.c.q_lo);
+    const float half_sig = kSig * window.scale;
     const int x_row = L.xstride;
 
     for (int tile = 0; tile < J.tiles; tile++) {
@@ -285,7 +307,7 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
                 const VoxTerm v = {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
                 const EnergyTerm t = energy_term(q, v);
                 int k0, k1;
-                bin_window(lut, scale, q_lo, t.w_hi, kSig * t.sigma, &k0, &k1);
+                bin_window(window, t.w_hi, half_sig * t.sigma, &k0, &k1);
                 if (k0 <= k1 && t.pref != 0.f) {   // pref 0: attenuation underflow, no contribution
                     float2 acc = make_float2(0.f, 0.f);
                     const float2 *x2 = (const float2 *)xs + i;
@@ -446,7 +468,8 @@ k_vox_adj(const VoxBatch B)
         const int v = min(chunk * 32 + lane, nv - 1);   // a lane past the last voxel repeats it
         const int xy = J.op.vox_xy[v];
         const ff c1 = {J.op.c1, J.op.c1l};
-        const float scale = J.op.lut_scale, q_lo = J.c.q_lo;
+        const WindowTable window = window_table(lut, J.op.lut_scale, J.c.q_lo);
+        const float half_sig = kSigAdj * window.scale;
         // this lane's column of the partial row: sums of two bins and their low parts
         float4 *row = J.part + ((int64_t)by * chunks + chunk) * K2 * 32 + lane;
         for (int k = 0; k < K2; k++) sums[32 * k] = make_float2(0.f, 0.f);
@@ -471,8 +494,8 @@ k_vox_adj(const VoxBatch B)
                 const float ct = ws[el] * t.pref, cu = el + 1 < E ? ws[e1] * u.pref : 0.f;
                 // the bins within 13.25 sigma: every term FP32 can represent
                 int k0, k1, l0, l1;
-                bin_window(lut, scale, q_lo, t.w_hi, kSigAdj * t.sigma, &k0, &k1);
-                bin_window(lut, scale, q_lo, u.w_hi, kSigAdj * u.sigma, &l0, &l1);
+                bin_window(window, t.w_hi, half_sig * t.sigma, &k0, &k1);
+                bin_window(window, u.w_hi, half_sig * u.sigma, &l0, &l1);
                 if (ct == 0.f || k0 > k1) k0 = 0xffff, k1 = -1;
                 if (cu == 0.f || l0 > l1) l0 = 0xffff, l1 = -1;
                 k0 = min(k0, l0) >> 1;
