@@ -814,6 +814,23 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         CK(launch_prep_map(P, (const float *)d_a1, (const float *)d_a2, (const float *)d_S2, B, st, &ctx->launches,
                            (const float *)d_S1, (const float *)d_spec, T.win_lo, (float *)tmp, true));
     }
+    // The pairs of a tile: whole groups of 32 pixels of every view (32 entries of a
+    // list), as many as the walk's table has room for.
+    const int64_t unit = ray_list ? 32 : 32 * (int64_t)p->n_src;
+    auto tile_pairs = [&](int64_t voxels, int64_t n_total) {
+        const int64_t fit = std::min<int64_t>(kWalkTableBytes / (voxels * (int64_t)sizeof(float2)), (int64_t)1 << 30);
+        return std::min<int64_t>(n_total, std::max<int64_t>(unit, fit / unit * unit));
+    };
+    // when one tile holds every pair however many voxels there are, the pairs'
+    // records need not wait for the count
+    const int64_t all_pairs = (int64_t)p->n_src * P.n_det;
+    const bool pairs_first = !plain && !ray_list && tile_pairs(nvox, all_pairs) == all_pairs;
+    void *drec = nullptr;
+    if (pairs_first) {
+        if ((rc = get_buf(ctx, S_PREC, pair_rec_bytes() * (size_t)all_pairs, &drec))) return rc;
+        ProfScope ps(ctx, XRDT_KERNEL_WALK);
+        CK(launch_pair_table(P, d_srcg, nullptr, 0, all_pairs, (PairRec *)drec, st, &ctx->launches, true));
+    }
     // (a stream in capture refuses the wait, and the call ends as a refused capture)
     if (cudaEventSynchronize(ctx->counted) != cudaSuccess) {
         cudaGetLastError();
@@ -864,23 +881,19 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         // pairs go through in tiles: the detector-side integrals of a tile
         // (k_walk.cu), then the projector over the same pairs
         auto project = [&](const int2 *list, int64_t n_total, float *oN, float *oC, float *oA) -> int {
-            // whole groups of 32 pixels of every view (32 entries of a list)
-            const int64_t unit = list ? 32 : 32 * (int64_t)p->n_src;
-            const int64_t fit = std::min<int64_t>(kWalkTableBytes / ((int64_t)nv * (int64_t)sizeof(float2)),
-                                                  (int64_t)1 << 30);
-            const int64_t tile = std::min<int64_t>(n_total, std::max<int64_t>(unit, fit / unit * unit));
+            const int64_t tile = tile_pairs(nv, n_total);
             void *dtab;
             int r = get_buf(ctx, S_WALK, sizeof(float2) * (size_t)tile * nv, &dtab);
             if (r) return r;
-            void *drec;
             if ((r = get_buf(ctx, S_PREC, pair_rec_bytes() * (size_t)tile, &drec))) return r;
             const PairRec *recs = (const PairRec *)drec;
             for (int64_t p0 = 0; p0 < n_total; p0 += tile) {
                 const int64_t n = std::min(tile, n_total - p0);
                 {
                     ProfScope ps(ctx, XRDT_KERNEL_WALK);
-                    CK(launch_pair_table(P, d_srcg, list ? list + p0 : nullptr, p0, n,
-                                         (PairRec *)drec, st, &ctx->launches, !list && p0 == 0));
+                    if (!pairs_first)
+                        CK(launch_pair_table(P, d_srcg, list ? list + p0 : nullptr, p0, n,
+                                             (PairRec *)drec, st, &ctx->launches, !list && p0 == 0));
                     CK(launch_det_walk(P, recs, list != nullptr, n, B.vox_xy, nv, B.cells, (float2 *)dtab, st,
                                        &ctx->launches, true));
                 }

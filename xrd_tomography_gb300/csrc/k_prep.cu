@@ -58,6 +58,7 @@ k_build_cells(int nx, int ny, const float *__restrict__ a1, const float *__restr
                               const int *__restrict__ win_lo, float *__restrict__ rf_win, int nrg_src, int nrf, int W,
                               int tiles)
 {
+    allow_dependents();
     if ((int)blockIdx.x >= tiles) {
         // ---- the blocks behind the cells: the tables ----
         const int i0 = ((int)blockIdx.x - tiles) * blockDim.x + threadIdx.x;
