@@ -25,9 +25,10 @@
 //
 //  * forward (k_vox_fwd): one item = one (source, pixel) pair, as in
 //    k_fwd.cu: tiles of voxels with their scattering geometry and their
-//    coefficients x[v, k] dq_k in shared memory, runs of 32-voxel steps of one
-//    energy off a counter, lane = voxel; a lane sums the coarse bins within
-//    7.5 sigma of its wavevector transfer, two per instruction.  The banded
+//    coefficients x[v, k] dq_k in shared memory, runs of 32-voxel steps of two
+//    neighbouring energies off a counter, lane = voxel; a lane sums the coarse
+//    bins within 7.5 sigma of either wavevector transfer, two per instruction,
+//    and reads a voxel's constants and a bin's coefficient once for both.  The banded
 //    spectrum weights give the detector bins.  In MLEM mode the block goes on
 //    to form the ratios y / (Av x + c + 1e-20) of main.m:162 for its detector
 //    bins and folds them back through the same weights, what[pair, e].
@@ -43,7 +44,8 @@
 // Both are bound by instruction issue.  The bins of a window come from a table
 // over the wavevector axis (VoxOp::qlut) instead of two square roots and
 // quotients, whose index is clamped by the addition that forms it.  Measured on
-// 128x128 voxels, 32 views x 128 px, 40 energies, 32 bins: forward 5.3 ms (5.5 with
+// 128x128 voxels, 32 views x 128 px, 40 energies, 32 bins: forward 4.6 ms (5.3 with
+// one energy at a time, which kept shared memory busy 58 % of the time; 5.5 with
 // integer clamps and renormalised pairs), 10.1 with lane = energy; 7.9 before the scattering geometry lost
 // its component-wise form (vox_geom) and the coefficients' transposition moved
 // out of the tiles.  Adjoint of 96x78 voxels, 27 views x 110 px, 40 energies, 40
@@ -56,6 +58,9 @@ namespace xrdt {
 
 namespace {
 
+// Two blocks of 8 warps per SM at 128 registers: two energies at a time spill at
+// 80 (three blocks: 4.9 ms against 4.75 at 128x128, 4.6 with the larger tiles; 10
+// and 12 warps 4.6 and 5.0).
 constexpr int kFwdWarps = 8;
 constexpr int kFwdThreads = 32 * kFwdWarps;
 constexpr int kMaxSteps = 24;   // 32-voxel steps of a tile
@@ -291,36 +296,54 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        // ---- lane = voxel: runs of 32-voxel steps of one energy, the widest windows first ----
+        // ---- lane = voxel: runs of 32-voxel steps of two neighbouring energies,
+        // the widest windows first ----
+        const int EP = (E + 1) >> 1;
         for (;;) {
             int item = 0;
             if (lane == 0) item = atomicAdd(&next_run, 1);
             item = __shfl_sync(0xffffffffu, item, 0);
-            if (item >= E * H) break;
-            const int el = E - 1 - item / H, row = el * H + item % H;
-            const int s0 = item % H * run_len, s1 = min(s0 + run_len, steps);
-            const VoxEnergy q = load_energy(en, el);
-            float sum = 0.f;
+            if (item >= EP * H) break;
+            const int el = 2 * (EP - 1 - item / H), run = item % H;
+            const int two = el + 1 < E;   // 0: the second energy is the first again, not kept
+            const int s0 = run * run_len, s1 = min(s0 + run_len, steps);
+            const VoxEnergy q = load_energy(en, el), q1 = load_energy(en, el + two);
+            float sum = 0.f, sum1 = 0.f;
             for (int st = s0; st < s1; st++) {
                 const int i = 32 * st + lane;
                 const float4 r0 = rec[i], r1 = rec[32 * nst + i], r2 = rec[64 * nst + i];
                 const VoxTerm v = {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
-                const EnergyTerm t = energy_term(q, v);
-                int k0, k1;
+                const EnergyTerm t = energy_term(q, v), u = energy_term(q1, v);
+                // Both take the bins of both windows, which lie a source bin
+                // apart: a fraction of their length, as sigma holds the width of
+                // the source bin.  (pref 0: attenuation underflow, no contribution)
+                int k0, k1, l0, l1;
                 bin_window(window, t.w_hi, half_sig * t.sigma, &k0, &k1);
-                if (k0 <= k1 && t.pref != 0.f) {   // pref 0: attenuation underflow, no contribution
-                    float2 acc = make_float2(0.f, 0.f);
+                bin_window(window, u.w_hi, half_sig * u.sigma, &l0, &l1);
+                if (k0 > k1) k0 = 0xffff, k1 = -1;
+                if (l0 > l1) l0 = 0xffff, l1 = -1;
+                k0 = min(k0, l0) >> 1;
+                k1 = max(k1, l1) >> 1;
+                if (k0 <= k1 && (t.pref != 0.f || u.pref != 0.f)) {
+                    float2 acc = make_float2(0.f, 0.f), bcc = make_float2(0.f, 0.f);
                     const float2 *x2 = (const float2 *)xs + i;
-                    for (int k = k0 >> 1; k <= k1 >> 1; k++)
-                        acc = __ffma2_rn(gauss2(t, cq[k]), x2[k * (x_row >> 1)], acc);
+                    for (int k = k0; k <= k1; k++) {
+                        const float4 b = cq[k];
+                        const float2 x = x2[k * (x_row >> 1)];
+                        acc = __ffma2_rn(gauss2(t, b), x, acc);
+                        bcc = __ffma2_rn(gauss2(u, b), x, bcc);
+                    }
                     sum = fmaf(t.pref, acc.x + acc.y, sum);
+                    sum1 = fmaf(u.pref, bcc.x + bcc.y, sum1);
                 }
             }
             sum = warp_sum(sum);
-            if (lane == 0) {
-                float2 k = TNs[row];
-                kahan_add(k.x, k.y, sum);
-                TNs[row] = k;
+            sum1 = warp_sum(sum1);
+            if (lane <= two) {
+                const int at = (el + lane) * H + run;
+                float2 k = TNs[at];
+                kahan_add(k.x, k.y, lane ? sum1 : sum);
+                TNs[at] = k;
             }
         }
     }
@@ -360,7 +383,7 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
 
 // Persistent forward over the pairs of every job (offsets off[0 .. n]).
 template <bool MLEM>
-__global__ void __launch_bounds__(kFwdThreads, 3)
+__global__ void __launch_bounds__(kFwdThreads, 2)
 k_vox_fwd(const VoxBatch B)
 {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -761,7 +784,7 @@ size_t vox_limit_smem(const DevProblem &P)
            sizeof(PairRec) + sizeof(float) * E + 16 + sizeof(int2) * E + 2 * K;
 }
 
-// The forward's tiles and runs: as many voxels per tile as three blocks per SM
+// The forward's tiles and runs: as many voxels per tile as two blocks per SM
 // leave room for (up to 768; a voxel takes 48 bytes and 4 per coarse bin), fewer
 // blocks only where not even one step of 32 voxels would fit; four runs or
 // more per warp.  They depend on the problem alone, so that a batch gives
@@ -772,12 +795,12 @@ size_t vox_fwd_split(const DevProblem &P, int nv, int *steps, int *tiles, int *r
     const int chunks = nv > 0 ? (nv + 31) / 32 : 1;
     const size_t stat = vox_fwd_static_smem() + 1024;
     auto runs_of = [&](int st) {
-        const int r = (4 * kFwdWarps + E - 1) / E;
+        const int ep = (E + 1) / 2, r = (4 * kFwdWarps + ep - 1) / ep;
         return r < 1 ? 1 : (r > st ? st : r);
     };
     int cap = 1;
     for (int st = 2; st <= kMaxSteps; st++)
-        if (vox_fwd_layout(P, E, st, runs_of(st)).total + stat <= 76 * 1024) cap = st;
+        if (vox_fwd_layout(P, E, st, runs_of(st)).total + stat <= 113 * 1024) cap = st;
     *tiles = (chunks + cap - 1) / cap;
     *steps = (chunks + *tiles - 1) / *tiles;
     *runs = runs_of(*steps);
