@@ -15,11 +15,13 @@
 // groups of 32 bins that none of the four windows (7.5 sigma) reaches.  Sums
 // stay in registers while the material stays the same.
 //
-// Bound by FMA and instruction issue: about half of the bins evaluated lie
-// beyond 7.5 sigma of their own term, and the two packed pair differences and
-// products cost more than the exp2.  64x64 voxels, 32 views x 128 px, 40
-// energies, 4 materials x 64 bins, the projection (1.9 ms) included: 6.2 ms; two
-// voxels at a time instead of four 8.0 ms; lane = energy with shared-memory float
+// Bound by instruction issue: about half of the bins evaluated lie beyond 7.5
+// sigma of their own term, the two packed pair differences and products cost
+// more than the exp2, and four voxels' window tests and materials nearly as much
+// again.  64x64 voxels, 32 views x 128 px, 40 energies, 4 materials x 64 bins: 3.5
+// ms, and 3.8 with the groups' range compared per group instead of a bit each;
+// the projection (1.8 ms) included 5.8 ms; two voxels at a time instead of four
+// (6.2 then) 8.0 ms; lane = energy with shared-memory float
 // atomics per (energy, material, bin) -- compare-and-swap loops here -- 21.4 ms.
 #include <algorithm>
 
@@ -33,8 +35,8 @@ constexpr int kMaxMatrixWarps = 24;
 static_assert(sizeof(PairRec) + 16 <= 256, "the static part of a block's shared memory");
 
 // words of four voxels' terms: pref, w_hi, w_lo and the exponent's scale of each
-// voxel, then the bin groups they reach (first | last << 16, -1: none), their
-// common material (-1: they differ) and the four materials; a stride of 20 words
+// voxel, then the bin groups of the pass they reach (a bit each), their common
+// material (-1: they differ) and the four materials; a stride of 20 words
 // keeps the stores of lane = voxel free of bank conflicts
 constexpr int kQuad = 20;
 
@@ -174,21 +176,17 @@ k_matrix(const MatrixArgs args)
                             const float sig2 = fmaf(er.sig_c2, r0.z, er.sig_c1 * (sh * sh));
                             const float rs = rsqrt_approx(sig2);
                             const float pref = PP * r0.w * rs;
-                            int g0 = 0x7fff, g1 = -1;
+                            // bit g: the window reaches group gb + g
+                            unsigned groups = 0;
                             if (pref != 0.f) {
                                 int klo, khi;
                                 coarse_window(w_hi, kSig * sig2 * rs, c.q_lo, c.qpar_a, c.qpar_b, K, &klo, &khi);
-                                if (klo <= khi) {
-                                    g0 = klo >> 5;
-                                    g1 = khi >> 5;
-                                }
+                                const int g0 = max((klo >> 5) - gb, 0), g1 = min((khi >> 5) - gb, NG - 1);
+                                if (klo <= khi && g0 <= g1) groups = (2u << g1) - (1u << g0);
                             }
-                            if (g1 < 0) g0 = 0x7fff;
-                            const float pr = g1 < 0 ? 0.f : pref;
-                            g0 = min(g0, __shfl_xor_sync(0xffffffffu, g0, 1));
-                            g0 = min(g0, __shfl_xor_sync(0xffffffffu, g0, 2));
-                            g1 = max(g1, __shfl_xor_sync(0xffffffffu, g1, 1));
-                            g1 = max(g1, __shfl_xor_sync(0xffffffffu, g1, 2));
+                            const float pr = groups ? pref : 0.f;
+                            groups |= __shfl_xor_sync(0xffffffffu, groups, 1);
+                            groups |= __shfl_xor_sync(0xffffffffu, groups, 2);
                             const int m0 = __float_as_int(r1.z), m1 = __shfl_xor_sync(0xffffffffu, m0, 1);
                             const int m01 = m0 | m1 << 16, m23 = __shfl_xor_sync(0xffffffffu, m01, 2);
                             __syncwarp();   // the last step's terms have been read
@@ -199,17 +197,16 @@ k_matrix(const MatrixArgs args)
                             t[12] = -0.5f * kLog2e * rs * rs;
                             if (!(lane & 3)) {
                                 const bool same = m01 == m23 && m0 == m1;
-                                *(int4 *)(t + 16) = make_int4(g1 < 0 ? -1 : g0 | g1 << 16, same ? m0 : -1, m01, m23);
+                                *(int4 *)(t + 16) = make_int4((int)groups, same ? m0 : -1, m01, m23);
                             }
                             __syncwarp();
                         }
                         // lane = coarse bin: four voxels at a time
+#pragma unroll 2
                         for (int v = 0; v < 8; v++) {
                             const float4 *t = (const float4 *)(term + kQuad * v);
                             const int4 info = *(const int4 *)(t + 4);
-                            if (info.x < 0) continue;   // no window holds a bin
-                            const int g0 = (info.x & 0xffff) - gb, g1 = (info.x >> 16) - gb;
-                            if (g1 < 0 || g0 >= NG) continue;
+                            if (!info.x) continue;   // no window reaches these groups
                             const float4 pr = t[0], wh = t[1], wl = t[2], sc = t[3];
                             // the Gaussians of two voxels at a bin
                             auto gauss = [&](float2 h, float2 l, float2 c2, float b, float bl) {
@@ -225,7 +222,7 @@ k_matrix(const MatrixArgs args)
                                 }
 #pragma unroll
                                 for (int g = 0; g < NG; g++)
-                                    if (g0 <= g && g <= g1) {
+                                    if (info.x & 1 << g) {
                                         acc[g] = __ffma2_rn(make_float2(pr.x, pr.y),
                                                             gauss(make_float2(wh.x, wh.y), make_float2(wl.x, wl.y),
                                                                   make_float2(sc.x, sc.y), qh[g], ql[g]),
@@ -241,7 +238,7 @@ k_matrix(const MatrixArgs args)
 #pragma unroll
                                 for (int g = 0; g < NG; g++) {
                                     const int k = 32 * (gb + g) + lane;
-                                    if (g0 <= g && g <= g1 && k < K) {
+                                    if ((info.x & 1 << g) && k < K) {
                                         const float2 a = gauss(make_float2(wh.x, wh.y), make_float2(wl.x, wl.y),
                                                                make_float2(sc.x, sc.y), qh[g], ql[g]);
                                         const float2 b = gauss(make_float2(wh.z, wh.w), make_float2(wl.z, wl.w),
