@@ -48,10 +48,10 @@ FLUSH_BYTES = 256 << 20
 # ncu capture of a single launch on the 128x128 workload (4096 pairs x 5009
 # voxels); the traffic is the launch's walk table plus a fixed part, so the
 # 256x256 figure below is that rate times the pair-voxels of its mean launch
-K_FWD_DRAM_BYTES_PER_PAIR_VOXEL = (166727936 + 4232704) / (4096 * 5009)   # 8.33 B (read + write)
+K_FWD_DRAM_BYTES_PER_PAIR_VOXEL = (166310400 + 4509952) / (4096 * 5009)   # 8.33 B (read + write)
 # issue slots busy in k_fwd (ncu, the same capture): the kernel is bound by
 # instruction issue, not by the SFU rate of the roofline below
-K_FWD_ISSUE_BUSY = 0.8392
+K_FWD_ISSUE_BUSY = 0.7981
 
 
 def parse():
@@ -304,7 +304,7 @@ def mlem_stored_bench(xt, synth, ctx, stream, dev, iters=200):
     peak, src = hbm_peak_gbs()
     gbs = traffic / (per_iter_ms * 1e-3) / 1e9
     return {"workload": f"explicit model matrix of the 64x64 workload: {p.rays} rays x {K} coefficients "
-                        f"({a_bytes / 1e6:.0f} MB), {iters} iterations, CUDA-graph replay",
+                        f"({a_bytes / 1e6:.0f} MB), {iters} iterations; part of A is still in L2 from the pass before",
             "iter_per_s": 1e3 / per_iter_ms, "ms_per_iter": per_iter_ms,
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
                          "traffic": None, "algorithmic_bytes_per_iter": traffic, "peak_source": src}}

@@ -304,8 +304,8 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
  * reshape).  y[rays] are measured counts, c[rays] the Compton bias
  * (main.m:162 uses Cphotons(:)).  K must be a multiple of 4, at most 1024;
  * device arrays A and x must be 16-byte aligned (XRDT_ERR_UNSUPPORTED).
- * The iteration body is a fused pass over A (one read of A per iteration)
- * and an FP64 reduction/update, replayed as a CUDA graph. */
+ * The iteration body is a fused pass over A (one read of A per iteration, the
+ * first of which also sums sum(A,1)) and an FP64 reduction/update. */
 int32_t xrdt_mlem_matrix(xrdt_ctx *ctx, const float *A, int64_t rays, int32_t K,
                          const float *y, const float *c, float *x, int32_t iters,
                          uint32_t flags);
