@@ -24,15 +24,16 @@
 //  * passes go over a warp's rows forwards and backwards in turn, so that what
 //    a pass read last, still in L2, is what the next one reads first (131072 x
 //    256: 500 -> 440 us for ten iterations, with the loop as it then was).
-// 131072 x 256, ten iterations: 217 us, against 198 for ten readings of A from
+// 131072 x 256, ten iterations: 220 us, against 198 for ten readings of A from
 // HBM; with loads into registers, 11 passes and separate launches 344.
-// 100000 x 64: 202 -> 87, 500 x 32: 99 -> 50 (the launches), 300000 x 256, five
-// iterations: 353 -> 237, 40000 x 1024, ten: 322 -> 267.  A row per warp with
+// 100000 x 64: 202 -> 90, 500 x 32: 99 -> 51 (the launches), 300000 x 256, five
+// iterations: 353 -> 239, 40000 x 1024, ten: 322 -> 265.  A row per warp with
 // its own division and reductions, and 64-bit addresses formed per row, issued
 // twice the instructions: 425 us on the first.
 #include <algorithm>
 
 #include "xrdt_device.cuh"
+#include "ff.cuh"
 
 namespace xrdt {
 
@@ -150,8 +151,8 @@ k_mlem_pass(const float *__restrict__ A, long long rays, int K, const float *__r
     bool on;
     auto load_yc = [&]() {
         on = yvisit < mine && (G == 1 || yrow < rays);
-        yn = on ? __ldg(y + yrow) : 0.f;
-        cn = on ? __ldg(c + yrow) : 0.f;
+        yn = on ? __ldcg(y + yrow) : 0.f;
+        cn = on ? __ldcg(c + yrow) : 0.f;
         yrow += P * drow;
         yvisit += P;
     };
@@ -191,14 +192,27 @@ k_mlem_pass(const float *__restrict__ A, long long rays, int K, const float *__r
         }
         const float sum = sum_lanes<L, P>(t, lane);
         const float own_ratio = oc ? yc / (sum + cc + 1e-20f) : 0.f;
+        // a step's rows add up among themselves first: the long sums then round
+        // once per step
+        float4 add[KC], ones[FIRST ? KC : 1];
 #pragma unroll
         for (int p = 0; p < P; p++) {
             const float ratio = L == 1 ? own_ratio : __shfl_sync(0xffffffffu, own_ratio, (lane & ~(L - 1)) + p * (L / P));
 #pragma unroll
             for (int i = 0; i < KC; i++) {
-                add4(g[i], ratio, a[p][i]);
-                if (FIRST) add4(h[i], 1.f, a[p][i]);
+                if (p == 0) {
+                    add[i] = make_float4(ratio * a[0][i].x, ratio * a[0][i].y, ratio * a[0][i].z, ratio * a[0][i].w);
+                    if (FIRST) ones[i] = a[0][i];
+                } else {
+                    add4(add[i], ratio, a[p][i]);
+                    if (FIRST) add4(ones[i], 1.f, a[p][i]);
+                }
             }
+        }
+#pragma unroll
+        for (int i = 0; i < KC; i++) {
+            add4(g[i], 1.f, add[i]);
+            if (FIRST) add4(h[i], 1.f, ones[i]);
         }
         free_slot = slot;
         slot = slot == S::kSteps - 1 ? 0 : slot + 1;
@@ -225,10 +239,19 @@ k_mlem_pass(const float *__restrict__ A, long long rays, int K, const float *__r
     for (int j = threadIdx.x; j < (FIRST ? 2 : 1) * KC * L; j += S::kWarps * 32) {
         const int at = j / (KC * L), q = j - at * KC * L;   // chunk q of the row
         if (q >= K4) continue;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int w = 0; w < S::kWarps; w++)
-            add4(s, 1.f, ring[((at * S::kWarps + w) * KC + q / L) * 32 + (q & (L - 1))]);
-        reinterpret_cast<float4 *>(partial + ((size_t)at * gridDim.x + blockIdx.x) * K)[q] = s;
+        // (as float pairs: a partial row is rounded once)
+        ff s[4] = {};
+        for (int w = 0; w < S::kWarps; w++) {
+            const float4 v = ring[((at * S::kWarps + w) * KC + q / L) * 32 + (q & (L - 1))];
+            const float t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const ff u = two_sum(s[i].hi, t[i]);
+                s[i] = ff{u.hi, s[i].lo + u.lo};
+            }
+        }
+        const float4 sum = make_float4(s[0].hi + s[0].lo, s[1].hi + s[1].lo, s[2].hi + s[2].lo, s[3].hi + s[3].lo);
+        reinterpret_cast<float4 *>(partial + ((size_t)at * gridDim.x + blockIdx.x) * K)[q] = sum;
     }
 }
 
