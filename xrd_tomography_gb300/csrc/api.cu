@@ -275,15 +275,8 @@ F32Consts make_f32_consts(const DevProblem &P)
     c.nxf = (float)P.nx;
     c.nyf = (float)P.ny;
     c.rsqrt2pi = (float)P.rsqrt2pi;
-    c.dqf_hi = (float)P.dq_fine;
-    c.dqf_lo = (float)(P.dq_fine - (double)c.dqf_hi);
-    c.inv_dqf = (float)(1.0 / P.dq_fine);
     c.q_lo = (float)P.q_lo;
-    c.q_hi = (float)P.q_hi;
     c.kn0 = (float)P.kn0;
-    c.kn1 = (float)P.kn1;
-    c.kn2 = (float)P.kn2;
-    c.edmin = (float)P.e_det_min;
     c.inv_dEd = (float)(1.0 / P.dEd);
     c.inv_dEs = (float)(1.0 / P.dEs);
     c.dEd = (float)P.dEd;
@@ -315,11 +308,6 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         r.Esrc2 = P.e_src_min + (double)(e + 1) * P.dEs;
         r.Esrc = 0.5 * (r.Esrc1 + r.Esrc2);
         r.ein = r.Esrc / P.mec2;
-        const double f1 = r.ein * r.ein * r.ein, f2 = P.kn0 + P.kn1 * r.ein + P.kn2 * r.ein * r.ein;
-        r.inv_f1 = (float)(1.0 / f1);
-        r.inv_f2 = (float)(1.0 / f2);
-        r.inv_f1_lo = (float)(1.0 / f1 - (double)r.inv_f1);
-        r.inv_f2_lo = (float)(1.0 / f2 - (double)r.inv_f2);
         const double wf = 2.0 * r.Esrc / P.hbarc;
         r.wfac_hi = (float)wf;
         r.wfac_lo = (float)(wf - (double)r.wfac_hi);
@@ -330,8 +318,6 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         r.sig_c1_lo = (float)(c1 - (double)r.sig_c1);
         r.sig_c2_lo = (float)(c2 - (double)r.sig_c2);
         r.einf = (float)r.ein;
-        r.Esrc1f = (float)r.Esrc1;
-        r.Esrc2f = (float)r.Esrc2;
     }
     // spectrum windows: detector bin n takes source bins win_lo[n] .. + W-1
     // with weights RF = spectrum[e + n*nrg_src]; win_n[e] = the detector bins
@@ -405,12 +391,6 @@ void build_host_tables(const xrdt_problem *p, const DevProblem &P, const float *
         const EnergyRow &r = t->energy[e];
         const FwdEnergy &q = t->fwd_energy[e];
         t->vox_energy[e] = VoxEnergy{q.f1, q.f1l, q.f2, q.f2l, r.wfac_hi, r.wfac_lo, r.sig_c2, r.sig_c2_lo};
-    }
-    t->fine_q.resize(p->nqf);
-    for (int j = 0; j < p->nqf; j++) {
-        const double q = P.q_lo + P.dq_fine * (0.5 + (double)j);
-        t->fine_q[j].x = (float)q;
-        t->fine_q[j].y = (float)(q - (double)t->fine_q[j].x);
     }
     // coarse bins of wvt_value.cu:8-22: centre as a pair, width
     t->coarse_q.resize(p->nwt);
@@ -798,7 +778,6 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         pack.add(ht.offs_e, &T.offs_e);
         pack.add(ht.win_lo, &T.win_lo);
         pack.add(ht.win_n, &T.win_n);
-        pack.add(ht.fine_q, &T.fine_q);
         pack.add(ht.coarse_q, &T.coarse_q);
         T.sl = ht.sl;
     }

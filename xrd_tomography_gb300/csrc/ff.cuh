@@ -26,8 +26,6 @@ __host__ __device__ inline ff ff_from_double(double d)
     return {h, (float)(d - (double)h)};
 }
 
-__device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
-
 __device__ __forceinline__ ff fast_two_sum(float a, float b)
 {
     const float s = a + b;
@@ -74,14 +72,6 @@ __device__ __forceinline__ ff ff_mulf(ff a, float b)
     const float p = a.hi * b;
     float e = fmaf(a.hi, b, -p);
     e = fmaf(a.lo, b, e);
-    return fast_two_sum(p, e);
-}
-
-__device__ __forceinline__ ff ff_sqr(ff a)
-{
-    const float p = a.hi * a.hi;
-    float e = fmaf(a.hi, a.hi, -p);
-    e = fmaf(2.0f * a.hi, a.lo, e);
     return fast_two_sum(p, e);
 }
 

@@ -195,9 +195,6 @@ __device__ __forceinline__ int floor_nc(float x)
     return floor_nc(x, &fl);
 }
 
-// ceil(x) = -floor(-x), same range
-__device__ __forceinline__ int ceil_nc(float x) { return -floor_nc(-x); }
-
 // floor_nc without the clamp, for arguments bounded well inside |x| < 2^22
 // by construction.  Outside that range (infinite or NaN arguments included)
 // the result is an arbitrary int: every caller clamps it into a table or
@@ -211,14 +208,6 @@ __device__ __forceinline__ int floor_bounded(float x, float *fl)
     *fl = up ? r - 1.f : r;
     return up ? i - 1 : i;
 }
-
-__device__ __forceinline__ int floor_bounded(float x)
-{
-    float fl;
-    return floor_bounded(x, &fl);
-}
-
-__device__ __forceinline__ int ceil_bounded(float x) { return -floor_bounded(-x); }
 
 __device__ inline double warp_sum(double v)
 {

@@ -39,9 +39,8 @@ struct DevProblem {
 // at 1/64 of the FP32 rate.
 struct F32Consts {
     float vox, DQ, DQ_lo, inv_DQ, nxf, nyf, rsqrt2pi;
-    float dqf_hi, dqf_lo, inv_dqf, q_lo, q_hi;
-    float kn0, kn1, kn2;
-    float edmin, inv_dEd, dEd, dEs, inv_dEs;
+    float q_lo, kn0;
+    float inv_dEd, dEd, dEs, inv_dEs;
     float qmin_t, inv_dqt, inv_dqg;
     float bin_guard;   // 1/2 minus the error of a Compton table coordinate in FP32, in bins
     float qpar_a, qpar_b;   // coarse bin edges: edge(n) = q_lo + qpar_b n + qpar_a n^2
@@ -57,12 +56,10 @@ struct SrcGeom {
 // Energy-bin table of the source grid (integrate_diffraction.cu:269-292).
 struct EnergyRow {
     double Esrc1, Esrc2, Esrc, ein;
-    float inv_f1, inv_f2;       // 1/ein^3, 1/KN(ein)
     float wfac_hi, wfac_lo;     // 2*Esrc/hbarc as a float pair
     float sig_c1, sig_c2;       // sigma^2 = c1*s^2 + c2*sg/s^2
-    float einf, Esrc1f, Esrc2f;
+    float einf;
     float sig_c1_lo, sig_c2_lo; // low parts of c1, c2 as float pairs
-    float inv_f1_lo, inv_f2_lo; // low parts of 1/ein^3, 1/KN(ein)
 };
 
 // A source bin's constants as the forward projector reads them (k_fwd.cu),
@@ -106,7 +103,6 @@ struct HostTables {
     std::vector<VoxEnergy> vox_energy;   // [nrg_src]
     std::vector<unsigned> qlut;          // [kLutCells + 2]
     float lut_scale = 0.f;          // cells per wavevector unit
-    std::vector<float2> fine_q;     // [nqf]
     std::vector<float4> coarse_q;   // [nwt]
 };
 // spectrum: host copy [nrg_src][nrg_det] column-major as passed to Forward_XRD.
@@ -193,7 +189,6 @@ struct FwdTables {
                                // detector bins whose window holds e
     const int *win_lo;         // [nrg_det] first source bin of each window
     const int *win_n;          // [nrg_src][2] detector bins whose window holds e
-    const float2 *fine_q;      // [nqf] fine q axis as (hi, lo)
     const float4 *coarse_q;    // [nwt] (q_hi, q_lo, dq, 0)
     unsigned long long *work;  // nullable: counts the exp2 evaluations
 };
