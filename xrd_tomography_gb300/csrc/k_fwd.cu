@@ -36,8 +36,8 @@
 // constants loaded for every voxel, a voxel's constants shuffled, a window loop
 // as long as the warp's longest window) 32 terms took about 390 instructions;
 // here they take about 240, and k_fwd went from 12.5 to 7.1 ms on 128x128 voxels,
-// 32 views x 128 px, 40 energies, from 314 to 139 ms on the reference's own sizes
-// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 327 ms
+// 32 views x 128 px, 40 energies, from 314 to 135 ms on the reference's own sizes
+// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 318 ms
 // on 256x256 voxels, 45 views x 512 px, 64 energies.  Two neighbouring energies per
 // step, packed two to an instruction, took 18 % fewer instructions but no less
 // time (7.0, 147 and 314 ms at best): a packed FMA holds its pipe for two cycles.
@@ -64,10 +64,11 @@ constexpr float kMagic = 12582912.f;
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // How a launch is cut: warps per block, 32-voxel steps per energy and tile,
-// columns of the Compton cells, whether the tables sit in shared memory, and
-// the runs an energy's steps of a tile are cut into.
+// columns of the Compton cells, whether the tables sit in shared memory, the
+// highest energies whose steps of a tile are one run, and the runs that those of
+// each other energy are cut into.
 struct FwdSplit {
-    int warps, steps, columns, tables, runs;
+    int warps, steps, columns, tables, whole, runs;
 };
 
 struct Layout {
@@ -174,7 +175,7 @@ k_fwd(const FwdArgs args)
     const F32Consts &c = args.c;
     const int E = args.E, SL = args.sl, W = 2 * P.dnrg + 1;
     const int nw = args.split.warps, nst = args.split.steps, ncol = args.split.columns;
-    const int H = args.split.runs, run_len = (nst + H - 1) / H;
+    const int H = args.split.runs, whole = args.split.whole, run_len = (nst + H - 1) / H;
     const Layout L = fwd_layout(P, E, SL, args.split, TAB);
     float4 *rec = (float4 *)(sm + L.rec);          // [3][32 nst]
     const FwdEnergy *en = (const FwdEnergy *)(sm + L.en);
@@ -285,9 +286,10 @@ k_fwd(const FwdArgs args)
             int item = 0;
             if (lane == 0) item = atomicAdd(&next_run, 1);
             item = __shfl_sync(0xffffffffu, item, 0);
-            if (item >= E * H) break;
-            const int el = E - 1 - item / H, row = el * H + item % H;
-            const int s0 = item % H * run_len, s1 = min(s0 + run_len, steps);
+            if (item >= whole + (E - whole) * H) break;
+            const int part = max(item - whole, 0);   // 0 for an energy in one run
+            const int el = E - 1 - min(item, whole) - part / H, row = el * H + part % H;
+            const int s0 = part % H * run_len, s1 = item < whole ? steps : min(s0 + run_len, steps);
             const FwdEnergy q = en[el];
             const float *orow = offs + el * (SL + 2);
             float accN = 0.f;
@@ -474,7 +476,7 @@ k_fwd(const FwdArgs args)
             for (int j = 0; j < W; j++) {
                 const int el = winlo[n] + j - P.e_lo;
                 float t = 0.f;
-                for (int h = 0; h < H; h++) t += TC[(el * H + h) * SL + (n - wn[el])];
+                for (int h = 0; h < (el >= E - whole ? 1 : H); h++) t += TC[(el * H + h) * SL + (n - wn[el])];
                 s = fmaf(t, rf[n * W + j], s);
             }
             Cacc[n] += (double)s;
@@ -538,17 +540,27 @@ bool choose_split(const DevProblem &P, int E, int SL, int nv, int tab, FwdSplit 
     // a voxel's pattern row and table column share a word of its record
     if ((int64_t)P.nq * P.na > 65536 || (int64_t)P.n_mat * ((P.nqf + 3) & ~3) > 65536) return false;
     const int chunks = std::max(1, (nv + 31) / 32);
-    static const FwdSplit candidates[] = {{kMaxWarps, kMaxSteps, 32, 1, 1}, {kMaxWarps, 12, 32, 1, 1}, {8, 12, 32, 1, 1}, {kMaxWarps, 12, 32, 1, 1}, {8, 8, 32, 1, 1},
-                                          {4, 4, 32, 1, 1},   {2, 2, 32, 1, 1},   {1, 1, 32, 1, 1},  {1, 1, 1, 1, 1},    {1, 1, 1, 0, 1}};
+    static const FwdSplit candidates[] = {
+        {kMaxWarps, kMaxSteps, 32, 1, 0, 1}, {kMaxWarps, 18, 32, 1, 0, 1}, {kMaxWarps, 12, 32, 1, 0, 1},
+        {8, 12, 32, 1, 0, 1},                {kMaxWarps, 12, 32, 1, 0, 1}, {8, 8, 32, 1, 0, 1},
+        {4, 4, 32, 1, 0, 1},                 {2, 2, 32, 1, 0, 1},          {1, 1, 32, 1, 0, 1},
+        {1, 1, 1, 1, 0, 1},                  {1, 1, 1, 0, 0, 1}};
     for (int i = 0; i < (int)(sizeof candidates / sizeof candidates[0]); i++) {
         FwdSplit sp = candidates[i];
         // tiles of about equal length
         const int tiles = (chunks + sp.steps - 1) / sp.steps;
         sp.steps = (chunks + tiles - 1) / tiles;
-        // four runs or more per warp
+        // four runs or more per warp; where the energies by themselves give as
+        // many, the lowest, one for two warps, in two runs each, for the warps to
+        // end a tile together (reference sizes 138.8 -> 134.8 ms, 256x256 326.5 -> 318.2,
+        // 128x128 7.09 -> 7.08; one per warp 136.0, 321.4; every energy in two 136.3, 335)
         sp.runs = std::min(sp.steps, std::max(1, (4 * sp.warps + E - 1) / E));
+        if (sp.runs == 1 && sp.steps > 1 && sp.warps > 1) {
+            sp.runs = 2;
+            sp.whole = std::max(0, E - sp.warps / 2);
+        }
         const size_t total = fwd_layout(P, E, SL, sp, tab).total;
-        const size_t limit = (i < 3 ? 113 : 227) * 1024;
+        const size_t limit = (i < 4 ? 113 : 227) * 1024;
         if (total + sizeof(PairRec) + 1024 <= limit) {
             *out = sp;
             *smem = total;
