@@ -274,6 +274,7 @@ F32Consts make_f32_consts(const DevProblem &P)
     c.inv_DQ = (float)(1.0 / P.DQ);
     c.nxf = (float)P.nx;
     c.nyf = (float)P.ny;
+    c.inv_side = 1.f / (float)std::min(P.nx, P.ny);
     c.rsqrt2pi = (float)P.rsqrt2pi;
     c.q_lo = (float)P.q_lo;
     c.kn0 = (float)P.kn0;

@@ -86,20 +86,43 @@ __device__ __forceinline__ void walk_anchor_ff(const F32Consts &C, ff ex, ff ey,
     w->uy = ff_neg(ff_mul(Dy, iD));
 }
 
+// How far rounding may move the entry point, in voxels: `unit` times the size of
+// the endpoint and of the region, and as much more as the edge's length times
+// the other side over |den| -- a side over the ray's extent across the edge --
+// says that the ray grazes the edge.  Of 10^7 rays per scanner (endpoints at 0.8
+// to 10^5 sides, maps of 3 to 2048 voxels a side, SFU quotients an ulp off) no
+// FP32 entry point was further off than 3.8 units of 2^-24; the pairs' is taken
+// the same way.
+constexpr float kUnitF32 = 6.f / 16777216.f, kUnitPairs = 1e-12f;
+
+__device__ __forceinline__ float walk_extent(const F32Consts &C, float ex, float ey)
+{
+    return fmaf(0.25f, C.nxf + C.nyf, fabsf(ex) + fabsf(ey));
+}
+
+__device__ __forceinline__ float entry_error(const F32Consts &C, float extent_units, float inv_den)
+{
+    return extent_units * fmaf(0.5f * (C.nxf * C.nyf), fabsf(inv_den), 1.f);
+}
+
 // FP32 version of walk_setup for the endpoint (ex, ey) rounded to float.
 // Returns false when a decision is too close to its threshold for FP32 to be
 // trusted -- a nearly edge-parallel ray, a ray through an ROI corner, or a
 // length within a few FP32 errors of a multiple of DQ (axis-aligned rays hit
 // the latter exactly) -- and the caller then decides in float pairs or FP64
-// (walk_decide).  Endpoint rounding (|e| ~ 300 voxels -> 1.5e-5) dominates the
-// FP32 error; the guards are several times that.
+// (walk_decide).  The guards grow with the distances: rounding of the endpoint
+// and of the products moves the entry point by a few 2^-24 of them, and further
+// along an edge that the ray grazes (entry_error).  With fixed guards, set for
+// endpoints some 300 voxels away, 0.25 % of the walks from a source 5000 voxels
+// away took a sample too many or too few.
 __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Consts &C, float ex, float ey,
                                                float vx, float vy, WalkSetup *w)
 {
     const float NX = C.nxf, NY = C.nyf, DQ = C.DQ, inv_DQ = C.inv_DQ;
     const float eps = kEdgeEps;
-    const float G = 2e-4f;
     const float dx = vx - ex, dy = vy - ey;
+    const float units = kUnitF32 * walk_extent(C, ex, ey);
+    float err = 0.f;
     float rx = 0.f, ry = 0.f;
     bool found = false;
     int edge = -1;
@@ -111,8 +134,12 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
         const float y4 = (i == 1 || i == 2) ? NY : 0.f;
         const float x4_x3 = x4 - x3, y3_y1 = y3 - ey, y4_y3 = y4 - y3, x3_x1 = x3 - ex;
         const float den = x4_x3 * dy - dx * y4_y3;
-        if (fabsf(den) < 1e-2f) return false;     // edge-parallel within FP32 error
+        // edge-parallel within FP32 error: 1e-2, and where the side is long enough
+        // for the rounding of its coordinates to reach a hundredth of |den|
+        if (fabsf(den) < fmaxf(1e-2f, 4e-6f * (NX * NY))) return false;
         const float inv = __fdividef(1.f, den);
+        err = entry_error(C, units, inv);
+        const float G = fmaxf(2e-4f, err * C.inv_side);
         const float ua = (x4_x3 * y3_y1 - x3_x1 * y4_y3) * inv;
         if (fabsf(ua + eps) < G || fabsf(ua - (1.f + eps)) < G) return false;
         if (ua > -eps && ua < 1.f + eps) {
@@ -135,7 +162,7 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
     float ft;
     const int it = floor_nc(t, &ft);
     const float fr = t - ft;
-    const float gt = fmaf(4e-7f, t, 1e-3f);
+    const float gt = fmaf(4e-7f, t, fmaxf(1e-3f, err * inv_DQ));
     if (fr < gt || fr > 1.f - gt) return false;
     long long n = (long long)it + 1;
     if (n > P.kmax) n = P.kmax;
@@ -150,9 +177,9 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
 
 // The same decisions in float pairs, for the lanes that walk_setup_f32 leaves
 // open: about 48 bits against its 24, in FP32 instructions.  Returns false
-// within 1e-9 of a threshold (1e-8 of a step for the length, both well above
-// the pairs' error of some 2^-44 of the distance), where FP64 has
-// to round as the oracle does: rays along the grid, rays through a corner.
+// within 1e-9 of a threshold (1e-8 of a step for the length), or within the
+// pairs' error of some 2^-44 of the distances where that is more, and FP64 then
+// has to round as the oracle does: rays along the grid, rays through a corner.
 // FP64 issues at 1/64 of the FP32 rate, and the 0.6 % of the lanes that are
 // open sit in one warp of six.  Straight to FP64 instead, the walk of 256x256
 // voxels, 45 views x 512 px took 67.4 ms against 65.4, and the source side's, all
@@ -162,7 +189,8 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
 {
     const float NX = C.nxf, NY = C.nyf;
     const ff eps = {kEdgeEps, 0.f};
-    const float G = 1e-9f;
+    const float units = kUnitPairs * walk_extent(C, ex.hi, ey.hi);
+    float err = 0.f;
     const ff dx = ff_fsub(vx, ex), dy = ff_fsub(vy, ey);
     if (!(fabsf(dx.hi) * NY > 1e-4f) || !(fabsf(dy.hi) * NX > 1e-4f)) return false;   // edge-parallel
     // how far inside [-eps, 1 + eps] a parameter lies (negative: outside)
@@ -179,6 +207,8 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
         const ff fx = i == 1 || i == 2 ? ex1 : ff_neg(ex);   // edge's first corner minus the endpoint
         const ff fy = i >= 2 ? ey1 : ff_neg(ey);
         ua = horizontal ? ff_div(fy, dy) : ff_div(fx, dx);
+        err = entry_error(C, units, __fdividef(1.f, horizontal ? dy.hi * NX : dx.hi * NY));
+        const float G = fmaxf(1e-9f, err * C.inv_side);
         const float in_a = inside(ua);
         if (fabsf(in_a) < G) return false;
         if (!(in_a > 0.f)) continue;
@@ -204,7 +234,7 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
         ft -= 1.f;
         fr = (t.hi - ft) + t.lo;
     }
-    const float gt = fmaf(1e-12f, D.hi * C.inv_DQ, 1e-8f);
+    const float gt = fmaf(err, C.inv_DQ, 1e-8f);
     if (fr < gt || fr > 1.f - fmaxf(gt, 1e-7f)) return false;
     long long n = (long long)ft + 1;
     if (n > P.kmax) n = P.kmax;

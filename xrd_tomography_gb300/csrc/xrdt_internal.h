@@ -39,6 +39,7 @@ struct DevProblem {
 // at 1/64 of the FP32 rate.
 struct F32Consts {
     float vox, DQ, DQ_lo, inv_DQ, nxf, nyf, rsqrt2pi;
+    float inv_side;    // 1 / min(nx, ny)
     float q_lo, kn0;
     float inv_dEd, dEd, dEs, inv_dEs;
     float qmin_t, inv_dqt, inv_dqg;
