@@ -47,3 +47,36 @@ def test_decisions_with_distant_endpoints(ctx, oracle_lib, nx, ny, r_src, r_det,
     p.r_src, p.r_det, p.dq_step = r_src, r_det, step
     inp = full_map(p, 31)
     compare(inp, some_rays(p, rays, 32), ctx, oracle_lib)
+
+
+# a flat fan (wedge angle 0: no photon passes, every output is 0) and the
+# thinnest ones
+@pytest.mark.parametrize("wedge", [0.0, 1e-12, 1e-4, -0.01])
+def test_flat_fan(ctx, oracle_lib, wedge):
+    p = sized_problem(14, 11, 3, 21, 7, 7, 2, nwt=40)
+    p.wedge_angle = wedge
+    inp = synth.make_inputs(p, 41)
+    rays = np.arange(p.rays)
+    N, C, A = xt.forward(p, *inp.args(), ctx=ctx)
+    Nr, Cr, Ar, _ = oracle_lib.forward_rays(inp, rays, want_a=True)
+    got, want = [N, C, A], [Nr, Cr, np.asarray(Ar).reshape(-1)]
+    S1 = synth.coherent_table(inp)
+    for bilinear in (False, True):
+        got += xt.forward_tables(p, inp.spectrum, inp.seg, inp.a1, inp.a2, S1, inp.S2, *inp.args()[6:],
+                                 bilinear=bilinear, ctx=ctx)
+        want += oracle_lib.forward_tables(inp, S1, rays, bilinear=bilinear)
+    rng = np.random.default_rng(42)
+    x = rng.uniform(0.0, 1.0, (p.nx * p.ny, p.nwt)).astype(np.float32)
+    x[inp.seg == 0] = 0.0
+    w = rng.uniform(0.0, 2.0, p.rays).astype(np.float32)
+    y_ref, g_ref = oracle_lib.vox_rays(inp, rays, x=x.reshape(-1), w=w)
+    op = xt.Operator(p, inp.spectrum, inp.seg, inp.a1, inp.a2, ctx=ctx)
+    got += [op.forward(x.reshape(-1)), op.adjoint(w)]
+    want += [y_ref, g_ref.reshape(-1)]
+    op.close()
+    for a, b in zip(got, want):
+        assert np.asarray(a).shape == np.asarray(b).shape
+        if wedge == 0.0:
+            assert not np.asarray(b).any() and not np.asarray(a).any()
+        else:
+            assert max_rel_err(a, b) < FAST_RTOL

@@ -220,10 +220,11 @@ __device__ __forceinline__ void pair_geom(const DevProblem &P, const SrcGeom &g,
     G->nsx = (float)nsx;
     G->nsy = (float)nsy;
     G->nsz = (float)nsz;
-    // Rvox_z = -(a . nsrc_xy) tan(geomphi/2) / |nsrc_xy|, Hvox with tan(geomphi)
+    // Rvox_z = -(a . nsrc_xy) tan(geomphi/2) / |nsrc_xy|, Hvox with tan(geomphi):
+    // their ratio by the double angle, finite at a wedge angle of 0 too
     G->mx = ff_from_double(-nsx * P.tan_half / nsxy);
     G->my = ff_from_double(-nsy * P.tan_half / nsxy);
-    G->hz = ff_from_double(-P.tan_full / P.tan_half);
+    G->hz = ff_from_double(-2.0 / (1.0 - P.tan_half * P.tan_half));
     G->ndx = (float)g.sphi;
     G->ndy = (float)(-g.cphi);
     G->Dn = ff_from_double(Dx * (double)G->ndx + Dy * (double)G->ndy);
