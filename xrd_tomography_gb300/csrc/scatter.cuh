@@ -18,9 +18,9 @@ namespace xrdt {
 // Per-(source, pixel) constants of the scattering geometry.
 struct PairGeom {
     ff Rsx, Rsy, Rdx, Rdy;        // source and detector positions (in plane)
-    ff Dx, Dy, Dz, DD;            // source -> detector vector and its square
+    ff Rdz;                       // detector height over the source
+    ff DD;                        // square of the source -> detector distance
     ff mx, my;                    // the voxel's height over the source: az = ax mx + ay my
-    ff Dn;                        // D . n_det
     ff hz;                        // Hvox = az hz
     float nsx, nsy, nsz, ndx, ndy, sphi, cphi;
     float tan_full, adet12, focal2_12;
@@ -211,9 +211,7 @@ __device__ __forceinline__ void pair_geom(const DevProblem &P, const SrcGeom &g,
     G->Rdx = ff_from_double(*Rdet_x);
     G->Rdy = ff_from_double(*Rdet_y);
     const double Dx = *Rdet_x - g.Rsrc_x, Dy = *Rdet_y - g.Rsrc_y;   // Rsrc_z = 0
-    G->Dx = ff_from_double(Dx);
-    G->Dy = ff_from_double(Dy);
-    G->Dz = ff_from_double(Rdz);
+    G->Rdz = ff_from_double(Rdz);
     G->DD = ff_from_double(Dx * Dx + Dy * Dy + Rdz * Rdz);
     const double nsx = -g.sphi * P.sta, nsy = g.cphi * P.sta, nsz = -P.cta;
     const double nsxy = sqrt(nsx * nsx + nsy * nsy);
@@ -227,7 +225,6 @@ __device__ __forceinline__ void pair_geom(const DevProblem &P, const SrcGeom &g,
     G->hz = ff_from_double(-2.0 / (1.0 - P.tan_half * P.tan_half));
     G->ndx = (float)g.sphi;
     G->ndy = (float)(-g.cphi);
-    G->Dn = ff_from_double(Dx * (double)G->ndx + Dy * (double)G->ndy);
     G->sphi = (float)g.sphi;
     G->cphi = (float)g.cphi;
     G->tan_full = (float)P.tan_full;
@@ -236,21 +233,23 @@ __device__ __forceinline__ void pair_geom(const DevProblem &P, const SrcGeom &g,
     G->focal2_12 = (float)(P.focal * P.focal / 12.0);
 }
 
-// integrate_diffraction.cu:196-255 for one voxel.  a = voxel - source as
-// float pairs, b = detector - voxel = D - a; 1 - cos(theta) from the cross
-// product a x b = a x D, |a x b|^2 / (|a||b| (|a||b| + a.b)), which has no
-// cancellation at small angles.  The blur vectors S = ((a x b) x a)/|a|^2,
+// integrate_diffraction.cu:196-255 for one voxel.  a = voxel - source and b =
+// detector - voxel as float pairs; 1 - cos(theta) from the cross product,
+// |a x b|^2 / (|a||b| (|a||b| + a.b)), which has no cancellation at small
+// angles.  (Everything from a and b themselves: with D = a + b in b's place, three
+// products less, the errors grow with |D|/|b| and its square, sin(theta/2) to 6e-11
+// with the source 5000 voxels away and 2e-9 from 10^5 on.)  The blur vectors S = ((a x b) x a)/|a|^2,
 // D' = ((a x b) x b)/|b|^2 and V = -(S + D') = u x (a x b), u = a/|a|^2 +
 // b/|b|^2, are perpendicular to a, b and a x b in turn, so with c = a x b
 //   |S|^2 = |c|^2/|a|^2,  |D'|^2 = |c|^2/|b|^2,  |V|^2 = |D|^2 |c|^2/(|a|^2 |b|^2)
-// and only their components along the source's, the detector's and the z axis
-// are left to find.  (The z component is no small one where the detector sits
+// and of the pairs only the components along the source's, the detector's and the
+// z axis are left to find.  (The z component is no small one where the detector sits
 // high over the fan plane.)
 // SIGMA_PAIR: the terms that make up most of sigma^2 as pairs (the per-voxel
 // operator, whose adjoint sums deep Gaussian tails: a tail amplifies sigma^2's
 // relative error by (q distance / sigma)^2 / 2, and FP32 leaves it about two
 // ulps off); otherwise in FP32 (the material forward projector, whose counts
-// are dominated by the Gaussians' cores).  About 500 and 300 instructions per
+// are dominated by the Gaussians' cores).  About 550 and 350 instructions per
 // voxel; component by component with correctly rounded quotients and roots
 // they were 2700 and 700, a third of the operator's forward and a tenth of
 // the projector.
@@ -259,14 +258,14 @@ __device__ __forceinline__ VoxGeom vox_geom(const PairGeom &G, float vx, float v
 {
     const ff ax = ff_fsub(vx, G.Rsx), ay = ff_fsub(vy, G.Rsy);
     const ff az = ffl_dot2(ax, G.mx, ay, G.my);
-    const ff aD = ffl_dot3(ax, G.Dx, ay, G.Dy, az, G.Dz);
-    const ff an = ffl_dot3(ax, ax, ay, ay, az, az);
-    const ff ab = ffl_sub(aD, an), bD = ffl_sub(G.DD, aD);
+    const ff bx = ff_neg(ff_fsub(vx, G.Rdx)), by = ff_neg(ff_fsub(vy, G.Rdy)), bz = ff_sub(G.Rdz, az);
     // (tight where terms cancel: these high parts are used as floats, too)
-    const ff bn = ff_sub(bD, ab);
-    const ff cx = ff_dot2(ay, G.Dz, ff_neg(az), G.Dy);
-    const ff cy = ff_dot2(az, G.Dx, ff_neg(ax), G.Dz);
-    const ff cz = ff_dot2(ax, G.Dy, ff_neg(ay), G.Dx);
+    const ff an = ffl_dot3(ax, ax, ay, ay, az, az);
+    const ff bn = ff_tight(ffl_dot3(bx, bx, by, by, bz, bz));
+    const ff ab = ffl_dot3(ax, bx, ay, by, az, bz);
+    const ff cx = ff_dot2(ay, bz, ff_neg(az), by);
+    const ff cy = ff_dot2(az, bx, ff_neg(ax), bz);
+    const ff cz = ff_dot2(ax, by, ff_neg(ay), bx);
     const ff cn = ffl_dot3(cx, cx, cy, cy, cz, cz);
     const ff nab = ffl_sqrt(ffl_mul(an, bn));
     VoxGeom r;
@@ -278,30 +277,30 @@ __device__ __forceinline__ VoxGeom vox_geom(const PairGeom &G, float vx, float v
     r.cos2 = costh * costh;
     // FP32 remainder of the geometry
     const float Ax = ax.hi, Ay = ay.hi, Az = az.hi, Cx = cx.hi, Cy = cy.hi, Cz = cz.hi;
-    // (from the pixel: D - a would round at the size of D)
-    const float Bx = (G.Rdx.hi - vx) + G.Rdx.lo, By = (G.Rdy.hi - vy) + G.Rdy.lo;
+    const float Bx = bx.hi, By = by.hi;
     const ff ian = ff_rcp(an), ibn = ff_rcp(bn);
     const float ia = ian.hi, ib = ibn.hi;
     const float Sn = ((Cy * Az - Cz * Ay) * G.nsx + (Cz * Ax - Cx * Az) * G.nsy + (Cx * Ay - Cy * Ax) * G.nsz) * ia;
     const float sS2 = (cn.hi * ia - Sn * Sn) * G.focal2_12;
     if (!SIGMA_PAIR) {
-        const float ux = fmaf(Ax, ia, Bx * ib), uy = fmaf(Ay, ia, By * ib);
-        const float Vz = ux * Cy - uy * Cx, Bz = G.Dz.hi - Az;
+        // (V by components: |V|^2 - Vz^2 would cancel where V points along z)
+        const float Bz = bz.hi, H = Az * G.hz.hi;
+        const float ux = fmaf(Ax, ia, Bx * ib), uy = fmaf(Ay, ia, By * ib), uz = fmaf(Az, ia, Bz * ib);
+        const float Vx = uy * Cz - uz * Cy, Vy = uz * Cx - ux * Cz, Vz = ux * Cy - uy * Cx;
         const float Dn = ((Cy * Bz - Cz * By) * G.ndx + (Cz * Bx - Cx * Bz) * G.ndy) * ib;
-        const float cb = cn.hi * ib;
-        const float H = Az * G.hz.hi;
-        const float rest = fmaf(Vz * Vz, fmaf(H * H, 1.f / 12.f, -G.vox2_12.hi), sS2);
-        r.sg = ff{fmaf(G.DD.hi * (cb * ia), G.vox2_12.hi, fmaf(cb - Dn * Dn, G.adet12, rest)) * ia * ib, 0.f};
+        const float rest = fmaf((H * H) * (1.f / 12.f), Vz * Vz, sS2);
+        r.sg = ff{fmaf(fmaf(Vx, Vx, Vy * Vy), G.vox2_12.hi, fmaf(fmaf(cn.hi, ib, -Dn * Dn), G.adet12, rest)) * ia * ib, 0.f};
     } else {
         const ff cb = ffl_mul(cn, ibn);
         const ff VV = ffl_mul(G.DD, ffl_mul(cb, ian));
-        // Vz of V = a (u.D) - D (u.a)
-        const ff ua = ffl_add(ff{1.f, 0.f}, ffl_mul(ab, ibn));
-        const ff Vz = ffl_dot2(az, ffl_dot2(aD, ian, bD, ibn), ff_neg(G.Dz), ua);
+        // Vz of V = u x c
+        const ff ux = ffl_dot2(ax, ian, bx, ibn), uy = ffl_dot2(ay, ian, by, ibn);
+        const ff Vz = ffl_dot2(ux, cy, ff_neg(uy), cx);
         const ff Vz2 = ffl_mul(Vz, Vz);
-        // D'.n_det = c.(b x n)/|b|^2 = ((a.b)(D.n) - (a.n)(D.b))/|b|^2
+        // D'.n_det = ((a.b) (b.n) - (a.n) |b|^2)/|b|^2
         const ff adn = ffl_dot2(ax, ff{G.ndx, 0.f}, ay, ff{G.ndy, 0.f});
-        const ff Dn = ffl_mul(ffl_dot2(ab, G.Dn, ff_neg(adn), bD), ibn);
+        const ff bdn = ffl_dot2(bx, ff{G.ndx, 0.f}, by, ff{G.ndy, 0.f});
+        const ff Dn = ffl_sub(ffl_mul(ffl_mul(ab, ibn), bdn), adn);
         const ff dD = ffl_sub(cb, ffl_mul(Dn, Dn));
         const ff H = ffl_mul(az, G.hz);
         const ff blur = ffl_add(ffl_dot3(ffl_sub(VV, Vz2), G.vox2_12, ffl_mul(Vz2, ffl_mul(H, H)),
