@@ -93,3 +93,15 @@ def test_scattering_angles_far_away(ctx, oracle_lib, r_src, r_det):
     p.r_src, p.r_det = r_src, r_det
     p.nq, p.na = 65536, 1
     compare(full_map(p, 51), some_rays(p, 300, 52), ctx, oracle_lib)
+
+
+# voxel centres that no float holds, on rays along the grid, whose lengths are
+# multiples of the sample step; and sides that a float holds
+@pytest.mark.parametrize("side", [0.7, 0.3, 0.9, 0.5, 0.75])
+def test_decisions_at_any_voxel_side(ctx, oracle_lib, side):
+    p = sized_problem(26, 18, 4, 9, 6, 6, 1)
+    p.cx, p.cy = 0.5 * side * (p.nx + 1), 0.5 * side * (p.ny + 1)   # on a voxel centre
+    p.r_src, p.r_det = 64.0, 60.0
+    p.col_pitch = side
+    p.vox_side = side
+    compare(full_map(p, 61), np.arange(p.rays), ctx, oracle_lib)

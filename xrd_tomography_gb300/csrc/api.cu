@@ -275,6 +275,9 @@ F32Consts make_f32_consts(const DevProblem &P)
     c.nxf = (float)P.nx;
     c.nyf = (float)P.ny;
     c.inv_side = 1.f / (float)std::min(P.nx, P.ny);
+    int exponent;
+    const double mantissa = 256.0 * frexp(P.vox, &exponent);
+    c.vox_exact = mantissa == floor(mantissa) && exponent > -100 && exponent < 100;
     c.rsqrt2pi = (float)P.rsqrt2pi;
     c.q_lo = (float)P.q_lo;
     c.kn0 = (float)P.kn0;

@@ -245,21 +245,26 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
     return true;
 }
 
-static __device__ __noinline__ void walk_setup_f64(const DevProblem &P, double ex, double ey, double vx, double vy,
+// In FP64, from the voxel's exact centre: (vx, vy) is that rounded to float, which
+// for a side of more than eight bits is no multiple of half a side any more.
+static __device__ __noinline__ void walk_setup_f64(const DevProblem &P, double ex, double ey, float vx, float vy,
                                             WalkSetup *w)
 {
-    walk_setup(P, ex, ey, vx, vy, w);
+    walk_setup(P, ex, ey, (rint((double)vx / P.vox - 0.5) + 0.5) * P.vox,
+               (rint((double)vy / P.vox - 0.5) + 0.5) * P.vox, w);
 }
 
 // A walk's decisions and its voxel-anchored form, from the endpoint as float
-// pairs (and in double for the last resort).
+// pairs (and in double for the last resort).  Pairs decide for voxel centres that
+// a float holds, as with a side of 1; for others FP64 does: a centre off by 1e-7
+// of itself takes a sample too many or too few where a length is a multiple of DQ.
 __device__ __forceinline__ void walk_decide(const DevProblem &P, const F32Consts &C, ff ex, ff ey,
                                             const double *exd, const double *eyd, float vx, float vy, WalkSetup *w)
 {
     bool ok = walk_setup_f32(P, C, ex.hi, ey.hi, vx, vy, w);
-    if (!ok) ok = walk_setup_pairs(P, C, ex, ey, vx, vy, w);
+    if (!ok && C.vox_exact) ok = walk_setup_pairs(P, C, ex, ey, vx, vy, w);
     if (ok) walk_anchor_ff(C, ex, ey, vx, vy, w);
-    else walk_setup_f64(P, *exd, *eyd, (double)vx, (double)vy, w);
+    else walk_setup_f64(P, *exd, *eyd, vx, vy, w);
 }
 
 // Sum of the n samples times DQ, walked cell by cell by one lane.  Cell (ci,

@@ -40,6 +40,7 @@ struct DevProblem {
 struct F32Consts {
     float vox, DQ, DQ_lo, inv_DQ, nxf, nyf, rsqrt2pi;
     float inv_side;    // 1 / min(nx, ny)
+    int vox_exact;     // every voxel centre is a float: a side of at most 8 significant bits
     float q_lo, kn0;
     float inv_dEd, dEd, dEs, inv_dEs;
     float qmin_t, inv_dqt, inv_dqg;
