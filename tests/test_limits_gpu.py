@@ -1,6 +1,8 @@
 """Geometries, sizes and values at the ends of what the entry points accept:
 distant sources and detectors, a flat fan, voxels of any side, tables of any
 shape, infinite unknowns, calls that fail half way -- against the FP64 oracle."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -105,3 +107,40 @@ def test_decisions_at_any_voxel_side(ctx, oracle_lib, side):
     p.col_pitch = side
     p.vox_side = side
     compare(full_map(p, 61), np.arange(p.rays), ctx, oracle_lib)
+
+
+def test_calls_of_different_sizes_on_two_threads(oracle_lib):
+    """Kernels whose shared memory follows the problem's size, called with a
+    small and a large one by two threads, each with a context of its own: the
+    calls neither fail nor change."""
+    small = synth.make_inputs(sized_problem(9, 7, 3, 11, 6, 6, 1, nwt=8, nqf=32), 71)
+    large = synth.make_inputs(sized_problem(12, 10, 3, 13, 120, 100, 4, nwt=64, nqf=768, mats=6), 72)
+    ctxs = [xt.Context(0), xt.Context(0)]
+    errors = []
+
+    def calls(inp, c):
+        p = inp.problem
+        T, G = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=c)
+        return [T, G, *xt.forward(p, *inp.args(), ctx=c)]
+
+    try:
+        want = [[a.copy() for a in calls(inp, c)] for inp, c in zip((small, large), ctxs)]
+
+        def work(inp, c, ref, n):
+            try:
+                for _ in range(n):
+                    for a, b in zip(calls(inp, c), ref):
+                        if not np.array_equal(a, b):
+                            raise AssertionError("a call's result changed")
+            except Exception as e:   # noqa: BLE001 - reported by the main thread
+                errors.append(e)
+
+        threads = [threading.Thread(target=work, args=(inp, c, ref, 400)) for inp, c, ref in zip((small, large), ctxs, want)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        for c in ctxs:
+            c.close()
+    assert not errors, errors

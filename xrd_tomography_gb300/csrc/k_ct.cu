@@ -145,6 +145,7 @@ __device__ __noinline__ void chord_setup_f64(const DevProblem &P, const SrcGeom 
 }
 
 constexpr int kCtWarps = 4;
+constexpr int kCtMaxSmem = 200 * 1024;
 
 // A detector's position per column pitch and a source's trigonometry as pairs.
 struct CtConsts {
@@ -318,7 +319,7 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
     size_t smem = bin_bytes * warps * E + tables;
     if (smem > 56 * 1024) {   // four blocks per SM
         warps = 1;
-        e_pass = tables < 200 * 1024 ? std::min<int64_t>(E, (int64_t)((200 * 1024 - tables) / bin_bytes)) : 0;
+        e_pass = tables < kCtMaxSmem ? std::min<int64_t>(E, (int64_t)((kCtMaxSmem - tables) / bin_bytes)) : 0;
         smem = bin_bytes * (size_t)e_pass + tables;
     }
     const bool staged = e_pass >= W;
@@ -328,7 +329,8 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
         smem = 0;
     }
     auto *kernel = staged ? k_ct_sinogram<true> : k_ct_sinogram<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit of every size: one call must not lower it between another thread's setting and launch)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtMaxSmem);
     if (e != cudaSuccess) return e;
     const int64_t nch = (int64_t)(32 >> lg_split) * warps;
     // strips of kStrip views where a lane has a chord to itself (38400 chords,

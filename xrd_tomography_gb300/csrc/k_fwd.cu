@@ -57,6 +57,7 @@ namespace xrdt {
 namespace {
 
 constexpr int kMaxWarps = 12;      // 384 threads, two blocks per SM at 80 registers
+constexpr int kMaxSmem = 226 * 1024 - (int)sizeof(PairRec);   // dynamic, of a block by itself
 constexpr int kMaxSteps = 24;      // 32-voxel steps per energy and tile: 768 voxels, 36 KB of records
 constexpr unsigned kMagicBits = 0x4B400000u;   // 1.5 * 2^23: adding it rounds to an integer in the mantissa
 constexpr float kMagic = 12582912.f;
@@ -520,7 +521,8 @@ template <int TAB, bool FAST, bool COUNT>
 cudaError_t launch_variant(const FwdArgs &a, int n_pairs, size_t smem, cudaStream_t s)
 {
     auto *kernel = k_fwd<TAB, FAST, COUNT>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit of every size: one call must not lower it between another thread's setting and launch)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     // early: the tables are staged while the walk ends
     return launch_after(kernel, n_pairs, 32 * a.split.warps, smem, s, true, a);
@@ -566,8 +568,8 @@ bool choose_split(const DevProblem &P, int E, int SL, int nv, int tab, FwdSplit 
             sp.whole = std::max(0, E - sp.warps / 2);
         }
         const size_t total = fwd_layout(P, E, SL, sp, tab).total;
-        const size_t limit = (i < 4 ? 113 : 227) * 1024;
-        if (total + sizeof(PairRec) + 1024 <= limit) {
+        const size_t limit = i < 4 ? (113 - 1) * 1024 - sizeof(PairRec) : kMaxSmem;
+        if (total <= limit) {
             *out = sp;
             *smem = total;
             return true;

@@ -32,7 +32,9 @@ namespace xrdt {
 namespace {
 
 constexpr int kMaxMatrixWarps = 24;
-static_assert(sizeof(PairRec) + 16 <= 256, "the static part of a block's shared memory");
+constexpr int kStaticSmem = 256;   // of a block, rounded up; 1 KB more is the system's
+constexpr int kMaxSmem = 227 * 1024 - kStaticSmem;   // dynamic, of a block by itself
+static_assert(sizeof(PairRec) + 16 <= kStaticSmem, "the static part of a block's shared memory");
 
 // words of four voxels' terms: pref, w_hi, w_lo and the exponent's scale of each
 // voxel, then the bin groups of the pass they reach (a bit each), their common
@@ -291,7 +293,8 @@ template <int NG>
 cudaError_t launch_groups(const MatrixArgs &a, int n_pairs, size_t smem, cudaStream_t s)
 {
     auto *kernel = a.T.work ? k_matrix<NG, true> : k_matrix<NG, false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit of every size: one call must not lower it between another thread's setting and launch)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     // early: it reads nothing of the projection's, so the two overlap
     return launch_after(kernel, n_pairs, 32 * a.split.warps, smem, s, true, a);
@@ -316,7 +319,7 @@ bool choose_split(const DevProblem &P, int E, int nv, MatrixSplit *out, size_t *
         if (h.blocks == 3 && h.steps == 20 && rounds(8) > rounds(12)) continue;
         const int tiles = (chunks + h.steps - 1) / h.steps;
         MatrixSplit sp = {h.warps, (chunks + tiles - 1) / tiles, 0};
-        const size_t limit = (size_t)228 * 1024 / h.blocks - 1024 - 256;   // 1 KB per block and the static part
+        const size_t limit = h.blocks == 1 ? kMaxSmem : (size_t)228 * 1024 / h.blocks - 1024 - kStaticSmem;
         const size_t base = matrix_layout(P, sp).total + 16;
         if (base + per_e > limit) continue;
         const int64_t fit = (int64_t)((limit - base) / per_e);
