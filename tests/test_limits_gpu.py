@@ -144,3 +144,53 @@ def test_calls_of_different_sizes_on_two_threads(oracle_lib):
         for c in ctxs:
             c.close()
     assert not errors, errors
+
+
+def test_infinite_unknowns_stay_in_their_energies_windows(ctx):
+    """With detector bins that take one source bin each, a ray sees its own
+    energy's window alone: an infinite coefficient reaches the same rays, and an
+    infinite weight the same unknowns, whether the kernels take two energies
+    together or the operator holds only one."""
+    def operator(e0, e1, n):
+        p = sized_problem(6, 5, 3, 65, n, n, 0, nwt=24)
+        p.e_src_min = p.e_det_min = e0
+        p.e_src_max = p.e_det_max = e1
+        # far away, for windows narrower than the q grid
+        p.r_src, p.r_det, p.col_pitch, p.z0 = 10 * p.r_src, 10 * p.r_det, 10 * p.col_pitch, 10 * p.z0
+        inp = full_map(p, 81)
+        inp.spectrum = np.eye(n, dtype=np.float32).reshape(-1)
+        return p, xt.Operator(p, inp.spectrum, inp.seg, inp.a1, inp.a2, ctx=ctx)
+
+    both, parts = operator(40.0, 44.0, 2), [operator(40.0, 42.0, 1), operator(42.0, 44.0, 1)]
+    p, op = both
+    pairs = p.rays // 2
+    rng = np.random.default_rng(82)
+    x = rng.uniform(0.1, 1.0, (p.nx * p.ny, p.nwt)).astype(np.float32)
+    reached = 0
+    for k in range(p.nwt):
+        xi = x.copy()
+        xi[k % (p.nx * p.ny), k] = np.inf
+        y = op.forward(xi.reshape(-1)).reshape(2, pairs)
+        for e, (_, one) in enumerate(parts):
+            want = one.forward(xi.reshape(-1))
+            assert np.array_equal(np.isnan(y[e]), np.isnan(want)) and np.array_equal(np.isinf(y[e]), np.isinf(want))
+            ok = np.isfinite(want)
+            assert max_rel_err(y[e][ok], want[ok]) < FAST_RTOL
+            reached += int((~ok).sum())
+    assert reached
+    partly = 0
+    for r in range(0, pairs, 13):
+        for e in range(2):
+            w = rng.uniform(0.5, 1.0, (2, pairs)).astype(np.float32)
+            w[1 - e, r], w[e, r] = 1.0, np.inf
+            g = op.adjoint(w.reshape(-1))
+            want = parts[e][1].adjoint(w[e])
+            assert np.array_equal(np.isfinite(g), np.isfinite(want))
+            ok = np.isfinite(want)
+            partly += bool(0 < (~ok).sum() < ok.size)
+            w[e, r] = 0.0
+            if ok.any():
+                assert max_rel_err(g[ok], op.adjoint(w.reshape(-1))[ok]) < FAST_RTOL
+    assert partly > 10
+    for _, o in (both, *parts):
+        o.close()

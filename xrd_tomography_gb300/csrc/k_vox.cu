@@ -240,6 +240,42 @@ __host__ __device__ inline FwdLayout vox_fwd_layout(const DevProblem &P, int E, 
     return L;
 }
 
+// A voxel's constants from its record i of a tile of 32 nst voxels.
+__device__ __forceinline__ VoxTerm load_term(const float4 *rec, int nst, int i)
+{
+    const float4 r0 = rec[i], r1 = rec[32 * nst + i], r2 = rec[64 * nst + i];
+    return {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
+}
+
+// Component k & 1 of a pair of bins.
+__device__ __forceinline__ float bin_of(float2 v, int k) { return k & 1 ? v.y : v.x; }
+
+// A run's sum at one energy, bin by bin over that energy's own window: for runs
+// whose sum is not finite.  An infinite coefficient outside the window -- within a
+// neighbouring energy's, or beside it in a pair -- must not reach the sum, nor one
+// whose term underflows, as 0 x inf.
+__device__ __noinline__ float run_by_window(const float4 *rec, const float *xs, const float4 *cq, int x_row,
+                                            const VoxEnergy *en, int el, int nst, int s0, int s1, WindowTable window)
+{
+    const int lane = threadIdx.x & 31;
+    const VoxEnergy q = load_energy(en, el);
+    float sum = 0.f;
+    for (int st = s0; st < s1; st++) {
+        const int i = 32 * st + lane;
+        const EnergyTerm t = energy_term(q, load_term(rec, nst, i));
+        if (t.pref == 0.f) continue;
+        int k0, k1;
+        bin_window(window, t.w_hi, kSig * window.scale * t.sigma, &k0, &k1);
+        float acc = 0.f;
+        for (int k = k0; k <= k1; k++) {
+            const float g = bin_of(gauss2(t, cq[k >> 1]), k);
+            if (g != 0.f) acc = fmaf(g, xs[(k >> 1) * x_row + 2 * i + (k & 1)], acc);
+        }
+        sum = fmaf(t.pref, acc, sum);
+    }
+    return warp_sum(sum);
+}
+
 // One (source, pixel) pair of job J, by the whole block; the job's tables are
 // staged.
 template <bool MLEM>
@@ -311,8 +347,7 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
             float sum = 0.f, sum1 = 0.f;
             for (int st = s0; st < s1; st++) {
                 const int i = 32 * st + lane;
-                const float4 r0 = rec[i], r1 = rec[32 * nst + i], r2 = rec[64 * nst + i];
-                const VoxTerm v = {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
+                const VoxTerm v = load_term(rec, nst, i);
                 const EnergyTerm t = energy_term(q, v), u = energy_term(q1, v);
                 // Both take the bins of both windows, which lie a source bin
                 // apart: a fraction of their length, as sigma holds the width of
@@ -339,6 +374,10 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
             }
             sum = warp_sum(sum);
             sum1 = warp_sum(sum1);
+            if (!(isfinite(sum) && isfinite(sum1))) {
+                sum = run_by_window(rec, xs, cq, x_row, en, el, nst, s0, s1, window);
+                sum1 = run_by_window(rec, xs, cq, x_row, en, el + two, nst, s0, s1, window);
+            }
             if (lane <= two) {
                 const int at = (el + lane) * H + run;
                 float2 k = TNs[at];
@@ -435,6 +474,29 @@ __host__ __device__ inline AdjLayout vox_adj_layout(const DevProblem &P, int E, 
     return L;
 }
 
+// What a pair adds to this lane's column of sums, energy by energy over each one's own
+// window: for pairs with a weight that is not finite (run_by_window).  Returns the first
+// and the last pair of bins touched.
+__device__ __noinline__ int2 pair_by_window(VoxTerm v, const VoxEnergy *en, const float4 *cq, const float *ws, int E,
+                                            WindowTable window, float2 *sums)
+{
+    int2 r = {0xffff, -1};
+    for (int el = 0; el < E; el++) {
+        const EnergyTerm t = energy_term(load_energy(en, el), v);
+        const float ct = ws[el] * t.pref;
+        int k0, k1;
+        bin_window(window, t.w_hi, kSigAdj * window.scale * t.sigma, &k0, &k1);
+        if (ct == 0.f || k0 > k1) continue;
+        r = make_int2(min(r.x, k0 >> 1), max(r.y, k1 >> 1));
+        for (int k = k0; k <= k1; k++) {
+            const float g = bin_of(gauss2(t, cq[k >> 1]), k);
+            float *s = (float *)(sums + 32 * (k >> 1)) + (k & 1);
+            if (g != 0.f) *s = fmaf(ct, g, *s);
+        }
+    }
+    return r;
+}
+
 // Adjoint tile (voxel-chunk block bx, pair group by) of job J.  A pair's sums
 // over the energies are plain FP32 sums in shared memory, two energies per
 // visit to a bin (the visits' loads and stores would bind before the FMA
@@ -505,12 +567,22 @@ k_vox_adj(const VoxBatch B)
             __syncwarp();   // the previous pair's constants are no longer read
             for (int i = lane; i < (int)(sizeof(PairRec) / 4); i += 32)
                 reinterpret_cast<int *>(&pr)[i] = reinterpret_cast<const int *>(J.op.pairs + pp)[i];
-            for (int i = lane; i < E; i += 32) ws[i] = __ldg(J.what + pp * E + i);
-            __syncwarp();
+            bool finite = true;
+            for (int i = lane; i < E; i += 32) {
+                const float w = __ldg(J.what + pp * E + i);
+                ws[i] = w;
+                finite &= isfinite(w);
+            }
+            const int by_two = __all_sync(0xffffffffu, finite);
             const VoxTerm vt = vox_term(pr.G, J.c, c1, xy, J.op.atten_src[(int64_t)pr.src * nv + v],
                                         J.op.walk[(pp - J.pair0) * nv + v]);
             int kmin = K2, kmax = -1;   // the pairs of bins this lane adds to
-            for (int el = 0; el < E; el += 2) {
+            if (!by_two) {
+                const int2 k = pair_by_window(vt, en, cq, ws, E, window, sums);
+                kmin = min(kmin, k.x);
+                kmax = k.y;
+            }
+            for (int el = by_two ? 0 : E; el < E; el += 2) {
                 const EnergyTerm t = energy_term(load_energy(en, el), vt);
                 const int e1 = min(el + 1, E - 1);
                 const EnergyTerm u = energy_term(load_energy(en, e1), vt);
