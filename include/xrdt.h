@@ -42,7 +42,8 @@ typedef enum xrdt_status {
     XRDT_ERR_INPUT = 4,       /* bad input values (material id > n_mat, ...)  */
     XRDT_ERR_CUDA = 5,        /* a CUDA runtime call failed                    */
     XRDT_ERR_ALLOC = 6,       /* device or pinned allocation failed            */
-    XRDT_ERR_UNSUPPORTED = 7, /* a flag combination that is not implemented    */
+    XRDT_ERR_UNSUPPORTED = 7, /* a flag combination that is not implemented, or
+                               * tables larger than one block has room for     */
     XRDT_ERR_TIMEOUT = 8,     /* a bounded device wait gave up                 */
     XRDT_ERR_IO = 9           /* a file could not be written or read           */
 } xrdt_status;

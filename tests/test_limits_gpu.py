@@ -194,3 +194,38 @@ def test_infinite_unknowns_stay_in_their_energies_windows(ctx):
     assert partly > 10
     for _, o in (both, *parts):
         o.close()
+
+
+@pytest.mark.parametrize("bilinear", [False, True])
+def test_table_path_takes_any_number_of_pattern_bins(ctx, oracle_lib, bilinear):
+    """The table path reads no patterns: 100 materials of 768 fine bins, more
+    than a block could hold, do not concern it."""
+    p = sized_problem(16, 13, 3, 21, 9, 7, 2, nqf=768, mats=100)
+    inp = synth.make_inputs(p, 91)
+    S1 = synth.coherent_table(inp)
+    N, C = xt.forward_tables(p, inp.spectrum, inp.seg, inp.a1, inp.a2, S1, inp.S2, *inp.args()[6:],
+                             bilinear=bilinear, ctx=ctx)
+    Nr, Cr = oracle_lib.forward_tables(inp, S1, np.arange(p.rays), bilinear=bilinear)
+    assert max_rel_err(N, Nr) < FAST_RTOL
+    assert max_rel_err(C, Cr) < FAST_RTOL
+
+
+@pytest.mark.parametrize("what,change", [("patterns", dict(nqf=768, mats=100)), ("matrix", dict(nwt=4096, mats=15)),
+                                         ("table", dict())])
+def test_tables_that_no_block_holds_are_refused(ctx, what, change):
+    """As unsupported, not as a failed launch; the context goes on; an empty
+    phantom needs no tables and is 0 at any size."""
+    p = sized_problem(10, 8, 2, 7, 4, 4, 1, **change)
+    if what == "table":
+        p.nq, p.na = 257, 256
+    inp = synth.make_inputs(p, 92)
+    matrix = what == "matrix"
+    for call in ([lambda: xt.forward(p, *inp.args(), want_amatrix=matrix, ctx=ctx),
+                  lambda: xt.forward_rays(p, np.arange(3), *inp.args(), want_amatrix=matrix, ctx=ctx)]):
+        with pytest.raises(xt.XrdtError) as e:
+            call()
+        assert e.value.status == 7
+    if matrix:
+        assert xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)[0].max() > 0
+    inp.seg = np.zeros_like(inp.seg)
+    assert not any(a.any() for a in xt.forward(p, *inp.args(), want_amatrix=matrix, ctx=ctx) if a is not None)

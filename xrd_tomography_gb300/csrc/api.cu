@@ -864,6 +864,10 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         // pairs go through in tiles: the detector-side integrals of a tile
         // (k_walk.cu), then the projector over the same pairs
         auto project = [&](const int2 *list, int64_t n_total, float *oN, float *oC, float *oA) -> int {
+            if (!forward_fits(P, T.sl, nv, tab) || (oA && !matrix_fits(P, nv))) {
+                cudaStreamSynchronize(st);   // nothing reads the caller's arrays after a refusal
+                return fail(ctx, XRDT_ERR_UNSUPPORTED, "the problem's tables exceed the shared memory of one block");
+            }
             const int64_t tile = tile_pairs(nv, n_total);
             void *dtab;
             int r = get_buf(ctx, S_WALK, sizeof(float2) * (size_t)tile * nv, &dtab);

@@ -545,8 +545,9 @@ cudaError_t launch_tab(const FwdArgs &a, int n_pairs, size_t smem, cudaStream_t 
 // tables read through L1.
 bool choose_split(const DevProblem &P, int E, int SL, int nv, int tab, FwdSplit *out, size_t *smem)
 {
-    // a voxel's pattern row and table column share a word of its record
-    if ((int64_t)P.nq * P.na > 65536 || (int64_t)P.n_mat * ((P.nqf + 3) & ~3) > 65536) return false;
+    // a voxel's pattern row and table column share a word of its record (the table
+    // path reads no patterns)
+    if ((int64_t)P.nq * P.na > 65536 || (!tab && (int64_t)P.n_mat * ((P.nqf + 3) & ~3) > 65536)) return false;
     const int chunks = std::max(1, (nv + 31) / 32);
     static const FwdSplit candidates[] = {
         {kMaxWarps, kMaxSteps, 32, 1, 0, 1}, {kMaxWarps, 18, 32, 1, 0, 1}, {kMaxWarps, 12, 32, 1, 0, 1},
@@ -593,6 +594,13 @@ __global__ void k_gather_rays(const int64_t *__restrict__ idx, int64_t n, const 
 }
 
 } // namespace
+
+bool forward_fits(const DevProblem &P, int sl, int nv, int tab)
+{
+    FwdSplit sp;
+    size_t smem;
+    return choose_split(P, P.e_hi - P.e_lo + 1, sl, nv, tab, &sp, &smem);
+}
 
 cudaError_t launch_gather_rays(const int64_t *idx, int64_t n, const float *Nc, const float *Cc,
                                const float *Ac, int mw, float *N, float *C, float *A, cudaStream_t s,

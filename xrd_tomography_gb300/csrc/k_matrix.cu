@@ -336,6 +336,13 @@ bool choose_split(const DevProblem &P, int E, int nv, MatrixSplit *out, size_t *
 
 } // namespace
 
+bool matrix_fits(const DevProblem &P, int nv)
+{
+    MatrixSplit sp;
+    size_t smem;
+    return choose_split(P, P.e_hi - P.e_lo + 1, nv, &sp, &smem);
+}
+
 cudaError_t launch_matrix(const DevProblem &P, const PairRec *recs, const FwdTables &T, const PrepBuffers &B, int nv,
                           bool list, long long n_list, long long p0, int n_pairs, const float2 *walk, float *A,
                           cudaStream_t s, int64_t *launches)

@@ -203,6 +203,10 @@ cudaError_t launch_fast_forward(const DevProblem &P, const PairRec *recs, const 
                                 const PrepBuffers &B, int nv, const float *Ifine,
                                 bool list, long long n_list, long long p0, int n_pairs,
                                 const float2 *walk, float *N, float *C, cudaStream_t s, int64_t *launches, int tab);
+// Whether a block has room for the tables of a projection with nv voxels, sl
+// detector bins per window (launch_fast_forward; tab as there), and of its matrix.
+bool forward_fits(const DevProblem &P, int sl, int nv, int tab);
+bool matrix_fits(const DevProblem &P, int nv);
 // k_matrix.cu: the model matrix of the same pairs (rows of n_mat*nwt; the
 // compact layout [nrg_det][n_list][n_mat*nwt] for a list).
 cudaError_t launch_matrix(const DevProblem &P, const PairRec *recs, const FwdTables &T, const PrepBuffers &B, int nv,
