@@ -229,3 +229,40 @@ def test_tables_that_no_block_holds_are_refused(ctx, what, change):
         assert xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)[0].max() > 0
     inp.seg = np.zeros_like(inp.seg)
     assert not any(a.any() for a in xt.forward(p, *inp.args(), want_amatrix=matrix, ctx=ctx) if a is not None)
+
+
+def random_table(p, seed):
+    """Neighbouring bins differ by a third of their value, so that a term read
+    from the wrong one shows."""
+    return np.random.default_rng(seed).uniform(20.0, 255.0, p.nq * p.na).astype(np.float32)
+
+
+# tables of any shape: two bins, odd and unequal sides, as long as a record's word
+# holds, and too large for shared memory beside the rest; nearest lookups (and the
+# fine-q path's) on rough tables, where a bin is right or wrong, bilinear ones on
+# smooth ones
+@pytest.mark.parametrize("nq,na", [(2, 2), (37, 91), (91, 37), (300, 3), (1024, 16), (256, 250), (32768, 2)])
+def test_tables_of_any_shape(ctx, oracle_lib, nq, na):
+    p = sized_problem(22, 17, 3, 40, 12, 11, 2)
+    p.nq, p.na = nq, na
+    inp = synth.make_inputs(p, 101)
+    rays = np.arange(p.rays)
+    S1 = synth.coherent_table(inp)
+    got = xt.forward_tables(p, inp.spectrum, inp.seg, inp.a1, inp.a2, S1, inp.S2, *inp.args()[6:], bilinear=True, ctx=ctx)
+    for a, b in zip(got, oracle_lib.forward_tables(inp, S1, rays, bilinear=True)):
+        assert max_rel_err(a, b) < FAST_RTOL
+    inp.S2, S1 = random_table(p, 102), random_table(p, 103)
+    got = xt.forward_tables(p, inp.spectrum, inp.seg, inp.a1, inp.a2, S1, inp.S2, *inp.args()[6:], ctx=ctx)
+    for a, b in zip(got, oracle_lib.forward_tables(inp, S1, rays)):
+        assert max_rel_err(a, b) < FAST_RTOL
+    N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
+    assert max_rel_err(N, Nr) < FAST_RTOL
+    assert max_rel_err(C, Cr) < FAST_RTOL
+
+
+@pytest.mark.parametrize("nq,na", [(2, 3), (37, 91), (1024, 16), (256, 250), (32768, 2)])
+def test_table_bins_at_any_shape(ctx, oracle_lib, nq, na):
+    p = sized_problem(40, 33, 6, 40, 12, 11, 2)
+    p.nq, p.na = nq, na
+    compare(synth.make_inputs(p, 104), some_rays(p, 500, 105), ctx, oracle_lib)

@@ -287,13 +287,15 @@ F32Consts make_f32_consts(const DevProblem &P)
     c.dEs = (float)P.dEs;
     c.qmin_t = (float)P.q_min;
     c.inv_dqt = P.dq_tab > 0 ? (float)(1.0 / P.dq_tab) : 0.f;
-    // the coordinate (L - q_min) / dq: lg2.approx is good to 2^-22 of L or
-    // absolute, and with its argument's and its own rounding L to 3e-7 |L| + 6e-7;
+    // the coordinate (L - q_min) / dq of a table lookup: lg2.approx is good to 2^-22
+    // of L or absolute; with the roundings of its arguments the Compton table's L
+    // (two of them) is off by at most 3e-7 |L| + 9.3e-7, the coherent table's by less;
     // the difference and product round at the size of the table.  (A fixed guard
     // of 2e-4 sent four times as many terms of a 64-bin table to FP64, which
-    // took a fifth of the FP64 units' time: 7.27 against 7.03 ms of k_fwd at 128x128.)
+    // took a fifth of the FP64 units' time: 7.27 against 7.03 ms of k_fwd at 128x128;
+    // from 256 bins on it is too narrow.)
     const double q_far = std::max(std::fabs(P.q_min), std::fabs(P.q_min + (double)P.nq * P.dq_tab));
-    c.bin_guard = (float)(0.5 - 1.3 * ((3e-7 * q_far + 6e-7) * c.inv_dqt + 2.4e-7 * (double)P.nq));
+    c.bin_guard = (float)(0.5 - 1.3 * ((3e-7 * q_far + 8e-7) * c.inv_dqt + 2.4e-7 * (double)P.nq));
     c.inv_dqg = P.dq_grid > 0 ? (float)(1.0 / P.dq_grid) : 0.f;
     const double NWT = (double)P.nwt;
     c.qpar_b = (float)P.dq0;

@@ -317,8 +317,8 @@ k_fwd(const FwdArgs args)
                     // wvt = ein sin(theta/2) on the tables' log2 axis
                     float s1v;
                     if (TAB == 1)
-                        s1v = table1(coherent_bin(P, q.ein, sh, oh, r1.w, args.T.energy[P.e_lo + el].ein, qmin_t,
-                                                  inv_dqt) +
+                        s1v = table1(coherent_bin(P, q.ein, sh, oh, r1.w, args.T.energy + P.e_lo + el, qmin_t,
+                                                  inv_dqt, c.bin_guard) +
                                      __float_as_int(r2.w));
                     else
                         s1v = table_bilinear(table1, P.nq, P.na, (lg2_approx(q.ein * sh) - qmin_t) * c.inv_dqg, r2.w);

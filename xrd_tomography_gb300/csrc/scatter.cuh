@@ -161,8 +161,8 @@ __device__ __forceinline__ int compton_bin(const DevProblem &P, float ein, float
 // The cross-section table path (code the reference keeps commented out,
 // integrate_diffraction.cu:701-719): the coherent table's wavevector bin
 // nq = floor((log2(w) - q_min) / dq) with w = ein sin(theta/2), clamped to
-// [0, NQ), decided in FP32 from the hi part of sin(theta/2); within 2e-4 of a
-// bin edge again in FP64 from 1 - cos(theta) (pair (oh, ol)).
+// [0, NQ), decided as compton_bin: in FP32 from the hi part of sin(theta/2), near
+// a bin edge again in FP64 from 1 - cos(theta) (pair (oh, ol)).
 __device__ __noinline__ int coherent_bin_f64(const DevProblem &P, double ein, float omc_hi, float omc_lo)
 {
     const double omcd = (double)omc_hi + (double)omc_lo;
@@ -171,14 +171,13 @@ __device__ __noinline__ int coherent_bin_f64(const DevProblem &P, double ein, fl
 }
 
 __device__ __forceinline__ int coherent_bin(const DevProblem &P, float ein, float sh, float oh, float ol,
-                                            double ein_d, float qmin_t, float inv_dqt)
+                                            const EnergyRow *row, float qmin_t, float inv_dqt, float bin_guard)
 {
-    const float tq = (lg2_approx(ein * sh) - qmin_t) * inv_dqt;
-    float ftq;
-    int nq = floor_bounded(tq, &ftq);   // clamped to the table below
-    const float fr = tq - ftq;
-    if (!(fr > 2e-4f && fr < 1.f - 2e-4f)) nq = coherent_bin_f64(P, ein_d, oh, ol);
-    return nq < 0 ? 0 : (nq >= P.nq ? P.nq - 1 : nq);
+    const float h = (lg2_approx(ein * sh) - qmin_t) * inv_dqt - 0.5f;
+    const float t = h + 12582912.f;
+    int nq = __float_as_int(t) - 0x4B400000;            // as in compton_bin
+    if (!(fabsf(h - (t - 12582912.f)) < bin_guard)) nq = coherent_bin_f64(P, row->ein, oh, ol);
+    return max(0, min(nq, P.nq - 1));
 }
 
 // Bilinear value of a table [nq, na] (S(q + a*nq) as a float) at

@@ -44,7 +44,7 @@ struct F32Consts {
     float q_lo, kn0;
     float inv_dEd, dEd, dEs, inv_dEs;
     float qmin_t, inv_dqt, inv_dqg;
-    float bin_guard;   // 1/2 minus the error of a Compton table coordinate in FP32, in bins
+    float bin_guard;   // 1/2 minus the error of a table coordinate in FP32, in bins
     float qpar_a, qpar_b;   // coarse bin edges: edge(n) = q_lo + qpar_b n + qpar_a n^2
 };
 F32Consts make_f32_consts(const DevProblem &P);
