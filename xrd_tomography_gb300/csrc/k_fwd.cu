@@ -159,12 +159,6 @@ __device__ __forceinline__ float sum8(const float *x, int lane)
     return s + __shfl_xor_sync(0xffffffffu, s, 1);
 }
 
-// The scattering geometry out of line: once per voxel and tile, it need not share
-// the run loop's scheduling (inlined, the reference's own sizes took 149.5 ms
-// against 146.8, with 0.1 % more instructions than before the geometry was formed
-// from b; 128x128 the same either way).
-__device__ __noinline__ VoxGeom tile_geom(const PairGeom &G, float vx, float vy) { return vox_geom<false>(G, vx, vy); }
-
 // TAB: 0 the coherent term from the materials' fine-q patterns
 // (integrate_diffraction.cu:299-308); 1 from the coherent table S1 by nearest
 // bin, 2 with both tables read bilinearly (the cross-section table path).
@@ -261,7 +255,7 @@ k_fwd(const FwdArgs args)
             const int xy = args.vox_xy[v];
             const float vx = ((float)(xy & 0xffff) + 0.5f) * c.vox;
             const float vy = ((float)(xy >> 16) + 0.5f) * c.vox;
-            const VoxGeom vg = tile_geom(pair.G, vx, vy);
+            const VoxGeom vg = vox_geom<false>(pair.G, vx, vy);
             const float a2v = args.vox_a2[v];
             // labels as at integrate_diffraction.cu:259-260: the detector-side
             // integral feeds Pin, the source-side one Pout; the coherent term
