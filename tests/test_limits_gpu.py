@@ -266,3 +266,35 @@ def test_table_bins_at_any_shape(ctx, oracle_lib, nq, na):
     p = sized_problem(40, 33, 6, 40, 12, 11, 2)
     p.nq, p.na = nq, na
     compare(synth.make_inputs(p, 104), some_rays(p, 500, 105), ctx, oracle_lib)
+
+
+def test_a_call_that_fails_half_way_leaves_the_next_one_alone(ctx, monkeypatch):
+    """An allocation that fails after the tables are on their way: the call
+    returns when the device is through with them, so the next call, with other
+    tables in the same staging buffer, computes what it does on a context of its own."""
+    torch = pytest.importorskip("torch")
+    one = synth.make_inputs(sized_problem(30, 28, 40, 2, 16, 12, 2), 111)
+    many = synth.make_inputs(sized_problem(30, 28, 8, 300, 16, 12, 2), 112)      # more pairs: records to allocate
+    other = synth.make_inputs(sized_problem(30, 28, 37, 2, 16, 16, 3), 113)
+    many_out = [torch.empty(many.problem.rays, device="cuda") for _ in range(2)]
+    args = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in many.args()[:6]]
+    torch.cuda.synchronize()
+    want = xt.forward(other.problem, *other.args(), want_amatrix=False, ctx=ctx)[:2]
+    c = xt.Context(0)
+    try:
+        for inp in (one, other):
+            xt.forward(inp.problem, *inp.args(), want_amatrix=False, ctx=c)
+        for _ in range(10):
+            monkeypatch.setenv("XRDT_TEST_FAIL_ALLOC", "1")
+            with pytest.raises(xt.XrdtError) as e:
+                xt.forward(many.problem, *args, *many.args()[6:], Nphotons=many_out[0], Cphotons=many_out[1],
+                           want_amatrix=False, ctx=c)
+            assert e.value.status == 6
+            monkeypatch.delenv("XRDT_TEST_FAIL_ALLOC")
+            got = xt.forward(other.problem, *other.args(), want_amatrix=False, ctx=c)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        xt.forward(many.problem, *args, *many.args()[6:], Nphotons=many_out[0], Cphotons=many_out[1],
+                   want_amatrix=False, ctx=c)
+        assert float(many_out[0].max()) > 0
+    finally:
+        c.close()

@@ -121,10 +121,13 @@ int stage_in(xrdt_ctx *ctx, int slot, const void *p, size_t bytes, const void **
 // pinned buffer and copied to the device in one go.  (As ten copies from
 // pageable memory they took 27 us of a call and as many gaps between its
 // kernels.)  The buffer belongs to the context.  Each call that fills it
-// waits until the copy is through before it returns, so the next may overwrite it.
+// waits until the copy is through before it returns, so the next may overwrite it:
+// by an event or a synchronisation of its own (landed), and where it fails before
+// that, here -- what it queued may still read the tables, and the caller's arrays.
 struct TablePack {
-    xrdt_ctx *ctx;
+    xrdt_ctx *ctx = nullptr;
     size_t used = 0;
+    bool in_flight = false;
     std::vector<std::pair<const void **, size_t>> views;   // where each table's address goes, and its offset
     std::vector<std::pair<const void *, size_t>> sources;  // what is copied, and its size
 
@@ -157,7 +160,13 @@ struct TablePack {
             *views[i].first = (const char *)d + views[i].second;
         }
         CK(cudaMemcpyAsync(d, ctx->h_stage, used, cudaMemcpyHostToDevice, ctx->stream));
+        in_flight = true;
         return XRDT_OK;
+    }
+    void landed() { in_flight = false; }
+    ~TablePack()
+    {
+        if (in_flight && cudaStreamSynchronize(ctx->stream) != cudaSuccess) cudaGetLastError();
     }
 };
 
@@ -774,7 +783,8 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
     for (int s = 0; s < p->n_src; s++) src_geom(p, s, &hsg[s]);
     const SrcGeom *d_srcg;
     FwdTables T;
-    TablePack pack{ctx};
+    TablePack pack;
+    pack.ctx = ctx;
     pack.add(hsg, &d_srcg);
     HostTables ht;
     if (!plain) {
@@ -821,6 +831,7 @@ int forward_impl(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectrum, co
         cudaGetLastError();
         CK(cudaStreamSynchronize(st));
     }
+    pack.landed();
     const int nv = ctx->h_counters[0];
     if (ctx->h_counters[1]) {
         cudaStreamSynchronize(st);   // nothing reads the caller's arrays after a refusal
@@ -1226,7 +1237,8 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
     const FwdEnergy *d_energy;
     const int *d_wlo;
     void *d_rf;
-    TablePack pack{ctx};
+    TablePack pack;
+    pack.ctx = ctx;
     pack.add(hsg, &d_srcg);
     pack.add(ht.fwd_energy, &d_energy);
     pack.add(ht.win_lo, &d_wlo);
@@ -1248,6 +1260,7 @@ int32_t xrdt_ct_sinogram(xrdt_ctx *ctx, const xrdt_problem *p, const float *spec
     if (hostT) CK(cudaMemcpyAsync(Tphotons, dT, sizeof(float) * rays, cudaMemcpyDeviceToHost, st));
     if (hostG) CK(cudaMemcpyAsync(gain0, dG, sizeof(float) * rays, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    pack.landed();
     return XRDT_OK;
 }
 
