@@ -48,7 +48,6 @@ namespace {
 constexpr int kTileM = 128;
 constexpr int kBasisThreads = 256;
 constexpr int kBasisWarps = kBasisThreads / 32;
-constexpr int kMaxK = 64;
 constexpr unsigned kSpinLimit = 1u << 26;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -999,19 +999,17 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     HostTables ht;
     build_host_tables(p, P, hspec.data(), &ht);
     build_window_table(p, &ht);
-    EnergyRow *d_energy;
     float *d_rf;
     int *d_wlo, *d_wn;
     float4 *d_cq;
     VoxEnergy *d_ven;
     unsigned *d_lut;
-    if ((rc = op_alloc_t(op, ht.energy.size(), &d_energy)) || (rc = op_alloc_t(op, ht.rf_win.size(), &d_rf)) ||
+    if ((rc = op_alloc_t(op, ht.rf_win.size(), &d_rf)) ||
         (rc = op_alloc_t(op, ht.win_lo.size(), &d_wlo)) || (rc = op_alloc_t(op, ht.win_n.size(), &d_wn)) ||
         (rc = op_alloc_t(op, ht.coarse_q.size(), &d_cq)) || (rc = op_alloc_t(op, ht.vox_energy.size(), &d_ven)) ||
         (rc = op_alloc_t(op, ht.qlut.size(), &d_lut)))
         return bail(rc);
-    e = cudaMemcpyAsync(d_energy, ht.energy.data(), sizeof(EnergyRow) * ht.energy.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_rf, ht.rf_win.data(), sizeof(float) * ht.rf_win.size(), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(d_rf, ht.rf_win.data(), sizeof(float) * ht.rf_win.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_wlo, ht.win_lo.data(), sizeof(int) * ht.win_lo.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_wn, ht.win_n.data(), sizeof(int) * ht.win_n.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_ven, ht.vox_energy.data(), sizeof(VoxEnergy) * ht.vox_energy.size(), cudaMemcpyHostToDevice, st);
@@ -1041,7 +1039,6 @@ int32_t xrdt_op_create(xrdt_ctx *ctx, const xrdt_problem *p, const float *spectr
     op->v.P = P;
     op->v.nv = nv;
     op->v.pairs = d_pairs;
-    op->v.energy = d_energy;
     op->v.rf_win = d_rf;
     op->v.win_lo = d_wlo;
     op->v.win_n = d_wn;

@@ -56,7 +56,6 @@ constexpr float kSig = 7.5f;            // Gaussian window, in sigma (tail below
 // adds to it (main.m:162), so the adjoint cannot drop them.
 constexpr float kSigAdj = 13.25f;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLog2e_lo = (float)(1.4426950408889634074 - (double)kLog2e);
 
 __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
 {
@@ -99,7 +98,6 @@ __device__ __forceinline__ float rsqrt_approx(float x)
     return y;
 }
 
-constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kTwelfth_hi = (float)(1.0 / 12.0);
 constexpr float kTwelfth_lo = (float)(1.0 / 12.0 - (double)kTwelfth_hi);
 // 0.5 log2(e) as a float pair: the Gaussian exp(-d^2 / (2 sigma^2)) is

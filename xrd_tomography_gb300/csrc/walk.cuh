@@ -17,8 +17,7 @@ namespace xrdt {
 constexpr float kEdgeEps = 0.00001f;   // GetIntersection's margin about an edge
 
 struct WalkSetup {
-    float rx, ry;   // ROI entry point (GetIntersection) minus one voxel in x and y
-    float Lx, Ly;   // DQ times the unit direction entry -> voxel
+    float Lx, Ly;   // along the ray, of any length
     int n;          // number of samples: k = 0 .. n-1
     int edge;       // ROI edge entered (GetIntersection's order: bottom, right,
                     // top, left), -1 when the segment misses the ROI
@@ -51,10 +50,8 @@ __device__ inline void walk_setup(const DevProblem &P, double ex, double ey, dou
         n = k + 1;
         if (n > P.kmax) n = P.kmax;
     }
-    w->rx = (float)(rx - 1.0);
-    w->ry = (float)(ry - 1.0);
-    w->Lx = (float)(Lx * P.DQ);
-    w->Ly = (float)(Ly * P.DQ);
+    w->Lx = (float)Lx;
+    w->Ly = (float)Ly;
     w->n = (int)n;
     if (n > 0) {
         w->dlt = ff_from_double(Lr - P.DQ * (double)(n - 1));
@@ -118,7 +115,7 @@ __device__ __forceinline__ float entry_error(const F32Consts &C, float extent_un
 __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Consts &C, float ex, float ey,
                                                float vx, float vy, WalkSetup *w)
 {
-    const float NX = C.nxf, NY = C.nyf, DQ = C.DQ, inv_DQ = C.inv_DQ;
+    const float NX = C.nxf, NY = C.nyf, inv_DQ = C.inv_DQ;
     const float eps = kEdgeEps;
     const float dx = vx - ex, dy = vy - ey;
     const float units = kUnitF32 * walk_extent(C, ex, ey);
@@ -155,10 +152,8 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
         }
     }
     if (!found) return false;
-    float Lx = vx - rx, Ly = vy - ry;
-    const float L2 = fmaf(Lx, Lx, Ly * Ly);
-    const float rL = rsqrtf(L2);
-    const float t = sqrtf(L2) * inv_DQ;
+    const float Lx = vx - rx, Ly = vy - ry;
+    const float t = sqrtf(fmaf(Lx, Lx, Ly * Ly)) * inv_DQ;
     float ft;
     const int it = floor_nc(t, &ft);
     const float fr = t - ft;
@@ -166,10 +161,8 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
     if (fr < gt || fr > 1.f - gt) return false;
     long long n = (long long)it + 1;
     if (n > P.kmax) n = P.kmax;
-    w->rx = rx - 1.f;
-    w->ry = ry - 1.f;
-    w->Lx = Lx * rL * DQ;
-    w->Ly = Ly * rL * DQ;
+    w->Lx = dx;
+    w->Ly = dy;
     w->n = (int)n;
     w->edge = edge;
     return true;
@@ -240,7 +233,7 @@ static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const 
     if (n > P.kmax) n = P.kmax;
     w->n = (int)n;
     w->edge = edge;
-    w->Lx = dx.hi;   // the direction only
+    w->Lx = dx.hi;
     w->Ly = dy.hi;
     return true;
 }

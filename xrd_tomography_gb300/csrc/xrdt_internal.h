@@ -276,7 +276,6 @@ struct VoxOp {
     DevProblem P;
     int nv;                    // non-empty voxels
     const PairRec *pairs;      // [n_src * n_det]
-    const EnergyRow *energy;
     const float *rf_win;
     const int *win_lo, *win_n;
     const float4 *coarse_q;
