@@ -298,3 +298,26 @@ def test_a_call_that_fails_half_way_leaves_the_next_one_alone(ctx, monkeypatch):
         assert float(many_out[0].max()) > 0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("side", [300, 1024])
+def test_ct_on_rough_maps(ctx, oracle_lib, side):
+    """Every cell different from the next, so that a sample's position shows: the
+    chord's offsets hold it to 1e-7 voxel and the line integral to 8e-8 of itself
+    wherever the chord lies.  Exponents X below 8 (in log2) round to 6e-7 of
+    the transmission, the integral's error and rounding times X ln 2 are 8e-7,
+    exp2 is good to 2.4e-7 and the sum of one window's term to 6e-8: 1.7e-6."""
+    p = sized_problem(side, side, 7, 301, 3, 3, 0)
+    p.col_pitch *= 1.3
+    inp = synth.make_inputs(p, 121)
+    rng = np.random.default_rng(122)
+    rough = np.where(rng.uniform(size=side * side) < 0.5, 0.0, rng.uniform(1.0, 2.0, side * side))
+    inp.a1 = np.zeros(side * side, np.float32)
+    inp.a2 = (3.0 / side * rough).astype(np.float32)
+    T, G = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=ctx)
+    rays = some_rays(p, 4000, 123)
+    Tr, Gr = oracle_lib.ct_rays(inp, rays)
+    X = -np.log2(np.maximum(Tr, 1e-300) / np.maximum(Gr, 1e-300))
+    ok = (Gr > 0) & (Tr > 0)
+    assert 3.0 < X[ok].max() < 8.0
+    assert np.max(np.abs(T[rays][ok] / Tr[ok] - 1.0)) < 1.7e-6

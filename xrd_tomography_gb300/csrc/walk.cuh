@@ -325,7 +325,12 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
     // exit edge offset h = +-0.5 (towards the step) times the inverse step
     const float2 hinv = make_float2(L.x < 0.f ? 0.5f * ilx : -0.5f * ilx, L.y < 0.f ? 0.5f * ily : -0.5f * ily);
     const float lxly = L.x * L.y;
-    const float2 uhi = make_float2(w.ux.hi, w.uy.hi), ulo = make_float2(w.ux.lo, w.uy.lo), v2 = make_float2(vx, vy);
+    const float2 uhi = make_float2(w.ux.hi, w.uy.hi), ulo = make_float2(w.ux.lo, w.uy.lo);
+    // LOW: whole voxels of the anchor and the rest, for the differences below to be
+    // exact as they are for a voxel centre (from a float anchor the offset loses up
+    // to 2e-5 voxel 250 cells on; line integrals of rough maps 512 a side 1e-6, not 6e-8)
+    const float2 vt = make_float2(vx, vy), v2 = LOW ? make_float2(rintf(vx), rintf(vy)) : vt;
+    if (LOW) vlow = make_float2((vx - v2.x) + vlow.x, (vy - v2.y) + vlow.y);
     // the distance of the voxel's nearest sample is below one step unless the
     // sample count was capped: then a two-sum that needs no ordering
     const bool small_dlt = w.dlt.hi <= DQ;
@@ -356,7 +361,7 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
         if (LOW) e = __fadd2_rn(e, vlow);
         // the cell whose centre is nearest (any cell holding the point gives
         // the same value: the interpolant is continuous), then the offset
-        const float2 t = __fadd2_rn(__fadd2_rn(v2, p), make_float2(magic, magic));
+        const float2 t = __fadd2_rn(__fadd2_rn(vt, p), make_float2(magic, magic));
         const int ix = __float_as_int(t.x) - 0x4B400000, iy = __float_as_int(t.y) - 0x4B400000;
         const unsigned c = min((unsigned)(ix * sx + iy * sy), ncell_m1);
         float4 c0, c1;
