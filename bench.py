@@ -588,7 +588,7 @@ def run_batched_stated(args):
             "metric": "batched per-voxel MLEM iterations per second (forward + adjoint + update)",
             "value": 1e3 / ms_iter, "unit": "iter/s", "n_gpus": ws, "steps": args.iters, "warmup": 1,
             "ms_per_step": ms_iter, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32 (FP64 geometry decisions and global sums)", "data": "synthetic (seeded)",
+            "dtype": "f32 (geometry decisions in float pairs or FP64 near a threshold, FP64 global sums)", "data": "synthetic (seeded)",
             "config": {"workload": f"{what}, one xrdt_batch, detector-side tables streamed in tiles",
                        "pair_voxels_per_iter": int(sum(pv)), "rays": int(sum(i.problem.rays for i in inps)),
                        "sizes": [f"{i.problem.nx}^2/{i.problem.n_src}v/{i.problem.n_col}px" for i in inps]},
@@ -693,7 +693,7 @@ def run_ours(args):
         "metric": "forward projector throughput (reference-equivalent ray-voxel-q terms)",
         "value": value, "unit": "G ray-voxel-q/s", "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": 1e3 * total_s / args.steps, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f32 (FP64 geometry and integer decisions)",
+        "vs_baseline": None, "dtype": "f32 (integer decisions in float pairs or FP64 near a threshold)",
         "data": "synthetic (seeded phantom, patterns, spectrum)",
         "config": workload_config(inp, parallelism=f"replicas x{ws}" if ws > 1 else "single GPU",
                                   l2="flushed between steps (256 MB write)"),

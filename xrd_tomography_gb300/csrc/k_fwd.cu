@@ -37,7 +37,7 @@
 // as long as the warp's longest window) 32 terms took about 390 instructions;
 // here they take about 240, and k_fwd went from 12.5 to 7.1 ms on 128x128 voxels,
 // 32 views x 128 px, 40 energies, from 314 to 135 ms on the reference's own sizes
-// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 318 ms
+// (100x100, 32 views x 1024 px, 64 energies, 768 fine bins), and from 674 to 319 ms
 // on 256x256 voxels, 45 views x 512 px, 64 energies.  Two neighbouring energies per
 // step, packed two to an instruction, took 18 % fewer instructions but no less
 // time (7.0, 147 and 314 ms at best): a packed FMA holds its pipe for two cycles.

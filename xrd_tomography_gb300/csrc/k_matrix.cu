@@ -302,7 +302,7 @@ cudaError_t launch_groups(const MatrixArgs &a, int n_pairs, size_t smem, cudaStr
 
 // Two blocks of 12 warps per SM, or three of 8 -- whichever leaves fewer warps
 // without an energy in the last round of a tile (64x64 voxels, 40 energies: the
-// projection with its matrix 8.5 against 8.9 ms) -- when the sums of every energy fit beside the tile; else
+// projection with its matrix 5.8 against 6.0 ms) -- when the sums of every energy fit beside the tile; else
 // one block with as many energies per pass as fit (a pass repeats the geometry
 // and adds to the rows written before), with fewer warps and shorter tiles
 // only when a single energy's sums leave no room.

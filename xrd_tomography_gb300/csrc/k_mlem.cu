@@ -17,8 +17,8 @@
 //
 // What keeps HBM busy:
 //  * every lane has its own ring of 16-byte asynchronous copies in shared
-//    memory (160 KB in flight per SM), refilled as it is used, so no load
-//    waits for the arithmetic before it;
+//    memory (112 to 160 KB in flight per SM by the row's length, 128 at K = 256),
+//    refilled as it is used, so no load waits for the arithmetic before it;
 //  * the kernels of a call overlap (programmatic dependent launch): a pass
 //    fills its ring, which needs A alone, while the update before it runs;
 //  * passes go over a warp's rows forwards and backwards in turn, so that what

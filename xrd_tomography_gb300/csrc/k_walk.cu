@@ -11,14 +11,14 @@
 // Sampled one point per lane, the walk is bound by L1 wavefronts: a
 // warp-wide 16-byte load costs at least four, and every sample needs a
 // 32-byte cell.  Here each lane walks a whole ray cell by cell (walk_cells,
-// walk.cuh), one cell load per run of 3-4 samples.  A warp takes 32 rays
+// walk.cuh), one cell load per run of 3-4 samples or per uniform square.  A warp takes 32 rays
 // that end on 32 neighbouring pixels of one view and leave from the same
 // voxel, so its lanes take about the same number of steps and stay within a
 // few voxels of each other, side by side across the rays.  The warp reads
 // the copy of the cell map (row- or column-major) whose rows run across its
 // rays, so that neighbouring lanes mostly share cache lines.  Per voxel each
-// lane sets up its own ray (FP32 with the exact FP64 fallback) and stores its
-// float2; the stores of consecutive voxels of a row merge in L2.
+// lane sets up its own ray (in FP32, near a threshold in float pairs or FP64,
+// walk_decide) and stores its float2; the stores of consecutive voxels of a row merge in L2.
 #include <algorithm>
 
 #include "scatter.cuh"
@@ -56,8 +56,9 @@ __device__ __forceinline__ bool group_row(const DevProblem &P, int list, long lo
 }
 
 // 8 blocks (32 warps) per SM: the walk waits on L1 latency, and at 64
-// registers (8 bytes spilled around the FP64 fallback call) it ran 1016 ms on
-// the 256x256 workload against 1089 ms at 6 blocks and 80 registers.
+// registers (28 bytes spilled around the fallback calls) it takes 63.8 ms on
+// 256x256 voxels, 45 views x 512 px against 68.7 at 6 blocks and 80 registers, 2.54
+// against 2.72 on 128x128, 32 views x 128 px.
 __global__ void __launch_bounds__(kWalkThreads, 8)
 k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list,
            long long n_items, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,

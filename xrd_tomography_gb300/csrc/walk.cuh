@@ -173,10 +173,10 @@ __device__ __forceinline__ bool walk_setup_f32(const DevProblem &P, const F32Con
 // within 1e-9 of a threshold (1e-8 of a step for the length), or within the
 // pairs' error of some 2^-44 of the distances where that is more, and FP64 then
 // has to round as the oracle does: rays along the grid, rays through a corner.
-// FP64 issues at 1/64 of the FP32 rate, and the 0.6 % of the lanes that are
-// open sit in one warp of six.  Straight to FP64 instead, the walk of 256x256
-// voxels, 45 views x 512 px took 67.4 ms against 65.4, and the source side's, all
-// of it in FP64 before, 397 us against 206.
+// FP64 issues at 1/64 of the FP32 rate, and the 0.7 % of the lanes that are
+// open sit in one warp of five.  Straight to FP64 instead, the walk of 256x256
+// voxels, 45 views x 512 px took 3 % longer, and the source side's, all of it in FP64
+// before, 397 us against 206.
 static __device__ __noinline__ bool walk_setup_pairs(const DevProblem &P, const F32Consts &C, ff ex, ff ey, float vx, float vy,
                                               WalkSetup *w)
 {
@@ -277,17 +277,16 @@ __device__ __forceinline__ void walk_decide(const DevProblem &P, const F32Consts
 // sample.  A sample within rounding of an edge may fall on either side; the
 // interpolant is continuous there, so the sum changes only by rounding.  The
 // runs are added with Kahan compensation.  One cell load serves the 3-4
-// samples of a run (DQ = 1/4 voxel; more in a uniform square, below), where the cooperative walk loads a cell
-// per sample.  The samples are taken from the last (next to the voxel) to
-// the first: rays that end on one voxel then start together and part slowly,
+// samples of a run (DQ = 1/4 voxel), or all of a uniform square's (below).  The
+// samples are taken from the last (next to the voxel) to the first: rays that end on one voxel then start together and part slowly,
 // so the lanes of a warp walking such rays read neighbouring cells.
 // Cell (ci, cj) is cells[2 (ci sx + cj sy)]: sx = 1, sy = NX+1 for the
 // row-major map, sx = NY+1, sy = 1 for the column-major copy.  Each step
 // reads its 32-byte cell with one 256-bit load (sm_100 and later; cells are
 // 32-byte aligned in a device allocation): the L1 cost of a warp-wide load
 // follows the cache lines its lanes touch, so one load per cell instead of
-// two halves it.  Measured on the 256x256 workload: 1085 ms against 1140 ms
-// for two 16-byte loads.
+// two halves it.  256x256 voxels, 45 views x 512 px: 63.8 ms against 65.3 for two
+// 16-byte loads.
 __device__ __forceinline__ void ld_cell256(const float4 *p, float4 &c0, float4 &c1)
 {
     asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -302,8 +301,8 @@ __device__ __forceinline__ void ld_cell256(const float4 *p, float4 &c0, float4 &
 // place: below kReachLimit, where a coefficient counts as 0 (k_build_cells).
 // Segmented phantoms are uniform but for their materials' borders, and rays
 // cross them in about log2(size) steps per region instead of one per cell:
-// 256x256 voxels, 45 views x 512 px 360 -> 67 ms, 128x128, 32 views x 128 px
-// 6.6 -> 2.7 ms.  With noise on the materials 270 and 4.6 ms; on a map without a
+// 256x256 voxels, 45 views x 512 px 360 -> 64 ms, 128x128, 32 views x 128 px
+// 6.6 -> 2.5 ms.  With noise on the materials 261 and 4.4 ms; on a map without a
 // single uniform cell the wider test costs 2 % (367 and 6.7 ms).
 constexpr int kReach = 31;
 constexpr float kReachUnit = 0x1p-125f, kReachScale = 0x1p125f, kReachLimit = 0x1p-115f;
@@ -366,8 +365,8 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
         const unsigned c = min((unsigned)(ix * sx + iy * sy), ncell_m1);
         float4 c0, c1;
         ld_cell256(cells + 2 * c, c0, c1);
-        // the cell centre (exact) minus the anchor is exact, and it cancels
-        // p but for the offset (Sterbenz), so only e rounds
+        // the cell centre (exact) minus the anchor -- half or whole voxels --
+        // is exact, and it cancels p but for the offset (Sterbenz), so only e rounds
         const float2 r = __fadd2_rn(t, make_float2(-magic, -magic));
         const float2 d = __fadd2_rn(__fadd2_rn(__fadd2_rn(v2, make_float2(-r.x, -r.y)), p), e);
         // steps to each exit edge of the cell, or of the uniform square around it
