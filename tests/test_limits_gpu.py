@@ -321,3 +321,19 @@ def test_ct_on_rough_maps(ctx, oracle_lib, side):
     ok = (Gr > 0) & (Tr > 0)
     assert 3.0 < X[ok].max() < 8.0
     assert np.max(np.abs(T[rays][ok] / Tr[ok] - 1.0)) < 1.7e-6
+
+
+def test_more_samples_than_a_float_counts(ctx, oracle_lib):
+    """Steps of a millionth of a voxel: more than 2^24 samples on a ray."""
+    p = sized_problem(24, 24, 1, 3, 2, 2, 0, nwt=8)
+    p.dq_step = 1e-6
+    inp = synth.make_inputs(p, 141)
+    rays = np.arange(p.rays)
+    T, G = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=ctx)
+    Tr, Gr = oracle_lib.ct_rays(inp, rays)
+    assert max_rel_err(T, Tr) < FAST_RTOL and max_rel_err(G, Gr) < FAST_RTOL
+    inp.seg = np.zeros_like(inp.seg)
+    inp.seg[[24 * 3 + 20, 24 * 21 + 2]] = 1   # walks of 3e6 to 3e7 samples
+    N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
+    Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
+    assert max_rel_err(N, Nr) < FAST_RTOL and max_rel_err(C, Cr) < FAST_RTOL

@@ -284,6 +284,9 @@ F32Consts make_f32_consts(const DevProblem &P)
     c.nxf = (float)P.nx;
     c.nyf = (float)P.ny;
     c.inv_side = 1.f / (float)std::min(P.nx, P.ny);
+    c.grain = 1.f;
+    while ((double)c.grain * 16777216.0 < (double)P.kmax && c.grain < 0x1p40f) c.grain *= 2.f;
+    c.grain_magic = 12582912.f * c.grain;
     int exponent;
     const double mantissa = 256.0 * frexp(P.vox, &exponent);
     c.vox_exact = mantissa == floor(mantissa) && exponent > -100 && exponent < 100;

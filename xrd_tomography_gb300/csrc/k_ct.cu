@@ -160,7 +160,7 @@ constexpr int kStrip = 8;
 // [e_pass][chords of the warp], then (STAGED) the spectrum windows [nrg_det][W],
 // their sums and their first bins.  Windows too wide for that (!STAGED) are read
 // through L1, and every bin forms its own transmissions.
-template <bool STAGED>
+template <bool STAGED, bool FINE>
 __global__ void __launch_bounds__(32 * kCtWarps)
 k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__ sg, const float4 *__restrict__ cells,
               const FwdEnergy *__restrict__ energy, const float *__restrict__ rf_win, const int *__restrict__ win_lo,
@@ -218,7 +218,7 @@ k_ct_sinogram(DevProblem P, F32Consts c, CtConsts q, const SrcGeom *__restrict__
                 chord_setup_f64(P, g, det, &ws, &ax, &ay);
             const int per = (ws.n + split - 1) >> lg_split;
             ws.n = min(ws.n, (sub + 1) * per);
-            float2 A = walk_cells<true>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c.DQ,
+            float2 A = walk_cells<true, FINE>(cells, 1, P.nx + 1, (unsigned)(ncell - 1), ws, ax.hi, ay.hi, c,
                                         make_float2(ax.lo, ay.lo), (float)(sub * per));
             for (int o = split >> 1; o > 0; o >>= 1) {
                 A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
@@ -328,7 +328,9 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
         e_pass = 0;
         smem = 0;
     }
-    auto *kernel = staged ? k_ct_sinogram<true> : k_ct_sinogram<false>;
+    const F32Consts c = make_f32_consts(P);
+    auto *kernel = c.grain > 1.f ? (staged ? k_ct_sinogram<true, true> : k_ct_sinogram<false, true>)
+                                 : (staged ? k_ct_sinogram<true, false> : k_ct_sinogram<false, false>);
     // (the limit of every size: one call must not lower it between another thread's setting and launch)
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtMaxSmem);
     if (e != cudaSuccess) return e;
@@ -341,7 +343,7 @@ cudaError_t launch_ct_sinogram(const DevProblem &P, const SrcGeom *sg, const flo
     if (blocks > 64LL * current_sm_count()) blocks = 64LL * current_sm_count();
     const CtConsts q = {ff_from_double(P.cx), ff_from_double(P.cy), ff_from_double(P.r_det), ff_from_double(P.col_pitch),
                         P.n_col};
-    kernel<<<(int)blocks, 32 * warps, smem, s>>>(P, make_f32_consts(P), q, sg, cells, energy, rf_win, win_lo, T, G0,
+    kernel<<<(int)blocks, 32 * warps, smem, s>>>(P, c, q, sg, cells, energy, rf_win, win_lo, T, G0,
                                                  (int)e_pass, lg_split, strip_w);
     if (launches) (*launches)++;
     return cudaGetLastError();

@@ -288,6 +288,7 @@ __global__ void k_voxel_compton(DevProblem P, const float *__restrict__ a1, cons
 // integrate_diffraction.cu:260, decided as the detector side's (walk_decide)
 // and walked cell by cell from the voxel (walk_cells), each lane its share of the
 // samples.  A warp takes neighbouring voxels of one source.
+template <bool FINE>
 __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict__ sg, const int *__restrict__ vox_xy,
                             int nv, const float4 *__restrict__ cells, float2 *__restrict__ out, int lg_split)
 {
@@ -308,7 +309,7 @@ __global__ void k_src_atten(DevProblem P, F32Consts c, const SrcGeom *__restrict
         walk_decide(P, c, ff_from_double(g->Rsrc_x), ff_from_double(g->Rsrc_y), &g->Rsrc_x, &g->Rsrc_y, vx, vy, &ws);
         const int per = (ws.n + split - 1) >> lg_split;
         ws.n = min(ws.n, (sub + 1) * per);
-        float2 A = walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ, make_float2(0.f, 0.f), (float)(sub * per));
+        float2 A = walk_cells<false, FINE>(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c, make_float2(0.f, 0.f), (float)(sub * per));
         for (int o = split >> 1; o > 0; o >>= 1) {
             A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
             A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
@@ -402,7 +403,9 @@ cudaError_t launch_src_atten(const DevProblem &P, const SrcGeom *d_src, int nv, 
     while (lg_split < 3 && items << (lg_split + 1) <= 1024LL * sms) lg_split++;
     int64_t blocks = ((items << lg_split) + 127) / 128;
     if (blocks > (int64_t)sms * 16) blocks = (int64_t)sms * 16;
-    k_src_atten<<<(int)blocks, 128, 0, s>>>(P, make_f32_consts(P), d_src, B.vox_xy, nv, B.cells, B.atten_src, lg_split);
+    const F32Consts c = make_f32_consts(P);
+    auto *kernel = c.grain > 1.f ? k_src_atten<true> : k_src_atten<false>;
+    kernel<<<(int)blocks, 128, 0, s>>>(P, c, d_src, B.vox_xy, nv, B.cells, B.atten_src, lg_split);
     if (launches) (*launches)++;
     return cudaGetLastError();
 }

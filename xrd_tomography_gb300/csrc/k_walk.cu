@@ -59,6 +59,7 @@ __device__ __forceinline__ bool group_row(const DevProblem &P, int list, long lo
 // registers (28 bytes spilled around the fallback calls) it takes 63.8 ms on
 // 256x256 voxels, 45 views x 512 px against 68.7 at 6 blocks and 80 registers, 2.54
 // against 2.72 on 128x128, 32 views x 128 px.
+template <bool FINE>
 __global__ void __launch_bounds__(kWalkThreads, 8)
 k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list,
            long long n_items, int nd, long long n_groups, int strip_len, const int *__restrict__ vox_xy, int nv,
@@ -103,8 +104,8 @@ k_det_walk(DevProblem P, F32Consts c, const PairRec *__restrict__ recs, int list
             ws.n = min(ws.n, (sub + 1) * per);
             const float2 none = make_float2(0.f, 0.f);
             const float k0 = (float)(sub * per);
-            float2 A = colmajor ? walk_cells(cells_t, P.ny + 1, 1, ncell_m1, ws, vx, vy, c.DQ, none, k0)
-                                : walk_cells(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c.DQ, none, k0);
+            float2 A = colmajor ? walk_cells<false, FINE>(cells_t, P.ny + 1, 1, ncell_m1, ws, vx, vy, c, none, k0)
+                                : walk_cells<false, FINE>(cells, 1, P.nx + 1, ncell_m1, ws, vx, vy, c, none, k0);
             for (int o = split >> 1; o > 0; o >>= 1) {
                 A.x += __shfl_xor_sync(0xffffffffu, A.x, o);
                 A.y += __shfl_xor_sync(0xffffffffu, A.y, o);
@@ -144,8 +145,9 @@ cudaError_t launch_det_walk(const DevProblem &P, const PairRec *recs, bool list,
     long long blocks = (nwork + kWalkWarps - 1) / kWalkWarps;
     if (blocks > (long long)sms * 64) blocks = (long long)sms * 64;
     if (launches) (*launches)++;
-    return launch_after(k_det_walk, (int)blocks, kWalkThreads, 0, s, early, P, make_f32_consts(P), recs, list ? 1 : 0,
-                        n_items, nd, n_groups, strip, vox_xy, nv, cells, tab, lg_split);
+    const F32Consts c = make_f32_consts(P);
+    return launch_after(c.grain > 1.f ? k_det_walk<true> : k_det_walk<false>, (int)blocks, kWalkThreads, 0, s, early, P,
+                        c, recs, list ? 1 : 0, n_items, nd, n_groups, strip, vox_xy, nv, cells, tab, lg_split);
 }
 
 } // namespace xrdt

@@ -40,6 +40,8 @@ struct DevProblem {
 struct F32Consts {
     float vox, DQ, DQ_lo, inv_DQ, nxf, nyf, rsqrt2pi;
     float inv_side;    // 1 / min(nx, ny)
+    float grain, grain_magic;   // the float that counts a ray's samples counts in grains: 1 up to 2^24 samples, and
+                                // 1.5 2^23 times that
     int vox_exact;     // every voxel centre is a float: a side of at most 8 significant bits
     float q_lo, kn0;
     float inv_dEd, dEd, dEs, inv_dEs;
