@@ -323,6 +323,35 @@ def test_ct_on_rough_maps(ctx, oracle_lib, side):
     assert np.max(np.abs(T[rays][ok] / Tr[ok] - 1.0)) < 1.7e-6
 
 
+@pytest.mark.parametrize("side", [256, 1024])
+def test_ct_chords_that_graze_a_side(ctx, oracle_lib, side):
+    """Chords that leave through a side which they cross at 1e-3 of a voxel per
+    length, that length within millionths of a step of a multiple, on a map that is 0
+    but for the texels about the chord's end: a sample too many or too few is 10 % of T."""
+    p = sized_problem(side, side, 1, 3, 1, 1, 0)
+    p.col_pitch = 1.5e-3
+    inp = synth.make_inputs(p, 131)
+    inp.a1 = np.zeros(side * side, np.float32)
+    ray = np.array([2])   # the pixel at +1.5e-3
+    for j in range(24):
+        p.cx = side - 0.75e-3 * (1.0 + 0.02 * j)
+        sx, sy = p.cx, p.cy - p.r_src
+        dx, dy = p.cx + 1.5e-3, p.cy + p.r_det
+        ex, ey = dx - sx, dy - sy
+        t0, t1 = (0.0 - sy) / ey, (side - sx) / ex
+        length = (t1 - t0) * np.sqrt(ex * ex + ey * ey)
+        end = int(length)
+        a2 = np.zeros((side, side), np.float32)   # [y, x]
+        a2[end - 2:end + 3, side - 1] = 1.0
+        inp.a2 = a2.reshape(-1)
+        for eps in (2e-7, 5e-7, 1e-6, 2e-6, 4e-6, 1e-5):
+            for sign in (-1.0, 1.0):
+                p.dq_step = length / (np.rint(4.0 * length) + sign * eps)
+                T, _ = xt.ct_sinogram(p, inp.spectrum, inp.a1, inp.a2, ctx=ctx)
+                Tr, _ = oracle_lib.ct_rays(inp, ray)
+                assert max_rel_err(T[ray], Tr) < FAST_RTOL
+
+
 def test_more_samples_than_a_float_counts(ctx, oracle_lib):
     """Steps of a millionth of a voxel: more than 2^24 samples on a ray."""
     p = sized_problem(24, 24, 1, 3, 2, 2, 0, nwt=8)

@@ -86,8 +86,12 @@ __device__ void chord_setup(const DevProblem &P, double sx, double sy, double dx
     w->uy = ff_from_double(ey * inv);
 }
 
-// The same in float pairs (about 2^-44 of the lengths): false within 1e-9 of
-// a threshold, 1e-8 of a step for the sample count, and for rays along an axis.
+// The same in float pairs: false within 1e-9 of a threshold, 1e-8 of a step for the
+// sample count, or within the pairs' error where that is more, and for rays along
+// an axis.  Rounding moves a crossing along the chord by some 2^-44 of the distances
+// over the chord's extent across the side, so by more the flatter it crosses it:
+// where 256 voxels are left at 1e-3 of a voxel per length, by 2e-6 of a step, and on
+// 1024 voxels, or from a source 5000 away, by 3e-5.
 __device__ __forceinline__ bool chord_setup_pairs(const DevProblem &P, const F32Consts &C, ff sx, ff sy, ff dx, ff dy,
                                                   WalkSetup *w, ff *rx, ff *ry)
 {
@@ -106,7 +110,9 @@ __device__ __forceinline__ bool chord_setup_pairs(const DevProblem &P, const F32
     if (less(tx1, t1)) t1 = tx1;
     if (less(ty1, t1)) t1 = ty1;
     const ff dt = ff_sub(t1, t0);
-    if (!(fabsf(dt.hi) > 1e-9f)) return false;
+    const float err = 2.f * kUnitPairs * walk_extent(C, fabsf(sx.hi) + fabsf(ex.hi), fabsf(sy.hi) + fabsf(ey.hi)) *
+                      fmaxf(fabsf(ix.hi), fabsf(iy.hi));
+    if (!(fabsf(dt.hi) > fmaxf(1e-9f, err))) return false;
     w->n = 0;
     w->dlt = w->ux = w->uy = ff{0.f, 0.f};
     *rx = *ry = ff{0.f, 0.f};
@@ -120,7 +126,7 @@ __device__ __forceinline__ bool chord_setup_pairs(const DevProblem &P, const F32
         ft -= 1.f;
         fr = (t.hi - ft) + t.lo;
     }
-    const float gt = fmaf(1e-12f, len.hi * C.inv_DQ, 1e-8f);
+    const float gt = fmaf(err, len.hi * C.inv_DQ, 1e-8f);
     if (!(fr > gt && fr < 1.f - fmaxf(gt, 1e-7f))) return false;
     long long n = (long long)ft + 1;
     if (n > P.kmax) n = P.kmax;

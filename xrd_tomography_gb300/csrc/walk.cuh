@@ -307,7 +307,8 @@ __device__ __forceinline__ void ld_cell256(const float4 *p, float4 &c0, float4 &
 constexpr int kReach = 31;
 constexpr float kReachUnit = 0x1p-125f, kReachScale = 0x1p125f, kReachLimit = 0x1p-115f;
 
-// LOW: the anchor is the pair (v, vlow), not an exact float.  k0: the first sample to
+// LOW: the anchor is the pair (v, vlow), not an exact float, and the step a pair too:
+// its rounding moves samples by up to 6e-8 of their way.  k0: the first sample to
 // take.  FINE: a ray may have more than 2^24 samples, which a float counts in grains of
 // two or more (C.grain): runs are whole grains long, so that k0 + m is exact and every
 // run starts past the one before.  (A variant of its own: with the grain a constant of
@@ -348,7 +349,8 @@ __device__ __forceinline__ float2 walk_cells(const float4 *__restrict__ cells, i
         // (explicitly rounded operations, x and y packed in one instruction:
         // a contracted multiply-add would count a product's error twice)
         const float kq = __fmul_rn(k0, DQ);
-        const float kqe = fmaf(k0, DQ, -kq);
+        float kqe = fmaf(k0, DQ, -kq);
+        if (LOW) kqe = fmaf(k0, C.DQ_lo, kqe);
         const float sh = __fadd_rn(w.dlt.hi, kq);
         float sl;
         if (small_dlt) {
