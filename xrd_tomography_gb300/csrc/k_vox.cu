@@ -573,6 +573,7 @@ k_vox_adj(const VoxBatch B)
                 ws[i] = w;
                 finite &= isfinite(w);
             }
+            __syncwarp();   // (the vote orders no memory)
             const int by_two = __all_sync(0xffffffffu, finite);
             const VoxTerm vt = vox_term(pr.G, J.c, c1, xy, J.op.atten_src[(int64_t)pr.src * nv + v],
                                         J.op.walk[(pp - J.pair0) * nv + v]);
