@@ -366,3 +366,30 @@ def test_more_samples_than_a_float_counts(ctx, oracle_lib):
     N, C, _ = xt.forward(p, *inp.args(), want_amatrix=False, ctx=ctx)
     Nr, Cr = oracle_lib.forward_rays(inp, rays)[:2]
     assert max_rel_err(N, Nr) < FAST_RTOL and max_rel_err(C, Cr) < FAST_RTOL
+
+
+@pytest.mark.parametrize("side", [1.0, -1.0])
+def test_detector_of_negative_area(ctx, oracle_lib, side):
+    """A row pitch of the other sign makes the detector's area negative and sigma^2 with it,
+    for some voxels and energies or for all: what a NaN term belongs to is NaN, as in
+    the reference's arithmetic, not a finite sum without that term."""
+    nans = 0
+    for seed in range(6):
+        rng = np.random.default_rng(150 + seed)
+        p = sized_problem(12, 9, 3, 7, 7, 6, 2, nwt=24)
+        p.row_pitch *= side * np.exp(rng.uniform(-3.0, 3.0))
+        inp = synth.make_inputs(p, 151 + seed)
+        rays = np.arange(p.rays)
+        x = rng.uniform(0.1, 1.0, (p.nx * p.ny, p.nwt)).astype(np.float32)
+        x[inp.seg == 0] = 0.0
+        w = np.where(rng.uniform(size=p.rays) < 0.2, 1.0, 0.0).astype(np.float32)
+        N, C, A = xt.forward(p, *inp.args(), ctx=ctx)
+        op = xt.Operator(p, inp.spectrum, inp.seg, inp.a1, inp.a2, ctx=ctx)
+        got = [N, C, A, op.forward(x.reshape(-1)), op.adjoint(w)]
+        op.close()
+        Nr, Cr, Ar, _ = oracle_lib.forward_rays(inp, rays, want_a=True)
+        y_ref, g_ref = oracle_lib.vox_rays(inp, rays, x=x.reshape(-1), w=w)
+        for a, b in zip(got, [Nr, Cr, np.asarray(Ar).reshape(-1), y_ref, np.asarray(g_ref).reshape(-1)]):
+            assert np.array_equal(np.isnan(a), np.isnan(b))
+            nans += int(np.isnan(b).sum())
+    assert (nans > 0) == (side < 0)

@@ -352,6 +352,7 @@ k_fwd(const __grid_constant__ FwdArgs args)
                     // they are integers and floats at once
                     const int jb = max(__float_as_int((y - half) + kMagic) & ~3, (int)kMagicBits);
                     const int je = min(__float_as_int((y + half) + kMagic), jlast);
+                    float2 acc = make_float2(0.f, 0.f);
                     if (jb <= je && pref != 0.f) {
                         // c (u - frac)^2 as a quadratic in u = j - j0: near the
                         // peak it is A alone, far out C u^2 dominates, so the
@@ -363,7 +364,6 @@ k_fwd(const __grid_constant__ FwdArgs args)
                         const float2 C2 = make_float2(cq, cq);
                         const float u = __int_as_float(jb) - tj;
                         float2 U = make_float2(u, u + 1.f);
-                        float2 acc = make_float2(0.f, 0.f);
                         uint32_t a = ifine_a + 4u * (uint32_t)((__float_as_int(r2.w) & 0xffff) + jb);
                         const uint32_t end = a + 4u * (uint32_t)(je - jb);
                         if (COUNT) nexp += (unsigned)((je - jb + 4) & ~3);
@@ -376,8 +376,10 @@ k_fwd(const __grid_constant__ FwdArgs args)
                             acc = __ffma2_rn(make_float2(ex2_approx(g0.x), ex2_approx(g0.y)), make_float2(I.x, I.y), acc);
                             acc = __ffma2_rn(make_float2(ex2_approx(g1.x), ex2_approx(g1.y)), make_float2(I.z, I.w), acc);
                         }
-                        accN = fmaf(pref, acc.x + acc.y, accN);
                     }
+                    // (outside: where sigma^2 is negative, of a detector of negative area, the
+                    // window is empty and pref is NaN, as the sum then is)
+                    accN = fmaf(pref, acc.x + acc.y, accN);
                 }
                 // ---- Compton, :318-356 ----
                 // eratio without contraction: the table bin's check forms it the same way

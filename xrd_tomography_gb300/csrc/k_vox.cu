@@ -247,15 +247,28 @@ __device__ __forceinline__ VoxTerm load_term(const float4 *rec, int nst, int i)
     return {{r0.x, r2.y}, {r0.y, r2.z}, {r0.z, r0.w}, {r1.z, r1.w}, r1.x, r1.y, r2.x};
 }
 
+// The window bin by bin; every bin where sigma is NaN -- sigma^2 is negative for a
+// detector of negative area (adet12 < 0) -- whose term is NaN at each.
+__device__ __forceinline__ void own_window(const WindowTable &L, const EnergyTerm &t, float sigmas, int K, int *k0,
+                                           int *k1)
+{
+    bin_window(L, t.w_hi, sigmas * L.scale * t.sigma, k0, k1);
+    if (isnan(t.sigma)) {
+        *k0 = 0;
+        *k1 = K - 1;
+    }
+}
+
 // Component k & 1 of a pair of bins.
 __device__ __forceinline__ float bin_of(float2 v, int k) { return k & 1 ? v.y : v.x; }
 
 // A run's sum at one energy, bin by bin over that energy's own window: for runs
-// whose sum is not finite.  An infinite coefficient outside the window -- within a
+// whose sum is not finite and detectors of negative area.  An infinite coefficient outside the window -- within a
 // neighbouring energy's, or beside it in a pair -- must not reach the sum, nor one
 // whose term underflows, as 0 x inf.
 __device__ __noinline__ float run_by_window(const float4 *rec, const float *xs, const float4 *cq, int x_row,
-                                            const VoxEnergy *en, int el, int nst, int s0, int s1, WindowTable window)
+                                            const VoxEnergy *en, int el, int nst, int s0, int s1, WindowTable window,
+                                            int K)
 {
     const int lane = threadIdx.x & 31;
     const VoxEnergy q = load_energy(en, el);
@@ -265,7 +278,7 @@ __device__ __noinline__ float run_by_window(const float4 *rec, const float *xs, 
         const EnergyTerm t = energy_term(q, load_term(rec, nst, i));
         if (t.pref == 0.f) continue;
         int k0, k1;
-        bin_window(window, t.w_hi, kSig * window.scale * t.sigma, &k0, &k1);
+        own_window(window, t, kSig, K, &k0, &k1);
         float acc = 0.f;
         for (int k = k0; k <= k1; k++) {
             const float g = bin_of(gauss2(t, cq[k >> 1]), k);
@@ -374,9 +387,9 @@ __device__ __forceinline__ void vox_fwd_pair(const VoxJob &J, int64_t pidx, unsi
             }
             sum = warp_sum(sum);
             sum1 = warp_sum(sum1);
-            if (!(isfinite(sum) && isfinite(sum1))) {
-                sum = run_by_window(rec, xs, cq, x_row, en, el, nst, s0, s1, window);
-                sum1 = run_by_window(rec, xs, cq, x_row, en, el + two, nst, s0, s1, window);
+            if (!(isfinite(sum) && isfinite(sum1) && pair.G.adet12 >= 0.f)) {
+                sum = run_by_window(rec, xs, cq, x_row, en, el, nst, s0, s1, window, K);
+                sum1 = run_by_window(rec, xs, cq, x_row, en, el + two, nst, s0, s1, window, K);
             }
             if (lane <= two) {
                 const int at = (el + lane) * H + run;
@@ -475,17 +488,17 @@ __host__ __device__ inline AdjLayout vox_adj_layout(const DevProblem &P, int E, 
 }
 
 // What a pair adds to this lane's column of sums, energy by energy over each one's own
-// window: for pairs with a weight that is not finite (run_by_window).  Returns the first
-// and the last pair of bins touched.
+// window: for pairs with a weight that is not finite, or with a detector of negative area
+// (run_by_window).  Returns the first and the last pair of bins touched.
 __device__ __noinline__ int2 pair_by_window(VoxTerm v, const VoxEnergy *en, const float4 *cq, const float *ws, int E,
-                                            WindowTable window, float2 *sums)
+                                            WindowTable window, int K, float2 *sums)
 {
     int2 r = {0xffff, -1};
     for (int el = 0; el < E; el++) {
         const EnergyTerm t = energy_term(load_energy(en, el), v);
         const float ct = ws[el] * t.pref;
         int k0, k1;
-        bin_window(window, t.w_hi, kSigAdj * window.scale * t.sigma, &k0, &k1);
+        own_window(window, t, kSigAdj, K, &k0, &k1);
         if (ct == 0.f || k0 > k1) continue;
         r = make_int2(min(r.x, k0 >> 1), max(r.y, k1 >> 1));
         for (int k = k0; k <= k1; k++) {
@@ -574,12 +587,12 @@ k_vox_adj(const VoxBatch B)
                 finite &= isfinite(w);
             }
             __syncwarp();   // (the vote orders no memory)
-            const int by_two = __all_sync(0xffffffffu, finite);
+            const int by_two = __all_sync(0xffffffffu, finite && pr.G.adet12 >= 0.f);
             const VoxTerm vt = vox_term(pr.G, J.c, c1, xy, J.op.atten_src[(int64_t)pr.src * nv + v],
                                         J.op.walk[(pp - J.pair0) * nv + v]);
             int kmin = K2, kmax = -1;   // the pairs of bins this lane adds to
             if (!by_two) {
-                const int2 k = pair_by_window(vt, en, cq, ws, E, window, sums);
+                const int2 k = pair_by_window(vt, en, cq, ws, E, window, P.nwt, sums);
                 kmin = min(kmin, k.x);
                 kmax = k.y;
             }
